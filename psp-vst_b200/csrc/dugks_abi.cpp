@@ -55,16 +55,17 @@ double inv_norm_host(double RT, int D) {
 
 size_t real_size(const dugks_handle* h) { return h->precision == DUGKS_FP64 ? sizeof(double) : sizeof(float); }
 
-dugks::StepArgs make_args(const dugks_handle* h, double dt, double dt_next) {
+bool sharded(const dugks_handle* h) { return h->shard_world > 1 || h->shard_nccl; }
+
+dugks::StepArgs make_args(const dugks_handle* h, double dt) {
     dugks::StepArgs a{};
     a.dm = h->dm;
     a.ds = h->ds;
     a.dt = dt;
-    a.dt_next = dt_next;
     a.chunks = h->chunks;
-    a.chunk_begin = h->d_chunk_begin;
+    a.chunks_f = h->chunks_f;
     a.hzero = h->h_zero ? 1 : 0;
-    dugks::pass_config(h->D, h->precision, h->n1d, &a);
+    a.fused = sharded(h) ? 0 : 1;
     return a;
 }
 
@@ -115,8 +116,6 @@ int shard_allreduce(dugks_handle* h, double* buf, size_t n) {
     return DUGKS_OK;
 }
 
-bool sharded(const dugks_handle* h) { return h->shard_world > 1 || h->shard_nccl; }
-
 int check_device_errors(dugks_handle* h) {
     int err[4] = {0, 0, 0, 0};
     CUDA_TRY(h, cudaMemcpyAsync(err, h->ds.err, sizeof err, cudaMemcpyDeviceToHost, h->stream));
@@ -139,6 +138,24 @@ void dugks_default_options(dugks_options* opt) {
     std::memset(opt, 0, sizeof *opt);
     opt->precision = DUGKS_FP64;
     opt->ls_weighting = DUGKS_LS_MAGSF;
+}
+
+// 3-D and KInner = 0: h is identically zero unless a nonzero h~ is loaded
+// (DV lists carry it all the same)
+static bool can_skip_h(const dugks_handle* h) { return h->D == 3 && h->gas.K_inner == 0 && !h->dm.general_dv; }
+
+// the step arrays of h
+static int alloc_h(dugks_handle* h) {
+    if (h->ds.hbar) return DUGKS_OK;
+    const size_t rs = real_size(h);
+    const size_t nvc = static_cast<size_t>(h->dm.nv_loc) * h->nC, nfv = static_cast<size_t>(h->dm.nv_loc) * h->dm.nF;
+    unsigned char *b = nullptr, *f = nullptr;
+    if (int st = dev_alloc(h, &b, nvc * rs)) return st;
+    if (int st = dev_alloc(h, &f, nfv * rs)) return st;
+    CUDA_TRY(h, cudaMemset(f, 0, nfv * rs));
+    h->ds.hbar = b;
+    h->ds.fvh = f;
+    return DUGKS_OK;
 }
 
 // dv: a tensor-product set; dvl: a DV list (exactly one of them)
@@ -326,35 +343,15 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     for (double x : h->lsP)
         if (!std::isfinite(x)) return fail(DUGKS_ERR_ARG, "dugks_create: singular least-squares system");
 
-    // tiles: at most kMaxTile cells, kMaxLocal cells with the ring, and one
-    // item per thread.  By default greedy tiles as large as those limits
-    // allow; a given tile_cells cuts uniform tiles, shrunk until the largest
-    // fits
-    if (opt.tile_cells > 0) {
-        int tile = std::min(opt.tile_cells, dugks::kMaxTile);
-        for (;;) {
-            dugks::build_tiling(h, tile);
-            const bool fits = h->tiling.max_items <= dugks::kMaxItems && h->tiling.max_local <= dugks::kMaxLocal;
-            if (fits || tile <= 4) break;
-            tile = std::max(4, tile * 7 / 8);
-        }
-    } else {
-        dugks::build_tiling(h, 0);
-    }
-    if (h->tiling.max_items > dugks::kMaxItems || h->tiling.max_local > dugks::kMaxLocal)
+    dugks::build_tiling(h, opt.tile_cells);
+    if (!h->tiling.fits)
         return fail(DUGKS_ERR_UNSUPPORTED, "dugks_create: cells with too many faces for the tile layout");
-    // DV chunks: enough CTAs to fill the GPU several times over
     int dev_count = 0;
     if (cudaGetDeviceCount(&dev_count) != cudaSuccess || dev_count <= 0)
         return fail(DUGKS_ERR_CUDA, "dugks_create: no CUDA device");
     if (h->device < 0 || h->device >= dev_count) return fail(DUGKS_ERR_ARG, "dugks_create: bad device ordinal");
     cudaError_t ce = cudaSetDevice(h->device);
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(ce));
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-    // one CTA per SM runs at a time; aim at about two waves.  Chunks are
-    // whole DV rows (n1d DVs along x at fixed y, z): the passes walk a row in
-    // batches and factor the x direction out of their sums
     const int rows = h->nv / h->n1d;
     // velocity-space shard: this device's block of DV rows
     int row0 = 0, row1 = rows;
@@ -369,12 +366,17 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         row1 = static_cast<int>(static_cast<int64_t>(rows) * (shard->rank + 1) / shard->world);
     }
     const int rows_loc = row1 - row0;
-    int chunks = opt.dv_chunks > 0 ? opt.dv_chunks : (2 * sms + h->tiling.n_tiles - 1) / h->tiling.n_tiles;
-    chunks = std::max(1, std::min(chunks, rows_loc));
-    h->chunks = chunks;
-    h->chunk_begin.resize(chunks + 1);
-    for (int c = 0; c <= chunks; ++c)
-        h->chunk_begin[c] = row0 + static_cast<int32_t>((static_cast<int64_t>(rows_loc) * c) / chunks);
+    // DV segments, and DV chunks of the face and cell reductions: about three
+    // waves of 128-thread CTAs (four per SM), a chunk at least one segment per
+    // warp of its CTA; a given dv_chunks is taken as far as there are segments
+    const int seg_per_row = dvl ? 1 : (h->n1d + dugks::kSeg - 1) / dugks::kSeg;
+    const int n_seg = dvl ? (rows_loc + dugks::kSeg - 1) / dugks::kSeg : rows_loc * seg_per_row;
+    auto chunks_for = [&](int entities) {
+        const int nb = (entities + 31) / 32, want = (148 * 4 * 3 + nb - 1) / nb;
+        return opt.dv_chunks > 0 ? std::min(opt.dv_chunks, n_seg) : std::max(1, std::min(want, n_seg / 4));
+    };
+    h->chunks = chunks_for(nC);
+    h->chunks_f = chunks_for(nF);
 
     // ---- device layout ----
     const dugks::Tiling& t = h->tiling;
@@ -396,21 +398,25 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dm.prec = h->precision;
     dm.n1d = h->n1d;
     dm.general_dv = dvl ? 1 : 0;
-    dm.n_tiles = t.n_tiles;
-    dm.n_items = t.n_items();
-    dm.nb_max = t.nb_max;
-    dm.nf_max = t.nf_max;
+    dm.nF = nF;
+    dm.n_seg = n_seg;
     dm.xi_max_co = std::sqrt(static_cast<double>(h->D)) * h->xi_max;
     int st;
     ce = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(ce));
     cudaEventCreate(&h->ev0);
     cudaEventCreate(&h->ev1);
-    double *d_xi, *d_w, *d_grad_ls, *d_dtV, *d_dc, *d_bS, *d_geo;
-    int32_t *d_tb, *d_tlo, *d_lc, *d_tio, *d_gnb, *d_cfi, *d_fi, *d_bpl, *d_bpt, *d_bown;
-    int32_t *d_meta, *d_loc, *d_face, *d_other, *d_bmir;
-    std::vector<double> dtV(nC);
-    for (int c = 0; c < nC; ++c) dtV[c] = 1.0 / h->V[t.perm[c]];
+    double *d_xi, *d_w, *d_nls, *d_invV, *d_dc, *d_bS, *d_geo;
+    int32_t *d_nbr, *d_cf, *d_fo, *d_fn, *d_for, *d_bpl, *d_bpt, *d_bown, *d_bmir;
+    uint32_t* d_upw = nullptr;
+    int2* d_row_yz;
+    std::vector<int2> row_yz(dvl ? 1 : rows_loc);
+    for (size_t r = 0; r < row_yz.size(); ++r) {
+        const int gr = row0 + static_cast<int>(r);
+        row_yz[r] = make_int2(h->D == 3 ? gr % h->n1d : gr, h->D == 3 ? gr / h->n1d : 0);
+    }
+    std::vector<double> invV(nC);
+    for (int c = 0; c < nC; ++c) invV[c] = 1.0 / h->V[t.perm[c]];
     std::vector<double> bS(3 * static_cast<size_t>(nBF));
     std::vector<int32_t> bown(nBF);
     for (int b = 0; b < nBF; ++b) {
@@ -426,17 +432,14 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     }
     double *d_X1, *d_W1;
     if ((st = upload(h, &d_X1, h->X1)) || (st = upload(h, &d_W1, h->W1)) ||
-        (st = upload(h, &d_xi, h->xi)) || (st = upload(h, &d_w, h->w)) || (st = upload(h, &d_tb, t.tile_begin)) ||
-        (st = upload(h, &d_tlo, t.tile_loc_off)) || (st = upload(h, &d_lc, t.loc_cells)) ||
-        (st = upload(h, &d_tio, t.tile_item_off)) || (st = upload(h, &d_meta, t.it_meta)) ||
-        (st = upload(h, &d_loc, t.it_loc)) || (st = upload(h, &d_face, t.it_face)) ||
-        (st = upload(h, &d_other, t.it_other)) || (st = upload(h, &d_geo, t.it_geo)) ||
-        (st = upload(h, &d_gnb, t.grad_nb)) || (st = upload(h, &d_grad_ls, t.grad_ls)) ||
-        (st = upload(h, &d_cfi, t.cf_item)) || (st = upload(h, &d_dtV, dtV)) || (st = upload(h, &d_fi, t.face_items)) ||
-        (st = upload(h, &d_bpl, h->bface_patch_local)) || (st = upload(h, &d_bpt, h->bface_ptype)) ||
-        (st = upload(h, &d_bown, bown)) || (st = upload(h, &d_dc, h->dc)) || (st = upload(h, &d_bS, bS)) ||
-        (st = upload(h, &d_bmir, h->bface_mirror)) ||
-        (st = upload(h, &h->d_chunk_begin, h->chunk_begin))) {
+        (st = upload(h, &d_row_yz, row_yz)) || (st = upload(h, &d_xi, h->xi)) || (st = upload(h, &d_w, h->w)) ||
+        (st = upload(h, &d_nbr, t.nbr)) ||
+        (st = upload(h, &d_nls, t.nbr_ls)) || (st = upload(h, &d_cf, t.cface)) || (st = upload(h, &d_geo, t.fgeo)) ||
+        (st = upload(h, &d_fo, t.fown)) || (st = upload(h, &d_fn, t.fnei)) || (st = upload(h, &d_for, t.forig)) ||
+        (st = upload(h, &d_invV, invV)) || (st = upload(h, &d_bpl, h->bface_patch_local)) ||
+        (st = upload(h, &d_bpt, h->bface_ptype)) || (st = upload(h, &d_bown, bown)) || (st = upload(h, &d_dc, h->dc)) ||
+        (st = upload(h, &d_bS, bS)) || (st = upload(h, &d_bmir, h->bface_mirror)) ||
+        (st = dev_alloc(h, &d_upw, 2 * static_cast<size_t>(n_seg) * nF))) {
         *out = h;
         return st;
     }
@@ -444,20 +447,18 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dm.W1 = d_W1;
     dm.xi = d_xi;
     dm.w = d_w;
-    dm.tile_begin = d_tb;
-    dm.tile_loc_off = d_tlo;
-    dm.loc_cells = d_lc;
-    dm.tile_item_off = d_tio;
-    dm.it_meta = d_meta;
-    dm.it_loc = d_loc;
-    dm.it_face = d_face;
-    dm.it_other = d_other;
-    dm.it_geo = d_geo;
-    dm.grad_nb = d_gnb;
-    dm.grad_ls = d_grad_ls;
-    dm.cf_item = d_cfi;
-    dm.dtV = d_dtV;
-    dm.face_items = d_fi;
+    dm.nb_max = t.nb_max;
+    dm.nf_max = t.nf_max;
+    dm.row_yz = d_row_yz;
+    dm.nbr = d_nbr;
+    dm.nbr_ls = d_nls;
+    dm.cface = d_cf;
+    dm.invV = d_invV;
+    dm.fgeo = d_geo;
+    dm.fown = d_fo;
+    dm.fnei = d_fn;
+    dm.forig = d_for;
+    dm.upw = d_upw;
     dm.bface_patch_local = d_bpl;
     dm.bface_ptype = d_bpt;
     dm.bface_owner = d_bown;
@@ -506,35 +507,38 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dugks::DevState& ds = h->ds;
     const size_t rs = real_size(h);
     const size_t nvc = static_cast<size_t>(dm.nv_loc) * nC;
-    const size_t nfv = static_cast<size_t>(dm.nv_loc) * std::max(dm.n_items, 1);
+    const size_t nfv = static_cast<size_t>(dm.nv_loc) * std::max(nF, 1);
     unsigned char* p;
-    // One state buffer.  Pass B reads each (DV, cell) entry of its own L0
-    // cells once and then writes it, and no kernel of a step reads the old
-    // state after pass B, so the update runs in place: g[1], h[1] alias
-    // g[0], h[0] and the step's buffer flip changes nothing.  This halves
-    // the state's HBM (the FP64 64^3 x 20^3 cube fits one B200 with it).
+    // One state buffer: the update runs in place, as k_update reads each
+    // (DV, cell) entry once and then writes it and no kernel of a step reads
+    // the old state after it.
     if ((st = dev_alloc(h, &p, nvc * rs))) return *out = h, st;
-    ds.g[0] = ds.g[1] = p;
+    ds.g = p;
     if ((st = dev_alloc(h, &p, nvc * rs))) return *out = h, st;
-    ds.h[0] = ds.h[1] = p;
+    ds.h = p;
+    if ((st = dev_alloc(h, &p, nvc * rs))) return *out = h, st;
+    ds.gbar = p;
     if ((st = dev_alloc(h, &p, nfv * rs))) return *out = h, st;
     ds.fvg = p;
-    if ((st = dev_alloc(h, &p, nfv * rs))) return *out = h, st;
-    ds.fvh = p;
-    // face values start at zero: with h identically zero no pass writes fvh,
-    // and the symmetry pass reads its boundary slots
-    if (cudaMemset(ds.fvg, 0, nfv * rs) != cudaSuccess || cudaMemset(ds.fvh, 0, nfv * rs) != cudaSuccess)
-        return fail(DUGKS_ERR_CUDA, "cudaMemset of the face values");
-    ds.cur = 0;
-    if ((st = dev_alloc(h, &ds.partF, static_cast<size_t>(chunks) * dm.n_items * dugks::kNM)) ||
-        (st = dev_alloc(h, &ds.partC, static_cast<size_t>(chunks) * nC * dugks::kNM)) ||
-        (dvl && opt.macro_flux && (st = dev_alloc(h, &ds.partX, static_cast<size_t>(chunks) * nC * dugks::kFX))) ||
+    // face values start at zero: the slots of incoming boundary DVs are read
+    // (and not used) before any kernel writes them
+    if (cudaMemset(ds.fvg, 0, nfv * rs) != cudaSuccess) return fail(DUGKS_ERR_CUDA, "cudaMemset of the face values");
+    // where h stays identically zero its step arrays are left out until a
+    // nonzero h~ is loaded (alloc_h)
+    if (!can_skip_h(h) && (st = alloc_h(h))) return *out = h, st;
+    const int nbl = (nIF + 31) / 32 + (nBF + 31) / 32;
+    dm.done_cells = nbl;
+    const size_t n_done = static_cast<size_t>(nbl) + (nC + 31) / 32;
+    if ((st = dev_alloc(h, &ds.partF, static_cast<size_t>(h->chunks_f) * nF * dugks::kNM)) ||
+        (st = dev_alloc(h, &ds.partC, static_cast<size_t>(h->chunks) * nC * dugks::kNM)) ||
+        (st = dev_alloc(h, &ds.done, n_done)) ||
+        (dvl && opt.macro_flux && (st = dev_alloc(h, &ds.partX, static_cast<size_t>(h->chunks) * nC * dugks::kFX))) ||
         (dvl && opt.macro_flux && shard &&
          (st = dev_alloc(h, &ds.redC, static_cast<size_t>(nC) * (dugks::kNM + dugks::kFX)))) ||
         (st = dev_alloc(h, &ds.cellrec, static_cast<size_t>(dugks::REC_N) * nC)) ||
-        (st = dev_alloc(h, &ds.facerec, static_cast<size_t>(dugks::REC_N) * dm.n_items)) ||
+        (st = dev_alloc(h, &ds.facerec, static_cast<size_t>(dugks::REC_N) * nF)) ||
         (st = dev_alloc(h, &ds.ctab, static_cast<size_t>(h->D) * h->n1d * nC)) ||
-        (st = dev_alloc(h, &ds.ftab, static_cast<size_t>(h->D) * h->n1d * dm.n_items)) ||
+        (st = dev_alloc(h, &ds.ftab, static_cast<size_t>(h->D) * h->n1d * nF)) ||
         (st = dev_alloc(h, &ds.brec, nBF)) || (st = dev_alloc(h, &ds.bmom_in, static_cast<size_t>(nBF) * dugks::kNM)) ||
         (st = dev_alloc(h, &ds.cm, static_cast<size_t>(nC) * 9)) ||
         (st = dev_alloc(h, &ds.fm, static_cast<size_t>(nF) * 9)) || (st = dev_alloc(h, &ds.co, 2)) ||
@@ -545,7 +549,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     if (h->precision == DUGKS_FP32C && !dvl) {
         double *d_gref, *d_href;
         if ((st = dev_alloc(h, &d_gref, dm.nv_loc)) || (st = dev_alloc(h, &d_href, dm.nv_loc)) ||
-            (st = dev_alloc(h, &ds.refmom, static_cast<size_t>(chunks) * dugks::kNM))) {
+            (st = dev_alloc(h, &ds.refmom, dugks::kNM))) {
             *out = h;
             return st;
         }
@@ -557,11 +561,11 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     }
     ce = cudaMemset(ds.err, 0, 4 * sizeof(int));
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, cudaGetErrorString(ce));
-    ce = cudaMemset(ds.partF, 0, static_cast<size_t>(chunks) * dm.n_items * dugks::kNM * sizeof(double));
+    ce = cudaMemset(ds.done, 0, n_done * sizeof(int));
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, cudaGetErrorString(ce));
-    dugks::StepArgs a = make_args(h, 0.0, 0.0);
-    ce = dugks::configure_kernels(h->precision, a);
-    if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, std::string("configure kernels: ") + cudaGetErrorString(ce));
+    ce = dugks::launch_upwind_bits(dm, d_upw, h->stream);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);
+    if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, std::string("upwind bits: ") + cudaGetErrorString(ce));
     if (shard && shard->use_nccl) {
         // collective: every rank of the shard set makes this call
         const NcclApi& api = nccl_api();
@@ -627,7 +631,6 @@ int dugks_set_macros(dugks_handle* h, const double* rho, const double* U, const 
     const double R = h->gas.R;
     const dugks::Tiling& t = h->tiling;
     std::vector<double> cm(static_cast<size_t>(nC) * 9);
-    std::vector<double> cr(static_cast<size_t>(dugks::REC_N) * nC, 0.0);
     for (int c = 0; c < nC; ++c) {
         const int o = t.perm[c];
         // a non-finite or non-positive macroscopic state is refused as the
@@ -646,14 +649,6 @@ int dugks_set_macros(dugks_handle* h, const double* rho, const double* U, const 
         m[4] = T[o];
         m[5] = m[6] = m[7] = 0.0;
         m[8] = tau;
-        const double RT = R * T[o];
-        const size_t n = static_cast<size_t>(nC);
-        cr[dugks::REC_UX * n + c] = m[1];
-        cr[dugks::REC_UY * n + c] = m[2];
-        cr[dugks::REC_UZ * n + c] = m[3];
-        cr[dugks::REC_INVRT * n + c] = 1.0 / RT;
-        cr[dugks::REC_A * n + c] = rho[o] * inv_norm_host(RT, D);
-        cr[dugks::REC_RTH * n + c] = RT;  // relax factor and heat-flux terms stay 0 (q = 0)
     }
     // boundary records
     const double K3D = h->gas.K_inner + 3.0 - D;
@@ -696,8 +691,6 @@ int dugks_set_macros(dugks_handle* h, const double* rho, const double* U, const 
     std::memcpy(&co_host[0], &co_max, sizeof(double));
     co_host[1] = co_sum;
     CUDA_TRY(h, cudaMemcpyAsync(h->ds.cm, cm.data(), cm.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(h, cudaMemcpyAsync(h->ds.cellrec, cr.data(), cr.size() * sizeof(double), cudaMemcpyHostToDevice,
-                                h->stream));
     if (nBF > 0)
         CUDA_TRY(h, cudaMemcpyAsync(h->ds.brec, br.data(), br.size() * sizeof(dugks::BRec), cudaMemcpyHostToDevice,
                                     h->stream));
@@ -731,42 +724,37 @@ int dugks_set_macros(dugks_handle* h, const double* rho, const double* U, const 
                                     cudaMemcpyHostToDevice, h->stream));
         CUDA_TRY(h, cudaMemcpyAsync(const_cast<double*>(h->dm.href), h->href.data(), nl * sizeof(double),
                                     cudaMemcpyHostToDevice, h->stream));
-        // raw moments of the reference over each DV chunk (moment record layout)
-        std::vector<double> rm(static_cast<size_t>(h->chunks) * dugks::kNM, 0.0);
-        for (int ch = 0; ch < h->chunks; ++ch) {
-            double* m = &rm[static_cast<size_t>(ch) * dugks::kNM];
-            for (int r = h->chunk_begin[ch]; r < h->chunk_begin[ch + 1]; ++r)
-                for (int ix = 0; ix < h->n1d; ++ix) {
-                    const int d = (r - h->dm.row_base) * h->n1d + ix;
-                    const double* xi = &h->xi[3 * static_cast<size_t>(h->dm.dv_base + d)];
-                    const double wd = h->w[h->dm.dv_base + d];
-                    const double a = wd * h->gref[d], u = a * (xi[0] * xi[0] + xi[1] * xi[1] + xi[2] * xi[2]) +
-                                                          wd * h->href[d];
-                    m[dugks::MOM_M0] += a;
-                    m[dugks::MOM_W] += u;
-                    for (int k = 0; k < 3; ++k) {
-                        m[dugks::MOM_M1 + k] += a * xi[k];
-                        m[dugks::MOM_V3 + k] += u * xi[k];
-                    }
-                    m[dugks::MOM_M2] += a * xi[0] * xi[0];
-                    m[dugks::MOM_M2 + 1] += a * xi[0] * xi[1];
-                    m[dugks::MOM_M2 + 2] += a * xi[0] * xi[2];
-                    m[dugks::MOM_M2 + 3] += a * xi[1] * xi[1];
-                    m[dugks::MOM_M2 + 4] += a * xi[1] * xi[2];
-                    m[dugks::MOM_M2 + 5] += a * xi[2] * xi[2];
-                }
+        // raw moments of the reference (moment record layout)
+        std::vector<double> rm(dugks::kNM, 0.0);
+        double* m = rm.data();
+        for (int d = 0; d < nl; ++d) {
+            const double* xi = &h->xi[3 * static_cast<size_t>(h->dm.dv_base + d)];
+            const double wd = h->w[h->dm.dv_base + d];
+            const double a = wd * h->gref[d],
+                         u = a * (xi[0] * xi[0] + xi[1] * xi[1] + xi[2] * xi[2]) + wd * h->href[d];
+            m[dugks::MOM_M0] += a;
+            m[dugks::MOM_W] += u;
+            for (int k = 0; k < 3; ++k) {
+                m[dugks::MOM_M1 + k] += a * xi[k];
+                m[dugks::MOM_V3 + k] += u * xi[k];
+            }
+            m[dugks::MOM_M2] += a * xi[0] * xi[0];
+            m[dugks::MOM_M2 + 1] += a * xi[0] * xi[1];
+            m[dugks::MOM_M2 + 2] += a * xi[0] * xi[2];
+            m[dugks::MOM_M2 + 3] += a * xi[1] * xi[1];
+            m[dugks::MOM_M2 + 4] += a * xi[1] * xi[2];
+            m[dugks::MOM_M2 + 5] += a * xi[2] * xi[2];
         }
         CUDA_TRY(h, cudaMemcpyAsync(h->ds.refmom, rm.data(), rm.size() * sizeof(double), cudaMemcpyHostToDevice,
                                     h->stream));
         CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     }
-    h->ds.cur = 0;
-    dugks::StepArgs a = make_args(h, 0.0, 0.0);
+    dugks::StepArgs a = make_args(h, 0.0);
     CUDA_TRY(h, dugks::launch_init(a, h->precision, h->stream));
     h->launches += h->nBF > 0 ? 3 : 2;
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     h->initialised = true;
-    h->h_zero = h->D == 3 && h->gas.K_inner == 0;
+    h->h_zero = can_skip_h(h);
     h->last_step_ms = 0;
     return DUGKS_OK;
 }
@@ -818,9 +806,9 @@ static int enqueue_step(dugks_handle* h, const dugks::StepArgs& a, cudaEvent_t* 
     CUDA_TRY(h, dugks::launch_stage(a, h->precision, dugks::STAGE_PASS_A, h->stream, launches));
     if (sev) CUDA_TRY(h, cudaEventRecord(sev[1], h->stream));
     if (sh) {
-        const size_t n = static_cast<size_t>(h->dm.n_items) * dugks::kNM;
-        CUDA_TRY(h, dugks::launch_sum_chunks(h->ds.partF, h->chunks, n, h->stream));
-        if (h->chunks > 1) ++*launches;
+        const size_t n = static_cast<size_t>(h->dm.nF) * dugks::kNM;
+        CUDA_TRY(h, dugks::launch_sum_chunks(h->ds.partF, h->chunks_f, n, h->stream));
+        if (h->chunks_f > 1) ++*launches;
         const int st = shard_allreduce(h, h->ds.partF, n);
         if (st) return st;
     }
@@ -869,12 +857,7 @@ static int run_steps(dugks_handle* h, int32_t n_steps, const double* dt, double*
     CUDA_TRY(h, cudaEventRecord(h->ev0, h->stream));
     int launches = 0;
     for (int i = 0; i < n_steps; ++i) {
-        dugks::StepArgs a = make_args(h, dt[i], i + 1 < n_steps ? dt[i + 1] : 0.0);
-        if (h->cellrec_dt != dt[i]) {
-            CUDA_TRY(h, dugks::launch_cell_prep(a, h->stream));
-            ++launches;
-        }
-        CUDA_TRY(h, cudaMemsetAsync(h->ds.co, 0, 2 * sizeof(double), h->stream));
+        const dugks::StepArgs a = make_args(h, dt[i]);
         if (const int st = enqueue_step(h, a, stage_ms ? sev : nullptr, &launches, nullptr)) return st;
         if (stage_ms) {
             CUDA_TRY(h, cudaEventSynchronize(sev[4]));
@@ -884,8 +867,6 @@ static int run_steps(dugks_handle* h, int32_t n_steps, const double* dt, double*
                 stage_ms[stg] += ms;
             }
         }
-        h->cellrec_dt = a.dt_next;
-        h->ds.cur = 1 - h->ds.cur;
         h->steps_done++;
     }
     CUDA_TRY(h, cudaEventRecord(h->ev1, h->stream));
@@ -928,20 +909,15 @@ int dugks_step_adaptive(dugks_handle* h, int32_t n_steps, const dugks_adapt* ada
     // slot after its face combine; step 1's dt comes from the current faces
     auto slot = [&](int k) { return h->d_dt + (k & 1); };
     int launches = 0;
-    dugks::StepArgs a = make_args(h, 0.0, 0.0);
+    dugks::StepArgs a = make_args(h, 0.0);
     CUDA_TRY(h, dugks::launch_adapt(a, h->d_dt, slot(1), h->d_hist, adapt->max_co, adapt->max_delta_t, h->stream));
-    a.dtp = slot(1);
-    CUDA_TRY(h, dugks::launch_cell_prep(a, h->stream));
-    launches += 2;
+    launches += 1;
     for (int k = 1; k <= n_steps; ++k) {
-        a = make_args(h, 0.0, 0.0);
+        a = make_args(h, 0.0);
         a.dtp = slot(k);
-        a.dtnp = slot(k + 1);
-        CUDA_TRY(h, cudaMemsetAsync(h->ds.co, 0, 2 * sizeof(double), h->stream));
         const AdaptCall ac{slot(k), slot(k + 1), k < n_steps ? h->d_hist + k : nullptr, adapt->max_co,
                            adapt->max_delta_t};
         if (const int st = enqueue_step(h, a, nullptr, &launches, &ac)) return st;
-        h->ds.cur = 1 - h->ds.cur;
         h->steps_done++;
     }
     CUDA_TRY(h, cudaEventRecord(h->ev1, h->stream));
@@ -950,7 +926,6 @@ int dugks_step_adaptive(dugks_handle* h, int32_t n_steps, const dugks_adapt* ada
         CUDA_TRY(h, cudaMemcpyAsync(dt_history, h->d_hist, static_cast<size_t>(n_steps) * sizeof(double),
                                     cudaMemcpyDeviceToHost, h->stream));
     h->launches += launches;
-    h->cellrec_dt = 0.0;   // the records hold the next adaptive dt; a fixed step rebuilds them
     int st = check_device_errors(h);
     float ms = 0;
     cudaEventElapsedTime(&ms, h->ev0, h->ev1);
@@ -970,20 +945,17 @@ int dugks_shard_phase(dugks_handle* h, int32_t phase, double dt, double** part, 
     if (phase == 0) {
         if (!(dt > 0) || !std::isfinite(dt)) return set_error(h, DUGKS_ERR_ARG, "dugks_shard_phase: dt must be > 0");
         h->shard_dt = dt;
-        const dugks::StepArgs a = make_args(h, dt, 0.0);
-        if (h->cellrec_dt != dt) {
-            CUDA_TRY(h, dugks::launch_cell_prep(a, h->stream));
-            ++launches;
-        }
-        CUDA_TRY(h, cudaMemsetAsync(h->ds.co, 0, 2 * sizeof(double), h->stream));
+        dugks::StepArgs a = make_args(h, dt);
+        a.fused = 0;
         CUDA_TRY(h, dugks::launch_stage(a, h->precision, dugks::STAGE_PASS_A, h->stream, &launches));
-        const size_t n = static_cast<size_t>(h->dm.n_items) * dugks::kNM;
-        CUDA_TRY(h, dugks::launch_sum_chunks(h->ds.partF, h->chunks, n, h->stream));
-        if (h->chunks > 1) ++launches;
+        const size_t n = static_cast<size_t>(h->dm.nF) * dugks::kNM;
+        CUDA_TRY(h, dugks::launch_sum_chunks(h->ds.partF, h->chunks_f, n, h->stream));
+        if (h->chunks_f > 1) ++launches;
         *part = h->ds.partF;
         *n_part = static_cast<int64_t>(n);
     } else if (phase == 1) {
-        const dugks::StepArgs a = make_args(h, h->shard_dt, 0.0);
+        dugks::StepArgs a = make_args(h, h->shard_dt);
+        a.fused = 0;
         dugks::StepArgs one = a;
         one.chunks = 1;
         CUDA_TRY(h, dugks::launch_stage(one, h->precision, dugks::STAGE_FACE_COMBINE, h->stream, &launches));
@@ -994,15 +966,14 @@ int dugks_shard_phase(dugks_handle* h, int32_t phase, double dt, double** part, 
         *part = buf;
         *n_part = static_cast<int64_t>(n);
     } else {
-        dugks::StepArgs one = make_args(h, h->shard_dt, 0.0);
+        dugks::StepArgs one = make_args(h, h->shard_dt);
         one.chunks = 1;
+        one.fused = 0;
         if (h->ds.redC) {
             one.ds.partC = h->ds.redC;
             one.ds.partX = h->ds.redC + static_cast<size_t>(h->nC) * dugks::kNM;
         }
         CUDA_TRY(h, dugks::launch_stage(one, h->precision, dugks::STAGE_CELL_COMBINE, h->stream, &launches));
-        h->cellrec_dt = 0.0;   // the next phase 0 sets the relax factors for its dt
-        h->ds.cur = 1 - h->ds.cur;
         h->steps_done++;
     }
     h->launches += launches;
@@ -1086,17 +1057,8 @@ int dugks_batch_create(dugks_handle* const* handles, int32_t n, const double* dt
     for (int i = 0; i < n; ++i)
         if ((e = cudaEventCreateWithFlags(&b->joins[i], cudaEventDisableTiming)) != cudaSuccess)
             return cuda_fail(e, "cudaEventCreate");
-    // every handle's cell records carry the relax factors of its dt, as the
-    // graph's cell combines write them for the next step
-    for (int i = 0; i < n; ++i) {
-        dugks_handle* h = b->hs[i];
-        if (h->cellrec_dt != b->dt[i]) {
-            if ((e = dugks::launch_cell_prep(make_args(h, b->dt[i], 0.0), h->stream)) != cudaSuccess)
-                return cuda_fail(e, "cell prep");
-            h->cellrec_dt = b->dt[i];
-        }
-        if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
-    }
+    for (int i = 0; i < n; ++i)
+        if ((e = cudaStreamSynchronize(b->hs[i]->stream)) != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
     // capture: fork from s0 into every handle's stream, two steps each, join
     if ((e = cudaStreamBeginCapture(b->s0, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
         return cuda_fail(e, "cudaStreamBeginCapture");
@@ -1106,15 +1068,10 @@ int dugks_batch_create(dugks_handle* const* handles, int32_t n, const double* dt
     for (int i = 0; i < n && st == DUGKS_OK; ++i) {
         dugks_handle* h = b->hs[i];
         cudaStreamWaitEvent(h->stream, b->fork, 0);
-        const int cur0 = h->ds.cur;
         b->hzero.push_back(h->h_zero ? 1 : 0);
         for (int k = 0; k < 2 && st == DUGKS_OK; ++k) {
-            const dugks::StepArgs a = make_args(h, b->dt[i], b->dt[i]);
-            if (cudaMemsetAsync(h->ds.co, 0, 2 * sizeof(double), h->stream) != cudaSuccess) st = DUGKS_ERR_CUDA;
-            else st = enqueue_step(h, a, nullptr, &b->launches_per_pair[i], nullptr);
-            h->ds.cur = 1 - h->ds.cur;
+            st = enqueue_step(h, make_args(h, b->dt[i]), nullptr, &b->launches_per_pair[i], nullptr);
         }
-        h->ds.cur = cur0;
         cudaEventRecord(b->joins[i], h->stream);
         cudaStreamWaitEvent(b->s0, b->joins[i], 0);
     }
@@ -1160,13 +1117,9 @@ int dugks_batch_step(dugks_batch* b, int32_t n_steps) {
         h->steps_done += 2 * pairs;
         h->launches += static_cast<int64_t>(b->launches_per_pair[i]) * pairs;
         if (n_steps % 2) {
-            // the odd step on the handle's own stream, then the relax factors
-            // of its dt again for the next replay
-            int st = run_steps(h, 1, &b->dt[i], nullptr);
-            if (st == DUGKS_OK && (e = dugks::launch_cell_prep(make_args(h, b->dt[i], 0.0), h->stream)) != cudaSuccess)
-                st = set_error(h, DUGKS_ERR_CUDA, cudaGetErrorString(e));
+            // the odd step on the handle's own stream
+            const int st = run_steps(h, 1, &b->dt[i], nullptr);
             if (st != DUGKS_OK) return batch_fail(b, st, "handle " + std::to_string(i) + ": " + h->last_error);
-            h->cellrec_dt = b->dt[i];
         }
         const int st = check_device_errors(h);
         if (st != DUGKS_OK) return batch_fail(b, st, "handle " + std::to_string(i) + ": " + h->last_error);
@@ -1273,9 +1226,8 @@ int dugks_set_step_record(dugks_handle* h, const double* rec) {
                                     h->stream));
     CUDA_TRY(h, cudaMemcpyAsync(h->ds.cm, cm.data(), cm.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     CUDA_TRY(h, cudaMemcpyAsync(h->ds.co, co, 2 * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(h, dugks::launch_cell_records(make_args(h, 0.0, 0.0), h->stream));
+    CUDA_TRY(h, dugks::launch_cell_records(make_args(h, 0.0), h->stream));
     h->launches += 1;
-    h->cellrec_dt = 0;   // the next step sets the relax factors for its dt
     return check_device_errors(h);
 }
 
@@ -1348,7 +1300,7 @@ int dugks_get_df(dugks_handle* h, const int32_t* cells, int32_t n, double* g_out
             double* dst = which == 0 ? g_out : h_out;
             if (!dst) continue;
             const unsigned char* src =
-                static_cast<const unsigned char*>(which == 0 ? h->ds.g[h->ds.cur] : h->ds.h[h->ds.cur]) + c * rs;
+                static_cast<const unsigned char*>(which == 0 ? h->ds.g : h->ds.h) + c * rs;
             CUDA_TRY(h, cudaMemcpy2DAsync(col.data(), rs, src, static_cast<size_t>(h->nC) * rs, rs, h->dm.nv_loc,
                                           cudaMemcpyDeviceToHost, h->stream));
             CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -1376,7 +1328,7 @@ static int state_io(dugks_handle* h, double* g, double* hh, const double* gi, co
     std::vector<unsigned char> buf(nvc * rs);
     const std::vector<int32_t>& perm = h->tiling.perm;
     for (int which = 0; which < 2; ++which) {
-        void* dev = which == 0 ? h->ds.g[h->ds.cur] : h->ds.h[h->ds.cur];
+        void* dev = which == 0 ? h->ds.g : h->ds.h;
         const std::vector<double>& ref = which == 0 ? h->gref : h->href;
         if (get) {
             double* dst = which == 0 ? g : hh;
@@ -1423,17 +1375,25 @@ int dugks_set_state(dugks_handle* h, const double* g, const double* hh, double d
     // a nonzero h~ ends the g-only passes for this handle
     if (h->h_zero) {
         const size_t nvc = static_cast<size_t>(h->dm.nv_loc) * h->nC;
-        for (size_t i = 0; i < nvc && h->h_zero; ++i) h->h_zero = hh[i] == 0.0;
+        bool zero = true;
+        for (size_t i = 0; i < nvc && zero; ++i) zero = hh[i] == 0.0;
+        if (!zero && (st = alloc_h(h))) return st;
+        h->h_zero = zero;
     }
-    dugks::StepArgs a = make_args(h, dt_prev, 0.0);
+    dugks::StepArgs a = make_args(h, dt_prev);
     a.dm.macro_flux = 0;   // the macros of given DFs are their moments (macroFlux yes: restore the step record)
     // a new state replaces a poisoned one: its own check starts clear
     CUDA_TRY(h, cudaMemsetAsync(h->ds.err, 0, 4 * sizeof(int), h->stream));
-    CUDA_TRY(h, dugks::launch_state_moments(a, h->precision, h->stream));
-    if ((st = shard_allreduce(h, h->ds.partC, static_cast<size_t>(h->nC) * dugks::kNM))) return st;
-    CUDA_TRY(h, dugks::launch_cell_combine_one(a, 0.0, h->stream));
-    h->launches += 2;
-    h->cellrec_dt = 0;
+    CUDA_TRY(h, dugks::launch_pass(a, h->precision, dugks::KERNEL_STATE_MOMENTS, h->stream));
+    h->launches += 1;
+    if (!a.fused) {
+        const size_t nm = static_cast<size_t>(h->nC) * dugks::kNM;
+        CUDA_TRY(h, dugks::launch_sum_chunks(h->ds.partC, h->chunks, nm, h->stream));
+        if (h->chunks > 1) h->launches += 1;
+        if ((st = shard_allreduce(h, h->ds.partC, nm))) return st;
+        CUDA_TRY(h, dugks::launch_finish(a, false, h->stream));
+        h->launches += 1;
+    }
     return check_device_errors(h);
 }
 
@@ -1473,23 +1433,18 @@ void dugks_destroy(dugks_handle* h) {
 namespace dugks {
 
 // Rebuilds the cell records and Maxwellian tables from the cell macros in
-// ds.cm, as dugks_set_step_record does after restoring them; the next step
-// sets the relax factors for its dt.
+// ds.cm, as dugks_set_step_record does after restoring them.
 int rebuild_cell_records(dugks_handle* h) {
-    CUDA_TRY(h, launch_cell_records(make_args(h, 0.0, 0.0), h->stream));
+    CUDA_TRY(h, launch_cell_records(make_args(h, 0.0), h->stream));
     h->launches += 1;
-    h->cellrec_dt = 0;
     return DUGKS_OK;
 }
 
 int record_face_values(dugks_handle* h, double dt) {
-    const StepArgs a = make_args(h, dt, 0.0);
+    StepArgs a = make_args(h, dt);
+    a.fused = 0;
+    a.keep_co = 1;
     int launches = 0;
-    if (h->cellrec_dt != dt) {
-        CUDA_TRY(h, launch_cell_prep(a, h->stream));
-        ++launches;
-        h->cellrec_dt = dt;   // the relax factors are now dt's
-    }
     CUDA_TRY(h, launch_stage(a, h->precision, STAGE_PASS_A, h->stream, &launches));
     h->launches += launches;
     return DUGKS_OK;

@@ -1,8 +1,8 @@
 // dugks_adjoint_run: the discrete adjoint of the FP64 DUGKS step on the
-// GPU.  The forward steps between checkpoints are the library's tiled
-// passes (dugks_step); the step being reversed is recorded again by the
-// plain per-(DV, entity) kernels of dugks_adjoint.cuh from its start state,
-// then reversed by the kernels there.  All arrays are FP64 in HBM.
+// GPU.  The forward steps between checkpoints are the library's own
+// (dugks_step); the step being reversed is recorded again from its start
+// state by the step's face kernels and those of dugks_adjoint.cuh, then
+// reversed by the kernels there.  All arrays are FP64 in HBM.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -60,8 +60,8 @@ struct GpuEx {
         ADJ_TRY(h, cudaGetLastError());
         return DUGKS_OK;
     }
-    // the tiled pass A of the recorded step, into the handle's face-value buffer
-    int pass_a(const adj::View& v) { return dugks::record_face_values(h, v.dt); }
+    // face values and their moments of the recorded step, into the handle's buffers
+    int face_values(const adj::View& v) { return dugks::record_face_values(h, v.dt); }
 };
 
 // device allocations of one run, freed together
@@ -116,18 +116,16 @@ struct HandleOps {
 
     int save(int s) {
         double* d = slot[s];
-        const int c = h->ds.cur;
-        ADJ_TRY(h, cudaMemcpyAsync(d, h->ds.g[c], nvc * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-        ADJ_TRY(h, cudaMemcpyAsync(d + nvc, h->ds.h[c], nvc * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+        ADJ_TRY(h, cudaMemcpyAsync(d, h->ds.g, nvc * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+        ADJ_TRY(h, cudaMemcpyAsync(d + nvc, h->ds.h, nvc * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
         ADJ_TRY(h, cudaMemcpyAsync(d + 2 * nvc, h->ds.cm, 9 * static_cast<size_t>(h->nC) * sizeof(double),
                                    cudaMemcpyDeviceToDevice, h->stream));
         return DUGKS_OK;
     }
     int restore(int s) {
         const double* d = slot[s];
-        const int c = h->ds.cur;
-        ADJ_TRY(h, cudaMemcpyAsync(h->ds.g[c], d, nvc * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-        ADJ_TRY(h, cudaMemcpyAsync(h->ds.h[c], d + nvc, nvc * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+        ADJ_TRY(h, cudaMemcpyAsync(h->ds.g, d, nvc * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+        ADJ_TRY(h, cudaMemcpyAsync(h->ds.h, d + nvc, nvc * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
         ADJ_TRY(h, cudaMemcpyAsync(h->ds.cm, d + 2 * nvc, 9 * static_cast<size_t>(h->nC) * sizeof(double),
                                    cudaMemcpyDeviceToDevice, h->stream));
         return dugks::rebuild_cell_records(h);
@@ -147,9 +145,8 @@ struct HandleOps {
     }
     int reverse(int n) {
         adj::View w = v;
-        const int c = h->ds.cur;
-        w.g = static_cast<const double*>(h->ds.g[c]);
-        w.h = static_cast<const double*>(h->ds.h[c]);
+        w.g = static_cast<const double*>(h->ds.g);
+        w.h = static_cast<const double*>(h->ds.h);
         w.cm = h->ds.cm;
         w.wn = n >= window_start ? 1.0 / (n_steps - window_start) : 0.0;
         w.fold = n >= 1 ? 1 : 0;
@@ -192,17 +189,16 @@ int prepare(dugks_handle* h, const dugks_objective* obj, const char* who, Arena&
     const size_t nvc = static_cast<size_t>(nv) * nC, nvf = static_cast<size_t>(nv) * nF;
     // mesh tables in the handle's cell numbering
     const std::vector<int32_t>& perm = h->tiling.perm;
-    const std::vector<int32_t>& iperm = h->tiling.iperm;
-    std::vector<int32_t> own(nF), nei(nIF);
-    for (int f = 0; f < nF; ++f) own[f] = iperm[h->owner[f]];
-    for (int f = 0; f < nIF; ++f) nei[f] = iperm[h->neighbour[f]];
+    const std::vector<int32_t>&own = h->tiling.fown, &nei = h->tiling.fnei, &forig = h->tiling.forig;
+    std::vector<int32_t> blocal(nBF);
+    for (int b = 0; b < nBF; ++b) blocal[b] = h->tiling.fnew[h->bface_patch_local[b]];
     std::vector<double> Cn(3 * static_cast<size_t>(nC)), Vn(nC);
     for (int c = 0; c < nC; ++c) {
         for (int k = 0; k < 3; ++k) Cn[3 * c + k] = h->C[3 * static_cast<size_t>(perm[c]) + k];
         Vn[c] = h->V[perm[c]];
     }
     adj::HostTables t;
-    adj::build_tables(nC, nIF, nBF, own.data(), nei.data(), Vn.data(), h->bface_patch_local.data(), t);
+    adj::build_tables(nC, nIF, nBF, own.data(), nei.data(), Vn.data(), blocal.data(), t);
     std::vector<double> ha(nBF, 0.0), fw(3 * static_cast<size_t>(nBF), 0.0);
     if (obj->energy_weight) std::copy(obj->energy_weight, obj->energy_weight + nBF, ha.begin());
     if (obj->momentum_weight) std::copy(obj->momentum_weight, obj->momentum_weight + 3 * nBF, fw.begin());
@@ -211,8 +207,14 @@ int prepare(dugks_handle* h, const dugks_objective* obj, const char* who, Arena&
         for (int k = 0; k < 3; ++k) ok = ok && std::isfinite(fw[3 * b + k]);
         if (!ok) return set_error(h, DUGKS_ERR_ARG, std::string(who) + ": non-finite objective weight");
     }
-    std::vector<double> Sf(h->Sf.begin(), h->Sf.begin() + 3 * static_cast<size_t>(nF));
-    std::vector<double> Cf(h->Cf.begin(), h->Cf.begin() + 3 * static_cast<size_t>(nF));
+    auto by_face = [&](const std::vector<double>& a, int n) {
+        std::vector<double> r(3 * static_cast<size_t>(n));
+        for (int f = 0; f < n; ++f)
+            for (int k = 0; k < 3; ++k) r[3 * f + k] = a[3 * static_cast<size_t>(forig[f]) + k];
+        return r;
+    };
+    const std::vector<double> Sf = by_face(h->Sf, nF), Cf = by_face(h->Cf, nF), lsP = by_face(h->lsP, nIF),
+                              lsN = by_face(h->lsN, nIF);
 
     v = adj::View{};
     v.nC = nC;
@@ -239,9 +241,9 @@ int prepare(dugks_handle* h, const dugks_objective* obj, const char* who, Arena&
     int st;
     if ((st = ar.put(h, &d_own, own)) || (st = ar.put(h, &d_nei, nei)) || (st = ar.put(h, &d_cfo, t.cf_off)) ||
         (st = ar.put(h, &d_cfe, t.cf_ent)) || (st = ar.put(h, &d_tho, t.th_off)) || (st = ar.put(h, &d_the, t.th_ent)) ||
-        (st = ar.put(h, &d_bt, h->bface_ptype)) || (st = ar.put(h, &d_bl, h->bface_patch_local)) ||
+        (st = ar.put(h, &d_bt, h->bface_ptype)) || (st = ar.put(h, &d_bl, blocal)) ||
         (st = ar.put(h, &d_S, Sf)) || (st = ar.put(h, &d_Cf, Cf)) || (st = ar.put(h, &d_C, Cn)) ||
-        (st = ar.put(h, &d_iV, t.invV)) || (st = ar.put(h, &d_lsP, h->lsP)) || (st = ar.put(h, &d_lsN, h->lsN)) ||
+        (st = ar.put(h, &d_iV, t.invV)) || (st = ar.put(h, &d_lsP, lsP)) || (st = ar.put(h, &d_lsN, lsN)) ||
         (st = ar.put(h, &d_bU, h->bc_U)) || (st = ar.put(h, &d_bT, h->bc_T)) || (st = ar.put(h, &d_brho, h->bc_rho)) ||
         (st = ar.put(h, &d_ha, ha)) || (st = ar.put(h, &d_fw, fw)))
         return st;
@@ -264,11 +266,13 @@ int prepare(dugks_handle* h, const dugks_objective* obj, const char* who, Arena&
     v.brho = d_brho;
     v.ha = d_ha;
     v.fw = d_fw;
-    v.fvg = static_cast<const double*>(h->ds.fvg);
-    v.fvh = static_cast<const double*>(h->ds.fvh);
-    v.fitems = h->dm.face_items;
-    v.nI = h->dm.n_items;
-    if ((st = ar.get(h, &v.fg, nvf)) || (st = ar.get(h, &v.fh, nvf)) ||
+    v.fg = static_cast<double*>(h->ds.fvg);
+    v.fh = static_cast<double*>(h->ds.fvh);
+    v.fmom = h->ds.partF;
+    v.nchM = h->chunks_f;
+    v.bmom_in = h->ds.bmom_in;
+    // with h identically zero the step keeps no face values of it
+    if ((!v.fh && (st = ar.zeros(h, &v.fh, nvf))) ||
         (st = ar.get(h, &v.pf, static_cast<size_t>(v.nchF) * nF * adj::kP)) || (st = ar.get(h, &v.rhow, nBF)) ||
         (st = ar.get(h, &v.inby, nBF)) || (st = ar.get(h, &v.fmac, static_cast<size_t>(nF) * adj::kMac)) ||
         (st = ar.zeros(h, &v.Jb, nBF)))
@@ -413,9 +417,8 @@ extern "C" int dugks_boundary_fluxes(dugks_handle* h, double dt, double* flux) {
     double* d_out;
     if ((st = ar.get(h, &d_out, 5 * static_cast<size_t>(nBF)))) return st;
     GpuEx ex{h, sms};
-    const int c = h->ds.cur;
-    v.g = static_cast<const double*>(h->ds.g[c]);
-    v.h = static_cast<const double*>(h->ds.h[c]);
+    v.g = static_cast<const double*>(h->ds.g);
+    v.h = static_cast<const double*>(h->ds.h);
     v.cm = h->ds.cm;
     if ((st = ex.run(nBF, adj::FInBy{v}))) return st;
     if ((st = adj::record_step(ex, v))) return st;
@@ -447,9 +450,8 @@ extern "C" int dugks_objective_run(dugks_handle* h, const dugks_objective* obj, 
     }
     for (int n = obj->window_start; n < obj->n_steps; ++n) {
         adj::View w = v;
-        const int c = h->ds.cur;
-        w.g = static_cast<const double*>(h->ds.g[c]);
-        w.h = static_cast<const double*>(h->ds.h[c]);
+        w.g = static_cast<const double*>(h->ds.g);
+        w.h = static_cast<const double*>(h->ds.h);
         w.cm = h->ds.cm;
         w.wn = 1.0 / (obj->n_steps - obj->window_start);
         if ((st = adj::record_step(ex, w))) return st;

@@ -65,7 +65,7 @@ enum { CO_AL = 0, CO_BE = 1, CO_GA = 4, CO_AQ = 5, CO_U = 8 };
 struct View {
     int nC, nIF, nBF, nF, nv, D, K, nchF, nchC;
     double R, Pr, omega, Tref, mu, dt;
-    // mesh (cells in the handle's numbering; faces internal then boundary)
+    // mesh (cells and faces in the handle's numbering; faces internal then boundary)
     const int32_t* own;     // [nF]
     const int32_t* nei;     // [nIF]
     const double* S;        // [nF][3]
@@ -91,15 +91,14 @@ struct View {
     const double* g;        // [nv][nC]
     const double* h;
     const double* cm;       // [nC][9] rho U T q tau the step starts from
-    // the tiled pass A's face-value buffer [nv][n_items] and the items of
-    // every face ([nF][2], -1: none), from which the record takes its face values
-    const double* fvg;
-    const double* fvh;
-    const int32_t* fitems;
-    int64_t nI;
-    // forward record of the step
+    // forward record of the step: the handle's face-value buffers, faces in
+    // the order of the step's arrays, and the raw moments k_face_moments sums
+    // of them ([nchM][16][nF]) with the incoming wall DFs' per unit rho_w
     double* fg;             // [nv][nF] face values before the relaxation
     double* fh;
+    const double* fmom;
+    int nchM;
+    const double* bmom_in;  // [nBF][16]
     double* pf;             // [nchF][nF][kP]
     double* pc;             // [nchC][nC][kP]
     double* rhow;           // [nBF]
@@ -416,115 +415,41 @@ struct FInBy {
     }
 };
 
-// 1-3: the face values at the half step (wall incoming DVs come in stage 5)
-// from the tiled pass A of the step (gbar+, the least-squares gradients and
-// the upwind reconstruction, fvDVM.C:648-683, discreteVelocity.C:366-369,
-// fvDVM.C:755-1029), gathered from item to face order.  A tile-boundary face
-// has an item in each tile: the upwind tile writes the value into both, and
-// on an exactly tangential face each holds its own side's half.  Far-field
-// incoming DVs are not stored by pass A: rho_b M(U_owner, T_b) here.
-struct FFace {
-    View v;
-    static constexpr int kMinCtas = 4;  // 32 warps per SM: at most 64 registers
-    ADJ_HD void operator()(int64_t idx) const {
-        const int i = static_cast<int>(idx / v.nF), f = static_cast<int>(idx % v.nF);
-        const double* xi = v.xi + 3 * i;
-        const double xs = xs_of(xi, v.S + 3 * f);
-        const size_t r = static_cast<size_t>(i) * static_cast<size_t>(v.nI);
-        const int it0 = v.fitems[2 * f], it1 = v.fitems[2 * f + 1];
-        if (f < v.nIF) {
-            double g = v.fvg[r + it0], h = v.fvh[r + it0];
-            if (it1 >= 0 && !(xs >= kVSmall) && !(xs < -kVSmall)) {
-                g += v.fvg[r + it1];
-                h += v.fvh[r + it1];
-            }
-            v.fg[idx] = g;
-            v.fh[idx] = h;
-            return;
-        }
-        const int b = f - v.nIF, ow = v.own[f];
-        if (xs > 0) {
-            v.fg[idx] = v.fvg[r + it0];
-            v.fh[idx] = v.fvh[r + it0];
-        } else if (v.btype[b] == 2) {
-            const double Tb = v.bT[b];
-            const double gi = v.brho[b] * eq_by_rho(v, xi, v.cm + 9 * static_cast<size_t>(ow) + 1, Tb);
-            v.fg[idx] = gi;
-            v.fh[idx] = gi * (v.R * Tb) * static_cast<double>(v.K + 3 - v.D);
-        }
-    }
-};
-
-// 4: outgoing flux of the wall faces, per DV chunk (slot 14)
-struct FWallOut {
-    View v;
-    ADJ_HD void operator()(int64_t idx) const {
-        const int ch = static_cast<int>(idx / v.nBF), b = static_cast<int>(idx % v.nBF);
-        const int f = v.nIF + b;
-        double out = 0;
-        if (v.btype[b] == 1) {
-            const double* S = v.S + 3 * f;
-            for (int i = chunk_lo(v.nv, v.nchF, ch); i < chunk_lo(v.nv, v.nchF, ch + 1); ++i) {
-                const double xs = xs_of(v.xi + 3 * i, S);
-                if (xs > 0) out += v.w[i] * xs * v.fg[at(i, v.nF, f)];
-            }
-        }
-        v.pf[(static_cast<size_t>(ch) * v.nF + f) * kP + 14] = out;
-    }
-};
-
-// 4b: rho_w = outgoing / |inComingByRho|
-struct FWallRho {
-    View v;
-    ADJ_HD void operator()(int64_t b) const {
-        const int f = v.nIF + static_cast<int>(b);
-        double out = 0;
-        for (int ch = 0; ch < v.nchF; ++ch) out += v.pf[(static_cast<size_t>(ch) * v.nF + f) * kP + 14];
-        v.rhow[b] = v.btype[b] == 1 ? out / fabs(v.inby[b]) : 0.0;
-    }
-};
-
-// 5: incoming wall DFs
-struct FWallIn {
-    View v;
-    ADJ_HD void operator()(int64_t idx) const {
-        const int i = static_cast<int>(idx / v.nBF), b = static_cast<int>(idx % v.nBF);
-        if (v.btype[b] != 1) return;
-        const int f = v.nIF + b;
-        const double* xi = v.xi + 3 * i;
-        if (xs_of(xi, v.S + 3 * f) <= 0) {
-            const double Tb = v.bT[b];
-            const double gi = v.rhow[b] * eq_by_rho(v, xi, v.bU + 3 * b, Tb);
-            v.fg[at(i, v.nF, f)] = gi;
-            v.fh[at(i, v.nF, f)] = gi * (v.R * Tb) * static_cast<double>(v.K + 3 - v.D);
-        }
-    }
-};
-
-// 6: raw moments of the face values, per DV chunk (slots 0..13)
-struct FFaceMom {
-    View v;
-    static constexpr int kMinCtas = 4;  // 32 warps per SM: at most 64 registers
-    ADJ_HD void operator()(int64_t idx) const {
-        const int ch = static_cast<int>(idx / v.nF), f = static_cast<int>(idx % v.nF);
-        double m[14] = {0};
-        for (int i = chunk_lo(v.nv, v.nchF, ch); i < chunk_lo(v.nv, v.nchF, ch + 1); ++i)
-            add_moments(v.xi + 3 * i, v.w[i], v.fg[at(i, v.nF, f)], v.fh[at(i, v.nF, f)], m);
-        double* p = v.pf + (static_cast<size_t>(ch) * v.nF + f) * kP;
-        for (int k = 0; k < 14; ++k) p[k] = m[k];
-    }
-};
-
-// 6b: face macro records
+// 1-3 and the sums of 4 and 6 come from the step's own kernels (half step,
+// face values, face moments), which leave the face values at the half step in
+// fg, fh and their raw moments, far-field incoming DFs included, in fmom.
+// 4, 6: rho_w = outgoing / |inComingByRho| of the wall faces, whose incoming
+// DFs are rho_w times a fixed Maxwellian, and the face macro records
 struct FFaceMac {
     View v;
     ADJ_HD void operator()(int64_t f) const {
-        double m[14] = {0};
-        for (int ch = 0; ch < v.nchF; ++ch) {
-            const double* p = v.pf + (static_cast<size_t>(ch) * v.nF + f) * kP;
-            for (int k = 0; k < 14; ++k) m[k] += p[k];
+        double m[15] = {0};
+        for (int ch = 0; ch < v.nchM; ++ch)
+            for (int k = 0; k < 15; ++k) m[k] += v.fmom[(static_cast<size_t>(ch) * kP + k) * v.nF + f];
+        if (f >= v.nIF) {
+            const int64_t b = f - v.nIF;
+            v.rhow[b] = v.btype[b] == 1 ? m[14] / fabs(v.inby[b]) : 0.0;
+            if (v.btype[b] == 1)
+                for (int k = 0; k < 14; ++k) m[k] += v.rhow[b] * v.bmom_in[kP * b + k];
         }
         macros_from_moments(v, m, 0.5 * v.dt * v.Pr, v.fmac + kMac * static_cast<size_t>(f));
+    }
+};
+
+// 5: incoming DFs: wall rho_w M(U_w, T_w), far field rho_b M(U_owner, T_b)
+struct FIncoming {
+    View v;
+    ADJ_HD void operator()(int64_t idx) const {
+        const int i = static_cast<int>(idx / v.nBF), b = static_cast<int>(idx % v.nBF);
+        const int f = v.nIF + b;
+        const double* xi = v.xi + 3 * i;
+        if (xs_of(xi, v.S + 3 * f) > 0) return;
+        const bool wall = v.btype[b] == 1;
+        const double Tb = v.bT[b];
+        const double gi = wall ? v.rhow[b] * eq_by_rho(v, xi, v.bU + 3 * b, Tb)
+                               : v.brho[b] * eq_by_rho(v, xi, v.cm + 9 * static_cast<size_t>(v.own[f]) + 1, Tb);
+        v.fg[at(i, v.nF, f)] = gi;
+        v.fh[at(i, v.nF, f)] = gi * (v.R * Tb) * static_cast<double>(v.K + 3 - v.D);
     }
 };
 
@@ -985,15 +910,9 @@ struct RInBy {
 template <class Ex>
 int record_step(Ex& ex, const View& v) {
     int st;
-    if ((st = ex.pass_a(v))) return st;
-    if ((st = ex.run(static_cast<int64_t>(v.nv) * v.nF, FFace{v}))) return st;
-    if (v.nBF > 0) {
-        if ((st = ex.run(static_cast<int64_t>(v.nchF) * v.nBF, FWallOut{v}))) return st;
-        if ((st = ex.run(v.nBF, FWallRho{v}))) return st;
-        if ((st = ex.run(static_cast<int64_t>(v.nv) * v.nBF, FWallIn{v}))) return st;
-    }
-    if ((st = ex.run(static_cast<int64_t>(v.nchF) * v.nF, FFaceMom{v}))) return st;
-    return ex.run(v.nF, FFaceMac{v});
+    if ((st = ex.face_values(v))) return st;
+    if ((st = ex.run(v.nF, FFaceMac{v}))) return st;
+    return ex.run(static_cast<int64_t>(v.nv) * v.nBF, FIncoming{v});
 }
 
 // reverse of one step from its record: og/oh = adjoint of the state before

@@ -1,11 +1,10 @@
 // Host-side preparation of the DUGKS step: OpenFOAM mesh geometry,
 // surface-interpolation weights, least-squares gradient vectors, and the
-// tile layout the device passes work on.
+// cell and face order the device passes work in.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <numeric>
-#include <unordered_map>
 
 #include "dugks_internal.h"
 
@@ -247,9 +246,14 @@ namespace {
 // Recursive coordinate bisection: cut the cell set along the longest axis
 // of its bounding box so that the first part holds a whole number of tiles,
 // until every part is one tile.  Consecutive tiles are neighbours in space.
-void rcb_order(const std::vector<double>& C, std::vector<int32_t>& idx, size_t b, size_t e, int tile) {
+// by_index: within a tile the caller's order stays, whose runs along a grid
+// line make the neighbours of consecutive cells consecutive.
+void rcb_order(const std::vector<double>& C, std::vector<int32_t>& idx, size_t b, size_t e, int tile, bool by_index) {
     const size_t n = e - b;
-    if (n <= static_cast<size_t>(tile)) return;
+    if (n <= static_cast<size_t>(tile)) {
+        if (by_index) std::sort(idx.begin() + b, idx.begin() + e);
+        return;
+    }
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
     for (size_t i = b; i < e; ++i)
         for (int k = 0; k < 3; ++k) {
@@ -262,15 +266,14 @@ void rcb_order(const std::vector<double>& C, std::vector<int32_t>& idx, size_t b
     const size_t nt = (n + tile - 1) / tile;
     const size_t nl = (nt / 2) * static_cast<size_t>(tile);
     std::stable_sort(idx.begin() + b, idx.begin() + e, [&](int32_t p, int32_t q) { return C[3 * p + ax] < C[3 * q + ax]; });
-    rcb_order(C, idx, b, b + nl, tile);
-    rcb_order(C, idx, b + nl, e, tile);
+    rcb_order(C, idx, b, b + nl, tile, by_index);
+    rcb_order(C, idx, b + nl, e, tile, by_index);
 }
 
 // Greedy tile boundaries over the RCB cell order: each tile takes the next
 // cells in order while it keeps at most kMaxTile L0 cells, kMaxLocal cells
-// with its ring and kMaxItems faces.  A pass CTA costs about the same
-// whatever its tile's size, so the fewest tiles that fit is the aim; tiles
-// end where the ring, not a fixed size, runs out.
+// with its ring and kMaxItems faces.  Tiles end where the ring, not a fixed size, runs
+// out.
 std::vector<int32_t> greedy_bounds(int nC, int nIF, const std::vector<int64_t>& owner,
                                    const std::vector<int64_t>& neighbour, const std::vector<int32_t>& cfo,
                                    const std::vector<int32_t>& cfl, const std::vector<int32_t>& perm,
@@ -332,190 +335,173 @@ std::vector<int32_t> greedy_bounds(int nC, int nIF, const std::vector<int64_t>& 
     return bounds;
 }
 
+// whether every tile [bounds[i], bounds[i+1]) keeps the limits of greedy_bounds
+bool tiles_fit(int nIF, const std::vector<int64_t>& owner, const std::vector<int64_t>& neighbour,
+               const std::vector<int32_t>& cfo, const std::vector<int32_t>& cfl, const std::vector<int32_t>& perm,
+               const std::vector<int32_t>& iperm, const std::vector<int32_t>& bounds) {
+    std::vector<int32_t> seen(perm.size(), -1);
+    for (size_t t = 0; t + 1 < bounds.size(); ++t) {
+        const int b = bounds[t], e = bounds[t + 1];
+        int ring = 0, items = 0;
+        for (int c = b; c < e; ++c)
+            for (int k = cfo[perm[c]]; k < cfo[perm[c] + 1]; ++k) {
+                const int f = cfl[k];
+                const int n = f >= nIF ? -1 : iperm[owner[f] == perm[c] ? neighbour[f] : owner[f]];
+                const bool inside = n >= b && n < e;
+                if (!inside || c < n) ++items;
+                if (n >= 0 && !inside && seen[n] != static_cast<int>(t)) {
+                    seen[n] = static_cast<int>(t);
+                    ++ring;
+                }
+            }
+        if (e - b + ring > dugks::kMaxLocal || items > dugks::kMaxItems) return false;
+    }
+    return true;
+}
+
+// Compact tiles of the mesh, of at most tile_cells cells (0: as large as the
+// limits of greedy_bounds allow).  No kernel works tile by tile; dugks_layout
+// reports them, and FP32 rows round one product by them (DevMesh::cface).
+// Returns the tile of every (caller's) cell.
+std::vector<int32_t> tile_cells_of(const dugks_handle* h, int tile_cells, dugks::Tiling& t) {
+    const int nC = h->nC, nIF = h->nIF, nF = nIF + h->nBF;
+    std::vector<int32_t> cfo(nC + 1, 0);
+    for (int f = 0; f < nF; ++f) cfo[h->owner[f] + 1]++;
+    for (int f = 0; f < nIF; ++f) cfo[h->neighbour[f] + 1]++;
+    for (int c = 0; c < nC; ++c) cfo[c + 1] += cfo[c];
+    std::vector<int32_t> cfl(cfo[nC]), fill(cfo.begin(), cfo.end() - 1), perm(nC), iperm(nC), bounds;
+    for (int f = 0; f < nF; ++f) {
+        cfl[fill[h->owner[f]]++] = f;
+        if (f < nIF) cfl[fill[h->neighbour[f]]++] = f;
+    }
+    for (int tile = std::min(tile_cells, dugks::kMaxTile);; tile = std::max(4, tile * 7 / 8)) {
+        std::iota(perm.begin(), perm.end(), 0);
+        rcb_order(h->C, perm, 0, nC, tile_cells > 0 ? tile : 4, false);
+        for (int c = 0; c < nC; ++c) iperm[perm[c]] = c;
+        bounds.clear();
+        if (tile_cells <= 0) {
+            bounds = greedy_bounds(nC, nIF, h->owner, h->neighbour, cfo, cfl, perm, iperm);
+            break;
+        }
+        for (int b = 0; b < nC; b += tile) bounds.push_back(b);
+        bounds.push_back(nC);
+        if (tile <= 4 || tiles_fit(nIF, h->owner, h->neighbour, cfo, cfl, perm, iperm, bounds)) break;
+    }
+    t.fits = tiles_fit(nIF, h->owner, h->neighbour, cfo, cfl, perm, iperm, bounds);
+    t.n_tiles = static_cast<int>(bounds.size()) - 1;
+    t.tile_cells = 0;
+    std::vector<int32_t> tile_of(nC);
+    for (int i = 0; i < t.n_tiles; ++i) {
+        t.tile_cells = std::max(t.tile_cells, bounds[i + 1] - bounds[i]);
+        for (int c = bounds[i]; c < bounds[i + 1]; ++c) tile_of[perm[c]] = i;
+    }
+    return tile_of;
+}
+
 }  // namespace
 
 namespace dugks {
 
-// Tile layout.  Cells are renumbered by recursive coordinate bisection and
-// cut into tiles of `tile_cells` consecutive cells (L0), or, with
-// tile_cells = 0, into the greedy tiles of greedy_bounds.  Each tile also
-// holds its ring L1 (face neighbours of L0 outside it), and one item per
-// face touching L0, sorted by item kind.  Gradient stencils and flux lists
-// are stored slot-major ([slot][cell]) so that consecutive threads read
-// consecutive words.
+// Cell order, face order and the tables of the step's kernels.  Cells are
+// renumbered by recursive coordinate bisection down to 1,024 cells, so that a CTA's cells and their neighbours meet in L1 and L2.
+// Smaller parts cost the gathers more sectors than they save: on a 6 x 16^3
+// cubed sphere the face values' L1 load is 51 % with parts of 4, 44 % with 256,
+// 40 % with 1,024.  Internal faces are numbered by the
+// lower of their two cells: in blocks of 32 cells, the first faces of the
+// block's cells, then the second ones and so on, so that the k-th faces of
+// consecutive cells are nearly consecutive.  Boundary faces follow in the
+// caller's order.  Stencils and face lists are slot-major ([slot][cell]).
 void build_tiling(dugks_handle* h, int tile_cells) {
     Tiling& t = h->tiling;
-    const int nC = h->nC, nIF = h->nIF, nBF = h->nBF;
+    const int nC = h->nC, nIF = h->nIF, nBF = h->nBF, nF = nIF + nBF;
     t.perm.resize(nC);
     std::iota(t.perm.begin(), t.perm.end(), 0);
-    const bool greedy = tile_cells <= 0;
-    rcb_order(h->C, t.perm, 0, nC, greedy ? 4 : tile_cells);
+    const std::vector<int32_t> tile_of = tile_cells_of(h, tile_cells, t);
+    rcb_order(h->C, t.perm, 0, nC, 1024, true);
     t.iperm.assign(nC, 0);
     for (int c = 0; c < nC; ++c) t.iperm[t.perm[c]] = c;
 
-    // cell -> faces (original numbering)
+    // cell -> faces, those it owns first, each part in the caller's face order
+    // (the order the cell's gradient and fluxes are summed in)
     std::vector<int32_t> cfo(nC + 1, 0);
-    for (int f = 0; f < nIF + nBF; ++f) cfo[h->owner[f] + 1]++;
-    for (int f = 0; f < nIF; ++f) cfo[h->neighbour[f] + 1]++;
-    for (int c = 0; c < nC; ++c) cfo[c + 1] += cfo[c];
-    std::vector<int32_t> cfl(cfo[nC]), fill(cfo.begin(), cfo.end() - 1);
-    for (int f = 0; f < nIF + nBF; ++f) cfl[fill[h->owner[f]]++] = f;
-    for (int f = 0; f < nIF; ++f) cfl[fill[h->neighbour[f]]++] = f;
-    t.nb_max = t.nf_max = 0;
+    for (int f = 0; f < nF; ++f) cfo[t.iperm[h->owner[f]] + 1]++;
+    for (int f = 0; f < nIF; ++f) cfo[t.iperm[h->neighbour[f]] + 1]++;
+    t.nf_max = 0;
     for (int c = 0; c < nC; ++c) {
-        int nb = 0;
-        for (int k = cfo[c]; k < cfo[c + 1]; ++k) nb += cfl[k] < nIF;
+        t.nf_max = std::max(t.nf_max, cfo[c + 1]);
+        cfo[c + 1] += cfo[c];
+    }
+    std::vector<int32_t> cfl(cfo[nC]), fill(cfo.begin(), cfo.end() - 1);
+    for (int f = 0; f < nF; ++f) cfl[fill[t.iperm[h->owner[f]]]++] = f;
+    for (int f = 0; f < nIF; ++f) cfl[fill[t.iperm[h->neighbour[f]]]++] = f;
+
+    // face order
+    struct Key {
+        int block, rank, cell, face;
+        bool operator<(const Key& o) const {
+            if (block != o.block) return block < o.block;
+            if (rank != o.rank) return rank < o.rank;
+            return cell < o.cell;
+        }
+    };
+    std::vector<Key> keys;
+    keys.reserve(nIF);
+    t.nb_max = 0;
+    for (int c = 0; c < nC; ++c) {
+        int rank = 0, nb = 0;
+        for (int k = cfo[c]; k < cfo[c + 1]; ++k) {
+            const int f = cfl[k];
+            if (f >= nIF) continue;
+            ++nb;
+            const int o = t.iperm[h->owner[f]], n = t.iperm[h->neighbour[f]];
+            if (std::min(o, n) == c) keys.push_back({c / 32, rank++, c, f});
+        }
         t.nb_max = std::max(t.nb_max, nb);
-        t.nf_max = std::max(t.nf_max, cfo[c + 1] - cfo[c]);
+    }
+    std::sort(keys.begin(), keys.end());
+    t.forig.resize(nF);
+    t.fnew.resize(nF);
+    for (int i = 0; i < nF; ++i) {
+        t.forig[i] = i < nIF ? keys[i].face : i;
+        t.fnew[t.forig[i]] = i;
+    }
+    t.fown.resize(nF);
+    t.fnei.resize(std::max(nIF, 1));
+    t.fgeo.assign(9 * static_cast<size_t>(nF), 0.0);
+    for (int i = 0; i < nF; ++i) {
+        const int f = t.forig[i];
+        const int64_t o = h->owner[f];
+        t.fown[i] = t.iperm[o];
+        for (int q = 0; q < 3; ++q) {
+            t.fgeo[static_cast<size_t>(q) * nF + i] = h->Sf[3 * f + q];
+            t.fgeo[static_cast<size_t>(3 + q) * nF + i] = h->Cf[3 * f + q] - h->C[3 * o + q];
+        }
+        if (f >= nIF) continue;
+        const int64_t n = h->neighbour[f];
+        t.fnei[i] = t.iperm[n];
+        for (int q = 0; q < 3; ++q) t.fgeo[static_cast<size_t>(6 + q) * nF + i] = h->Cf[3 * f + q] - h->C[3 * n + q];
     }
 
-    std::vector<int32_t> bounds;
-    if (greedy) {
-        bounds = greedy_bounds(nC, nIF, h->owner, h->neighbour, cfo, cfl, t.perm, t.iperm);
-    } else {
-        for (int b = 0; b < nC; b += tile_cells) bounds.push_back(b);
-        bounds.push_back(nC);
-    }
-    t.n_tiles = static_cast<int>(bounds.size()) - 1;
-    t.tile_cells = 0;
-    for (int ti = 0; ti < t.n_tiles; ++ti) t.tile_cells = std::max(t.tile_cells, bounds[ti + 1] - bounds[ti]);
-    t.tile_begin.assign(t.n_tiles + 1, 0);
-    t.tile_loc_off.assign(t.n_tiles + 1, 0);
-    t.tile_item_off.assign(t.n_tiles + 1, 0);
-    t.loc_cells.clear();
-    t.it_meta.clear();
-    t.it_loc.clear();
-    t.it_face.clear();
-    t.it_other.clear();
-    std::vector<double> geo;  // item-major scratch [n_items][9]
-    t.grad_nb.assign(static_cast<size_t>(t.nb_max) * nC, -1);
-    t.grad_ls.assign(static_cast<size_t>(t.nb_max) * 3 * nC, 0.0);
-    t.cf_item.assign(static_cast<size_t>(t.nf_max) * nC, 0);
-    t.max_local = t.max_l0 = t.max_items = 0;
-    std::vector<int32_t> face_item0(nIF + nBF, -1), face_item1(nIF + nBF, -1);
-    std::vector<int32_t> local_of(nC, -1);
-    struct Pending {
-        int kind, f;
-    };
-    for (int ti = 0; ti < t.n_tiles; ++ti) {
-        const int b = bounds[ti], e = bounds[ti + 1], n0 = e - b;
-        t.tile_begin[ti] = b;
-        t.tile_loc_off[ti] = static_cast<int32_t>(t.loc_cells.size());
-        std::vector<int32_t> l1;
-        for (int c = b; c < e; ++c) {
-            const int o = t.perm[c];
-            for (int k = cfo[o]; k < cfo[o + 1]; ++k) {
-                const int f = cfl[k];
-                if (f >= nIF) continue;
-                const int other = h->owner[f] == o ? static_cast<int>(h->neighbour[f]) : static_cast<int>(h->owner[f]);
-                const int on = t.iperm[other];
-                if (on < b || on >= e) l1.push_back(on);
-            }
-        }
-        std::sort(l1.begin(), l1.end());
-        l1.erase(std::unique(l1.begin(), l1.end()), l1.end());
-        for (int c = b; c < e; ++c) {
-            local_of[c] = c - b;
-            t.loc_cells.push_back(c);
-        }
-        for (size_t i = 0; i < l1.size(); ++i) {
-            local_of[l1[i]] = n0 + static_cast<int>(i);
-            t.loc_cells.push_back(l1[i]);
-        }
-        // the tile's faces, sorted by kind
-        std::vector<Pending> pend;
-        for (int c = b; c < e; ++c) {
-            const int o = t.perm[c];
-            for (int k = cfo[o]; k < cfo[o + 1]; ++k) {
-                const int f = cfl[k];
-                int kind;
-                if (f < nIF) {
-                    const int own_new = t.iperm[h->owner[f]], nei_new = t.iperm[h->neighbour[f]];
-                    const bool own_in = own_new >= b && own_new < e, nei_in = nei_new >= b && nei_new < e;
-                    if (own_in && nei_in && own_new != c) continue;  // listed once, from the owner
-                    kind = (own_in && nei_in) ? ITEM_TILE_INTERNAL : (own_in ? ITEM_TB_OWN : ITEM_TB_NEI);
-                } else {
-                    kind = ITEM_MESH_BOUNDARY;
-                }
-                pend.push_back({kind, f});
-            }
-        }
-        std::stable_sort(pend.begin(), pend.end(), [](const Pending& p, const Pending& q) { return p.kind < q.kind; });
-        const int item0 = t.n_items();
-        t.tile_item_off[ti] = item0;
-        std::unordered_map<int, int> face_to_local_item;
-        for (const Pending& p : pend) {
-            const int f = p.f;
-            const int64_t fo = h->owner[f];
-            const int lo = local_of[t.iperm[fo]];
-            int ln = 0xffff, ptype = 0;
-            double g9[9];
-            for (int q = 0; q < 3; ++q) {
-                g9[q] = h->Sf[3 * f + q];
-                g9[3 + q] = h->Cf[3 * f + q] - h->C[3 * fo + q];
-                g9[6 + q] = 0.0;
-            }
+    // gradient stencils and face lists, slots in that order
+    t.nbr.resize(static_cast<size_t>(std::max(t.nb_max, 1)) * nC);
+    for (size_t i = 0; i < t.nbr.size(); ++i) t.nbr[i] = static_cast<int32_t>(i % nC);
+    t.nbr_ls.assign(static_cast<size_t>(std::max(t.nb_max, 1)) * 3 * nC, 0.0);
+    t.cface.assign(static_cast<size_t>(t.nf_max) * nC, -1);
+    for (int c = 0; c < nC; ++c) {
+        int sb = 0, sf = 0;
+        for (int k = cfo[c]; k < cfo[c + 1]; ++k) {
+            const int f = cfl[k], i = t.fnew[f];
+            const bool is_own = t.fown[i] == c;
             if (f < nIF) {
-                const int64_t fn = h->neighbour[f];
-                ln = local_of[t.iperm[fn]];
-                for (int q = 0; q < 3; ++q) g9[6 + q] = h->Cf[3 * f + q] - h->C[3 * fn + q];
-            } else {
-                ptype = h->bface_ptype[f - nIF];
+                t.nbr[static_cast<size_t>(sb) * nC + c] = is_own ? t.fnei[i] : t.fown[i];
+                const double* ls = is_own ? &h->lsP[3 * f] : &h->lsN[3 * f];
+                for (int q = 0; q < 3; ++q) t.nbr_ls[(static_cast<size_t>(sb) * 3 + q) * nC + c] = ls[q];
+                ++sb;
             }
-            t.it_meta.push_back(p.kind | (ptype << 4));
-            t.it_loc.push_back(lo | (ln << 16));
-            t.it_face.push_back(f < nIF ? f : f - nIF);
-            t.it_other.push_back(-1);
-            geo.insert(geo.end(), g9, g9 + 9);
-            const int li = t.n_items() - 1 - item0;
-            face_to_local_item[f] = li;
-            if (face_item0[f] < 0) face_item0[f] = item0 + li;
-            else face_item1[f] = item0 + li;
+            const bool in_tile = f < nIF && tile_of[h->owner[f]] == tile_of[h->neighbour[f]];
+            t.cface[static_cast<size_t>(sf) * nC + c] = 4 * i + (in_tile ? 2 : 0) + (is_own ? 0 : 1);
+            ++sf;
         }
-        // gradient stencils and flux lists of the L0 cells
-        for (int c = b; c < e; ++c) {
-            const int o = t.perm[c];
-            int sb = 0, sf = 0;
-            for (int k = cfo[o]; k < cfo[o + 1]; ++k) {
-                const int f = cfl[k];
-                const bool is_own = h->owner[f] == o;
-                if (f < nIF) {
-                    const int other = is_own ? static_cast<int>(h->neighbour[f]) : static_cast<int>(h->owner[f]);
-                    t.grad_nb[static_cast<size_t>(sb) * nC + c] = local_of[t.iperm[other]];
-                    const double* ls = is_own ? &h->lsP[3 * f] : &h->lsN[3 * f];
-                    for (int q = 0; q < 3; ++q) t.grad_ls[(static_cast<size_t>(sb) * 3 + q) * nC + c] = ls[q];
-                    ++sb;
-                }
-                const int li = face_to_local_item.at(f);
-                t.cf_item[static_cast<size_t>(sf) * nC + c] = is_own ? -(li + 1) : (li + 1);
-                ++sf;
-            }
-        }
-        for (int c = b; c < e; ++c) local_of[c] = -1;
-        for (int c : l1) local_of[c] = -1;
-        t.max_local = std::max(t.max_local, n0 + static_cast<int>(l1.size()));
-        t.max_l0 = std::max(t.max_l0, n0);
-        t.max_items = std::max(t.max_items, t.n_items() - item0);
-    }
-    t.tile_begin[t.n_tiles] = nC;
-    t.tile_loc_off[t.n_tiles] = static_cast<int32_t>(t.loc_cells.size());
-    t.tile_item_off[t.n_tiles] = t.n_items();
-    // the item of the other side of every tile-boundary face: pass B reads
-    // that side's share of the face value from the item's face-value slot
-    const int ni = t.n_items();
-    for (int i = 0; i < ni; ++i) {
-        const int kind = t.it_meta[i] & 15;
-        if (kind != ITEM_TB_OWN && kind != ITEM_TB_NEI) continue;
-        const int f = t.it_face[i];
-        t.it_other[i] = face_item0[f] == i ? face_item1[f] : face_item0[f];
-    }
-    t.it_geo.assign(static_cast<size_t>(9) * ni, 0.0);
-    for (int i = 0; i < ni; ++i)
-        for (int q = 0; q < 9; ++q) t.it_geo[static_cast<size_t>(q) * ni + i] = geo[static_cast<size_t>(i) * 9 + q];
-    t.face_items.assign(2 * static_cast<size_t>(nIF + nBF), -1);
-    for (int f = 0; f < nIF + nBF; ++f) {
-        t.face_items[2 * f] = face_item0[f];
-        t.face_items[2 * f + 1] = face_item1[f];
     }
 }
 

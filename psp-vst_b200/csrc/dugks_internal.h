@@ -12,10 +12,10 @@
 
 namespace dugks {
 
-constexpr int kThreads = 512;      // threads per CTA of the two tile passes
-constexpr int kMaxTile = 128;      // cells per tile (L0) at most
-constexpr int kMaxLocal = 256;     // L0 + L1 cells per tile at most
-constexpr int kMaxItems = kThreads - 1;  // items per tile at most (one per thread; one flux slot kept zero)
+constexpr int kMaxTile = 128;      // cells per tile at most
+constexpr int kMaxLocal = 256;     // cells of a tile with its ring of neighbours at most
+constexpr int kMaxItems = 511;     // faces of a tile's cells at most
+constexpr int kSeg = 32;           // DVs per segment at most (one bit each in DevMesh::upw)
 constexpr int kMaxN1d = 64;        // DV nodes per dimension at most
 constexpr int kNM = 16;            // stride of a partial-moment record (doubles)
 constexpr int kFX = 8;             // stride of a flux-moment record: M0, M1[3], W/2
@@ -31,15 +31,6 @@ enum {
     MOM_M0 = 0, MOM_M1 = 1, MOM_W = 4, MOM_V3 = 5, MOM_M2 = 8, MOM_OUT = 14
 };
 
-// item kinds of a tile (faces touching the tile's own cells); a tile lists
-// its items sorted by kind so that warps see one kind at a time
-enum : int32_t {
-    ITEM_TILE_INTERNAL = 0,   // owner and neighbour both in the tile
-    ITEM_TB_OWN = 1,          // tile-boundary face, owner side in the tile
-    ITEM_TB_NEI = 2,          // tile-boundary face, neighbour side in the tile
-    ITEM_MESH_BOUNDARY = 3    // boundary face of a non-empty patch
-};
-
 // Record fields of the structure-of-arrays coefficient tables.  Cell
 // records (gbar+ half step, fvDVM.C:668-679) and face records (face
 // relaxation, fvDVM.C:1374-1444) share the layout: field k of entity e is
@@ -48,7 +39,7 @@ enum {
     REC_UX = 0, REC_UY = 1, REC_UZ = 2,
     REC_INVRT = 3,   // 1/(R T)
     REC_A = 4,       // rho (2 pi R T)^(-D/2)
-    REC_R = 5,       // relax factor: cells 1.5 dt/(2 tau + dt), faces 0.5 dt/(2 tau + 0.5 dt)
+    REC_R = 5,       // faces: relax factor 0.5 dt/(2 tau + 0.5 dt); cells: tau (the factor follows the step's dt)
     REC_QX = 6, REC_QY = 7, REC_QZ = 8,   // (1-Pr) q / (5 rho (R T)^2)
     REC_RTH = 9,     // R T used by h^S (boundary faces: the internal-face T at the patch-local index)
     REC_N = 10
@@ -72,7 +63,7 @@ struct __align__(16) BRec {
 struct DevMesh {
     int D, K;
     double R, Pr, omega, Tref, muRef;
-    int nC, nIF, nBF, nv, n_tiles;
+    int nC, nIF, nBF, nF, nv;
     // DVs this device holds: global DVs dv_base .. dv_base + nv_loc - 1, the
     // DV rows row_base ..; the state and face-value arrays are [nv_loc][..]
     int nv_loc, dv_base, row_base;
@@ -84,25 +75,25 @@ struct DevMesh {
     int general_dv;        // 1: a DV list that is no tensor product (n1d is 1, a "row" is one DV)
     const double* X1;      // [n1d] one-dimensional nodes
     const double* W1;      // [n1d] one-dimensional weights
-    // tiles
-    const int32_t* tile_begin;     // [n_tiles+1] L0 = [begin, begin+n0) (renumbered cells)
-    const int32_t* tile_loc_off;   // [n_tiles+1] into loc_cells
-    const int32_t* loc_cells;      // local cells (L0 then L1), renumbered ids
-    const int32_t* tile_item_off;  // [n_tiles+1] into the item arrays
-    // items (structure of arrays over all tiles' items)
-    const int32_t* it_meta;        // kind | ptype << 4
-    const int32_t* it_loc;         // lo | ln << 16 (0xffff: none); local indices
-    const int32_t* it_face;        // internal face id, or boundary face id
-    const int32_t* it_other;       // tile-boundary items: the item of the face's other side
-    const double* it_geo;          // [9][n_items]: S, Cf - C_own, Cf - C_nei
-    // gradient stencils and flux lists, slot-major [slot][cell]
+    // DV segments: up to kSeg consecutive DVs of one row (of the list); the
+    // kernels walk DVs by segments and DV chunks are runs of segments
+    int n_seg;
+    const int2* row_yz;            // y and z index of every row of this device
+    // Cells in the renumbered order.  Faces in the order of the step's arrays:
+    // internal faces grouped by blocks of 32 cells, first faces of a block's
+    // cells first, so that neighbouring cells reach neighbouring faces; then
+    // the boundary faces in the caller's order.
     int nb_max, nf_max;
-    const int32_t* grad_nb;        // [nb_max][nC] local index of the neighbour, -1: none
-    const double* grad_ls;         // [nb_max][3][nC] least-squares vector
-    const int32_t* cf_item;        // [nf_max][nC] (local item + 1) * (+1 nei / -1 own), 0: none
-    const double* dtV;             // 1/V per renumbered cell
-    // combine maps
-    const int32_t* face_items;     // [nF*2] global item ids of each face (-1 none)
+    const int32_t* nbr;            // [nb_max][nC] neighbour cells (absent: the cell itself)
+    const double* nbr_ls;          // [nb_max][3][nC] least-squares vectors (absent: 0)
+    const int32_t* cface;          // [nf_max][nC] faces of a cell: 2 face + (1 if the cell is the neighbour), -1 none
+    const double* invV;            // [nC]
+    const double* fgeo;            // [9][nF]: S, Cf - C_own, Cf - C_nei
+    const int32_t* fown;           // [nF] owner cell
+    const int32_t* fnei;           // [nIF] neighbour cell
+    const int32_t* forig;          // [nF] the caller's face
+    const uint32_t* upw;           // [n_seg][nF][2] upwind bits of a segment's DVs: owner side, neighbour side
+    int done_cells;                // first cell-block counter in DevState::done (face blocks before it)
     const int32_t* bface_patch_local;  // [nBF] index within its patch
     const int32_t* bface_ptype;    // [nBF]
     const int32_t* bface_owner;    // [nBF] renumbered owner cell
@@ -117,7 +108,6 @@ struct DevMesh {
     const double* mf_V;            // [nC] renumbered
     const double* dc;              // [nIF] deltaCoeffs
     const double* bS;              // [nBF*3] boundary face area vectors
-    int n_items;
     double xi_max_co;              // sqrt(D) * xiMax
     // FP32 storage of a tensor DV set: g~, gbar+, the face values and the
     // fluxes are stored as deviations from a per-DV reference Maxwellian,
@@ -129,56 +119,55 @@ struct DevMesh {
 
 // Mutable device state
 struct DevState {
-    void* g[2];        // state g~ [nv][nC] (Real); g[1] aliases g[0]: pass B updates in place
-    void* h[2];
-    int cur;
-    // face values [nv][n_items] (Real): pass A's upwind reconstruction at the
-    // half step of every item, weighted by the side's share on tile-boundary
-    // faces; pass B relaxes them instead of reconstructing again
+    void* g;           // state g~ [nv][nC] (Real), updated in place
+    void* h;
+    void* gbar;        // gbar+ of the step [nv][nC] (Real)
+    void* hbar;        // (null while h is identically zero)
+    // face values [nv][nF] (Real): the upwind reconstruction at the half step,
+    // then, relaxed and multiplied by xi.S, the flux
     void* fvg;
-    void* fvh;
-    double* partF;     // [chunks][n_items][kNM]
-    double* partC;     // [chunks][nC][kNM]
-    double* partX;     // [chunks][nC][kFX] DV-list macroFlux: moments of the flux term (else null)
-    double* redC;      // sharded DV-list macroFlux: [nC][kNM] cell moments then [nC][kFX] flux moments, reduced together
+    void* fvh;         // (null while h is identically zero)
+    double* partF;     // [chunks_f][kNM][nF]
+    double* partC;     // [chunks][kNM][nC]
+    double* partX;     // [chunks][kFX][nC] DV-list macroFlux: moments of the flux term (else null)
+    double* redC;      // sharded DV-list macroFlux: [kNM][nC] cell moments then [kFX][nC] flux moments, reduced together
+    int* done;         // chunks finished per face block, then per cell block; zero between launches
     double* cellrec;   // [REC_N][nC]
-    // face records in item order (each face's record is written to its one
-    // or two items, so that a tile reads its faces' records contiguously)
-    double* facerec;   // [REC_N][n_items]
+    double* facerec;   // [REC_N][nF]
     // one-dimensional Maxwellian factors, FP64 for both precisions (the
     // equilibrium and the relaxation are evaluated in FP64, so that the FP32
     // path injects no rounding bias into the conserved moments): table k of
     // entity e at node i is tab[(k * n1d + i) * n + e] = exp(-(X_i - U_k)^2 /
     // (2 R T)), the x table multiplied by A = rho (2 pi R T)^(-D/2)
     double* ctab;      // [D][n1d][nC]
-    double* ftab;      // [D][n1d][n_items]  (item order, as facerec)
+    double* ftab;      // [D][n1d][nF]
     BRec* brec;        // [nBF]
     double* bmom_in;   // [nBF][kNM] incoming wall moments per unit rho_w
     double* cm;        // cell macros [nC][9]: rho U(3) T q(3) tau (renumbered)
     // FP32 storage of a tensor DV set: the raw moments of the reference
-    // Maxwellian over each DV chunk, [chunks][kNM] (null otherwise); a face
-    // or cell whose DVs all count in full adds them once instead of per DV
+    // Maxwellian over this device's DVs, [kNM] (null otherwise); a face or
+    // cell whose DVs all count in full adds them once instead of per DV
     double* refmom;
-    double* fm;        // face macros [nF][9]
+    double* fm;        // face macros [nF][9], the caller's face order
     double* co;        // [2] Courant max (as ordered bits) and sum
     int* err;          // [4] device error flags
 };
 
+// Cell and face order of the device arrays and the tables built on them
 struct Tiling {
     int n_tiles = 0;
-    int tile_cells = 0;
-    int max_local = 0, max_l0 = 0, max_items = 0;
+    int tile_cells = 0;             // cells of the largest tile
+    bool fits = true;               // every tile keeps the limits above
     int nb_max = 0, nf_max = 0;
     std::vector<int32_t> perm;      // new -> old cell
     std::vector<int32_t> iperm;     // old -> new
-    std::vector<int32_t> tile_begin, tile_loc_off, loc_cells, tile_item_off;
-    std::vector<int32_t> it_meta, it_loc, it_face, it_other;
-    std::vector<double> it_geo;     // [9][n_items]
-    std::vector<int32_t> grad_nb;   // [nb_max][nC]
-    std::vector<double> grad_ls;    // [nb_max][3][nC]
-    std::vector<int32_t> cf_item;   // [nf_max][nC]
-    std::vector<int32_t> face_items;
-    int n_items() const { return static_cast<int>(it_meta.size()); }
+    std::vector<int32_t> forig;     // new -> caller's face
+    std::vector<int32_t> fnew;      // caller's -> new face
+    std::vector<int32_t> fown, fnei;
+    std::vector<double> fgeo;       // [9][nF]
+    std::vector<int32_t> nbr;       // [nb_max][nC]
+    std::vector<double> nbr_ls;     // [nb_max][3][nC]
+    std::vector<int32_t> cface;     // [nf_max][nC]
 };
 
 }  // namespace dugks
@@ -201,8 +190,7 @@ struct dugks_handle {
     std::vector<int64_t> owner, neighbour;
     std::vector<double> C, V, Cf, Sf, weights, dc, lsP, lsN, lsB;
     dugks::Tiling tiling;
-    int chunks = 1;
-    std::vector<int32_t> chunk_begin;   // DV chunk boundaries in global DV rows [chunks+1]
+    int chunks = 1, chunks_f = 1;       // DV chunks of the cell and of the face reductions
     // velocity-space shard (world 1: the whole DV set)
     int shard_rank = 0, shard_world = 1;
     bool shard_nccl = false;
@@ -215,7 +203,6 @@ struct dugks_handle {
     dugks::DevMesh dm{};
     dugks::DevState ds{};
     std::vector<void*> allocations;
-    int32_t* d_chunk_begin = nullptr;
     double* d_dt = nullptr;         // [2] device time steps of adaptive stepping (ping-pong)
     double* d_hist = nullptr;       // time steps of the last adaptive call
     int32_t hist_cap = 0;
@@ -224,7 +211,6 @@ struct dugks_handle {
     // every formula that feeds h (initial state, equilibria, boundary
     // DFs), so h stays zero unless dugks_set_state loads a nonzero h~
     bool h_zero = false;
-    double cellrec_dt = 0;          // time step the cell records' relax factors were built for
     long steps_done = 0;
     int64_t launches = 0;           // kernels launched by this handle
     double last_step_ms = 0;
@@ -237,9 +223,10 @@ namespace dugks {
 void compute_weights_and_ls(dugks_handle* h, int weighting);
 void build_tiling(dugks_handle* h, int tile_cells);
 int set_error(dugks_handle* h, int code, const std::string& msg);
-// ABI helper (dugks_abi.cpp): cell records and tables from ds.cm
+// ABI helpers (dugks_abi.cpp): cell records and tables from ds.cm
 int rebuild_cell_records(dugks_handle* h);
-// pass A of a step of size dt from the current state: the face-value buffer
-// then holds the step's upwind face values at the half step
+// the step's face values at the half step (DevState::fvg, fvh) and their raw
+// moments (partF, chunks_f chunks) for a step of size dt from the current
+// state, which stays as it is
 int record_face_values(dugks_handle* h, double dt);
 }  // namespace dugks

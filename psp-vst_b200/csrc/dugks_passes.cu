@@ -1,161 +1,159 @@
-// The two tile passes of the DUGKS step (sm_100a).
+// The kernels of one DUGKS step over (DV, cell) and (DV, face) arrays (sm_100a).
 //
-// Discrete velocities are walked in batches of NB consecutive DVs of one DV
-// row (the n1d DVs along x at fixed y and z).  Within a batch xi = (x_j, Y, Z)
-// varies in x only, so xi.S, the Shakhov exponent and the raw moments split
-// into a part computed once per batch (Y, Z) and a short per-DV part in x.
+// Every array of the step is DV-major, [dv][cell] or [dv][face], so that a
+// warp of consecutive cells or faces reads and writes contiguously; a thread
+// keeps one cell's or face's geometry and coefficients in registers and walks
+// DVs.  DVs are walked in segments (DevMesh::n_seg): up to 32 consecutive DVs
+// of one row of the tensor product (the n1d DVs along x at fixed y and z), or
+// of the DV list.  Within a row xi = (x_j, Y, Z) varies in x only, so xi.S, the
+// Shakhov exponent and the raw moments split into a part computed once per
+// segment (Y, Z) and a short per-DV part in x.
 //
-// Pass A: one CTA of 512 threads per (tile, DV chunk).  A tile is up to 128
-// L0 cells, their L1 ring (up to 256 local cells in all) and its items = the
-// faces touching L0 (up to 512, one per thread), sorted by kind.  Per batch:
-//   stage 0  cp.async of the NEXT batch's g~, h~ (and, for DV sets of more
-//            than 2 NB nodes per dimension, x Maxwellian factors) of the
-//            local cells into shared memory, overlapping this batch's stages
-//   stage 1  gbar+/hbar+ of the local cells (updateGHbarPvol,
-//            fvDVM.C:648-683); the y and z Maxwellian factors of the row are
-//            computed here from the cell record: two exponentials per cell
-//            cost less than gathering them for the ring cells
-//   stage 2  least-squares gradients of the L0 cells (leastSquaresGrad;
-//            the zero-gradient boundary terms vanish, fvDVM.C:456-485,
-//            :775-809)
-//   stage 3  per item: upwind reconstruction at the half step
-//            (updateGHbarSurf, fvDVM.C:755-1029); raw face moments in
-//            registers (updateMacroSurf, :1181-1297) and the wall out-flux;
-//            the reconstructed value goes to the face-value buffer
-// Pass B: one CTA per (tile, DV chunk), L0 cells and items only.  Per batch:
-//   stage 3  per item: relaxation of the stored face value (updateGHsurf,
-//            :1362-1457), incoming boundary DFs, flux xi.S g_f to shared memory
-//   stage 4  per L0 cell: gbar+ of the cell, flux gather and g~/h~ update
-//            (updateGHtildeVol, :1462-1519), raw cell moments (updateMacroVol,
-//            :1528-1554)
+//   k_half_step     cells  gbar+ = relaxed g~ (updateGHbarPvol, fvDVM.C:648-683)
+//   k_face_values   cells  least-squares gradient of gbar+ and, for every face the
+//                          cell is the upwind side of, the reconstruction at the
+//                          half step (fvDVM.C:456-485, :755-1029)
+//   k_face_moments  faces  raw face moments (updateMacroSurf, :1181-1297) and the
+//                          wall out-flux; incoming boundary DFs; then face macros
+//   k_face_flux     faces  relaxation of the face value (updateGHsurf, :1362-1457),
+//                          flux xi.S g_f in place
+//   k_update        cells  flux gather and g~ update (updateGHtildeVol, :1462-1519),
+//                          raw cell moments (updateMacroVol, :1528-1554), then the
+//                          cell macros
+//
+// Why five streaming kernels: the step moves per (cell, DV) and field 2 reals
+// (half step), 1 + D (face values written), D (moments), 2 D (flux) and D + 2
+// (update), 2.5 times what tiles in shared memory would, but each kernel is a
+// plain stream at high occupancy.  The tiled form (two passes of 512-thread CTAs,
+// 16 warps per SM, two or three CTA barriers per 8 to 16 DVs) issued on 30 % of
+// the cycles and recomputed gbar+ of each tile's ring.
+#include <algorithm>
+#include <type_traits>
+
 #include "dugks_device.cuh"
 
 namespace dugks {
 
 namespace {
 
-constexpr int kSL = kMaxLocal;           // row stride of local-cell arrays in shared memory
-constexpr int kS0 = kMaxTile;            // row stride of L0-cell arrays
-constexpr int kSI = kMaxItems + 1;       // row stride of item arrays (slot kSI - 1: zero flux)
-constexpr int kPartsL = kThreads / kSL;  // threads per local cell in stages 0-1
-constexpr int kParts0 = kThreads / kS0;  // threads per L0 cell in stages 2 and 4
-// Hex cells have at most 6 face neighbours: such stencils are kept in
-// shared memory for the whole CTA (larger ones are read from global memory)
-constexpr int kMaxRegStencil = 6;
-
-// batch widths: pass A (narrow, wide), pass B (narrow, wide)
-template <typename Real>
-struct Width;
-template <>
-struct Width<double> {
-    static constexpr int A0 = 8, A1 = 8, B0 = 8, B1 = 8;
-};
-template <>
-struct Width<float> {
-    static constexpr int A0 = 8, A1 = 8, B0 = 8, B1 = 8;
-};
+constexpr int kLanes = 32;      // entities per CTA of the reducing kernels
+constexpr int kParts = 4;       // warps per CTA of the reducing kernels: segments interleaved
+constexpr int kStream = 128;    // threads per CTA of k_half_step and k_face_flux
+constexpr int kCells = 256;     // threads per CTA of k_face_values: its L1 holds the block's ring
+constexpr int kFast = 6;        // neighbours and faces of a cell kept in registers (a hexahedron)
 
 // FP32 storage holds deviations from the per-DV reference Maxwellian
-// (DevMesh::gref, href): g = stored + ref.  These add and remove the
-// reference; for FP64 storage they are the identity and read nothing.
-template <typename Real>
+// (DevMesh::gref, href): g = stored + ref.  DV lists store absolute values.
+template <typename Real, bool GEN>
 __device__ __forceinline__ double dv_ref(const double* ref, int d) {
-    if constexpr (sizeof(Real) == 4) return __ldg(ref + d);
+    if constexpr (sizeof(Real) == 4 && !GEN) return __ldg(ref + d);
     else return 0.0;
 }
-template <typename Real>
-__device__ __forceinline__ double plus_ref(double x, double r) {
-    if constexpr (sizeof(Real) == 4) return x + r;
-    else return x;
-}
-template <typename Real>
-__device__ __forceinline__ double minus_ref(double x, double r) {
-    if constexpr (sizeof(Real) == 4) return x - r;
-    else return x;
-}
 
 // ---------------------------------------------------------------------
-// asynchronous global -> shared copies (cp.async, L1-allocating)
+// segments
 // ---------------------------------------------------------------------
-template <typename Real>
-__device__ __forceinline__ void cp_async(Real* sdst, const Real* gsrc) {
-    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
-    if (sizeof(Real) == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// ---------------------------------------------------------------------
-// batches
-// ---------------------------------------------------------------------
-struct TileRange {
-    int b, n0, loff, nloc, ioff, nit, r0, r1;
+struct Seg {
+    int ix0, len, d0, iy, iz;   // first x index, DVs, first local DV, row indices
 };
 
-__device__ __forceinline__ TileRange tile_range(const DevMesh& m, const int32_t* chunk_begin) {
-    TileRange t;
-    const int tile = blockIdx.x, chunk = blockIdx.y;
-    t.b = __ldg(m.tile_begin + tile);
-    t.n0 = __ldg(m.tile_begin + tile + 1) - t.b;
-    t.loff = __ldg(m.tile_loc_off + tile);
-    t.nloc = __ldg(m.tile_loc_off + tile + 1) - t.loff;
-    t.ioff = __ldg(m.tile_item_off + tile);
-    t.nit = __ldg(m.tile_item_off + tile + 1) - t.ioff;
-    t.r0 = __ldg(chunk_begin + chunk);
-    t.r1 = __ldg(chunk_begin + chunk + 1);
-    return t;
+// (d0, len and ix0 by arithmetic on the segment's number, which is uniform
+// over the warp: the row addresses they lead to stay in uniform registers)
+template <bool GEN>
+__device__ __forceinline__ Seg seg_at(const DevMesh& m, int s) {
+    Seg q;
+    if constexpr (GEN) {
+        q.ix0 = q.iy = q.iz = 0;
+        q.d0 = s * kSeg;
+        q.len = min(kSeg, m.nv_loc - q.d0);
+    } else {
+        const int two = m.n1d > kSeg, row = s >> two, k = s & two;   // n1d <= 64: one or two segments a row
+        q.ix0 = k * kSeg;
+        q.d0 = row * m.n1d + q.ix0;
+        q.len = min(kSeg, m.n1d - q.ix0);
+        const int2 t = __ldg(m.row_yz + row);
+        q.iy = t.x;
+        q.iz = t.y;
+    }
+    return q;
 }
 
-// position of batch k of a chunk: first x index, width, first DV of this
-// device's DV block (the state and face-value row), row indices
-struct BatchPos {
-    int ix0, nb, d0, iy, iz;
-};
+// p + off bytes: with p uniform over the warp the offset is part of the load
+template <typename T>
+__device__ __forceinline__ T* at(T* p, unsigned off) {
+    return reinterpret_cast<T*>(reinterpret_cast<char*>(const_cast<std::remove_const_t<T>*>(p)) + off);
+}
 
-// walks the batches of a chunk of DV rows in order (x batches of a row,
-// then the next row) without integer divisions per batch
-template <int D, int NB>
-struct BatchWalk {
-    int row, iy, iz, kb, nbr, n1d, rb;
-    // r0: first global row of the chunk; base: first global row this device holds
-    __device__ __forceinline__ BatchWalk(int r0, int n, int base)
-        : row(r0), kb(0), nbr((n + NB - 1) / NB), n1d(n), rb(base) {
-        iy = D == 3 ? r0 % n : r0;
-        iz = D == 3 ? r0 / n : 0;
-    }
-    __device__ __forceinline__ BatchPos pos() const {
-        BatchPos p;
-        p.ix0 = kb * NB;
-        p.nb = min(NB, n1d - p.ix0);
-        p.d0 = (row - rb) * n1d + p.ix0;
-        p.iy = iy;
-        p.iz = iz;
-        return p;
-    }
-    __device__ __forceinline__ void next() {
-        if (++kb == nbr) {
-            kb = 0;
-            ++row;
-            if (++iy == n1d && D == 3) {
-                iy = 0;
-                ++iz;
-            }
+// row j of an array of rows of n bytes each
+template <typename T>
+__device__ __forceinline__ T* row_of(T* p, int j, unsigned n) {
+    return at(p, static_cast<unsigned>(j) * n);
+}
+
+// this thread's warp in its CTA, known to be uniform
+__device__ __forceinline__ int warp_id() { return __shfl_sync(0xffffffffu, threadIdx.x / kLanes, 0); }
+
+// calls f(j, U) for groups of U consecutive DVs of a segment, then narrower
+// groups for the rest: the loads of a group are issued together
+template <int U, class F>
+__device__ __forceinline__ void groups(int len, F&& f) {
+    int j = 0;
+    for (; j + U <= len; j += U) f(j, std::integral_constant<int, U>{});
+    if constexpr (U >= 8) {
+        if (j + 4 <= len) {
+            f(j, std::integral_constant<int, 4>{});
+            j += 4;
         }
     }
-};
+    if constexpr (U >= 4) {
+        if (j + 2 <= len) {
+            f(j, std::integral_constant<int, 2>{});
+            j += 2;
+        }
+    }
+    if (U > 1 && j < len) f(j, std::integral_constant<int, 1>{});
+}
 
-// per-batch DV constants: the y, z velocity and weight of the row and the
+// one-dimensional nodes and weights of the DV set in shared memory
+__device__ __forceinline__ void load_nodes(const DevMesh& m, double* x1, double* w1) {
+    for (int i = threadIdx.x; i < m.n1d; i += blockDim.x) {
+        x1[i] = __ldg(m.X1 + i);
+        w1[i] = __ldg(m.W1 + i);
+    }
+    __syncthreads();
+}
+
+// velocity and weight of DV j of a segment
+struct Dv {
+    double x, y, z, w;
+};
+template <int D, bool GEN>
+__device__ __forceinline__ Dv dv_at(const DevMesh& m, const Seg& q, const double* x1, int j) {
+    Dv v;
+    if constexpr (GEN) {
+        const int d = m.dv_base + q.d0 + j;
+        v.x = __ldg(m.xi + 3 * d);
+        v.y = __ldg(m.xi + 3 * d + 1);
+        v.z = D == 3 ? __ldg(m.xi + 3 * d + 2) : 0.0;
+        v.w = __ldg(m.w + d);
+    } else {
+        v.x = x1[q.ix0 + j];
+        v.y = x1[q.iy];
+        v.z = D == 3 ? x1[q.iz] : 0.0;
+        v.w = 0.0;
+    }
+    return v;
+}
+
+// per-segment DV constants of a row: its y, z velocity and weight and the
 // products the moment fold needs.  The DV weight is w1[iz] w1[iy] w1[ix]
 // (3-D) or w1[iy] w1[ix] (2-D), as the tensor product is formed.
 struct RowConst {
-    double Y, Z, wyz, R2, cY, cZ, cYY, cYZ, cZZ;
+    double Y, Z, R2, wyz, cY, cZ, cYY, cYZ, cZZ;
 };
 
 template <int D>
-__device__ __forceinline__ RowConst row_const(const double* x1, const double* w1, const BatchPos& p) {
+__device__ __forceinline__ RowConst row_const(const double* x1, const double* w1, const Seg& p) {
     RowConst q;
     q.Y = x1[p.iy];
     q.Z = D == 3 ? x1[p.iz] : 0.0;
@@ -169,18 +167,16 @@ __device__ __forceinline__ RowConst row_const(const double* x1, const double* w1
     return q;
 }
 
-// Raw moments of one batch, summed along x (a = w_x g, b = w_x h):
+// Raw moments of one segment, summed along x (a = w_x g, b = w_x h):
 // S_k = sum a x^k (k = 0..3), B_k = sum b x^k (k = 0, 1), O = sum a xi.S
 // over outgoing wall DVs.  row_fold turns them into the moment record
 // (layout in dugks_internal.h) with |xi|^2 = x^2 + Y^2 + Z^2.
 struct RowSums {
-    double S0, S1, S2, S3, B0, B1, O;
+    double S0 = 0, S1 = 0, S2 = 0, S3 = 0, B0 = 0, B1 = 0, O = 0;
 };
 
-__device__ __forceinline__ void row_zero(RowSums& r) { r.S0 = r.S1 = r.S2 = r.S3 = r.B0 = r.B1 = r.O = 0.0; }
-
 // HZ: h is identically zero (D = 3, KInner = 0); its sums stay zero
-template <bool HZ = false>
+template <bool HZ>
 __device__ __forceinline__ double row_add(RowSums& r, double wx, double x, double g, double h) {
     const double a = wx * g;
     r.S0 += a;
@@ -197,8 +193,47 @@ __device__ __forceinline__ double row_add(RowSums& r, double wx, double x, doubl
     return a;
 }
 
-template <int D>
-__device__ __forceinline__ void row_fold(double* acc, const RowSums& r, const RowConst& q) {
+// A CTA of the reducing kernels holds 32 faces (or cells) and kParts warps
+// that share the segments of its DV chunk.  Their sums meet in shared memory
+// in a fixed order, the chunk's sums go to memory, and the CTA that finishes an
+// entity block last (a counter per block) adds the chunks in order and forms
+// the macros: no launch of its own, no wait.
+struct Finish {
+    double red[kParts][15][kLanes];
+    double tot[15][kLanes];
+    double mac[5][kLanes];   // U, 1/RT, A of the entity
+    int last;
+};
+
+// moment sums of one thread: its column of Finish::red (rows, updated once
+// per segment: 30 registers less in the DV loops), or registers (DV lists,
+// updated once per DV) that put() copies there
+struct SumsShared {
+    double* p;
+    __device__ __forceinline__ explicit SumsShared(Finish& f) : p(&f.red[threadIdx.x / kLanes][0][threadIdx.x % kLanes]) {
+#pragma unroll
+        for (int j = 0; j < 15; ++j) p[j * kLanes] = 0.0;
+    }
+    __device__ __forceinline__ double& operator[](int j) { return p[j * kLanes]; }
+    __device__ __forceinline__ void put(Finish&) {}
+};
+struct SumsRegs {
+    double v[15];
+    __device__ __forceinline__ explicit SumsRegs(Finish&) {
+#pragma unroll
+        for (int j = 0; j < 15; ++j) v[j] = 0.0;
+    }
+    __device__ __forceinline__ double& operator[](int j) { return v[j]; }
+    __device__ __forceinline__ void put(Finish& f) {
+#pragma unroll
+        for (int j = 0; j < 15; ++j) f.red[threadIdx.x / kLanes][j][threadIdx.x % kLanes] = v[j];
+    }
+};
+template <bool GEN>
+using Sums = std::conditional_t<GEN, SumsRegs, SumsShared>;
+
+template <int D, typename Acc>
+__device__ __forceinline__ void row_fold(Acc& acc, const RowSums& r, const RowConst& q) {
     const double c = q.wyz;
     const double Wb = r.S2 + fma(q.R2, r.S0, r.B0);   // sum a |xi|^2 + b
     const double Vx = r.S3 + fma(q.R2, r.S1, r.B1);   // sum (a |xi|^2 + b) x
@@ -221,1247 +256,1281 @@ __device__ __forceinline__ void row_fold(double* acc, const RowSums& r, const Ro
     acc[MOM_OUT] = fma(c, r.O, acc[MOM_OUT]);
 }
 
+// moments of one DV of a segment: along the row, or straight into acc (DV list)
+template <int D, bool HZ, bool GEN, typename Acc>
+__device__ __forceinline__ double add_dv(Acc& acc, RowSums& rs, const double* w1, const Seg& q, const Dv& v, int j,
+                                         double g, double h) {
+    if constexpr (GEN) {
+        const double xi[3] = {v.x, v.y, v.z};
+        accum<D>(acc.v, v.w, xi, v.x * v.x + v.y * v.y + v.z * v.z, g, h);
+        return v.w * g;
+    } else {
+        return row_add<HZ>(rs, w1[q.ix0 + j], v.x, g, h);
+    }
+}
+
 // xi.S rounded as the reference evaluates it, ((x Sx + y Sy) + z Sz) without
-// fused multiply-adds, with the y and z products of the row precomputed
-__device__ __forceinline__ double xs_row(double x, double Sx, double p2, double p3) {
-    return __dadd_rn(__dadd_rn(__dmul_rn(x, Sx), p2), p3);
+// fused multiply-adds
+__device__ __forceinline__ double xs_dv(const Dv& v, const double* S) {
+    return __dadd_rn(__dadd_rn(__dmul_rn(v.x, S[0]), __dmul_rn(v.y, S[1])), __dmul_rn(v.z, S[2]));
 }
 
 // ---------------------------------------------------------------------
-// Shakhov relaxation pair of one DV from the per-batch parts of a record
+// Shakhov relaxation of one entity over the DVs of a segment
 //   gbar = (1-r) g + r gS,  hbar = (1-r) h + r hS   (fvDVM.C:668-679, :1374-1391)
 //   gS = E (1 + s (cs - D - 2)),  hS = E RTh (K3D + s ((cs - D) K3D - 2 K))
 //   cs = |xi-U|^2 / RT = (x-Ux)^2 / RT + Cyz,  s = (xi-U).qv = (x-Ux) qx + Syz
-//   r E = (A e_x(x)) (r e_y(Y) e_z(Z))
+//   r E = (A e_x(x)) (r e_y(Y) e_z(Z)) from the entity's one-dimensional tables
 // ---------------------------------------------------------------------
-template <typename Real>
-struct Shk {
-    Real Ux, invRT, qx, RTh, omr;   // per entity
-    Real Cyz, Syz, eyzr;            // per entity and batch
-};
-
-template <int D, typename Real>
-__device__ __forceinline__ void shk_batch(Shk<Real>& s, Real Uy, Real Uz, Real qy, Real qz, Real r, double Y, double Z,
-                                          Real ey, Real ez) {
-    const Real cy = Real(Y) - Uy;
-    const Real cz = D == 3 ? Real(Z) - Uz : Real(0);
-    s.Cyz = (cy * cy + cz * cz) * s.invRT;
-    s.Syz = D == 3 ? cy * qy + cz * qz : cy * qy;
-    s.eyzr = D == 3 ? r * ey * ez : r * ey;
-}
-
-template <int D, typename Real>
-__device__ __forceinline__ void shk_relax(const Shk<Real>& s, Real x, Real ex, Real g, Real h, Real K3D, Real c0h,
-                                          Real& go, Real& ho) {
-    const Real cx = x - s.Ux;
-    const Real cs = fma(cx * cx, s.invRT, s.Cyz);
-    const Real sq = fma(cx, s.qx, s.Syz);
-    const Real Er = ex * s.eyzr;
-    const Real pg = fma(sq, cs - Real(D + 2), Real(1));
-    const Real ph = fma(sq, fma(cs, K3D, c0h), K3D);
-    go = fma(s.omr, g, Er * pg);
-    ho = fma(s.omr, h, (Er * s.RTh) * ph);
-}
-
-// ---------------------------------------------------------------------
-// Shared memory
-// ---------------------------------------------------------------------
-enum { CR_UX, CR_UY, CR_UZ, CR_INVRT, CR_QX, CR_QY, CR_QZ, CR_RTH, CR_OMR, CR_R, CR_N };
-
-template <int D, typename Real, int NB, bool HZ = false>
-struct SmemA {
-    // DF arrays per local cell: g~ and h~, or g~ alone when h is identically zero
-    static constexpr int NH = HZ ? 1 : 2;
-    // rows of stgx: [2][NB] staged per batch, or the resident table [n1d];
-    // the g-only 16-wide pass runs on DV sets of at most NB nodes per
-    // dimension and keeps the resident table only
-    static constexpr int XR = (HZ && NB >= 16) ? NB : 2 * NB;
-    double* x1;     // [kMaxN1d] 1-D nodes
-    double* w1;     // [kMaxN1d] 1-D weights
-    double* crec;   // [CR_N][kSL] records of the local cells
-    // e_x of the local cells: when the DV set has at most 2 NB nodes per
-    // dimension, the whole table [n1d][kSL] is loaded once per CTA (e_x does
-    // not depend on the row); otherwise [2][NB][kSL] staged per batch
-    double* stgx;
-    Real* stg;      // [2][NH][NB][kSL] staged g~ (and h~)
-    // FP32 storage: gbar+ is double-buffered by batch parity ([2][NB][kSL])
-    static constexpr int GB = sizeof(Real) == 4 ? 2 : 1;
-    Real* gB;       // [GB][NB][kSL] gbar+
-    Real* hB;       // (null when h is identically zero)
-    Real* Gg;       // [NB][D][kS0] gradients of the L0 cells
-    Real* Gh;       // (null when h is identically zero)
-    int* snb;       // [kMaxRegStencil][kS0] gradient stencils of the L0 cells: local neighbour
-    Real* sls;      // [kMaxRegStencil][D][kS0] and least-squares vector
-    static constexpr size_t bytes() {
-        return 2 * kMaxN1d * sizeof(double) + static_cast<size_t>(kMaxRegStencil) * kS0 * sizeof(int) +
-               (static_cast<size_t>(CR_N) * kSL + static_cast<size_t>(XR) * kSL) * sizeof(double) +
-               (2 * NH * static_cast<size_t>(NB) * kSL + GB * NH * NB * kSL + NH * NB * D * kS0 +
-                static_cast<size_t>(kMaxRegStencil) * D * kS0) *
-                   sizeof(Real);
-    }
-};
-
-template <int D, typename Real, int NB, bool HZ = false>
-__device__ __forceinline__ SmemA<D, Real, NB, HZ> carve_a(unsigned char* base) {
-    using S = SmemA<D, Real, NB, HZ>;
-    S s;
-    s.x1 = reinterpret_cast<double*>(base);
-    s.w1 = s.x1 + kMaxN1d;
-    s.crec = s.w1 + kMaxN1d;
-    s.stgx = s.crec + CR_N * kSL;
-    Real* p = reinterpret_cast<Real*>(s.stgx + S::XR * kSL);
-    s.stg = p;
-    p += 2 * S::NH * NB * kSL;
-    s.gB = p;
-    p += S::GB * NB * kSL;
-    s.hB = HZ ? nullptr : p;
-    if (!HZ) p += S::GB * NB * kSL;
-    s.Gg = p;
-    p += NB * D * kS0;
-    s.Gh = HZ ? nullptr : p;
-    if (!HZ) p += NB * D * kS0;
-    s.sls = p;
-    p += kMaxRegStencil * D * kS0;
-    s.snb = reinterpret_cast<int*>(p);
-    return s;
-}
-
-template <typename Real, int NB, bool HZ = false>
-struct SmemB {
-    // DF arrays per item: g and h, or g alone when h is identically zero
-    static constexpr int NH = HZ ? 1 : 2;
-    // rows of stx: e_x of the items does not depend on the row, so a DV set
-    // of at most XR nodes per dimension keeps the whole table [n1d][kSI],
-    // loaded once per CTA; larger sets stage [NB][kSI] per batch.  Where h is
-    // identically zero, 8-DV batches keep 16 rows in the shared memory h
-    // would take (16- and 20-wide batches hold a whole row already; for
-    // 10-DV batches on 20-node sets the resident table measured slower than
-    // staging)
-    static constexpr int XR = (HZ && 2 * NB <= 16) ? 2 * NB : NB;
-    double* x1;
-    double* w1;
-    double* frec;  // [CR_N][kSI] face records of the items
-    double* crec;  // [CR_N][kS0] records of the L0 cells
-    double* stx;   // [XR][kSI] e_x of the items: the resident table, or staged per batch
-    Real* st;      // [NH][NB][kSI] staged face values g (and h) of the items
-    Real* Fg;      // [NB][kSI] fluxes xi.S g_f of the items
-    Real* Fh;      // (null when h is identically zero)
-    double* red;   // end-of-CTA reduction of the split cell moments (aliases stx and st)
-    static constexpr size_t bytes() {
-        return 2 * kMaxN1d * sizeof(double) +
-               (static_cast<size_t>(CR_N) * (kSI + kS0) + static_cast<size_t>(XR) * kSI) * sizeof(double) +
-               2 * NH * static_cast<size_t>(NB) * kSI * sizeof(Real);
-    }
-};
-
-template <typename Real, int NB, bool HZ = false>
-__device__ __forceinline__ SmemB<Real, NB, HZ> carve_b(unsigned char* base) {
-    using S = SmemB<Real, NB, HZ>;
-    S s;
-    s.x1 = reinterpret_cast<double*>(base);
-    s.w1 = s.x1 + kMaxN1d;
-    s.frec = s.w1 + kMaxN1d;
-    s.crec = s.frec + CR_N * kSI;
-    s.stx = s.crec + CR_N * kS0;
-    s.st = reinterpret_cast<Real*>(s.stx + S::XR * kSI);
-    s.Fg = s.st + S::NH * NB * kSI;
-    s.Fh = HZ ? nullptr : s.Fg + NB * kSI;
-    s.red = s.stx;
-    return s;
-}
-
-// a coefficient record (structure of arrays over n entities) into shared
-// memory: U, 1/RT, qv, RTh, 1 - r, r
-template <typename Real>
-__device__ __forceinline__ void stash_rec(Real* dst, int stride, int l, const double* __restrict__ rec, size_t n, int e) {
-    dst[CR_UX * stride + l] = Real(__ldg(rec + REC_UX * n + e));
-    dst[CR_UY * stride + l] = Real(__ldg(rec + REC_UY * n + e));
-    dst[CR_UZ * stride + l] = Real(__ldg(rec + REC_UZ * n + e));
-    dst[CR_INVRT * stride + l] = Real(__ldg(rec + REC_INVRT * n + e));
-    dst[CR_QX * stride + l] = Real(__ldg(rec + REC_QX * n + e));
-    dst[CR_QY * stride + l] = Real(__ldg(rec + REC_QY * n + e));
-    dst[CR_QZ * stride + l] = Real(__ldg(rec + REC_QZ * n + e));
-    dst[CR_RTH * stride + l] = Real(__ldg(rec + REC_RTH * n + e));
-    const double r = __ldg(rec + REC_R * n + e);
-    dst[CR_OMR * stride + l] = Real(1.0 - r);
-    dst[CR_R * stride + l] = Real(r);
-}
-
-// the Shakhov parts of a stashed record for one batch
-template <int D, typename Real>
-__device__ __forceinline__ Shk<Real> shk_from(const Real* src, int stride, int l, const RowConst& q, Real ey, Real ez) {
-    Shk<Real> s;
-    s.Ux = src[CR_UX * stride + l];
-    s.invRT = src[CR_INVRT * stride + l];
-    s.qx = src[CR_QX * stride + l];
-    s.RTh = src[CR_RTH * stride + l];
-    s.omr = src[CR_OMR * stride + l];
-    shk_batch<D, Real>(s, src[CR_UY * stride + l], src[CR_UZ * stride + l], src[CR_QY * stride + l],
-                       src[CR_QZ * stride + l], src[CR_R * stride + l], q.Y, q.Z, ey, ez);
-    return s;
-}
-static_assert(static_cast<size_t>(kParts0 - 1) * kS0 * 15 * sizeof(double) <=
-                  static_cast<size_t>(Width<double>::B0) * kSI * (sizeof(double) + 2 * sizeof(double)),
-              "the cell-moment reduction must fit in the staging arrays");
-static_assert(static_cast<size_t>(kParts0 - 1) * kS0 * 15 * sizeof(double) <=
-                  static_cast<size_t>(Width<float>::B0) * kSI * (sizeof(double) + 2 * sizeof(float)),
-              "the cell-moment reduction must fit in the staging arrays");
-
-__device__ __forceinline__ void load_dv_tables(const DevMesh& m, double* x1, double* w1) {
-    if (threadIdx.x < m.n1d) {
-        x1[threadIdx.x] = __ldg(m.X1 + threadIdx.x);
-        w1[threadIdx.x] = __ldg(m.W1 + threadIdx.x);
-    }
-}
-
-// ---------------------------------------------------------------------
-// Items
-// ---------------------------------------------------------------------
-// Per-item registers.  la/da: the side reconstructed here (internal items:
-// the owner; tile-boundary items: the side in the tile; boundary items: the
-// owner), lb/db: the neighbour of internal items.
-struct Item {
-    int kind, ptype, la, lb, gi, face, other;
-    double S[3], da[3], db[3];
-};
-
-__device__ __forceinline__ Item load_item(const DevMesh& m, int gi) {
-    Item v;
-    const int meta = __ldg(m.it_meta + gi), loc = __ldg(m.it_loc + gi);
-    v.kind = meta & 15;
-    v.ptype = meta >> 4;
-    v.gi = gi;
-    v.face = __ldg(m.it_face + gi);
-    v.other = __ldg(m.it_other + gi);
-    const int lo = loc & 0xffff, ln = (loc >> 16) & 0xffff;
-    const size_t n = static_cast<size_t>(m.n_items);
-    double dO[3], dN[3];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        v.S[q] = __ldg(m.it_geo + q * n + gi);
-        dO[q] = __ldg(m.it_geo + (3 + q) * n + gi);
-        dN[q] = __ldg(m.it_geo + (6 + q) * n + gi);
-    }
-    const bool nei_here = v.kind == ITEM_TB_NEI;
-    v.la = nei_here ? ln : lo;
-    v.lb = ln;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        v.da[q] = nei_here ? dN[q] : dO[q];
-        v.db[q] = dN[q];
-    }
-    return v;
-}
-
-// reconstruction at the half step from local L0 cell l (fvDVM.C:832-836):
-// gbar+_l + grad_l . v,  v = Cf - C_l - xi dt/2
-template <int D, typename Real, int NB, bool HZ = false>
-__device__ __forceinline__ void recon(const SmemA<D, Real, NB, HZ>& sm, int j, int l, Real vx, Real vy, Real vz, Real& g,
-                                      Real& h) {
-    const Real* Gg = sm.Gg + j * D * kS0 + l;
-    Real gg = fma(Gg[0], vx, sm.gB[j * kSL + l]);
-    gg = fma(Gg[kS0], vy, gg);
-    if (D == 3) gg = fma(Gg[2 * kS0], vz, gg);
-    g = gg;
-    if constexpr (HZ) {
-        h = Real(0);
-    } else {
-        const Real* Gh = sm.Gh + j * D * kS0 + l;
-        Real hh = fma(Gh[0], vx, sm.hB[j * kSL + l]);
-        hh = fma(Gh[kS0], vy, hh);
-        if (D == 3) hh = fma(Gh[2 * kS0], vz, hh);
-        h = hh;
-    }
-}
-
-// ---------------------------------------------------------------------
-// Pass A stages
-// ---------------------------------------------------------------------
-// cp.async of batch bp's inputs of local cell l (thread part `part` of it)
-template <int D, typename Real, int NB, bool FULL, bool HZ>
-__device__ __forceinline__ void stage0(const DevMesh& m, const SmemA<D, Real, NB, HZ>& sm, int buf, const BatchPos& bp,
-                                       const Real* __restrict__ g, const Real* __restrict__ h,
-                                       const double* __restrict__ ctab, int l, int part, int c, bool active,
-                                       bool ex_res) {
-    if (active) {
-        constexpr int H = NB / kPartsL;
-        Real* sg = sm.stg + static_cast<size_t>(buf) * SmemA<D, Real, NB, HZ>::NH * NB * kSL;
-        double* sx = sm.stgx + static_cast<size_t>(buf) * NB * kSL;
-        const size_t nC = static_cast<size_t>(m.nC);
-#pragma unroll
-        for (int jj = 0; jj < H; ++jj) {
-            const int j = part * H + jj;
-            if (FULL || j < bp.nb) {
-                cp_async(sg + j * kSL + l, g + static_cast<size_t>(bp.d0 + j) * nC + c);
-                if (!HZ) cp_async(sg + (NB + j) * kSL + l, h + static_cast<size_t>(bp.d0 + j) * nC + c);
-                if (!ex_res) cp_async(sx + j * kSL + l, ctab + static_cast<size_t>(bp.ix0 + j) * nC + c);
-            }
-        }
-
-    }
-    cp_commit();
-}
-
-template <int D, typename Real, int NB, bool FULL, bool HZ>
-__device__ __forceinline__ void stage1(const SmemA<D, Real, NB, HZ>& sm, int buf, const BatchPos& bp, const RowConst& q,
-                                       int l, int part, bool active, double K3D, double c0h, bool ex_res,
-                                       const double* gref, const double* href, double& ey, double& ez) {
-    if (!active) return;
-    Shk<double> s;
-    s.Ux = sm.crec[CR_UX * kSL + l];
-    s.invRT = sm.crec[CR_INVRT * kSL + l];
-    s.qx = sm.crec[CR_QX * kSL + l];
-    s.RTh = sm.crec[CR_RTH * kSL + l];
-    s.omr = sm.crec[CR_OMR * kSL + l];
-    // the y and z Maxwellian factors of the batch's row, as the combine
-    // kernels tabulate them (write_maxwell_tables): exp(-x^2/2 invRT); the
-    // thread's cell is the same in every batch, so the g-only pass, which
-    // has the registers to spare, computes them on the row's first batch
-    // and keeps them for the others
-    const double uy = sm.crec[CR_UY * kSL + l], uz = sm.crec[CR_UZ * kSL + l];
-    if (!HZ || bp.ix0 == 0) {
-        const double yy = q.Y - uy, zz = q.Z - uz;
-        ey = exp(-0.5 * yy * yy * s.invRT);
-        ez = D == 3 ? exp(-0.5 * zz * zz * s.invRT) : 1.0;
-    }
-    shk_batch<D, double>(s, uy, uz, sm.crec[CR_QY * kSL + l], sm.crec[CR_QZ * kSL + l], sm.crec[CR_R * kSL + l], q.Y,
-                         q.Z, ey, ez);
-    const Real* sg = sm.stg + static_cast<size_t>(buf) * SmemA<D, Real, NB, HZ>::NH * NB * kSL;
-    const double* sx = sm.stgx + (ex_res ? bp.ix0 : buf * NB) * kSL;
-    constexpr int H = NB / kPartsL;
-#pragma unroll
-    for (int jj = 0; jj < H; ++jj) {
-        const int j = part * H + jj;
-        if (FULL || j < bp.nb) {
-            double go, ho;
-            const double gr = dv_ref<Real>(gref, bp.d0 + j), hr = dv_ref<Real>(href, bp.d0 + j);
-            const double hin = HZ ? 0.0 : plus_ref<Real>(double(sg[(NB + j) * kSL + l]), hr);
-            shk_relax<D, double>(s, sm.x1[bp.ix0 + j], sx[j * kSL + l], plus_ref<Real>(double(sg[j * kSL + l]), gr),
-                                 hin, K3D, c0h, go, ho);
-            sm.gB[j * kSL + l] = Real(minus_ref<Real>(go, gr));
-            if (!HZ) sm.hB[j * kSL + l] = Real(minus_ref<Real>(ho, hr));
+// What depends on the row only is formed per segment from the record in
+// memory (it stays in L1), so that a thread holds five numbers per entity.
+template <int D, bool HZ, bool GEN>
+struct Relax {
+    const double* rec;   // records and tables of all entities (stride n)
+    const double* tab;
+    unsigned n8, e8;     // bytes of a row of them; the entity's offset in one
+    double Ux, invRT, qx, RTh, r;
+    double Cyz, Syz, eyzr;                  // rows
+    double Uy, Uz, qy, qz, rA;              // DV lists
+    const double* ex;
+    __device__ __forceinline__ Relax(const double* rec_, const double* tab_, int n_, int e, double r_) {
+        rec = rec_;
+        tab = tab_;
+        n8 = 8u * n_;
+        e8 = 8u * e;
+        Ux = field(REC_UX);
+        invRT = field(REC_INVRT);
+        qx = field(REC_QX);
+        RTh = HZ ? 0.0 : field(REC_RTH);
+        r = r_;
+        if constexpr (GEN) {
+            Uy = field(REC_UY);
+            Uz = field(REC_UZ);
+            qy = field(REC_QY);
+            qz = field(REC_QZ);
+            rA = r * field(REC_A);
         }
     }
-}
-
-
-template <int D, typename Real, int NB, bool HZ>
-__device__ __forceinline__ void grad_one(const SmemA<D, Real, NB, HZ>& sm, int j, int l, const int* nbi,
-                                         const Real (*ls)[D], int nk) {
-    const Real* gB = sm.gB + j * kSL;
-    const Real* hB = HZ ? nullptr : sm.hB + j * kSL;
-    const Real g0 = gB[l], h0 = HZ ? Real(0) : hB[l];
-    Real gx[D], hx[D];
-#pragma unroll
-    for (int q = 0; q < D; ++q) gx[q] = hx[q] = Real(0);
-#pragma unroll
-    for (int k = 0; k < kMaxRegStencil; ++k) {
-        if (k < nk) {
-            const Real dg = gB[nbi[k]] - g0;
-#pragma unroll
-            for (int q = 0; q < D; ++q) gx[q] = fma(ls[k][q], dg, gx[q]);
-            if constexpr (!HZ) {
-                const Real dh = hB[nbi[k]] - h0;
-#pragma unroll
-                for (int q = 0; q < D; ++q) hx[q] = fma(ls[k][q], dh, hx[q]);
-            }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < D; ++q) {
-        sm.Gg[(j * D + q) * kS0 + l] = gx[q];
-        if (!HZ) sm.Gh[(j * D + q) * kS0 + l] = hx[q];
-    }
-}
-
-template <int D, typename Real, int NB, bool FULL, bool HZ>
-__device__ __forceinline__ void stage2(const DevMesh& m, const SmemA<D, Real, NB, HZ>& sm, const BatchPos& bp,
-                                       const TileRange& t, int* err) {
-    const int l = threadIdx.x % kS0, part = threadIdx.x / kS0;
-    if (l >= t.n0) return;
-    const int c = t.b + l;
-    constexpr int H = (NB + kParts0 - 1) / kParts0;
-    if (m.nb_max <= kMaxRegStencil) {
-        // stencil from shared memory (absent neighbours: the cell itself
-        // with a zero vector)
-        int nbi[kMaxRegStencil];
-        Real ls[kMaxRegStencil][D];
-#pragma unroll
-        for (int k = 0; k < kMaxRegStencil; ++k) {
-            nbi[k] = sm.snb[k * kS0 + l];
-#pragma unroll
-            for (int q = 0; q < D; ++q) ls[k][q] = sm.sls[(k * D + q) * kS0 + l];
-        }
-#pragma unroll
-        for (int jj = 0; jj < H; ++jj) {
-            const int j = part + kParts0 * jj;
-            if (FULL || j < bp.nb) grad_one<D, Real, NB, HZ>(sm, j, l, nbi, ls, kMaxRegStencil);
-        }
-    } else {
-#pragma unroll 1
-        for (int jj = 0; jj < H; ++jj) {
-            const int j = part + kParts0 * jj;
-            if (!FULL && j >= bp.nb) break;
-            const Real* gB = sm.gB + j * kSL;
-            const Real* hB = HZ ? nullptr : sm.hB + j * kSL;
-            const Real g0 = gB[l], h0 = HZ ? Real(0) : hB[l];
-            Real gx[D], hx[D];
-#pragma unroll
-            for (int q = 0; q < D; ++q) gx[q] = hx[q] = Real(0);
-            for (int k = 0; k < m.nb_max; ++k) {
-                const int n0 = __ldg(m.grad_nb + static_cast<size_t>(k) * m.nC + c);
-                if (n0 < 0) continue;
-                const int n = chk(n0, 0, t.nloc, err);
-                const Real dg = gB[n] - g0, dh = HZ ? Real(0) : hB[n] - h0;
-#pragma unroll
-                for (int q = 0; q < D; ++q) {
-                    const Real lsq = Real(__ldg(m.grad_ls + (static_cast<size_t>(k) * 3 + q) * m.nC + c));
-                    gx[q] = fma(lsq, dg, gx[q]);
-                    hx[q] = fma(lsq, dh, hx[q]);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < D; ++q) {
-                sm.Gg[(j * D + q) * kS0 + l] = gx[q];
-                if (!HZ) sm.Gh[(j * D + q) * kS0 + l] = hx[q];
-            }
-        }
-    }
-}
-
-// ---------------------------------------------------------------------
-// Pass A: face reconstruction, raw face moments, face values
-// ---------------------------------------------------------------------
-// HZ: h is identically zero (D = 3 and KInner = 0 make K + 3 - D = 0 in
-// every h formula, fvDVM.C:414-426, :673-679, :1079-1092): the pass reads,
-// reconstructs and writes g alone; its results are those of the full pass
-template <int D, typename Real, int NB, bool FULL, bool HZ>
-__global__ void __launch_bounds__(kThreads, 1) k_pass_a(const StepArgs a) {
-    const DevMesh& m = a.dm;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    SmemA<D, Real, NB, HZ> sm = carve_a<D, Real, NB, HZ>(smem_raw);
-    // FP32 storage: gbar+ double-buffered by batch parity, so stage 1 of a
-    // batch overwrites no buffer the previous batch's stage 3 still reads,
-    // and the loop needs no barrier before stage 1.  Used where it costs no
-    // register spills (2-D, and 3-D rows that do not split into whole
-    // batches); measured 1.96 -> 1.68 ms on a 256^2 x 28^2 cavity, while the
-    // spilling 3-D 16-wide variant lost 4 %
-    constexpr bool kDbl = SmemA<D, Real, NB, HZ>::GB == 2 && (D == 2 || !FULL);
-    const TileRange t = tile_range(m, a.chunk_begin);
-    const Real* g = reinterpret_cast<const Real*>(a.ds.g[a.ds.cur]);
-    const Real* h = reinterpret_cast<const Real*>(a.ds.h[a.ds.cur]);
-    const double* ctab = a.ds.ctab;
-    Real* const fvg = reinterpret_cast<Real*>(a.ds.fvg);
-    Real* const fvh = reinterpret_cast<Real*>(a.ds.fvh);
-    const double K3D = m.K + 3.0 - m.D, c0h = -(m.D * (m.K + 3.0 - m.D) + 2.0 * m.K);
-    const Real hdt = Real(0.5 * step_dt(a));
-    const size_t nI = static_cast<size_t>(m.n_items);
-
-    // CTA set-up: DV tables, records of the local cells, this thread's cell
-    // of stages 0-1 and its item
-    load_dv_tables(m, sm.x1, sm.w1);
-    const int l1 = threadIdx.x % kSL, p1 = threadIdx.x / kSL;
-    const bool act1 = l1 < t.nloc;
-    const int c1 = act1 ? chk(__ldg(m.loc_cells + t.loff + l1), 0, m.nC, a.ds.err) : 0;
-    if (act1 && p1 == 0) {
-        const double* cr = a.ds.cellrec;
-        const size_t n = static_cast<size_t>(m.nC);
-        sm.crec[CR_UX * kSL + l1] = __ldg(cr + REC_UX * n + c1);
-        sm.crec[CR_UY * kSL + l1] = __ldg(cr + REC_UY * n + c1);
-        sm.crec[CR_UZ * kSL + l1] = __ldg(cr + REC_UZ * n + c1);
-        sm.crec[CR_INVRT * kSL + l1] = __ldg(cr + REC_INVRT * n + c1);
-        sm.crec[CR_QX * kSL + l1] = __ldg(cr + REC_QX * n + c1);
-        sm.crec[CR_QY * kSL + l1] = __ldg(cr + REC_QY * n + c1);
-        sm.crec[CR_QZ * kSL + l1] = __ldg(cr + REC_QZ * n + c1);
-        sm.crec[CR_RTH * kSL + l1] = __ldg(cr + REC_RTH * n + c1);
-        const double r = __ldg(cr + REC_R * n + c1);
-        sm.crec[CR_OMR * kSL + l1] = 1.0 - r;
-        sm.crec[CR_R * kSL + l1] = r;
-    }
-    const bool ex_res = m.n1d <= 2 * NB;
-    if (ex_res && act1)
-        for (int ix = p1; ix < m.n1d; ix += kPartsL)
-            sm.stgx[ix * kSL + l1] = __ldg(ctab + static_cast<size_t>(ix) * m.nC + c1);
-    // gradient stencils of the L0 cells (slot-major tables, -1: none)
-    if (threadIdx.x < kS0 && m.nb_max <= kMaxRegStencil) {
-        const int l = threadIdx.x;
-        const int c = t.b + l;
-#pragma unroll
-        for (int k = 0; k < kMaxRegStencil; ++k) {
-            const int n = (l < t.n0 && k < m.nb_max) ? __ldg(m.grad_nb + static_cast<size_t>(k) * m.nC + c) : -1;
-            sm.snb[k * kS0 + l] = n >= 0 ? chk(n, 0, t.nloc, a.ds.err) : l;
-#pragma unroll
-            for (int q = 0; q < D; ++q)
-                sm.sls[(k * D + q) * kS0 + l] =
-                    n >= 0 ? Real(__ldg(m.grad_ls + (static_cast<size_t>(k) * 3 + q) * m.nC + c)) : Real(0);
-        }
-    }
-    const int it = threadIdx.x;
-    const bool has_item = it < t.nit;
-    Item v{};
-    if (has_item) {
-        v = load_item(m, t.ioff + it);
-        v.la = chk(v.la, 0, t.nloc, a.ds.err);
-        if (v.kind != ITEM_MESH_BOUNDARY) v.lb = chk(v.lb, 0, t.nloc, a.ds.err);
-        else v.face = chk(v.face, 0, m.nBF, a.ds.err);
-        if (v.kind == ITEM_TB_OWN || v.kind == ITEM_TB_NEI) v.other = chk(v.other, 0, m.n_items, a.ds.err);
-    }
-    double acc[15];
-#pragma unroll
-    for (int j = 0; j < 15; ++j) acc[j] = 0.0;
-
-    BatchWalk<D, NB> walk(t.r0, m.n1d, m.row_base), ahead(t.r0, m.n1d, m.row_base);
-    const int nbt = (t.r1 - t.r0) * walk.nbr;
-    double ey1 = 1.0, ez1 = 1.0;   // y, z Maxwellian factors of this thread's local cell and row
-    if (nbt > 0) stage0<D, Real, NB, FULL, HZ>(m, sm, 0, ahead.pos(), g, h, ctab, l1, p1, c1, act1, ex_res);
-    if constexpr (kDbl) __syncthreads();  // the CTA set-up above is visible to every thread
-    for (int k = 0; k < nbt; ++k, walk.next()) {
-        const int buf = k & 1;
-        const BatchPos bp = walk.pos();
-        // this thread's staged entries of batch k (stage 1 reads only what the
-        // same thread staged)
-        cp_wait_all();
-        if constexpr (kDbl) {
-            const SmemA<D, Real, NB, HZ> s0 = carve_a<D, Real, NB, HZ>(smem_raw);
-            sm.gB = s0.gB + buf * NB * kSL;
-            if (!HZ) sm.hB = s0.hB + buf * NB * kSL;
-        } else {
-            __syncthreads();  // the previous batch's stage 3 is done with gbar+ (and the set-up is visible)
-        }
-        if (k + 1 < nbt) {
-            ahead.next();
-            stage0<D, Real, NB, FULL, HZ>(m, sm, buf ^ 1, ahead.pos(), g, h, ctab, l1, p1, c1, act1, ex_res);
-        }
-        const RowConst q = row_const<D>(sm.x1, sm.w1, bp);
-        stage1<D, Real, NB, FULL, HZ>(sm, buf, bp, q, l1, p1, act1, K3D, c0h, ex_res, m.gref, m.href, ey1, ez1);
-        __syncthreads();
-        stage2<D, Real, NB, FULL, HZ>(m, sm, bp, t, a.ds.err);
-        __syncthreads();
-        if (!has_item) continue;
-        // stage 3
-        const double p2 = __dmul_rn(q.Y, v.S[1]);
-        const double p3 = D == 3 ? __dmul_rn(q.Z, v.S[2]) : 0.0;
-        const Real ay = Real(v.da[1]) - hdt * Real(q.Y), az = Real(v.da[2]) - hdt * Real(q.Z);
-        RowSums rs;
-        row_zero(rs);
-        Real* fg = fvg + static_cast<size_t>(bp.d0) * nI + v.gi;
-        Real* fh = fvh + static_cast<size_t>(bp.d0) * nI + v.gi;
-        if (v.kind == ITEM_TILE_INTERNAL) {
-            const Real by = Real(v.db[1]) - hdt * Real(q.Y), bz = Real(v.db[2]) - hdt * Real(q.Z);
-#pragma unroll
-            for (int j = 0; j < NB; ++j) {
-                if (FULL || j < bp.nb) {
-                    const double x = sm.x1[bp.ix0 + j];
-                    const double xs = xs_row(x, v.S[0], p2, p3);
-                    const bool own_up = xs >= kVSmall, nei_up = xs < -kVSmall;
-                    const Real hx = hdt * Real(x);
-                    Real gg, hh;
-                    if (own_up || nei_up) {
-                        recon<D, Real, NB, HZ>(sm, j, own_up ? v.la : v.lb, Real(own_up ? v.da[0] : v.db[0]) - hx,
-                                               own_up ? ay : by, own_up ? az : bz, gg, hh);
-                    } else {
-                        // exactly tangential: both sides averaged (fvDVM.C:847-863)
-                        Real g1, h1, g2, h2;
-                        recon<D, Real, NB, HZ>(sm, j, v.la, Real(v.da[0]) - hx, ay, az, g1, h1);
-                        recon<D, Real, NB, HZ>(sm, j, v.lb, Real(v.db[0]) - hx, by, bz, g2, h2);
-                        gg = Real(0.5) * (g2 + g1);
-                        hh = Real(0.5) * (h2 + h1);
-                    }
-                    // FP32 storage: the deviations only; the reference part is added once below
-                    row_add<HZ>(rs, sm.w1[bp.ix0 + j], x, double(gg), double(hh));
-                    fg[j * nI] = gg;
-                    if (!HZ) fh[j * nI] = hh;
-                }
-            }
-        } else if (v.kind != ITEM_MESH_BOUNDARY) {
-            // tile-boundary face: this tile's side only, weighted 1 upwind,
-            // 1/2 tangential, 0 downwind; the other tile adds its side.  The
-            // upwind tile writes the face value into both items' slots, so
-            // that each tile's pass B reads its own slot, coalesced (reading
-            // the other tile's slot instead cost pass B more than the
-            // second store costs here); tangential halves stay in their own
-            // slots
-            const bool own_side = v.kind == ITEM_TB_OWN;
-            Real* og = fvg + static_cast<size_t>(bp.d0) * nI + v.other;
-            Real* oh = fvh + static_cast<size_t>(bp.d0) * nI + v.other;
-#pragma unroll
-            for (int j = 0; j < NB; ++j) {
-                if (FULL || j < bp.nb) {
-                    const double x = sm.x1[bp.ix0 + j];
-                    const double xs = xs_row(x, v.S[0], p2, p3);
-                    const bool own_up = xs >= kVSmall, nei_up = xs < -kVSmall;
-                    const bool up = own_side ? own_up : nei_up;
-                    const bool tang = !own_up && !nei_up;
-                    // the downwind side contributes nothing; neighbouring
-                    // tile-boundary faces share their orientation, so whole
-                    // warps skip together
-                    if (up || tang) {
-                        const Real cs = up ? Real(1) : Real(0.5);
-                        Real gg, hh;
-                        recon<D, Real, NB, HZ>(sm, j, v.la, Real(v.da[0]) - hdt * Real(x), ay, az, gg, hh);
-                        gg *= cs;
-                        hh *= cs;
-                        // this side's share of the face value and of its reference part
-                        const double gr = double(cs) * dv_ref<Real>(m.gref, bp.d0 + j);
-                        const double hr = double(cs) * dv_ref<Real>(m.href, bp.d0 + j);
-                        row_add<HZ>(rs, sm.w1[bp.ix0 + j], x, plus_ref<Real>(double(gg), gr), plus_ref<Real>(double(hh), hr));
-                        fg[j * nI] = gg;
-                        if (!HZ) fh[j * nI] = hh;
-                        if (up) {
-                            og[j * nI] = gg;
-                            if (!HZ) oh[j * nI] = hh;
-                        }
-                    }
-                }
-            }
-        } else {
-            // mesh boundary, by patch type (fvDVM.C:866-1027)
-            const int pt = v.ptype;
-            const bool wall = pt == DUGKS_PATCH_MAXWELL_WALL;
-            const bool zero_grad = pt == DUGKS_PATCH_ZERO_GRADIENT;
-            const bool sym = pt == DUGKS_PATCH_SYMMETRY || pt == DUGKS_PATCH_DVM_SYMMETRY;
-            // incoming DFs computed here: far field and pressure patches
-            // rho_b M(xi; U_owner, T_b) (fvDVM.C:926-938); mixed patches the
-            // Maxwellian of the patch rho, U, T kept from the start
-            // (discreteVelocity.C:226-258)
-            const bool eq_in = !wall && !zero_grad && !sym;
-            double bK = 0, bInv = 0, bHf = 0, bU[3] = {0, 0, 0};
-            if (eq_in) {
-                const BRec* br = a.ds.brec + v.face;
-                bK = __ldg(&br->rho_in) * __ldg(&br->K_in);
-                bInv = __ldg(&br->invRT_in);
-                bHf = __ldg(&br->hfac);
-                if (pt == DUGKS_PATCH_MIXED) {
-                    for (int i = 0; i < 3; ++i) bU[i] = __ldg(&br->U[i]);
-                } else {
-                    const int own = chk(__ldg(m.bface_owner + v.face), 0, m.nC, a.ds.err);
-                    const size_t n = static_cast<size_t>(m.nC);
-                    for (int i = 0; i < 3; ++i) bU[i] = __ldg(a.ds.cellrec + (REC_UX + i) * n + own);
-                }
-            }
-            const double cyz = (q.Y - bU[1]) * (q.Y - bU[1]) + (q.Z - bU[2]) * (q.Z - bU[2]);
-            if (zero_grad || sym) {
-                // (a loop of its own: the rare types stay off the common path)
-#pragma unroll 1
-                for (int j = 0; j < NB; ++j) {
-                    if (FULL || j < bp.nb) {
-                        const double x = sm.x1[bp.ix0 + j];
-                        const double xs = xs_row(x, v.S[0], p2, p3);
-                        const double wx = sm.w1[bp.ix0 + j];
-                        Real gg, hh;
-                        if (zero_grad) {
-                            // every DV: the owner cell's gbar+ (fvDVM.C:887-891)
-                            gg = sm.gB[j * kSL + v.la];
-                            hh = HZ ? Real(0) : sm.hB[j * kSL + v.la];
-                        } else if (xs > -kVSmall) {
-                            // outgoing and tangential: upwind from the owner
-                            // (fvDVM.C:1013-1023); incoming ones are the mirror
-                            // DVs' values, added by the symmetry pass after this one
-                            recon<D, Real, NB, HZ>(sm, j, v.la, Real(v.da[0]) - hdt * Real(x), ay, az, gg, hh);
-                        } else {
-                            continue;
-                        }
-                        const double gr = dv_ref<Real>(m.gref, bp.d0 + j), hr = dv_ref<Real>(m.href, bp.d0 + j);
-                        row_add<HZ>(rs, wx, x, plus_ref<Real>(double(gg), gr), plus_ref<Real>(double(hh), hr));
-                        fg[j * nI] = gg;
-                        if (!HZ) fh[j * nI] = hh;
-                    }
-                }
-            } else
-#pragma unroll
-            for (int j = 0; j < NB; ++j) {
-                if (FULL || j < bp.nb) {
-                    const double x = sm.x1[bp.ix0 + j];
-                    const double xs = xs_row(x, v.S[0], p2, p3);
-                    const double wx = sm.w1[bp.ix0 + j];
-                    const double gr = dv_ref<Real>(m.gref, bp.d0 + j), hr = dv_ref<Real>(m.href, bp.d0 + j);
-                    if (xs > 0) {
-                        // outgoing: upwind from the owner (fvDVM.C:916-923, :950-961)
-                        Real gg, hh;
-                        recon<D, Real, NB, HZ>(sm, j, v.la, Real(v.da[0]) - hdt * Real(x), ay, az, gg, hh);
-                        const double aw =
-                            row_add<HZ>(rs, wx, x, plus_ref<Real>(double(gg), gr), plus_ref<Real>(double(hh), hr));
-                        if (wall) rs.O = fma(aw, xs, rs.O);
-                        fg[j * nI] = gg;
-                        if (!HZ) fh[j * nI] = hh;
-                    } else if (eq_in) {
-                        const double cx = x - bU[0];
-                        const double ge = bK * exp(-0.5 * (cx * cx + cyz) * bInv);
-                        // rounded as pass B rounds the same incoming DF
-                        row_add<HZ>(rs, wx, x, plus_ref<Real>(double(Real(minus_ref<Real>(ge, gr))), gr),
-                                plus_ref<Real>(double(Real(minus_ref<Real>(ge * bHf, hr))), hr));
-                    }
-                    // incoming wall DFs enter through rho_w in the face combine
-                }
-            }
-        }
-        row_fold<D>(acc, rs, q);
-    }
-    if (has_item) {
-        if constexpr (sizeof(Real) == 4) {
-            // a tile-internal face counts every DV of the chunk in full: its
-            // moments gain the reference's chunk moments once
-            if (v.kind == ITEM_TILE_INTERNAL) {
-                const double* rm = a.ds.refmom + static_cast<size_t>(blockIdx.y) * kNM;
-#pragma unroll
-                for (int j = 0; j < 14; ++j) acc[j] += __ldg(rm + j);
-            }
-        }
-        double* p = a.ds.partF + (static_cast<size_t>(blockIdx.y) * m.n_items + v.gi) * kNM;
-#pragma unroll
-        for (int j = 0; j < 15; ++j) p[j] = acc[j];
-    }
-}
-
-// ---------------------------------------------------------------------
-// Pass B: face relaxation, volume update, raw cell moments
-// ---------------------------------------------------------------------
-// faces of a cell whose flux list stays in registers (hex cells have 6)
-constexpr int kRegFaces = 6;
-
-// v with its sign flipped when neg is 1
-__device__ __forceinline__ double flip_sign(double v, unsigned neg) {
-    return __hiloint2double(__double2hiint(v) ^ static_cast<int>(neg << 31), __double2loint(v));
-}
-__device__ __forceinline__ float flip_sign(float v, unsigned neg) {
-    return __int_as_float(__float_as_int(v) ^ static_cast<int>(neg << 31));
-}
-
-// cp.async of an item's own face-value slot and Maxwellian x factors for a
-// batch (each thread stages and later reads only its own item's entries)
-template <typename Real, int NB, bool FULL, bool HZ>
-__device__ __forceinline__ void stage_items(const SmemB<Real, NB, HZ>& sm, const BatchPos& bp, const Real* __restrict__ fvg,
-                                            const Real* __restrict__ fvh, const double* __restrict__ ftab, size_t nI,
-                                            int it, int gi, bool x_res) {
-    const size_t base = static_cast<size_t>(bp.d0) * nI + gi;
-    const size_t tb = static_cast<size_t>(bp.ix0) * nI + gi;
-#pragma unroll
-    for (int j = 0; j < NB; ++j) {
-        if (FULL || j < bp.nb) {
-            cp_async(sm.st + j * kSI + it, fvg + base + j * nI);
-            if (!HZ) cp_async(sm.st + (NB + j) * kSI + it, fvh + base + j * nI);
-            if (!x_res) cp_async(sm.stx + j * kSI + it, ftab + tb + j * nI);
-        }
-    }
-    cp_commit();
-}
-
-// the L0 cell's g~, h~ and Maxwellian x factors of its DVs of a batch, into
-// registers one batch ahead
-template <typename Real, int NB, bool FULL, bool HZ>
-__device__ __forceinline__ void fetch_cells(const BatchPos& bp, const Real* __restrict__ g, const Real* __restrict__ h,
-                                            const double* __restrict__ ctab, size_t nC, int c, int part, Real* pg,
-                                            Real* ph, double* pe) {
-    constexpr int H = (NB + kParts0 - 1) / kParts0;
-#pragma unroll
-    for (int jj = 0; jj < H; ++jj) {
-        const int j = part + kParts0 * jj;
-        if (FULL || j < bp.nb) {
-            const size_t idx = static_cast<size_t>(bp.d0 + j) * nC + c;
-            pg[jj] = __ldg(g + idx);
-            ph[jj] = HZ ? Real(0) : __ldg(h + idx);
-            pe[jj] = __ldg(ctab + static_cast<size_t>(bp.ix0 + j) * nC + c);
-        }
-    }
-}
-
-// HZ: as for pass A, g alone (h stays identically zero)
-template <int D, typename Real, int NB, bool FULL, bool HZ>
-__global__ void __launch_bounds__(kThreads, 1) k_pass_b(const StepArgs a) {
-    const DevMesh& m = a.dm;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const SmemB<Real, NB, HZ> sm = carve_b<Real, NB, HZ>(smem_raw);
-    const TileRange t = tile_range(m, a.chunk_begin);
-    const Real* g = reinterpret_cast<const Real*>(a.ds.g[a.ds.cur]);
-    const Real* h = reinterpret_cast<const Real*>(a.ds.h[a.ds.cur]);
-    Real* gn = reinterpret_cast<Real*>(a.ds.g[1 - a.ds.cur]);
-    Real* hn = reinterpret_cast<Real*>(a.ds.h[1 - a.ds.cur]);
-    const Real* fvg = reinterpret_cast<const Real*>(a.ds.fvg);
-    const Real* fvh = reinterpret_cast<const Real*>(a.ds.fvh);
-    const double* ctab = a.ds.ctab;
-    const double* ftab = a.ds.ftab;
-    const double K3D = m.K + 3.0 - m.D, c0h = -(m.D * (m.K + 3.0 - m.D) + 2.0 * m.K);
-    const size_t nI = static_cast<size_t>(m.n_items), nC = static_cast<size_t>(m.nC);
-    load_dv_tables(m, sm.x1, sm.w1);
-
-    // item of stage 3; its face record (item order) goes to shared memory
-    const int it = threadIdx.x;
-    const bool has_item = it < t.nit;
-    const int gi = t.ioff + (has_item ? it : 0);
-    int kind = 0, other = 0;
-    double S[3] = {0, 0, 0};
-    if (has_item) {
-        kind = __ldg(m.it_meta + gi) & 15;
-        other = __ldg(m.it_other + gi);
-        if (kind == ITEM_TB_OWN || kind == ITEM_TB_NEI) other = chk(other, 0, m.n_items, a.ds.err);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) S[q] = __ldg(m.it_geo + q * nI + gi);
-        stash_rec(sm.frec, kSI, it, a.ds.facerec, nI, gi);
-    }
-    // e_x of this thread's item for every node, when the table fits (each
-    // thread reads back only its own item's column)
-    // (a variant whose table is only a batch wide stages: decided at compile time)
-    constexpr int kXR = SmemB<Real, NB, HZ>::XR;
-    const bool x_res = (kXR > NB || NB >= 16) && m.n1d <= kXR;
-    if (x_res && has_item)
-        for (int ix = 0; ix < m.n1d; ++ix) sm.stx[ix * kSI + it] = __ldg(ftab + static_cast<size_t>(ix) * nI + gi);
-    // L0 cell of stage 4 (kParts0 threads per cell, DVs interleaved)
-    const int lc = threadIdx.x % kS0, part = threadIdx.x / kS0;
-    const bool has_cell = lc < t.n0;
-    const int c = t.b + (has_cell ? lc : 0);
-    if (has_cell && part == 0) stash_rec(sm.crec, kS0, lc, a.ds.cellrec, nC, c);
-    const double dtV = has_cell ? step_dt(a) * __ldg(m.dtV + c) : 0.0;
-    // flux list of the cell: item slot and sign (owner side: outflow, negated
-    // by flipping the sign bit); absent entries read the zero slot kSI - 1,
-    // which no item uses
-    int ent_off[kRegFaces];
-    unsigned ent_neg[kRegFaces];
-#pragma unroll
-    for (int s = 0; s < kRegFaces; ++s) {
-        const int e = (has_cell && s < m.nf_max) ? __ldg(m.cf_item + static_cast<size_t>(s) * nC + c) : 0;
-        ent_off[s] = e == 0 ? kSI - 1 : chk((e > 0 ? e : -e) - 1, 0, t.nit, a.ds.err);
-        ent_neg[s] = e < 0 ? 1u : 0u;
-    }
-    if (threadIdx.x == kThreads - 1) {
-        for (int j = 0; j < NB; ++j) {
-            sm.Fg[j * kSI + kSI - 1] = Real(0);
-            if (!HZ) sm.Fh[j * kSI + kSI - 1] = Real(0);
-        }
-    }
-    double acc[15];
-#pragma unroll
-    for (int j = 0; j < 15; ++j) acc[j] = 0.0;
-
-    constexpr int H = (NB + kParts0 - 1) / kParts0;
-    Real pg[H], ph[H];
-    double pe[H];
-    BatchWalk<D, NB> walk(t.r0, m.n1d, m.row_base), ahead(t.r0, m.n1d, m.row_base);
-    const int nbt = (t.r1 - t.r0) * walk.nbr;
-    if (nbt > 0) {
-        if (has_item) stage_items<Real, NB, FULL, HZ>(sm, walk.pos(), fvg, fvh, ftab, nI, it, gi, x_res);
-        if (has_cell) fetch_cells<Real, NB, FULL, HZ>(walk.pos(), g, h, ctab, nC, c, part, pg, ph, pe);
-    }
-    for (int k = 0; k < nbt; ++k, walk.next()) {
-        const BatchPos bp = walk.pos();
-        if (k + 1 < nbt) ahead.next();
-        __syncthreads();  // records stashed; the previous batch's stage 4 is done with the fluxes
-        const RowConst q = row_const<D>(sm.x1, sm.w1, bp);
-        // stage 3: relaxed face DFs and fluxes of the items
-        if (has_item) {
-            const double p2 = __dmul_rn(q.Y, S[1]);
-            const double p3 = D == 3 ? __dmul_rn(q.Z, S[2]) : 0.0;
-            const double ey = __ldg(ftab + static_cast<size_t>(m.n1d + bp.iy) * nI + gi);
-            const double ez = D == 3 ? __ldg(ftab + static_cast<size_t>(2 * m.n1d + bp.iz) * nI + gi) : 1.0;
-            const Shk<double> fs = shk_from<D, double>(sm.frec, kSI, it, q, ey, ez);
-            const double* sx = sm.stx + (x_res ? bp.ix0 * kSI : 0) + it;
-            cp_wait_all();  // this item's staged entries of batch k
-            const Real* sg = sm.st + it;
-            if (kind != ITEM_MESH_BOUNDARY) {
-                // internal and tile-boundary faces: the staged slot holds the
-                // upwind face value; on an exactly tangential tile-boundary
-                // face it holds this side's half and the other slot the rest
-                const bool tb = kind != ITEM_TILE_INTERNAL;
-#pragma unroll
-                for (int j = 0; j < NB; ++j) {
-                    if (FULL || j < bp.nb) {
-                        const double x = sm.x1[bp.ix0 + j];
-                        const double xs = xs_row(x, S[0], p2, p3);
-                        Real rg = sg[j * kSI], rh = HZ ? Real(0) : sg[(NB + j) * kSI];
-                        if (tb && !(xs >= kVSmall) && !(xs < -kVSmall)) {
-                            const size_t o = static_cast<size_t>(bp.d0 + j) * nI + other;
-                            rg += __ldg(fvg + o);
-                            if (!HZ) rh += __ldg(fvh + o);
-                        }
-                        const double gr = dv_ref<Real>(m.gref, bp.d0 + j), hr = dv_ref<Real>(m.href, bp.d0 + j);
-                        double gf, hf;
-                        shk_relax<D, double>(fs, x, sx[j * kSI], plus_ref<Real>(double(rg), gr),
-                                             plus_ref<Real>(double(rh), hr), K3D, c0h, gf, hf);
-                        // the reference part of the fluxes cancels over a closed cell (sum of +-Sf = 0)
-                        sm.Fg[j * kSI + it] = Real(xs * minus_ref<Real>(gf, gr));
-                        if (!HZ) sm.Fh[j * kSI + it] = Real(xs * minus_ref<Real>(hf, hr));
-                    }
-                }
+    __device__ __forceinline__ double field(int k) const { return __ldg(at(row_of(rec, k, n8), e8)); }
+    __device__ __forceinline__ void row(const DevMesh& m, const Seg& q, double Y, double Z) {
+        if constexpr (!GEN) {
+            const double cy = Y - field(REC_UY), vy = field(REC_QY);
+            const double ey = __ldg(at(row_of(tab, m.n1d + q.iy, n8), e8));
+            if constexpr (D == 3) {
+                const double cz = Z - field(REC_UZ), vz = field(REC_QZ);
+                const double ez = __ldg(at(row_of(tab, 2 * m.n1d + q.iz, n8), e8));
+                Cyz = (cy * cy + cz * cz) * invRT;
+                Syz = cy * vy + cz * vz;
+                eyzr = r * ey * ez;
             } else {
-                // mesh boundary, by patch type.  Outgoing DFs are relaxed with
-                // the boundary face's record, whose h uses the internal-face T
-                // at the patch-local index (fvDVM.C:1367, :1413, :1429-1444).
-                // Incoming ones are not relaxed: wall rho_w M(U_w, T_w)
-                // (fvDVM.C:1079-1092), far field and pressure rho_b M(U_owner,
-                // T_b) (fvDVM.C:926-938) and mixed rho_b M(U_b, T_b) computed
-                // here; zero-gradient and symmetry ones come from the face-value
-                // buffer.  DVMsymmetry relaxes every DV once more
-                // (fvDVM.C:1445-1453).  Read per batch: boundary items are few.
-                const int face = chk(__ldg(m.it_face + gi), 0, m.nBF, a.ds.err);
-                const int pt = __ldg(m.it_meta + gi) >> 4;
-                const bool stored_in = pt == DUGKS_PATCH_ZERO_GRADIENT || pt == DUGKS_PATCH_SYMMETRY ||
-                                       pt == DUGKS_PATCH_DVM_SYMMETRY;
-                const bool again = pt == DUGKS_PATCH_DVM_SYMMETRY;
-                const BRec* br = a.ds.brec + face;
-                const double bK = br->rho_in * __ldg(&br->K_in);
-                const double bInv = __ldg(&br->invRT_in), bHf = __ldg(&br->hfac);
-                double bU[3];
-                if (pt == DUGKS_PATCH_MAXWELL_WALL || pt == DUGKS_PATCH_MIXED) {
-                    for (int i = 0; i < 3; ++i) bU[i] = __ldg(&br->U[i]);
-                } else {
-                    const int own = chk(__ldg(m.bface_owner + face), 0, m.nC, a.ds.err);
-                    for (int i = 0; i < 3; ++i) bU[i] = __ldg(a.ds.cellrec + (REC_UX + i) * nC + own);
-                }
-                const double cyz = (q.Y - bU[1]) * (q.Y - bU[1]) + (q.Z - bU[2]) * (q.Z - bU[2]);
-                if (again) {
-                    // DVMsymmetry: every DV relaxed once more after the outgoing
-                    // ones (a loop of its own: the rare type stays off the common path)
-#pragma unroll 1
-                    for (int j = 0; j < NB; ++j) {
-                        if (FULL || j < bp.nb) {
-                            const double x = sm.x1[bp.ix0 + j];
-                            const double xs = xs_row(x, S[0], p2, p3);
-                            const double gr = dv_ref<Real>(m.gref, bp.d0 + j), hr = dv_ref<Real>(m.href, bp.d0 + j);
-                            double gf = plus_ref<Real>(double(sg[j * kSI]), gr);
-                            double hf = plus_ref<Real>(double(HZ ? Real(0) : sg[(NB + j) * kSI]), hr);
-                            if (xs > 0) shk_relax<D, double>(fs, x, sx[j * kSI], gf, hf, K3D, c0h, gf, hf);
-                            shk_relax<D, double>(fs, x, sx[j * kSI], gf, hf, K3D, c0h, gf, hf);
-                            sm.Fg[j * kSI + it] = Real(xs * minus_ref<Real>(gf, gr));
-                            if (!HZ) sm.Fh[j * kSI + it] = Real(xs * minus_ref<Real>(hf, hr));
-                        }
-                    }
-                } else
+                Cyz = cy * cy * invRT;
+                Syz = cy * vy;
+                eyzr = r * ey;
+            }
+            ex = row_of(tab, q.ix0, n8);
+        }
+    }
+    // the Maxwellian factor of DV j of the segment
+    __device__ __forceinline__ double factor(int j) const {
+        if constexpr (GEN) return 0.0;
+        else return __ldg(at(row_of(ex, j, n8), e8));
+    }
+    __device__ __forceinline__ void operator()(const Dv& v, double e, double g, double h, double K3D, double c0h,
+                                               double& go, double& ho) const {
+        const double cx = v.x - Ux;
+        double cs, sq, Er;
+        if constexpr (GEN) {
+            const double cy = v.y - Uy, cz = D == 3 ? v.z - Uz : 0.0;
+            cs = (cx * cx + cy * cy + cz * cz) * invRT;
+            sq = cx * qx + cy * qy + (D == 3 ? cz * qz : 0.0);
+            Er = rA * exp(-0.5 * cs);
+        } else {
+            cs = fma(cx * cx, invRT, Cyz);
+            sq = fma(cx, qx, Syz);
+            Er = e * eyzr;
+        }
+        const double omr = 1.0 - r;
+        go = fma(omr, g, Er * fma(sq, cs - double(D + 2), 1.0));
+        if constexpr (HZ) ho = 0.0;
+        else ho = fma(omr, h, (Er * RTh) * fma(sq, fma(cs, K3D, c0h), K3D));
+    }
+};
+
+// K + 3 - D and -(D (K + 3 - D) + 2 K) of h^S
+template <int D>
+__device__ __forceinline__ double k3d(const DevMesh& m) { return m.K + 3.0 - D; }
+template <int D>
+__device__ __forceinline__ double c0h_of(const DevMesh& m) { return -(D * (m.K + 3.0 - D) + 2.0 * m.K); }
+
+// a cell's relax factor of this step (fvDVM.C:668); its record holds tau
+__device__ __forceinline__ double cell_r(const StepArgs& a, int c) {
+    const double dt = step_dt(a), tau = __ldg(a.ds.cellrec + REC_R * static_cast<size_t>(a.dm.nC) + c);
+    return 1.5 * dt / (2.0 * tau + dt);
+}
+
+// ---------------------------------------------------------------------
+// k_half_step
+// ---------------------------------------------------------------------
+// Reads g~ and writes gbar+: 16 B per (cell, DV) and FP64 field, bound by HBM.
+template <int D, typename Real, bool HZ, bool GEN>
+__global__ void __launch_bounds__(kStream) k_half_step(const __grid_constant__ StepArgs a) {
+    const DevMesh& m = a.dm;
+    __shared__ double x1[kMaxN1d], w1[kMaxN1d];
+    load_nodes(m, x1, w1);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2 && !a.keep_co) a.ds.co[threadIdx.x] = 0.0;
+    const int c = blockIdx.x * kStream + threadIdx.x;
+    if (c >= m.nC) return;
+    const size_t nC = static_cast<size_t>(m.nC);
+    const unsigned cb = sizeof(Real) * c, rb = sizeof(Real) * m.nC;
+    const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
+    Relax<D, HZ, GEN> rx(a.ds.cellrec, a.ds.ctab, m.nC, c, cell_r(a, c));
+    const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
+    for (int s = s0; s < s1; ++s) {
+        const Seg q = seg_at<GEN>(m, s);
+        rx.row(m, q, x1[q.iy], x1[q.iz]);
+        const size_t base = static_cast<size_t>(q.d0) * nC;
+        const Real* __restrict__ gs = reinterpret_cast<const Real*>(a.ds.g) + base;
+        const Real* __restrict__ hs = reinterpret_cast<const Real*>(a.ds.h) + base;
+        Real* __restrict__ gd = reinterpret_cast<Real*>(a.ds.gbar) + base;
+        Real* __restrict__ hd = reinterpret_cast<Real*>(a.ds.hbar) + base;
+        groups<4>(q.len, [&](int j, auto uc) {
+            constexpr int U = decltype(uc)::value;
+            Real gi[U], hi[U];
+            double e[U];
 #pragma unroll
-                for (int j = 0; j < NB; ++j) {
-                    if (FULL || j < bp.nb) {
-                        const double x = sm.x1[bp.ix0 + j];
-                        const double xs = xs_row(x, S[0], p2, p3);
-                        const double gr = dv_ref<Real>(m.gref, bp.d0 + j), hr = dv_ref<Real>(m.href, bp.d0 + j);
-                        double gf, hf;
-                        if (xs > 0) {
-                            shk_relax<D, double>(fs, x, sx[j * kSI], plus_ref<Real>(double(sg[j * kSI]), gr),
-                                                 plus_ref<Real>(double(HZ ? Real(0) : sg[(NB + j) * kSI]), hr), K3D, c0h, gf, hf);
-                        } else if (stored_in) {
-                            gf = plus_ref<Real>(double(sg[j * kSI]), gr);
-                            hf = plus_ref<Real>(double(HZ ? Real(0) : sg[(NB + j) * kSI]), hr);
+            for (int u = 0; u < U; ++u) {
+                gi[u] = __ldcs(at(row_of(gs, j + u, rb), cb));
+                if (!HZ) hi[u] = __ldcs(at(row_of(hs, j + u, rb), cb));
+                e[u] = rx.factor(j + u);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j + u), hr = dv_ref<Real, GEN>(m.href, q.d0 + j + u);
+                double go, ho;
+                rx(dv_at<D, GEN>(m, q, x1, j + u), e[u], double(gi[u]) + gr, HZ ? 0.0 : double(hi[u]) + hr, K3D, c0h, go,
+                   ho);
+                *at(row_of(gd, j + u, rb), cb) = Real(go - gr);
+                if (!HZ) *at(row_of(hd, j + u, rb), cb) = Real(ho - hr);
+            }
+        });
+    }
+}
+
+// ---------------------------------------------------------------------
+// k_face_values
+// ---------------------------------------------------------------------
+// Reconstruction at the half step from one side of a face
+// (fvDVM.C:832-836): gbar+ + grad . v, v = Cf - C - xi dt/2, x first, one
+// fused multiply-add per dimension and one for each component of v.
+template <int D, typename Real>
+__device__ __forceinline__ Real recon(Real gb, const Real* G, const Real* v) {
+    Real r = fma(G[0], v[0], gb);
+    r = fma(G[1], v[1], r);
+    if (D == 3) r = fma(G[D - 1], v[D - 1], r);
+    return r;
+}
+
+// One component of v = Cf - C - xi dt/2 in the storage type.  FP32 results
+// are held to the last bit, and this decides them: along a row the x product
+// is fused and the y and z products are rounded first; a DV list rounds all.
+template <typename Real>
+__device__ __forceinline__ Real fused_dist(Real d, Real hdt, double x) {
+    return fma(-hdt, Real(x), d);
+}
+template <typename Real>
+__device__ __forceinline__ Real rounded_dist(Real d, Real hdt, double x) {
+    if constexpr (sizeof(Real) == 4) return __fsub_rn(d, __fmul_rn(hdt, Real(x)));
+    else return fma(-hdt, x, d);
+}
+// (2-D rows that do not split into eights round the x product too at the
+// first and last of every eight nodes, on faces inside a tile: in_tile)
+template <int D, typename Real, bool GEN>
+__device__ __forceinline__ bool rounds_rows(const DevMesh& m) {
+    return D == 2 && sizeof(Real) == 4 && !GEN && (m.n1d & 7) != 0;
+}
+template <int D, typename Real, bool GEN>
+__device__ __forceinline__ void half_dist(const Real* d, double hdt, const Dv& v, int ix, bool in_tile, Real* r) {
+    if constexpr (GEN && sizeof(Real) == 4) {
+        r[0] = d[0] - Real(hdt * v.x);
+        r[1] = d[1] - Real(hdt * v.y);
+        if (D == 3) r[D - 1] = d[D - 1] - Real(hdt * v.z);
+    } else {
+        const Real h = Real(hdt);
+        r[0] = in_tile && ((ix + 1) & 6) == 0 ? rounded_dist<Real>(d[0], h, v.x) : fused_dist<Real>(d[0], h, v.x);
+        r[1] = rounded_dist<Real>(d[1], h, v.y);
+        if (D == 3) r[D - 1] = rounded_dist<Real>(d[D - 1], h, v.z);
+    }
+}
+
+// gradient of cell c's gbar+ (field f of DV row pointer) from the tables in
+// memory: cells with more than kFast neighbours, and tangential faces
+template <int D, typename Real>
+__device__ __forceinline__ void grad_mem(const DevMesh& m, const Real* f, int c, Real* G, int k0, int* err) {
+    const size_t nC = static_cast<size_t>(m.nC);
+    const Real f0 = f[c];
+    for (int k = k0; k < m.nb_max; ++k) {
+        const int n = chk(__ldg(m.nbr + k * nC + c), 0, m.nC, err);
+        const Real df = f[n] - f0;
+#pragma unroll
+        for (int q = 0; q < D; ++q) G[q] = fma(Real(__ldg(m.nbr_ls + (k * 3 + q) * nC + c)), df, G[q]);
+    }
+}
+
+// the reconstruction from one side of face f, everything from memory
+template <int D, typename Real, bool GEN>
+__device__ __forceinline__ Real recon_mem(const DevMesh& m, const Real* row, int f, int side, int c, double hdt,
+                                          const Dv& v, int ix, bool in_tile, int* err) {
+    const size_t nF = static_cast<size_t>(m.nF);
+    Real G[D];
+#pragma unroll
+    for (int q = 0; q < D; ++q) G[q] = Real(0);
+    grad_mem<D, Real>(m, row, c, G, 0, err);
+    Real d[D], r[D];
+#pragma unroll
+    for (int q = 0; q < D; ++q) d[q] = Real(__ldg(m.fgeo + (3 + 3 * side + q) * nF + f));
+    half_dist<D, Real, GEN>(d, hdt, v, ix, in_tile, r);
+    return recon<D, Real>(row[c], G, r);
+}
+
+// One thread per cell: the gradient from its neighbours' gbar+ (gathered
+// through L1: a CTA's cells are a compact block of the mesh) and the value of
+// every face it is upwind of (one bit per face and DV, DevMesh::upw).  The
+// gradient never leaves registers.  On an exactly tangential internal face
+// no side is upwind; k_face_moments averages both there.
+template <int D, typename Real, bool HZ, bool GEN, int NS>
+__global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant__ StepArgs a) {
+    const DevMesh& m = a.dm;
+    __shared__ double x1[kMaxN1d], w1[kMaxN1d];
+    load_nodes(m, x1, w1);
+    const int c = blockIdx.x * kCells + threadIdx.x;
+    if (c >= m.nC) return;
+    const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF);
+    const Real* __restrict__ gbar = reinterpret_cast<const Real*>(a.ds.gbar);
+    const Real* __restrict__ hbar = reinterpret_cast<const Real*>(a.ds.hbar);
+    Real* __restrict__ fvg = reinterpret_cast<Real*>(a.ds.fvg);
+    Real* __restrict__ fvh = reinterpret_cast<Real*>(a.ds.fvh);
+    const double hdt = 0.5 * step_dt(a);
+    // FP64 folds the DV's part of v once per cell, gbar+ - G.xi dt/2; FP32
+    // keeps the reference's order, one v per face
+    constexpr bool kFold = sizeof(Real) == 8;
+    const unsigned cr = sizeof(Real) * m.nC, fr = sizeof(Real) * m.nF, own = sizeof(Real) * c;
+    unsigned nb[NS], fo[NS];   // byte offsets in a row of cells, of faces
+    int code[NS];
+    Real ls[NS][D], dist[NS][D];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+        nb[k] = sizeof(Real) * (k < m.nb_max ? chk(__ldg(m.nbr + k * nC + c), 0, m.nC, a.ds.err) : c);
+        code[k] = k < m.nf_max ? chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err) : -1;
+#pragma unroll
+        for (int q = 0; q < D; ++q) {
+            ls[k][q] = k < m.nb_max ? Real(__ldg(m.nbr_ls + (k * 3 + q) * nC + c)) : Real(0);
+            fo[k] = code[k] < 0 ? 0u : sizeof(Real) * (code[k] >> 2);
+            dist[k][q] = code[k] < 0 ? Real(0) : Real(__ldg(m.fgeo + (3 + 3 * (code[k] & 1) + q) * nF + (code[k] >> 2)));
+        }
+    }
+    unsigned in_tile = 0;
+    if (rounds_rows<D, Real, GEN>(m)) {
+#pragma unroll
+        for (int k = 0; k < NS; ++k)
+            if (code[k] >= 0 && (code[k] & 2)) in_tile |= 1u << k;
+    }
+    const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
+    const bool more = m.nb_max > NS || m.nf_max > NS;
+    for (int s = s0; s < s1; ++s) {
+        const Seg q = seg_at<GEN>(m, s);
+        const double Y = x1[q.iy], Z = x1[q.iz];
+        unsigned up[NS];   // the segment's upwind bits
+#pragma unroll
+        for (int k = 0; k < NS; ++k)
+            up[k] = code[k] < 0 ? 0u : __ldg(m.upw + (static_cast<size_t>(s) * nF + (code[k] >> 2)) * 2 + (code[k] & 1));
+        const Real *gr = gbar + static_cast<size_t>(q.d0) * nC, *hr = hbar + static_cast<size_t>(q.d0) * nC;
+        Real *fg = fvg + static_cast<size_t>(q.d0) * nF, *fh = fvh + static_cast<size_t>(q.d0) * nF;
+        groups<kFold && D == 3 && !HZ ? 1 : 2>(q.len, [&](int j0, auto uc) {
+            constexpr int U = decltype(uc)::value;
+            Real g0[U], h0[U], dg[U][NS], dh[U][NS];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const Real *gj = row_of(gr, j0 + u, cr), *hj = row_of(hr, j0 + u, cr);
+                g0[u] = __ldg(at(gj, own));
+                if (!HZ) h0[u] = __ldg(at(hj, own));
+#pragma unroll
+                for (int k = 0; k < NS; ++k) {
+                    dg[u][k] = __ldg(at(gj, nb[k]));
+                    if (!HZ) dh[u][k] = __ldg(at(hj, nb[k]));
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int j = j0 + u;
+                Real G[D], H[D];
+#pragma unroll
+                for (int p = 0; p < D; ++p) G[p] = H[p] = Real(0);
+#pragma unroll
+                for (int k = 0; k < NS; ++k) {
+                    const Real x = dg[u][k] - g0[u];
+#pragma unroll
+                    for (int p = 0; p < D; ++p) G[p] = fma(ls[k][p], x, G[p]);
+                    if (!HZ) {
+                        const Real y = dh[u][k] - h0[u];
+#pragma unroll
+                        for (int p = 0; p < D; ++p) H[p] = fma(ls[k][p], y, H[p]);
+                    }
+                }
+                if (more) {
+                    grad_mem<D, Real>(m, gr + j * m.nC, c, G, NS, a.ds.err);
+                    if (!HZ) grad_mem<D, Real>(m, hr + j * m.nC, c, H, NS, a.ds.err);
+                }
+                Dv v = dv_at<D, GEN>(m, q, x1, j);
+                if constexpr (!GEN) {
+                    v.y = Y;
+                    v.z = Z;
+                }
+                Real gc = g0[u], hc = HZ ? Real(0) : h0[u];
+                if constexpr (kFold) {
+                    const Real t[3] = {Real(-hdt * v.x), Real(-hdt * v.y), Real(-hdt * v.z)};
+                    gc = recon<D, Real>(gc, G, t);
+                    if (!HZ) hc = recon<D, Real>(hc, H, t);
+                }
+                Real *fgj = row_of(fg, j, fr), *fhj = row_of(fh, j, fr);
+#pragma unroll
+                for (int k = 0; k < NS; ++k) {
+                    if (up[k] & (1u << j)) {
+                        Real vk[D];
+                        if constexpr (kFold) {
+#pragma unroll
+                            for (int p = 0; p < D; ++p) vk[p] = dist[k][p];
                         } else {
-                            const double cx = x - bU[0];
-                            const double ge = bK * exp(-0.5 * (cx * cx + cyz) * bInv);
-                            gf = plus_ref<Real>(double(Real(minus_ref<Real>(ge, gr))), gr);
-                            hf = plus_ref<Real>(double(Real(minus_ref<Real>(ge * bHf, hr))), hr);
+                            half_dist<D, Real, GEN>(dist[k], hdt, v, q.ix0 + j, (in_tile >> k) & 1u, vk);
                         }
-                        sm.Fg[j * kSI + it] = Real(xs * minus_ref<Real>(gf, gr));
-                        if (!HZ) sm.Fh[j * kSI + it] = Real(xs * minus_ref<Real>(hf, hr));
+                        *at(fgj, fo[k]) = recon<D, Real>(gc, G, vk);
+                        if (!HZ) *at(fhj, fo[k]) = recon<D, Real>(hc, H, vk);
+                    }
+                }
+                if (more) {
+                    for (int k = NS; k < m.nf_max; ++k) {
+                        const int cd = chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err);
+                        if (cd < 0) break;
+                        const int f = cd >> 2, side = cd & 1;
+                        if ((__ldg(m.upw + (static_cast<size_t>(s) * nF + f) * 2 + side) >> j) & 1u) {
+                            Real dk[D], vk[D];
+#pragma unroll
+                            for (int p = 0; p < D; ++p) dk[p] = Real(__ldg(m.fgeo + (3 + 3 * side + p) * nF + f));
+                            half_dist<D, Real, GEN>(dk, hdt, v, q.ix0 + j, (cd & 2) && rounds_rows<D, Real, GEN>(m), vk);
+                            fgj[f] = recon<D, Real>(g0[u], G, vk);
+                            if (!HZ) fhj[f] = recon<D, Real>(h0[u], H, vk);
+                        }
                     }
                 }
             }
-            // this thread has read its staged entries: stage the next batch
-            if (k + 1 < nbt) stage_items<Real, NB, FULL, HZ>(sm, ahead.pos(), fvg, fvh, ftab, nI, it, gi, x_res);
+        });
+    }
+}
+
+// upwind bits of every face and segment (geometry and DV set only; once at
+// creation).  Bit j of word (s, f, side): DV j of segment s leaves through
+// face f from that side -- internal faces by the switch of fvDVM.C:829-863
+// (neither side on an exactly tangential face), boundary faces the outgoing
+// DVs (:916-923), symmetry faces the tangential ones too (:1013-1023);
+// zero-gradient faces take the cell's value for every DV instead.
+template <int D, bool GEN>
+__global__ void k_upwind_bits(const DevMesh m, uint32_t* upw) {
+    __shared__ double x1[kMaxN1d], w1[kMaxN1d];
+    load_nodes(m, x1, w1);
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= m.nF) return;
+    const size_t nF = static_cast<size_t>(m.nF);
+    const double S[3] = {__ldg(m.fgeo + f), __ldg(m.fgeo + nF + f), __ldg(m.fgeo + 2 * nF + f)};
+    const int pt = f < m.nIF ? 0 : __ldg(m.bface_ptype + f - m.nIF);
+    const bool sym = pt == DUGKS_PATCH_SYMMETRY || pt == DUGKS_PATCH_DVM_SYMMETRY;
+    for (int s = blockIdx.y; s < m.n_seg; s += gridDim.y) {
+        const Seg q = seg_at<GEN>(m, s);
+        uint32_t own = 0, nei = 0;
+        for (int j = 0; j < q.len; ++j) {
+            const double xs = xs_dv(dv_at<D, GEN>(m, q, x1, j), S);
+            if (pt == 0) {
+                if (xs >= kVSmall) own |= 1u << j;
+                else if (xs < -kVSmall) nei |= 1u << j;
+            } else if (pt != DUGKS_PATCH_ZERO_GRADIENT) {
+                if (sym ? xs > -kVSmall : xs > 0) own |= 1u << j;
+            }
         }
-        __syncthreads();
-        // stage 4: g~ <- -g~/3 + 4/3 gbar+ - dt/V sum_f (+-)(xi.S) g_f, cell moments
-        if (has_cell) {
-            const double ey = __ldg(ctab + static_cast<size_t>(m.n1d + bp.iy) * nC + c);
-            const double ez = D == 3 ? __ldg(ctab + static_cast<size_t>(2 * m.n1d + bp.iz) * nC + c) : 1.0;
-            const Shk<double> cs = shk_from<D, double>(sm.crec, kS0, lc, q, ey, ez);
-            RowSums rs;
-            row_zero(rs);
+        uint32_t* w = upw + (static_cast<size_t>(s) * nF + f) * 2;
+        w[0] = own;
+        w[1] = nei;
+    }
+}
+
+// ---------------------------------------------------------------------
+// Reductions of the face and cell kernels
+// ---------------------------------------------------------------------
+// this CTA's chunk, from its warps' sums in f.red, into part [chunk][kNM][n];
+// true in the CTA that completes the entity block
+__device__ __forceinline__ bool reduce_chunk(Finish& f, double* part, size_t n, int e0, int count, int* done, bool fused) {
+    const int lane = threadIdx.x % kLanes, w = threadIdx.x / kLanes;
+    __syncthreads();
+    for (int j = w; j < 15; j += kParts) {
+        double v = f.red[0][j][lane];
+        for (int p = 1; p < kParts; ++p) v += f.red[p][j][lane];
+        if (lane < count) part[(static_cast<size_t>(blockIdx.y) * kNM + j) * n + e0 + lane] = v;
+    }
+    if (!fused) return false;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int k = gridDim.y > 1 ? atomicAdd(done, 1) : 0;
+        f.last = k == static_cast<int>(gridDim.y) - 1;
+        if (f.last && gridDim.y > 1) *done = 0;   // for the next launch
+    }
+    __syncthreads();
+    if (!f.last) return false;
+    __threadfence();
+    return true;
+}
+
+// chunk sums of the block's entities, added in chunk order, into f.tot
+__device__ __forceinline__ void sum_chunks(Finish& f, const double* part, size_t n, int e0, int count, int chunks) {
+    const int lane = threadIdx.x % kLanes, w = threadIdx.x / kLanes;
+    for (int j = w; j < 15; j += kParts) {
+        double v = 0.0;
+        if (lane < count) {
+#pragma unroll 4
+            for (int ch = 0; ch < chunks; ++ch) v += __ldcg(part + (static_cast<size_t>(ch) * kNM + j) * n + e0 + lane);
+        }
+        f.tot[j][lane] = v;
+    }
+    __syncthreads();
+}
+
+// one-dimensional Maxwellian factors of the block's entities (layout in
+// dugks_internal.h): D * n1d exponentials each, shared by the CTA's warps
+__device__ __forceinline__ void write_tables(const Finish& f, const DevMesh& m, double* tab, size_t n, int e0, int count) {
+    const int lane = threadIdx.x % kLanes, w = threadIdx.x / kLanes;
+    if (lane >= count) return;
+    for (int i = w; i < m.D * m.n1d; i += kParts) {
+        const int k = i / m.n1d;
+        const double x = __ldg(m.X1 + i - k * m.n1d) - f.mac[k][lane];
+        double v = exp(-0.5 * x * x * f.mac[3][lane]);
+        if (k == 0) v *= f.mac[4][lane];
+        tab[static_cast<size_t>(i) * n + e0 + lane] = v;
+    }
+}
+
+// Face macros and relaxation coefficients of the block's faces from the
+// chunk sums (updateMaxwellWallRho fvDVM.C:1032-1052,
+// calculatedMaxwellFvPatchField.C:140-164, updateMacroSurf :1248-1300).
+__device__ __noinline__ void finish_faces(Finish& sm, const StepArgs& a, const Consts& kc, int f0, int count, int chunks) {
+    const DevMesh& m = a.dm;
+    const size_t nF = static_cast<size_t>(m.nF);
+    sum_chunks(sm, a.ds.partF, nF, f0, count, chunks);
+    const int lane = threadIdx.x % kLanes;
+    if (threadIdx.x < kLanes) {
+        double co = 0.0;
+        if (lane < count) {
+            const int f = f0 + lane;
+            const double dt = step_dt(a);
+            double s[15];
+            for (int j = 0; j < 15; ++j) s[j] = sm.tot[j][lane];
+            if (f >= m.nIF && __ldg(m.bface_ptype + f - m.nIF) == DUGKS_PATCH_MAXWELL_WALL) {
+                // rho_w = outGoing / |inComingByRho|; the incoming wall DFs enter through it
+                BRec* br = a.ds.brec + (f - m.nIF);
+                const double rho_w = s[MOM_OUT] / fabs(br->inByRho);
+                br->rho_in = rho_w;
+                const double* mi = a.ds.bmom_in + static_cast<size_t>(f - m.nIF) * kNM;
+                for (int j = 0; j < 14; ++j) s[j] += rho_w * mi[j];
+            }
+            double rho, U[3], T, q[3], tau;
+            macros_from_moments(s, kc, rho, U, T, q, tau);
+            const double fac = 2.0 * tau / (2.0 * tau + 0.5 * dt * kc.Pr);  // fvDVM.C:1300
+            for (int i = 0; i < 3; ++i) q[i] *= fac;
+            const int fo = __ldg(m.forig + f);
+            double* fm = a.ds.fm + static_cast<size_t>(fo) * 9;
+            fm[0] = rho;
+            fm[4] = T;
+            fm[8] = tau;
+            const double RT = kc.R * T, A = rho * inv_norm(RT, kc.D);
+            const double qs = kc.Pr1 / (5.0 * rho * RT * RT);
+            double* fr = a.ds.facerec + f;
+            for (int i = 0; i < 3; ++i) {
+                fm[1 + i] = U[i];
+                fm[5 + i] = q[i];
+                fr[(REC_UX + i) * nF] = U[i];
+                fr[(REC_QX + i) * nF] = q[i] * qs;
+                sm.mac[i][lane] = U[i];
+            }
+            fr[REC_INVRT * nF] = 1.0 / RT;
+            fr[REC_A * nF] = A;
+            fr[REC_R * nF] = 0.5 * dt / (2.0 * tau + 0.5 * dt);
+            fr[REC_RTH * nF] = RT;
+            sm.mac[3][lane] = 1.0 / RT;
+            sm.mac[4][lane] = A;
+            if (f < m.nIF)  // getCoNum, fvDVM.C:2180-2182
+                co = __ldg(m.dc + fo) * (sqrt(U[0] * U[0] + U[1] * U[1] + U[2] * U[2]) + m.xi_max_co);
+        }
+        double vmax = co, vsum = co;
+        for (int o = 16; o > 0; o >>= 1) {
+            vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+            vsum += __shfl_xor_sync(0xffffffffu, vsum, o);
+        }
+        if (lane == 0) {
+            // non-negative doubles order like their bit patterns
+            atomicMax(reinterpret_cast<unsigned long long*>(a.ds.co), static_cast<unsigned long long>(__double_as_longlong(vmax)));
+            atomicAdd(a.ds.co + 1, vsum);
+        }
+    }
+    __syncthreads();
+    if (!m.general_dv) write_tables(sm, m, a.ds.ftab, nF, f0, count);
+}
+
+// the coefficient record of the next half step
+__device__ __noinline__ void write_cellrec(const StepArgs& a, const Consts& k, int c, double rho, const double* U,
+                                           double T, const double* q, double tau) {
+    const double RT = k.R * T;
+    const double qs = k.Pr1 / (5.0 * rho * RT * RT);
+    const size_t n = static_cast<size_t>(a.dm.nC);
+    double* cr = a.ds.cellrec + c;
+    for (int i = 0; i < 3; ++i) {
+        cr[(REC_UX + i) * n] = U[i];
+        cr[(REC_QX + i) * n] = q[i] * qs;
+    }
+    cr[REC_INVRT * n] = 1.0 / RT;
+    cr[REC_A * n] = rho * inv_norm(RT, k.D);
+    cr[REC_R * n] = tau;
+    cr[REC_RTH * n] = RT;
+}
+
+// macroFlux yes (fvDVM.C:1523-1526, :1613-1679): the cell's old rho, rho U,
+// rho E advanced by this step's face macro fluxes, faces in face order.  The
+// face stress is zero (its sum is commented out, fvDVM.C:1270, :1305); the
+// boundary momentum flux takes Sf of the internal face at the patch-local
+// index (fvDVM.C:1668-1669); "X & Sf*dt/V" is X & ((Sf dt)/V).
+__device__ __forceinline__ void macro_flux_update(const StepArgs& a, const Consts& k, int c, double& rho, double rU[3],
+                                                  double& rE) {
+    const DevMesh& m = a.dm;
+    const double* cm = a.ds.cm + static_cast<size_t>(c) * 9;
+    const double U0[3] = {cm[1], cm[2], cm[3]};
+    rho = cm[0];
+    for (int i = 0; i < 3; ++i) rU[i] = rho * U0[i];
+    rE = rho * (0.5 * (U0[0] * U0[0] + U0[1] * U0[1] + U0[2] * U0[2]) + (k.Kin + 3) / 2.0 * k.R * cm[4]);
+    const double V = __ldg(m.mf_V + c), dt = k.dt;
+    for (int e = __ldg(m.mf_off + c); e < __ldg(m.mf_off + c + 1); ++e) {
+        const int code = __ldg(m.mf_ent + e), f = chk(code >> 2, 0, m.nIF + m.nBF, a.ds.err);
+        const bool add = code & 1;
+        const double* fm = a.ds.fm + static_cast<size_t>(f) * 9;
+        const double rf = fm[0], Uf[3] = {fm[1], fm[2], fm[3]}, qf[3] = {fm[5], fm[6], fm[7]};
+        const double* S = m.mf_Sf + 3 * static_cast<size_t>(f);
+        const double* Sm = f < m.nIF ? S
+                                     : m.mf_Sf + 3 * static_cast<size_t>(chk(__ldg(m.bface_patch_local + f - m.nIF), 0,
+                                                                             m.nIF + m.nBF, a.ds.err));
+        const double rUf[3] = {__dmul_rn(rf, Uf[0]), __dmul_rn(rf, Uf[1]), __dmul_rn(rf, Uf[2])};
+        const double rEf = __dmul_rn(rf, __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(Uf[0], Uf[0]), __dmul_rn(Uf[1], Uf[1])),
+                                                             __dmul_rn(Uf[2], Uf[2])),
+                                                   __dmul_rn(__dmul_rn((k.Kin + 3) / 2.0, k.R), fm[4])));
+        double ev[3], Sd[3], Smd[3];
+        for (int i = 0; i < 3; ++i) {
+            ev[i] = __dadd_rn(__dmul_rn(rEf, Uf[i]), qf[i]);
+            Sd[i] = __ddiv_rn(__dmul_rn(__ldg(S + i), dt), V);
+            Smd[i] = __ddiv_rn(__dmul_rn(__ldg(Sm + i), dt), V);
+        }
+        const double mr = __ddiv_rn(__dmul_rn(xi_dot_s(rUf, S), dt), V);
+        const double mE = xi_dot_s(ev, Sd);
+        double mU[3];
+        for (int i = 0; i < 3; ++i) {
+            const double t[3] = {__dmul_rn(rUf[i], Uf[0]), __dmul_rn(rUf[i], Uf[1]), __dmul_rn(rUf[i], Uf[2])};
+            mU[i] = xi_dot_s(t, Smd);
+        }
+        if (add) {
+            rho += mr;
+            for (int i = 0; i < 3; ++i) rU[i] += mU[i];
+            rE += mE;
+        } else {
+            rho -= mr;
+            for (int i = 0; i < 3; ++i) rU[i] -= mU[i];
+            rE -= mE;
+        }
+    }
+}
+
+// cell macros and record from the moment sums s
+__device__ __noinline__ void cell_macros(const StepArgs& a, const Consts& k, int c, const double* s, int chunks) {
+    const DevMesh& m = a.dm;
+    double rho, U[3], T, q[3], tau;
+    if (!m.macro_flux) {
+        macros_from_moments(s, k, rho, U, T, q, tau);
+    } else {
+        // rho, U, T from the fluxes; q from the DF moments about that U:
+        // q = 1/2 [V3 - 2 M2.U + |U|^2 M1 - U W + 2 U (M1.U) - U |U|^2 M0]
+        double rU[3], rE;
+        if (!m.general_dv) {
+            macro_flux_update(a, k, c, rho, rU, rE);
+        } else {
+            // the velocity-mesh branch (fvDVM.C:1562-1611): the old rho, rho U,
+            // rho E plus the moments of the update's flux term (pass B)
+            const double* cm = a.ds.cm + static_cast<size_t>(c) * 9;
+            double f[5] = {0, 0, 0, 0, 0};
+            for (int ch = 0; ch < chunks; ++ch)
+                for (int j = 0; j < 5; ++j)
+                    f[j] += __ldcg(a.ds.partX + (static_cast<size_t>(ch) * kFX + j) * m.nC + c);
+            const double U0[3] = {cm[1], cm[2], cm[3]};
+            rho = cm[0] + f[0];
+            for (int i = 0; i < 3; ++i) rU[i] = cm[0] * U0[i] + f[1 + i];
+            rE = cm[0] * (0.5 * (U0[0] * U0[0] + U0[1] * U0[1] + U0[2] * U0[2]) + (k.Kin + 3) / 2.0 * k.R * cm[4]) +
+                 f[4];
+        }
+        for (int i = 0; i < 3; ++i) U[i] = rU[i] / rho;
+        const double u2 = U[0] * U[0] + U[1] * U[1] + U[2] * U[2];
+        T = (rE - 0.5 * rho * u2) / ((k.Kin + 3.0) / 2.0 * k.R * rho);
+        tau = k.muRef * exp(k.omega * log(T / k.Tref)) / rho / T / k.R;
+        const double* M2 = s + MOM_M2;
+        const double M2U[3] = {M2[0] * U[0] + M2[1] * U[1] + M2[2] * U[2], M2[1] * U[0] + M2[3] * U[1] + M2[4] * U[2],
+                               M2[2] * U[0] + M2[4] * U[1] + M2[5] * U[2]};
+        const double M1U = s[MOM_M1] * U[0] + s[MOM_M1 + 1] * U[1] + s[MOM_M1 + 2] * U[2];
+        for (int i = 0; i < 3; ++i)
+            q[i] = 0.5 * (s[MOM_V3 + i] - 2.0 * M2U[i] + u2 * s[MOM_M1 + i] - U[i] * s[MOM_W] + 2.0 * U[i] * M1U -
+                          U[i] * u2 * s[MOM_M0]);
+    }
+    const double fac = 2.0 * tau / (2.0 * tau + k.dt * k.Pr);  // fvDVM.C:1742
+    for (int i = 0; i < 3; ++i) q[i] *= fac;
+    if (!(rho > 0.0) || !(T > 0.0) || !isfinite(rho + T + U[0] + U[1] + U[2])) atomicOr(a.ds.err, 1);
+    double* cm = a.ds.cm + static_cast<size_t>(c) * 9;
+    cm[0] = rho;
+    cm[1] = U[0];
+    cm[2] = U[1];
+    cm[3] = U[2];
+    cm[4] = T;
+    cm[5] = q[0];
+    cm[6] = q[1];
+    cm[7] = q[2];
+    cm[8] = tau;
+    write_cellrec(a, k, c, rho, U, T, q, tau);
+}
+
+// record factors of the block's cells for their tables
+__device__ __forceinline__ void tables_of_records(Finish& sm, const StepArgs& a, int c0, int count) {
+    const size_t nC = static_cast<size_t>(a.dm.nC);
+    const int lane = threadIdx.x % kLanes;
+    if (threadIdx.x < kLanes && lane < count) {
+        const double* cr = a.ds.cellrec + c0 + lane;
+        for (int i = 0; i < 3; ++i) sm.mac[i][lane] = cr[(REC_UX + i) * nC];
+        sm.mac[3][lane] = cr[REC_INVRT * nC];
+        sm.mac[4][lane] = cr[REC_A * nC];
+    }
+    __syncthreads();
+    if (!a.dm.general_dv) write_tables(sm, a.dm, a.ds.ctab, nC, c0, count);
+}
+
+// Cell macros (updateMacroVol, fvDVM.C:1682-1742) and the coefficient
+// records of the next half step, of the block's cells from the chunk sums.
+__device__ __noinline__ void finish_cells(Finish& sm, const StepArgs& a, const Consts& kc, int c0, int count, int chunks) {
+    sum_chunks(sm, a.ds.partC, static_cast<size_t>(a.dm.nC), c0, count, chunks);
+    const int lane = threadIdx.x % kLanes;
+    if (threadIdx.x < kLanes && lane < count) {
+        Consts k = kc;
+        k.dt = step_dt(a);
+        double s[15];
+        for (int j = 0; j < 15; ++j) s[j] = sm.tot[j][lane];
+        cell_macros(a, k, c0 + lane, s, chunks);
+    }
+    tables_of_records(sm, a, c0, count);
+}
+
+// cell records and tables from the cell macros in cm
+__global__ void __launch_bounds__(kLanes* kParts) k_cell_records(const __grid_constant__ StepArgs a,
+                                                                 const __grid_constant__ Consts k) {
+    __shared__ Finish sm;
+    const int c0 = blockIdx.x * kLanes, count = min(kLanes, a.dm.nC - c0), lane = threadIdx.x % kLanes;
+    if (threadIdx.x < kLanes && lane < count) {
+        const double* cm = a.ds.cm + static_cast<size_t>(c0 + lane) * 9;
+        const double U[3] = {cm[1], cm[2], cm[3]}, q[3] = {cm[5], cm[6], cm[7]};
+        write_cellrec(a, k, c0 + lane, cm[0], U, cm[4], q, cm[8]);
+    }
+    tables_of_records(sm, a, c0, count);
+}
+
+// ---------------------------------------------------------------------
+// k_face_moments
+// ---------------------------------------------------------------------
+// the Maxwellian a boundary face's incoming DFs take (fvDVM.C:926-938,
+// :1079-1092; mixed patches discreteVelocity.C:226-258)
+struct Incoming {
+    double rK, inv, hf, U[3];
+    template <int D>
+    __device__ __forceinline__ void at(const Dv& v, double& g, double& h) const {
+        const double cx = v.x - U[0], cy = v.y - U[1], cz = v.z - U[2];
+        g = rK * exp(-0.5 * (cx * cx + cy * cy + cz * cz) * inv);
+        h = g * hf;
+    }
+};
+
+__device__ __forceinline__ Incoming load_incoming(const StepArgs& a, int b, int pt) {
+    const BRec* br = a.ds.brec + b;
+    Incoming t;
+    t.rK = br->rho_in * br->K_in;
+    t.inv = br->invRT_in;
+    t.hf = br->hfac;
+    if (pt == DUGKS_PATCH_MAXWELL_WALL || pt == DUGKS_PATCH_MIXED) {
+        for (int i = 0; i < 3; ++i) t.U[i] = br->U[i];
+    } else {
+        const size_t nC = static_cast<size_t>(a.dm.nC);
+        const int own = chk(__ldg(a.dm.bface_owner + b), 0, a.dm.nC, a.ds.err);
+        for (int i = 0; i < 3; ++i) t.U[i] = a.ds.cellrec[(REC_UX + i) * nC + own];
+    }
+    return t;
+}
+
+// boundary faces of one chunk: by patch type (fvDVM.C:866-1027)
+template <int D, typename Real, bool HZ, bool GEN>
+__device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x1, const double* w1, int f, int s0,
+                                              int s1, int w, Finish& sm) {
+    const DevMesh& m = a.dm;
+    Sums<GEN> acc(sm);
+    const size_t nF = static_cast<size_t>(m.nF), nC = static_cast<size_t>(m.nC);
+    Real* fg = reinterpret_cast<Real*>(a.ds.fvg) + f;
+    Real* fh = reinterpret_cast<Real*>(a.ds.fvh) + f;
+    const int b = f - m.nIF, pt = __ldg(m.bface_ptype + b);
+    const bool wall = pt == DUGKS_PATCH_MAXWELL_WALL, zero_grad = pt == DUGKS_PATCH_ZERO_GRADIENT;
+    const bool sym = pt == DUGKS_PATCH_SYMMETRY || pt == DUGKS_PATCH_DVM_SYMMETRY;
+    const double S[3] = {__ldg(m.fgeo + f), __ldg(m.fgeo + nF + f), __ldg(m.fgeo + 2 * nF + f)};
+    const int own = chk(__ldg(m.bface_owner + b), 0, m.nC, a.ds.err);
+    const int axis = sym ? __ldg(m.bface_mirror + b) : -1;
+    double S0[3] = {0, 0, 0};
+    if (axis >= 0) {
+        const int b0 = chk(b - __ldg(m.bface_patch_local + b), 0, m.nBF, a.ds.err);
+        for (int i = 0; i < 3; ++i) S0[i] = __ldg(m.bS + 3 * b0 + i);
+    }
+    Incoming in{};
+    if (!wall && !zero_grad && !sym) in = load_incoming(a, b, pt);
+    for (int s = s0 + w; s < s1; s += kParts) {
+        const Seg q = seg_at<GEN>(m, s);
+        RowSums rs;
+        for (int j = 0; j < q.len; ++j) {
+            const int d = q.d0 + j;
+            const size_t o = static_cast<size_t>(d) * nF;
+            const Dv v = dv_at<D, GEN>(m, q, x1, j);
+            const double xs = xs_dv(v, S);
+            const double gr = dv_ref<Real, GEN>(m.gref, d), hr = dv_ref<Real, GEN>(m.href, d);
+            double g, h = 0.0;
+            if (zero_grad) {
+                // every DV: the owner cell's gbar+ (fvDVM.C:887-891)
+                const size_t oc = static_cast<size_t>(d) * nC + own;
+                const Real gv = reinterpret_cast<const Real*>(a.ds.gbar)[oc];
+                fg[o] = gv;
+                g = double(gv) + gr;
+                if (!HZ) {
+                    const Real hv = reinterpret_cast<const Real*>(a.ds.hbar)[oc];
+                    fh[o] = hv;
+                    h = double(hv) + hr;
+                }
+            } else if (sym) {
+                // incoming through the patch's first face (updateGHbarSurfSymmetryIn,
+                // fvDVM.C:1100-1179, discreteVelocity.C:691-773): the face value of the
+                // mirror DV along the patch's axis; a DV that is its own mirror stays
+                bool counted = xs > -kVSmall;
+                if constexpr (!GEN) {
+                    if (!(xs_dv(v, S0) > 0)) {
+                        const int n = m.n1d, st = axis == 0 ? 1 : axis == 1 ? n : n * n;
+                        const int i = axis == 0 ? q.ix0 + j : axis == 1 ? q.iy : q.iz;
+                        const int t = d + (n - 1 - 2 * i) * st;
+                        if (t != d) {
+                            counted = true;
+                            // of two mirrors that are both incoming the later one keeps its value
+                            Dv vt = v;
+                            (axis == 0 ? vt.x : axis == 1 ? vt.y : vt.z) = x1[n - 1 - i];
+                            if (xs_dv(vt, S0) > 0 || t > d) {
+                                const size_t ot = static_cast<size_t>(t) * nF;
+                                const double grt = dv_ref<Real, GEN>(m.gref, t), hrt = dv_ref<Real, GEN>(m.href, t);
+                                fg[o] = Real((double(fg[ot]) + grt) - gr);
+                                if (!HZ) fh[o] = Real((double(fh[ot]) + hrt) - hr);
+                            }
+                        }
+                    }
+                }
+                if (!counted) continue;
+                g = double(fg[o]) + gr;
+                if (!HZ) h = double(fh[o]) + hr;
+            } else if (xs > 0) {
+                // outgoing: upwind from the owner (fvDVM.C:916-923, :950-961)
+                g = double(fg[o]) + gr;
+                if (!HZ) h = double(fh[o]) + hr;
+            } else if (wall) {
+                continue;   // incoming wall DFs enter through rho_w
+            } else {
+                in.at<D>(v, g, h);
+                // rounded as k_face_flux rounds the same incoming DF
+                g = double(Real(g - gr)) + gr;
+                h = double(Real(h - hr)) + hr;
+            }
+            const double aw = add_dv<D, HZ, GEN>(acc, rs, w1, q, v, j, g, h);
+            if (wall) {
+                if constexpr (GEN) acc[MOM_OUT] = fma(aw, xs, acc[MOM_OUT]);
+                else rs.O = fma(aw, xs, rs.O);
+            }
+        }
+        if constexpr (!GEN) row_fold<D>(acc, rs, row_const<D>(x1, w1, q));
+    }
+    acc.put(sm);
+}
+
+template <int D, typename Real, bool HZ, bool GEN>
+__global__ void __launch_bounds__(kLanes* kParts, 8) k_face_moments(const __grid_constant__ StepArgs a,
+                                                                 const __grid_constant__ Consts kc) {
+    const DevMesh& m = a.dm;
+    __shared__ double x1[kMaxN1d], w1[kMaxN1d];
+    __shared__ Finish sm;
+    load_nodes(m, x1, w1);
+    // boundary face blocks first: they evaluate exponentials and take longest
+    const int nbB = (m.nBF + kLanes - 1) / kLanes, bx = blockIdx.x;
+    const bool bnd = bx < nbB;
+    const int f0 = bnd ? m.nIF + bx * kLanes : (bx - nbB) * kLanes;
+    const int count = min(kLanes, (bnd ? m.nF : m.nIF) - f0);
+    const int lane = threadIdx.x % kLanes, f = f0 + lane;
+    const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF);
+    const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
+    const int w = warp_id();
+    Sums<GEN> acc(sm);
+    if (bnd) {
+        if (lane < count) boundary_moments<D, Real, HZ, GEN>(a, x1, w1, f, s0, s1, w, sm);
+    } else {
+        if (lane < count) {
+            Real* fg = reinterpret_cast<Real*>(a.ds.fvg);
+            Real* fh = reinterpret_cast<Real*>(a.ds.fvh);
+            const unsigned fb = sizeof(Real) * f, fr = sizeof(Real) * m.nF;
+            for (int s = s0 + w; s < s1; s += kParts) {
+                const Seg q = seg_at<GEN>(m, s);
+                const uint2 up = __ldg(reinterpret_cast<const uint2*>(m.upw) + static_cast<size_t>(s) * nF + f);
+                unsigned tang = ~(up.x | up.y) & (q.len == 32 ? 0xffffffffu : (1u << q.len) - 1u);
+                while (tang) {
+                    // exactly tangential: both sides averaged (fvDVM.C:847-863)
+                    const int j = __ffs(tang) - 1;
+                    tang &= tang - 1;
+                    const int o = chk(__ldg(m.fown + f), 0, m.nC, a.ds.err), n = chk(__ldg(m.fnei + f), 0, m.nC, a.ds.err);
+                    const double hdt = 0.5 * step_dt(a);
+                    const Dv v = dv_at<D, GEN>(m, q, x1, j);
+                    bool in_tile = false;
+                    if (rounds_rows<D, Real, GEN>(m))
+                        for (int k = 0; k < m.nf_max; ++k) {
+                            const int code = __ldg(m.cface + k * nC + o);
+                            if (code >= 0 && (code >> 2) == f) in_tile = code & 2;
+                        }
+                    const size_t rc = static_cast<size_t>(q.d0 + j) * nC, rf = static_cast<size_t>(q.d0 + j) * nF + f;
+                    const Real* g = reinterpret_cast<const Real*>(a.ds.gbar) + rc;
+                    fg[rf] = Real(0.5) * (recon_mem<D, Real, GEN>(m, g, f, 1, n, hdt, v, q.ix0 + j, in_tile, a.ds.err) +
+                                          recon_mem<D, Real, GEN>(m, g, f, 0, o, hdt, v, q.ix0 + j, in_tile, a.ds.err));
+                    if (!HZ) {
+                        const Real* h = reinterpret_cast<const Real*>(a.ds.hbar) + rc;
+                        fh[rf] = Real(0.5) * (recon_mem<D, Real, GEN>(m, h, f, 1, n, hdt, v, q.ix0 + j, in_tile, a.ds.err) +
+                                              recon_mem<D, Real, GEN>(m, h, f, 0, o, hdt, v, q.ix0 + j, in_tile, a.ds.err));
+                    }
+                }
+                RowSums rs;
+                const Real *gs = fg + static_cast<size_t>(q.d0) * nF, *hs = fh + static_cast<size_t>(q.d0) * nF;
+                // FP32 storage: the deviations only; the reference part is added once below
+                groups<HZ ? 8 : 4>(q.len, [&](int j, auto uc) {
+                    constexpr int U = decltype(uc)::value;
+                    Real gi[U], hi[U];
 #pragma unroll
-            for (int jj = 0; jj < H; ++jj) {
-                const int j = part + kParts0 * jj;
-                if (FULL || j < bp.nb) {
-                    const Real gt = pg[jj], ht = ph[jj];
-                    const double x = sm.x1[bp.ix0 + j];
-                    const double gr = dv_ref<Real>(m.gref, bp.d0 + j), hr = dv_ref<Real>(m.href, bp.d0 + j);
+                    for (int u = 0; u < U; ++u) {
+                        gi[u] = *at(row_of(gs, j + u, fr), fb);
+                        if (!HZ) hi[u] = *at(row_of(hs, j + u, fr), fb);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        add_dv<D, HZ, GEN>(acc, rs, w1, q, dv_at<D, GEN>(m, q, x1, j + u), j + u, double(gi[u]),
+                                           HZ ? 0.0 : double(hi[u]));
+                });
+                if constexpr (!GEN) row_fold<D>(acc, rs, row_const<D>(x1, w1, q));
+            }
+            if constexpr (sizeof(Real) == 4 && !GEN) {
+                // an internal face counts every DV in full: the reference's moments once
+                if (blockIdx.y == 0 && threadIdx.x < kLanes)
+                    for (int j = 0; j < 14; ++j) acc[j] += __ldg(a.ds.refmom + j);
+            }
+        }
+        acc.put(sm);
+    }
+    if (reduce_chunk(sm, a.ds.partF, nF, f0, count, a.ds.done + bx, a.fused != 0))
+        finish_faces(sm, a, kc, f0, count, gridDim.y);
+}
+
+// the finishing part alone, for sharded handles: the chunk sums of all
+// shards have been added into chunk 0
+__global__ void __launch_bounds__(kLanes* kParts) k_finish_faces(const __grid_constant__ StepArgs a,
+                                                                 const __grid_constant__ Consts kc) {
+    __shared__ Finish sm;
+    const int f0 = blockIdx.x * kLanes;
+    finish_faces(sm, a, kc, f0, min(kLanes, a.dm.nF - f0), 1);
+}
+__global__ void __launch_bounds__(kLanes* kParts) k_finish_cells(const __grid_constant__ StepArgs a,
+                                                                 const __grid_constant__ Consts kc) {
+    __shared__ Finish sm;
+    const int c0 = blockIdx.x * kLanes;
+    finish_cells(sm, a, kc, c0, min(kLanes, a.dm.nC - c0), 1);
+}
+
+// ---------------------------------------------------------------------
+// k_face_flux
+// ---------------------------------------------------------------------
+// Reads a face value, relaxes it and writes the flux xi.S g_f in its place:
+// 16 B per (face, DV) and FP64 field, bound by HBM; the face's e_x column
+// is read back through L1 once per row.  FP32 storage keeps the flux of the
+// deviation: the reference's cancels over a closed cell (sum of +-Sf = 0).
+template <int D, typename Real, bool HZ, bool GEN, bool BND>
+__device__ __forceinline__ void face_flux(const StepArgs& a, const double* x1, int f) {
+    const DevMesh& m = a.dm;
+    const int n = m.nF;
+    const size_t nF = static_cast<size_t>(n);
+    Real* fg = reinterpret_cast<Real*>(a.ds.fvg);
+    Real* fh = reinterpret_cast<Real*>(a.ds.fvh);
+    const unsigned fb = sizeof(Real) * f, fr = sizeof(Real) * n;
+    const double S[3] = {__ldg(m.fgeo + f), __ldg(m.fgeo + nF + f), __ldg(m.fgeo + 2 * nF + f)};
+    const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
+    Relax<D, HZ, GEN> rx(a.ds.facerec, a.ds.ftab, n, f, __ldg(a.ds.facerec + REC_R * nF + f));
+    // boundary faces, by patch type.  Outgoing DFs are relaxed, h with the
+    // internal-face T at the patch-local index (fvDVM.C:1367, :1413,
+    // :1429-1444).  Incoming ones are not: wall rho_w M(U_w, T_w)
+    // (fvDVM.C:1079-1092), far field and pressure rho_b M(U_owner, T_b)
+    // (fvDVM.C:926-938) and mixed rho_b M(U_b, T_b); zero-gradient and
+    // symmetry ones are stored.  DVMsymmetry relaxes every DV once more
+    // (fvDVM.C:1445-1453).
+    Incoming in{};
+    bool stored = false, again = false;
+    if constexpr (BND) {
+        const int b = f - m.nIF, pt = __ldg(m.bface_ptype + b);
+        const int li = chk(__ldg(m.bface_patch_local + b), 0, m.nIF, a.ds.err);
+        rx.RTh = m.R * a.ds.fm[static_cast<size_t>(li) * 9 + 4];
+        stored = pt == DUGKS_PATCH_ZERO_GRADIENT || pt == DUGKS_PATCH_SYMMETRY || pt == DUGKS_PATCH_DVM_SYMMETRY;
+        again = pt == DUGKS_PATCH_DVM_SYMMETRY;
+        if (!stored) in = load_incoming(a, b, pt);
+    }
+    const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
+    for (int s = s0; s < s1; ++s) {
+        const Seg q = seg_at<GEN>(m, s);
+        const double Y = x1[q.iy], Z = x1[q.iz];
+        rx.row(m, q, Y, Z);
+        const double p2 = __dmul_rn(Y, S[1]), p3 = D == 3 ? __dmul_rn(Z, S[2]) : 0.0;
+        Real *gs = fg + static_cast<size_t>(q.d0) * nF, *hs = fh + static_cast<size_t>(q.d0) * nF;
+        groups<4>(q.len, [&](int j, auto uc) {
+            constexpr int U = decltype(uc)::value;
+            Real gi[U], hi[U];
+            double e[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                gi[u] = __ldcs(at(row_of(gs, j + u, fr), fb));
+                if (!HZ) hi[u] = __ldcs(at(row_of(hs, j + u, fr), fb));
+                e[u] = rx.factor(j + u);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const Dv v = dv_at<D, GEN>(m, q, x1, j + u);
+                double xs;
+                if constexpr (GEN) xs = xs_dv(v, S);
+                else xs = __dadd_rn(__dadd_rn(__dmul_rn(v.x, S[0]), p2), p3);
+                const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j + u), hr = dv_ref<Real, GEN>(m.href, q.d0 + j + u);
+                double gf = double(gi[u]) + gr, hf = HZ ? 0.0 : double(hi[u]) + hr;
+                if (!BND || xs > 0) {
+                    rx(v, e[u], gf, hf, K3D, c0h, gf, hf);
+                } else if (!stored) {
+                    if constexpr (BND) {
+                        Dv w = v;
+                        if constexpr (!GEN) {
+                            w.y = Y;
+                            w.z = D == 3 ? Z : 0.0;
+                        }
+                        in.at<D>(w, gf, hf);
+                        gf = double(Real(gf - gr)) + gr;
+                        hf = double(Real(hf - hr)) + hr;
+                    }
+                }
+                if (BND && again) rx(v, e[u], gf, hf, K3D, c0h, gf, hf);
+                *at(row_of(gs, j + u, fr), fb) = Real(xs * (gf - gr));
+                if (!HZ) *at(row_of(hs, j + u, fr), fb) = Real(xs * (hf - hr));
+            }
+        });
+    }
+}
+
+template <int D, typename Real, bool HZ, bool GEN>
+__device__ __noinline__ void boundary_flux(const StepArgs& a, const double* x1, int f) {
+    face_flux<D, Real, HZ, GEN, true>(a, x1, f);
+}
+
+template <int D, typename Real, bool HZ, bool GEN>
+__global__ void __launch_bounds__(kStream, 6) k_face_flux(const __grid_constant__ StepArgs a) {
+    const DevMesh& m = a.dm;
+    __shared__ double x1[kMaxN1d], w1[kMaxN1d];
+    load_nodes(m, x1, w1);
+    // boundary face blocks first, as in k_face_moments
+    const int nbB = (m.nBF + kStream - 1) / kStream, bx = blockIdx.x;
+    if (bx < nbB) {
+        const int f = m.nIF + bx * kStream + threadIdx.x;
+        if (f < m.nF) boundary_flux<D, Real, HZ, GEN>(a, x1, f);
+    } else {
+        const int f = (bx - nbB) * kStream + threadIdx.x;
+        if (f < m.nIF) face_flux<D, Real, HZ, GEN, false>(a, x1, f);
+    }
+}
+
+// ---------------------------------------------------------------------
+// k_update
+// ---------------------------------------------------------------------
+// One thread per cell and DV segment: gathers the fluxes of the cell's faces
+// (owner side: outflow, negated), updates g~ in place and sums the cell's
+// moments.  A flux is read by the two cells of its face; the second read hits L2.
+template <int D, typename Real, bool HZ, bool GEN, int NS>
+__global__ void __launch_bounds__(kLanes* kParts, 5) k_update(const __grid_constant__ StepArgs a,
+                                                           const __grid_constant__ Consts kc) {
+    const DevMesh& m = a.dm;
+    __shared__ double x1[kMaxN1d], w1[kMaxN1d];
+    __shared__ Finish sm;
+    load_nodes(m, x1, w1);
+    const int c0 = blockIdx.x * kLanes, count = min(kLanes, m.nC - c0);
+    const int lane = threadIdx.x % kLanes, c = c0 + lane;
+    const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF);
+    const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
+    const int w = warp_id();
+    Sums<GEN> acc(sm);
+    // macroFlux yes with a DV list (fvDVM.C:1562-1611): the cell's rho, rho U,
+    // rho E gain sum_DV w (1, xi, |xi|^2/2 & h/2) times the flux term
+    // dt/V sum_f (+-)(xi.S) g_f of the update
+    double accx[5] = {0, 0, 0, 0, 0};
+    const bool fx = GEN && m.macro_flux;
+    if (lane < count) {
+        Real* g = reinterpret_cast<Real*>(a.ds.g);
+        Real* h = reinterpret_cast<Real*>(a.ds.h);
+        const unsigned cb = sizeof(Real) * c, cr = sizeof(Real) * m.nC, fr = sizeof(Real) * m.nF;
+        const Real* __restrict__ fvg = reinterpret_cast<const Real*>(a.ds.fvg);
+        const Real* __restrict__ fvh = reinterpret_cast<const Real*>(a.ds.fvh);
+        const double dtV = step_dt(a) * __ldg(m.invV + c);
+        const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
+        Relax<D, HZ, GEN> rx(a.ds.cellrec, a.ds.ctab, m.nC, c, cell_r(a, c));
+        // faces with their sign (owner side: outflow, -1); an absent slot
+        // repeats the first face with sign 0
+        unsigned fc[NS];
+        Real sign[NS];
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            const int code = k < m.nf_max ? chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err) : -1;
+            fc[k] = code < 0 ? fc[0] : sizeof(Real) * (code >> 2);
+            sign[k] = code < 0 ? Real(0) : (code & 1) ? Real(1) : Real(-1);
+        }
+        for (int s = s0 + w; s < s1; s += kParts) {
+            const Seg q = seg_at<GEN>(m, s);
+            rx.row(m, q, x1[q.iy], x1[q.iz]);
+            RowSums rs;
+            Real *gs = g + static_cast<size_t>(q.d0) * nC, *hs = h + static_cast<size_t>(q.d0) * nC;
+            const Real *fgs = fvg + static_cast<size_t>(q.d0) * nF, *fhs = fvh + static_cast<size_t>(q.d0) * nF;
+            groups<2>(q.len, [&](int j, auto uc) {
+                constexpr int U = decltype(uc)::value;
+                Real gi[U], hi[U], fg[U][NS], fh[U][NS];
+                double e[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    gi[u] = *at(row_of(gs, j + u, cr), cb);
+                    if (!HZ) hi[u] = *at(row_of(hs, j + u, cr), cb);
+                    e[u] = rx.factor(j + u);
+                    const Real *fgj = row_of(fgs, j + u, fr), *fhj = row_of(fhs, j + u, fr);
+#pragma unroll
+                    for (int k = 0; k < NS; ++k) {
+                        fg[u][k] = __ldg(at(fgj, fc[k]));
+                        if (!HZ) fh[u][k] = __ldg(at(fhj, fc[k]));
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const Dv v = dv_at<D, GEN>(m, q, x1, j + u);
+                    const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j + u), hr = dv_ref<Real, GEN>(m.href, q.d0 + j + u);
                     double gb, hb;
-                    shk_relax<D, double>(cs, x, pe[jj], plus_ref<Real>(double(gt), gr), plus_ref<Real>(double(ht), hr),
-                                         K3D, c0h, gb, hb);
-                    const Real* Fg = sm.Fg + j * kSI;
-                    const Real* Fh = HZ ? nullptr : sm.Fh + j * kSI;
+                    rx(v, e[u], double(gi[u]) + gr, HZ ? 0.0 : double(hi[u]) + hr, K3D, c0h, gb, hb);
+                    // (a product with +-1 is exact: the sum in slot order)
                     Real sg = 0, sh = 0;
 #pragma unroll
-                    for (int s = 0; s < kRegFaces; ++s) {
-                        sg += flip_sign(Fg[ent_off[s]], ent_neg[s]);
-                        if (!HZ) sh += flip_sign(Fh[ent_off[s]], ent_neg[s]);
+                    for (int k = 0; k < NS; ++k) {
+                        sg = fma(sign[k], fg[u][k], sg);
+                        if (!HZ) sh = fma(sign[k], fh[u][k], sh);
                     }
-                    for (int s = kRegFaces; s < m.nf_max; ++s) {
-                        const int e = __ldg(m.cf_item + static_cast<size_t>(s) * nC + c);
-                        if (e != 0) {
-                            const int i = chk((e > 0 ? e : -e) - 1, 0, t.nit, a.ds.err);
-                            sg += e > 0 ? Fg[i] : -Fg[i];
-                            if (!HZ) sh += e > 0 ? Fh[i] : -Fh[i];
+                    if (m.nf_max > NS) {
+                        for (int k = NS; k < m.nf_max; ++k) {
+                            const int code = chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err);
+                            if (code < 0) break;
+                            const int of = (j + u) * m.nF + (code >> 2);
+                            const Real sk = (code & 1) ? Real(1) : Real(-1);
+                            sg = fma(sk, __ldg(fgs + of), sg);
+                            if (!HZ) sh = fma(sk, __ldg(fhs + of), sh);
                         }
                     }
                     // the update in FP64, one rounding to the storage type; with a
                     // reference, -g/3 + 4/3 gbar+ - ref = -(g - ref)/3 + 4/3 (gbar+ - ref)
-                    const Real g_new =
-                        Real(fma(-1.0 / 3, double(gt), fma(4.0 / 3, minus_ref<Real>(gb, gr), double(sg) * dtV)));
-                    const Real h_new =
-                        Real(fma(-1.0 / 3, double(ht), fma(4.0 / 3, minus_ref<Real>(hb, hr), double(sh) * dtV)));
-                    const size_t idx = static_cast<size_t>(bp.d0 + j) * nC + c;
-                    gn[idx] = g_new;
-                    if (!HZ) hn[idx] = h_new;
-                    row_add<HZ>(rs, sm.w1[bp.ix0 + j], x, double(g_new), double(h_new));  // reference part below
+                    const Real gn = Real(fma(-1.0 / 3, double(gi[u]), fma(4.0 / 3, gb - gr, double(sg) * dtV)));
+                    *at(row_of(gs, j + u, cr), cb) = gn;
+                    Real hn = 0;
+                    if (!HZ) {
+                        hn = Real(fma(-1.0 / 3, double(hi[u]), fma(4.0 / 3, hb - hr, double(sh) * dtV)));
+                        *at(row_of(hs, j + u, cr), cb) = hn;
+                    }
+                    add_dv<D, HZ, GEN>(acc, rs, w1, q, v, j + u, double(gn), double(hn));
+                    if constexpr (GEN) {
+                        if (fx) {
+                            const double fgd = double(sg) * dtV, fhd = double(sh) * dtV, aw = v.w * fgd;
+                            accx[0] += aw;
+                            accx[1] += aw * v.x;
+                            accx[2] += aw * v.y;
+                            accx[3] += aw * v.z;
+                            accx[4] += 0.5 * v.w * (fgd * (v.x * v.x + v.y * v.y + v.z * v.z) + fhd);
+                        }
+                    }
                 }
+            });
+            if constexpr (!GEN) row_fold<D>(acc, rs, row_const<D>(x1, w1, q));
+        }
+        if constexpr (sizeof(Real) == 4 && !GEN) {
+            // FP32 storage: the reference's moments once
+            if (blockIdx.y == 0 && threadIdx.x < kLanes)
+                for (int j = 0; j < 14; ++j) acc[j] += __ldg(a.ds.refmom + j);
+        }
+    }
+    if constexpr (GEN) {
+        if (fx) {
+            // the flux term's moments of the chunk, in warp order
+            for (int j = 0; j < 5; ++j) sm.red[w][j][lane] = accx[j];
+            __syncthreads();
+            for (int j = w; j < 5; j += kParts) {
+                double v = sm.red[0][j][lane];
+                for (int p = 1; p < kParts; ++p) v += sm.red[p][j][lane];
+                if (lane < count) a.ds.partX[(static_cast<size_t>(blockIdx.y) * kFX + j) * nC + c] = v;
             }
-            row_fold<D>(acc, rs, q);
-            // the next batch's cell inputs fly during the barrier and stage 3
-            if (k + 1 < nbt) fetch_cells<Real, NB, FULL, HZ>(ahead.pos(), g, h, ctab, nC, c, part, pg, ph, pe);
+            __syncthreads();
         }
     }
-    // the cell moments of a cell are split over kParts0 threads: reduce them
-    // through shared memory in a fixed order
-    __syncthreads();
-    if (part > 0 && has_cell)
-        for (int j = 0; j < 15; ++j) sm.red[((part - 1) * kS0 + lc) * 15 + j] = acc[j];
-    __syncthreads();
-    if (part == 0 && has_cell) {
-        for (int p = 1; p < kParts0; ++p)
-            for (int j = 0; j < 15; ++j) acc[j] += sm.red[((p - 1) * kS0 + lc) * 15 + j];
-        if constexpr (sizeof(Real) == 4) {
-            // FP32 storage: the reference's moments over this chunk's DVs
-            const double* rm = a.ds.refmom + static_cast<size_t>(blockIdx.y) * kNM;
-            for (int j = 0; j < 14; ++j) acc[j] += __ldg(rm + j);
-        }
-        double* dst = a.ds.partC + (static_cast<size_t>(blockIdx.y) * m.nC + c) * kNM;
-#pragma unroll
-        for (int j = 0; j < 15; ++j) dst[j] = acc[j];
-    }
+    acc.put(sm);
+    if (reduce_chunk(sm, a.ds.partC, nC, c0, count, a.ds.done + m.done_cells + blockIdx.x, a.fused != 0))
+        finish_cells(sm, a, kc, c0, count, gridDim.y);
 }
 
-#include "dugks_passes_gen.cuh"
+// raw cell moments of the current state (set_state), as k_update sums them
+template <int D, typename Real, bool GEN>
+__global__ void __launch_bounds__(kLanes* kParts) k_state_moments(const __grid_constant__ StepArgs a,
+                                                                  const __grid_constant__ Consts kc) {
+    const DevMesh& m = a.dm;
+    __shared__ double x1[kMaxN1d], w1[kMaxN1d];
+    __shared__ Finish sm;
+    load_nodes(m, x1, w1);
+    const int c0 = blockIdx.x * kLanes, count = min(kLanes, m.nC - c0);
+    const int lane = threadIdx.x % kLanes, c = c0 + lane;
+    const size_t nC = static_cast<size_t>(m.nC);
+    const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
+    const int w = warp_id();
+    Sums<GEN> acc(sm);
+    if (lane < count) {
+        const Real* __restrict__ g = reinterpret_cast<const Real*>(a.ds.g) + c;
+        const Real* __restrict__ h = reinterpret_cast<const Real*>(a.ds.h) + c;
+        for (int s = s0 + w; s < s1; s += kParts) {
+            const Seg q = seg_at<GEN>(m, s);
+            RowSums rs;
+#pragma unroll 4
+            for (int j = 0; j < q.len; ++j) {
+                const size_t o = static_cast<size_t>(q.d0 + j) * nC;
+                const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j), hr = dv_ref<Real, GEN>(m.href, q.d0 + j);
+                add_dv<D, false, GEN>(acc, rs, w1, q, dv_at<D, GEN>(m, q, x1, j), j, double(__ldg(g + o)) + gr,
+                                      double(__ldg(h + o)) + hr);
+            }
+            if constexpr (!GEN) row_fold<D>(acc, rs, row_const<D>(x1, w1, q));
+        }
+    }
+    acc.put(sm);
+    if (reduce_chunk(sm, a.ds.partC, nC, c0, count, a.ds.done + m.done_cells + blockIdx.x, a.fused != 0))
+        finish_cells(sm, a, kc, c0, count, gridDim.y);
+}
 
-template <typename K>
-cudaError_t set_smem(K* kernel, size_t bytes);
+int blocks(int n, int per) { return (n + per - 1) / per; }
 
-// ---------------------------------------------------------------------
-// launch plumbing
-// ---------------------------------------------------------------------
-constexpr int kNbGen = 8;   // DVs per batch of the general-DV passes
+// CTAs along the DV segments for the kernels without a reduction: about
+// eight CTAs of 128 threads on each of 148 SMs, four times over, so that the
+// last wave is short
+int stream_chunks(const DevMesh& m, int nb) {
+    const int target = 148 * 8 * 4;
+    return std::max(1, std::min({m.n_seg, (target + nb - 1) / std::max(nb, 1), 65535}));
+}
 
-template <int D, typename Real>
-cudaError_t launch_gen(const StepArgs& a, bool pass_b, cudaStream_t s) {
-    const dim3 grid(a.dm.n_tiles, a.chunks);
-    if (!pass_b) k_pass_a_gen<D, Real, kNbGen><<<grid, kThreads, a.smemA, s>>>(a);
-    else k_pass_b_gen<D, Real, kNbGen><<<grid, kThreads, a.smemB, s>>>(a);
+template <int D, typename Real, bool HZ, bool GEN>
+cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
+    const DevMesh& m = a.dm;
+    const Consts k = make_consts(m, a.dt);
+    const int nbI = blocks(m.nIF, kLanes), nbB = blocks(m.nBF, kLanes);
+    const bool quad = m.nb_max <= 4 && m.nf_max <= 4;   // quadrilaterals, tetrahedra: shorter face lists
+    switch (which) {
+        case KERNEL_HALF_STEP: {
+            const int nb = blocks(m.nC, kStream);
+            k_half_step<D, Real, HZ, GEN><<<dim3(nb, stream_chunks(m, nb)), kStream, 0, s>>>(a);
+            break;
+        }
+        case KERNEL_FACE_VALUES: {
+            const int nb = blocks(m.nC, kCells);
+            const dim3 grid(nb, stream_chunks(m, nb));
+            if (quad) k_face_values<D, Real, HZ, GEN, 4><<<grid, kCells, 0, s>>>(a);
+            else k_face_values<D, Real, HZ, GEN, kFast><<<grid, kCells, 0, s>>>(a);
+            break;
+        }
+        case KERNEL_FACE_MOMENTS:
+            k_face_moments<D, Real, HZ, GEN><<<dim3(nbI + nbB, a.chunks_f), kLanes * kParts, 0, s>>>(a, k);
+            break;
+        case KERNEL_FACE_FLUX: {
+            const int nb = blocks(m.nIF, kStream) + blocks(m.nBF, kStream);
+            k_face_flux<D, Real, HZ, GEN><<<dim3(nb, stream_chunks(m, nb)), kStream, 0, s>>>(a);
+            break;
+        }
+        case KERNEL_UPDATE: {
+            const dim3 grid(blocks(m.nC, kLanes), a.chunks);
+            if (quad) k_update<D, Real, HZ, GEN, 4><<<grid, kLanes * kParts, 0, s>>>(a, k);
+            else k_update<D, Real, HZ, GEN, kFast><<<grid, kLanes * kParts, 0, s>>>(a, k);
+            break;
+        }
+        case KERNEL_STATE_MOMENTS:
+            k_state_moments<D, Real, GEN><<<dim3(blocks(m.nC, kLanes), a.chunks), kLanes * kParts, 0, s>>>(a, k);
+            break;
+        default:
+            return cudaErrorInvalidValue;
+    }
     return cudaGetLastError();
 }
 
 template <int D, typename Real>
-cudaError_t configure_gen(const StepArgs& a) {
-    cudaError_t e = set_smem(k_pass_a_gen<D, Real, kNbGen>, a.smemA);
-    return e != cudaSuccess ? e : set_smem(k_pass_b_gen<D, Real, kNbGen>, a.smemB);
-}
-template <int D, typename Real, int NA, int NBB, bool HZ>
-cudaError_t launch_nb_h(const StepArgs& a, bool pass_b, cudaStream_t s) {
-    const dim3 grid(a.dm.n_tiles, a.chunks);
-    if constexpr (HZ) {
-        if (!pass_b && a.wideA16) {
-            k_pass_a<D, Real, 16, true, true><<<grid, kThreads, a.smemA, s>>>(a);
-            return cudaGetLastError();
-        }
-        if constexpr (sizeof(Real) == 4) {
-            if (pass_b && a.wideB16) {
-                k_pass_b<D, Real, 16, true, true><<<grid, kThreads, a.smemB, s>>>(a);
-                return cudaGetLastError();
-            }
-        }
-        if constexpr (sizeof(Real) == 4) {
-            // FP32 storage, 20 nodes per dimension: a whole row per batch
-            if (a.row20) {
-                if (!pass_b) k_pass_a<D, Real, 20, true, true><<<grid, kThreads, a.smemA, s>>>(a);
-                else k_pass_b<D, Real, 20, true, true><<<grid, kThreads, a.smemB, s>>>(a);
-                return cudaGetLastError();
-            }
-        }
-        // 20 nodes per dimension: two batches of 10 per row (guarded: 10 DVs
-        // do not split evenly over the threads of a cell)
-        if (a.row10) {
-            if (!pass_b) k_pass_a<D, Real, 10, false, true><<<grid, kThreads, a.smemA, s>>>(a);
-            else k_pass_b<D, Real, 10, false, true><<<grid, kThreads, a.smemB, s>>>(a);
-            return cudaGetLastError();
-        }
-    }
-    if (!pass_b) {
-        if (a.fullA) k_pass_a<D, Real, NA, true, HZ><<<grid, kThreads, a.smemA, s>>>(a);
-        else k_pass_a<D, Real, NA, false, HZ><<<grid, kThreads, a.smemA, s>>>(a);
-    } else {
-        if (a.fullB) k_pass_b<D, Real, NBB, true, HZ><<<grid, kThreads, a.smemB, s>>>(a);
-        else k_pass_b<D, Real, NBB, false, HZ><<<grid, kThreads, a.smemB, s>>>(a);
-    }
-    return cudaGetLastError();
-}
-
-// h identically zero (StepArgs::hzero) exists in 3-D only
-template <int D, typename Real, int NA, int NBB>
-cudaError_t launch_nb(const StepArgs& a, bool pass_b, cudaStream_t s) {
+cudaError_t launch_d(const StepArgs& a, int which, cudaStream_t s) {
+    if (a.dm.general_dv) return launch_kernel<D, Real, false, true>(a, which, s);
     if constexpr (D == 3) {
-        if (a.hzero) return launch_nb_h<D, Real, NA, NBB, true>(a, pass_b, s);
+        if (a.hzero) return launch_kernel<D, Real, true, false>(a, which, s);
     }
-    return launch_nb_h<D, Real, NA, NBB, false>(a, pass_b, s);
+    return launch_kernel<D, Real, false, false>(a, which, s);
 }
-
-template <int D, typename Real>
-cudaError_t launch_pass_d(const StepArgs& a, bool pass_b, cudaStream_t s) {
-    using W = Width<Real>;
-    if (!pass_b) return a.wideA ? launch_nb<D, Real, W::A1, W::B0>(a, false, s) : launch_nb<D, Real, W::A0, W::B0>(a, false, s);
-    return a.wideB ? launch_nb<D, Real, W::A0, W::B1>(a, true, s) : launch_nb<D, Real, W::A0, W::B0>(a, true, s);
-}
-
-template <int D, typename Real>
-void smem_d(bool wideA, bool wideB, size_t* smemA, size_t* smemB) {
-    *smemA = wideA ? SmemA<D, Real, Width<Real>::A1>::bytes() : SmemA<D, Real, Width<Real>::A0>::bytes();
-    *smemB = wideB ? SmemB<Real, Width<Real>::B1>::bytes() : SmemB<Real, Width<Real>::B0>::bytes();
-}
-
-template <typename K>
-cudaError_t set_smem(K* kernel, size_t bytes) {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-}
-
-template <int D, typename Real, int NA, int NBB, bool HZ>
-cudaError_t configure_nb_h(const StepArgs& a, bool pass_b) {
-    if (!pass_b)
-        return a.fullA ? set_smem(k_pass_a<D, Real, NA, true, HZ>, a.smemA)
-                       : set_smem(k_pass_a<D, Real, NA, false, HZ>, a.smemA);
-    return a.fullB ? set_smem(k_pass_b<D, Real, NBB, true, HZ>, a.smemB)
-                   : set_smem(k_pass_b<D, Real, NBB, false, HZ>, a.smemB);
-}
-
-template <int D, typename Real, int NA, int NBB>
-cudaError_t configure_nb(const StepArgs& a, bool pass_b) {
-    cudaError_t e = configure_nb_h<D, Real, NA, NBB, false>(a, pass_b);
-    if constexpr (D == 3) {
-        if (e == cudaSuccess) e = configure_nb_h<D, Real, NA, NBB, true>(a, pass_b);
-        if (e == cudaSuccess && !pass_b)
-            e = set_smem(k_pass_a<D, Real, 16, true, true>, SmemA<D, Real, 16, true>::bytes());
-        if (e == cudaSuccess)
-            e = pass_b ? set_smem(k_pass_b<D, Real, 10, false, true>, SmemB<Real, 10, true>::bytes())
-                       : set_smem(k_pass_a<D, Real, 10, false, true>, SmemA<D, Real, 10, true>::bytes());
-        if constexpr (sizeof(Real) == 4) {
-            if (e == cudaSuccess && pass_b)
-                e = set_smem(k_pass_b<D, Real, 16, true, true>, SmemB<Real, 16, true>::bytes());
-            if (e == cudaSuccess)
-                e = pass_b ? set_smem(k_pass_b<D, Real, 20, true, true>, SmemB<Real, 20, true>::bytes())
-                           : set_smem(k_pass_a<D, Real, 20, true, true>, SmemA<D, Real, 20, true>::bytes());
-        }
-    }
-    return e;
-}
-
-template <int D, typename Real>
-cudaError_t configure_d(const StepArgs& a) {
-    using W = Width<Real>;
-    cudaError_t e = a.wideA ? configure_nb<D, Real, W::A1, W::B0>(a, false) : configure_nb<D, Real, W::A0, W::B0>(a, false);
-    if (e != cudaSuccess) return e;
-    return a.wideB ? configure_nb<D, Real, W::A0, W::B1>(a, true) : configure_nb<D, Real, W::A0, W::B0>(a, true);
-}
-
-// padding of the last batch of a row of n1d DVs at width nb
-int row_waste(int n1d, int nb) { return (n1d + nb - 1) / nb * nb - n1d; }
 
 }  // namespace
 
-// every launched layout fits the 227 KB of shared memory a B200 CTA may
-// opt into (cudaFuncAttributeMaxDynamicSharedMemorySize)
-constexpr size_t kSmemMax = 232448;
-template <int D, typename Real>
-constexpr bool fits_d() {
-    return SmemA<D, Real, 8>::bytes() <= kSmemMax && SmemA<D, Real, 8, true>::bytes() <= kSmemMax &&
-           SmemB<Real, 8>::bytes() <= kSmemMax && SmemB<Real, 8, true>::bytes() <= kSmemMax &&
-           SmemA<3, Real, 16, true>::bytes() <= kSmemMax && SmemA<3, Real, 10, true>::bytes() <= kSmemMax &&
-           SmemB<Real, 10, true>::bytes() <= kSmemMax && SmemAG<D, Real, kNbGen>::bytes() <= kSmemMax &&
-           SmemBG<Real, kNbGen>::bytes() <= kSmemMax;
-}
-static_assert(fits_d<2, double>() && fits_d<3, double>() && fits_d<2, float>() && fits_d<3, float>(),
-              "a pass layout exceeds the shared memory of a CTA");
-static_assert(SmemB<float, 16, true>::bytes() <= kSmemMax && SmemA<3, float, 20, true>::bytes() <= kSmemMax &&
-                  SmemB<float, 20, true>::bytes() <= kSmemMax,
-              "a wide FP32 pass layout exceeds the shared memory of a CTA");
-
-cudaError_t launch_pass(const StepArgs& a, int precision, bool pass_b, cudaStream_t s) {
-    if (a.dm.general_dv) {
-        if (precision == DUGKS_FP64)
-            return a.dm.D == 3 ? launch_gen<3, double>(a, pass_b, s) : launch_gen<2, double>(a, pass_b, s);
-        return a.dm.D == 3 ? launch_gen<3, float>(a, pass_b, s) : launch_gen<2, float>(a, pass_b, s);
-    }
-    if (precision == DUGKS_FP64)
-        return a.dm.D == 3 ? launch_pass_d<3, double>(a, pass_b, s) : launch_pass_d<2, double>(a, pass_b, s);
-    return a.dm.D == 3 ? launch_pass_d<3, float>(a, pass_b, s) : launch_pass_d<2, float>(a, pass_b, s);
+cudaError_t launch_pass(const StepArgs& a, int precision, int which, cudaStream_t s) {
+    if (precision == DUGKS_FP64) return a.dm.D == 3 ? launch_d<3, double>(a, which, s) : launch_d<2, double>(a, which, s);
+    return a.dm.D == 3 ? launch_d<3, float>(a, which, s) : launch_d<2, float>(a, which, s);
 }
 
-void pass_config(int D, int precision, int n1d, StepArgs* a) {
-    const bool f64 = precision == DUGKS_FP64;
-    if (a->dm.general_dv) {
-        a->wideA = a->wideB = a->fullA = a->fullB = 0;
-        if (f64) {
-            a->smemA = D == 3 ? SmemAG<3, double, kNbGen>::bytes() : SmemAG<2, double, kNbGen>::bytes();
-            a->smemB = SmemBG<double, kNbGen>::bytes();
-        } else {
-            a->smemA = D == 3 ? SmemAG<3, float, kNbGen>::bytes() : SmemAG<2, float, kNbGen>::bytes();
-            a->smemB = SmemBG<float, kNbGen>::bytes();
-        }
-        return;
-    }
-    const int a0 = f64 ? Width<double>::A0 : Width<float>::A0, a1 = f64 ? Width<double>::A1 : Width<float>::A1;
-    const int b0 = f64 ? Width<double>::B0 : Width<float>::B0, b1 = f64 ? Width<double>::B1 : Width<float>::B1;
-    // the wide batch unless it pads the rows more than the narrow one;
-    // rows that split into whole batches take the unguarded kernels
-    a->wideA = row_waste(n1d, a1) <= row_waste(n1d, a0) ? 1 : 0;
-    a->wideB = row_waste(n1d, b1) <= row_waste(n1d, b0) ? 1 : 0;
-    a->fullA = row_waste(n1d, a->wideA ? a1 : a0) == 0 ? 1 : 0;
-    a->fullB = row_waste(n1d, a->wideB ? b1 : b0) == 0 ? 1 : 0;
-    if (f64) {
-        if (D == 3) smem_d<3, double>(a->wideA, a->wideB, &a->smemA, &a->smemB);
-        else smem_d<2, double>(a->wideA, a->wideB, &a->smemA, &a->smemB);
+cudaError_t launch_finish(const StepArgs& a, bool faces, cudaStream_t s) {
+    const Consts k = make_consts(a.dm, a.dt);
+    if (faces) k_finish_faces<<<blocks(a.dm.nF, kLanes), kLanes * kParts, 0, s>>>(a, k);
+    else k_finish_cells<<<blocks(a.dm.nC, kLanes), kLanes * kParts, 0, s>>>(a, k);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_cell_records(const StepArgs& a, cudaStream_t s) {
+    k_cell_records<<<blocks(a.dm.nC, kLanes), kLanes * kParts, 0, s>>>(a, make_consts(a.dm, a.dt));
+    return cudaGetLastError();
+}
+
+cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, cudaStream_t s) {
+    const int nb = blocks(m.nF, 128);
+    const dim3 grid(nb, std::min(m.n_seg, std::max(1, 148 * 32 / std::max(nb, 1))));
+    if (m.general_dv) {
+        if (m.D == 3) k_upwind_bits<3, true><<<grid, 128, 0, s>>>(m, upw);
+        else k_upwind_bits<2, true><<<grid, 128, 0, s>>>(m, upw);
     } else {
-        if (D == 3) smem_d<3, float>(a->wideA, a->wideB, &a->smemA, &a->smemB);
-        else smem_d<2, float>(a->wideA, a->wideB, &a->smemA, &a->smemB);
+        if (m.D == 3) k_upwind_bits<3, false><<<grid, 128, 0, s>>>(m, upw);
+        else k_upwind_bits<2, false><<<grid, 128, 0, s>>>(m, upw);
     }
-    // the g-only instantiations' own sizes (no h arrays; pass B keeps its
-    // items' e_x table resident in part of that room)
-    if (D == 3 && a->hzero) {
-        using WD = Width<double>;
-        using WF = Width<float>;
-        if (f64) {
-            a->smemA = a->wideA ? SmemA<3, double, WD::A1, true>::bytes() : SmemA<3, double, WD::A0, true>::bytes();
-            a->smemB = a->wideB ? SmemB<double, WD::B1, true>::bytes() : SmemB<double, WD::B0, true>::bytes();
-        } else {
-            a->smemA = a->wideA ? SmemA<3, float, WF::A1, true>::bytes() : SmemA<3, float, WF::A0, true>::bytes();
-            a->smemB = a->wideB ? SmemB<float, WF::B1, true>::bytes() : SmemB<float, WF::B0, true>::bytes();
-        }
-    }
-    // g-only pass A in batches of 16 DVs (a whole row) for 16 nodes per
-    // dimension: half the per-batch work and barriers per DV, and the
-    // shared memory the h arrays would take holds the wider batch
-    a->wideA16 = a->wideB16 = a->row10 = a->row20 = 0;
-    if (D == 3 && a->hzero && n1d == 20) {
-        if (f64) {
-            // both passes in batches of 10 DVs: two per row instead of 8 + 8 + 4
-            a->row10 = 1;
-            a->smemA = SmemA<3, double, 10, true>::bytes();
-            a->smemB = SmemB<double, 10, true>::bytes();
-        } else {
-            // FP32 storage: a whole row per batch (the 20-wide FP64 staging
-            // does not fit in shared memory)
-            a->row20 = 1;
-            a->smemA = SmemA<3, float, 20, true>::bytes();
-            a->smemB = SmemB<float, 20, true>::bytes();
-        }
-    }
-    if (D == 3 && a->hzero && n1d == 16) {
-        a->wideA16 = 1;
-        a->smemA = f64 ? SmemA<3, double, 16, true>::bytes() : SmemA<3, float, 16, true>::bytes();
-        // pass B likewise with FP32 storage (in FP64 the 16-wide staging does
-        // not fit in shared memory)
-        if (!f64) {
-            a->wideB16 = 1;
-            a->smemB = SmemB<float, 16, true>::bytes();
-        }
-    }
-}
-
-cudaError_t configure_kernels(int precision, const StepArgs& a) {
-    if (a.dm.general_dv) {
-        if (precision == DUGKS_FP64) return a.dm.D == 3 ? configure_gen<3, double>(a) : configure_gen<2, double>(a);
-        return a.dm.D == 3 ? configure_gen<3, float>(a) : configure_gen<2, float>(a);
-    }
-    if (precision == DUGKS_FP64) return a.dm.D == 3 ? configure_d<3, double>(a) : configure_d<2, double>(a);
-    return a.dm.D == 3 ? configure_d<3, float>(a) : configure_d<2, float>(a);
+    return cudaGetLastError();
 }
 
 }  // namespace dugks
