@@ -813,7 +813,7 @@ __device__ __forceinline__ void macro_flux_update(const StepArgs& a, const Const
     rE = rho * (0.5 * (U0[0] * U0[0] + U0[1] * U0[1] + U0[2] * U0[2]) + (k.Kin + 3) / 2.0 * k.R * cm[4]);
     const double V = __ldg(m.mf_V + c), dt = k.dt;
     for (int e = __ldg(m.mf_off + c); e < __ldg(m.mf_off + c + 1); ++e) {
-        const int code = __ldg(m.mf_ent + e), f = chk(code >> 2, 0, m.nIF + m.nBF, a.ds.err);
+        const int code = __ldg(m.mf_ent + e), f = chk(code >> 1, 0, m.nIF + m.nBF, a.ds.err);
         const bool add = code & 1;
         const double* fm = a.ds.fm + static_cast<size_t>(f) * 9;
         const double rf = fm[0], Uf[3] = {fm[1], fm[2], fm[3]}, qf[3] = {fm[5], fm[6], fm[7]};
