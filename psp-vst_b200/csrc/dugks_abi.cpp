@@ -148,7 +148,7 @@ static bool can_skip_h(const dugks_handle* h) { return h->D == 3 && h->gas.K_inn
 static int alloc_h(dugks_handle* h) {
     if (h->ds.hbar) return DUGKS_OK;
     const size_t rs = real_size(h);
-    const size_t nvc = static_cast<size_t>(h->dm.nv_loc) * h->nC, nfv = static_cast<size_t>(h->dm.nv_loc) * h->dm.nF;
+    const size_t nvc = static_cast<size_t>(h->dm.nv_loc) * h->nC, nfv = static_cast<size_t>(h->dm.nv_loc) * h->dm.pF;
     unsigned char *b = nullptr, *f = nullptr;
     if (int st = dev_alloc(h, &b, nvc * rs)) return st;
     if (int st = dev_alloc(h, &f, nfv * rs)) return st;
@@ -375,8 +375,13 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         const int nb = (entities + 31) / 32, want = (148 * 4 * 3 + nb - 1) / nb;
         return opt.dv_chunks > 0 ? std::min(opt.dv_chunks, n_seg) : std::max(1, std::min(want, n_seg / 4));
     };
+    // (the face reduction: one thread per internal face)
+    auto chunks_f_for = [&](int entities) {
+        const int nb = (entities + 127) / 128, want = (148 * 5 * 4 + nb - 1) / nb;
+        return opt.dv_chunks > 0 ? std::min(opt.dv_chunks, n_seg) : std::max(1, std::min(want, n_seg));
+    };
     h->chunks = chunks_for(nC);
-    h->chunks_f = chunks_for(nF);
+    h->chunks_f = chunks_f_for(nF);
 
     // ---- device layout ----
     const dugks::Tiling& t = h->tiling;
@@ -399,6 +404,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dm.n1d = h->n1d;
     dm.general_dv = dvl ? 1 : 0;
     dm.nF = nF;
+    dm.pF = (nF + 31) / 32 * 32;
     dm.n_seg = n_seg;
     dm.xi_max_co = std::sqrt(static_cast<double>(h->D)) * h->xi_max;
     int st;
@@ -409,6 +415,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     double *d_xi, *d_w, *d_nls, *d_invV, *d_dc, *d_bS, *d_geo;
     int32_t *d_nbr, *d_cf, *d_fo, *d_fn, *d_for, *d_bpl, *d_bpt, *d_bown, *d_bmir;
     uint32_t* d_upw = nullptr;
+    unsigned long long* d_count = nullptr;
     int2* d_row_yz;
     std::vector<int2> row_yz(dvl ? 1 : rows_loc);
     for (size_t r = 0; r < row_yz.size(); ++r) {
@@ -439,7 +446,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         (st = upload(h, &d_invV, invV)) || (st = upload(h, &d_bpl, h->bface_patch_local)) ||
         (st = upload(h, &d_bpt, h->bface_ptype)) || (st = upload(h, &d_bown, bown)) || (st = upload(h, &d_dc, h->dc)) ||
         (st = upload(h, &d_bS, bS)) || (st = upload(h, &d_bmir, h->bface_mirror)) ||
-        (st = dev_alloc(h, &d_upw, 2 * static_cast<size_t>(n_seg) * nF))) {
+        (st = dev_alloc(h, &d_upw, 2 * static_cast<size_t>(n_seg) * nF)) || (st = dev_alloc(h, &d_count, 2))) {
         *out = h;
         return st;
     }
@@ -459,6 +466,8 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dm.fnei = d_fn;
     dm.forig = d_for;
     dm.upw = d_upw;
+    dm.tang = nullptr;
+    dm.n_tang = 0;
     dm.bface_patch_local = d_bpl;
     dm.bface_ptype = d_bpt;
     dm.bface_owner = d_bown;
@@ -507,7 +516,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dugks::DevState& ds = h->ds;
     const size_t rs = real_size(h);
     const size_t nvc = static_cast<size_t>(dm.nv_loc) * nC;
-    const size_t nfv = static_cast<size_t>(dm.nv_loc) * std::max(nF, 1);
+    const size_t nfv = static_cast<size_t>(dm.nv_loc) * dm.pF;
     unsigned char* p;
     // One state buffer: the update runs in place, as k_update reads each
     // (DV, cell) entry once and then writes it and no kernel of a step reads
@@ -526,7 +535,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     // where h stays identically zero its step arrays are left out until a
     // nonzero h~ is loaded (alloc_h)
     if (!can_skip_h(h) && (st = alloc_h(h))) return *out = h, st;
-    const int nbl = (nIF + 31) / 32 + (nBF + 31) / 32;
+    const int nbl = (nIF + 127) / 128 + (nBF + 31) / 32;
     dm.done_cells = nbl;
     const size_t n_done = static_cast<size_t>(nbl) + (nC + 31) / 32;
     if ((st = dev_alloc(h, &ds.partF, static_cast<size_t>(h->chunks_f) * nF * dugks::kNM)) ||
@@ -538,7 +547,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         (st = dev_alloc(h, &ds.cellrec, static_cast<size_t>(dugks::REC_N) * nC)) ||
         (st = dev_alloc(h, &ds.facerec, static_cast<size_t>(dugks::REC_N) * nF)) ||
         (st = dev_alloc(h, &ds.ctab, static_cast<size_t>(h->D) * h->n1d * nC)) ||
-        (st = dev_alloc(h, &ds.ftab, static_cast<size_t>(h->D) * h->n1d * nF)) ||
+        (st = dev_alloc(h, &ds.ftab, static_cast<size_t>(h->D) * h->n1d * dm.pF)) ||
         (st = dev_alloc(h, &ds.brec, nBF)) || (st = dev_alloc(h, &ds.bmom_in, static_cast<size_t>(nBF) * dugks::kNM)) ||
         (st = dev_alloc(h, &ds.cm, static_cast<size_t>(nC) * 9)) ||
         (st = dev_alloc(h, &ds.fm, static_cast<size_t>(nF) * 9)) || (st = dev_alloc(h, &ds.co, 2)) ||
@@ -563,8 +572,22 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, cudaGetErrorString(ce));
     ce = cudaMemset(ds.done, 0, n_done * sizeof(int));
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, cudaGetErrorString(ce));
-    ce = dugks::launch_upwind_bits(dm, d_upw, h->stream);
+    ce = dugks::configure_kernels(h->D, h->precision);
+    if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, std::string("configure kernels: ") + cudaGetErrorString(ce));
+    unsigned long long n_tang = 0;
+    ce = cudaMemsetAsync(d_count, 0, 2 * sizeof(unsigned long long), h->stream);
+    if (ce == cudaSuccess) ce = dugks::launch_upwind_bits(dm, d_upw, d_count, h->stream);
+    if (ce == cudaSuccess)
+        ce = cudaMemcpyAsync(&n_tang, d_count, sizeof n_tang, cudaMemcpyDeviceToHost, h->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);
+    if (ce == cudaSuccess && n_tang > 0) {
+        int2* d_tang = nullptr;
+        if ((st = dev_alloc(h, &d_tang, n_tang))) return *out = h, st;
+        ce = dugks::launch_list_tangential(dm, d_tang, d_count + 1, h->stream);
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);
+        dm.tang = d_tang;
+        dm.n_tang = static_cast<long long>(n_tang);
+    }
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, std::string("upwind bits: ") + cudaGetErrorString(ce));
     if (shard && shard->use_nccl) {
         // collective: every rank of the shard set makes this call

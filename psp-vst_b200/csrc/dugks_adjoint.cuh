@@ -63,7 +63,7 @@ enum {
 enum { CO_AL = 0, CO_BE = 1, CO_GA = 4, CO_AQ = 5, CO_U = 8 };
 
 struct View {
-    int nC, nIF, nBF, nF, nv, D, K, nchF, nchC;
+    int nC, nIF, nBF, nF, pF, nv, D, K, nchF, nchC;   // pF: pitch of the face rows
     double R, Pr, omega, Tref, mu, dt;
     // mesh (cells and faces in the handle's numbering; faces internal then boundary)
     const int32_t* own;     // [nF]
@@ -94,7 +94,7 @@ struct View {
     // forward record of the step: the handle's face-value buffers, faces in
     // the order of the step's arrays, and the raw moments k_face_moments sums
     // of them ([nchM][16][nF]) with the incoming wall DFs' per unit rho_w
-    double* fg;             // [nv][nF] face values before the relaxation
+    double* fg;             // [nv][pF] face values before the relaxation
     double* fh;
     const double* fmom;
     int nchM;
@@ -110,7 +110,7 @@ struct View {
     const double* lh;
     double* og;             // [nv][nC] adjoint of the state before the step (output)
     double* oh;
-    double* ag;             // [nv][nF] adjoint of the face values before the relaxation
+    double* ag;             // [nv][pF] adjoint of the face values before the relaxation
     double* ah;
     double* aGg;            // [3][nv][nC] adjoint of the gradients
     double* aGh;
@@ -448,8 +448,8 @@ struct FIncoming {
         const double Tb = v.bT[b];
         const double gi = wall ? v.rhow[b] * eq_by_rho(v, xi, v.bU + 3 * b, Tb)
                                : v.brho[b] * eq_by_rho(v, xi, v.cm + 9 * static_cast<size_t>(v.own[f]) + 1, Tb);
-        v.fg[at(i, v.nF, f)] = gi;
-        v.fh[at(i, v.nF, f)] = gi * (v.R * Tb) * static_cast<double>(v.K + 3 - v.D);
+        v.fg[at(i, v.pF, f)] = gi;
+        v.fh[at(i, v.pF, f)] = gi * (v.R * Tb) * static_cast<double>(v.K + 3 - v.D);
     }
 };
 
@@ -482,7 +482,7 @@ struct FCellMac {
 ADJ_HD bool relaxed_value(const View& v, int i, int f, double& gr, double& hr, double& gEq, double& hEq,
                           double& r) {
     const double* xi = v.xi + 3 * i;
-    const size_t id = at(i, v.nF, f);
+    const size_t id = at(i, v.pF, f);
     gr = v.fg[id];
     hr = v.fh[id];
     if (f >= v.nIF && !(xs_of(xi, v.S + 3 * f) > 0)) return false;
@@ -569,7 +569,7 @@ struct RRelax {
         for (int i = chunk_lo(v.nv, v.nchF, ch); i < chunk_lo(v.nv, v.nchF, ch + 1); ++i) {
             const double* xi = v.xi + 3 * i;
             const double xs = xs_of(xi, S);
-            const size_t id = at(i, v.nF, f);
+            const size_t id = at(i, v.pF, f);
             const double lgo = ro(v.lg + at(i, v.nC, ow)), lho = ro(v.lh + at(i, v.nC, ow));
             const double lgn = ro(v.lg + at(i, v.nC, ne)), lhn = ro(v.lh + at(i, v.nC, ne));
             const double pg = ro(v.fg + id), ph = ro(v.fh + id);
@@ -648,7 +648,7 @@ struct RFaceMom {
         double s[5] = {0, 0, 0, 0, 0};
         for (int i = chunk_lo(v.nv, v.nchF, ch); i < chunk_lo(v.nv, v.nchF, ch + 1); ++i) {
             const double* xi = v.xi + 3 * i;
-            const size_t id = at(i, v.nF, f);
+            const size_t id = at(i, v.pF, f);
             double a_g, a_h;
             moment_adjoint(co, xi, v.w[i], a_g, a_h);
             a_g += v.ag[id];
@@ -708,7 +708,7 @@ struct RWallOut {
         if (v.btype[b] != 1) return;
         const int f = v.nIF + b;
         const double xs = xs_of(v.xi + 3 * i, v.S + 3 * f);
-        if (xs > 0) v.ag[at(i, v.nF, f)] += v.aout[b] * v.w[i] * xs;
+        if (xs > 0) v.ag[at(i, v.pF, f)] += v.aout[b] * v.w[i] * xs;
     }
 };
 
@@ -732,7 +732,7 @@ struct RGradAdj {
             else if (xs < -kVSmall) share = is_nei ? 1.0 : 0.0;
             else share = 0.5;
             if (share == 0.0) continue;
-            const size_t id = at(i, v.nF, f);
+            const size_t id = at(i, v.pF, f);
             const double a_g = share * v.ag[id], a_h = share * v.ah[id];
             double d[3];
             recon_vec(v, f, c, xi, d);

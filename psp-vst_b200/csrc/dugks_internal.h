@@ -64,6 +64,7 @@ struct DevMesh {
     int D, K;
     double R, Pr, omega, Tref, muRef;
     int nC, nIF, nBF, nF, nv;
+    int pF;                // pitch of the face-value rows and of ftab: nF padded to a multiple of 32
     // DVs this device holds: global DVs dv_base .. dv_base + nv_loc - 1, the
     // DV rows row_base ..; the state and face-value arrays are [nv_loc][..]
     int nv_loc, dv_base, row_base;
@@ -93,6 +94,8 @@ struct DevMesh {
     const int32_t* fnei;           // [nIF] neighbour cell
     const int32_t* forig;          // [nF] the caller's face
     const uint32_t* upw;           // [n_seg][nF][2] upwind bits of a segment's DVs: owner side, neighbour side
+    const int2* tang;              // [n_tang] exactly tangential pairs: internal face, segment * kSeg + DV in it
+    long long n_tang;
     int done_cells;                // first cell-block counter in DevState::done (face blocks before it)
     const int32_t* bface_patch_local;  // [nBF] index within its patch
     const int32_t* bface_ptype;    // [nBF]
@@ -123,7 +126,7 @@ struct DevState {
     void* h;
     void* gbar;        // gbar+ of the step [nv][nC] (Real)
     void* hbar;        // (null while h is identically zero)
-    // face values [nv][nF] (Real): the upwind reconstruction at the half step,
+    // face values [nv][pF] (Real): the upwind reconstruction at the half step,
     // then, relaxed and multiplied by xi.S, the flux
     void* fvg;
     void* fvh;         // (null while h is identically zero)
@@ -140,7 +143,7 @@ struct DevState {
     // entity e at node i is tab[(k * n1d + i) * n + e] = exp(-(X_i - U_k)^2 /
     // (2 R T)), the x table multiplied by A = rho (2 pi R T)^(-D/2)
     double* ctab;      // [D][n1d][nC]
-    double* ftab;      // [D][n1d][nF]
+    double* ftab;      // [D][n1d][pF]
     BRec* brec;        // [nBF]
     double* bmom_in;   // [nBF][kNM] incoming wall moments per unit rho_w
     double* cm;        // cell macros [nC][9]: rho U(3) T q(3) tau (renumbered)

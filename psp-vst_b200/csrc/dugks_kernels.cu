@@ -165,6 +165,7 @@ cudaError_t launch_stage(const StepArgs& a, int precision, int stage, cudaStream
         case STAGE_PASS_A:
             pass(KERNEL_HALF_STEP);
             pass(KERNEL_FACE_VALUES);
+            if (a.dm.n_tang > 0) pass(KERNEL_TANGENTIAL);
             pass(KERNEL_FACE_MOMENTS);
             break;
         case STAGE_FACE_COMBINE:

@@ -27,7 +27,7 @@ enum { STAGE_PASS_A = 0, STAGE_FACE_COMBINE = 1, STAGE_PASS_B = 2, STAGE_CELL_CO
 // kernels of dugks_passes.cu
 enum {
     KERNEL_HALF_STEP = 0, KERNEL_FACE_VALUES = 1, KERNEL_FACE_MOMENTS = 2, KERNEL_FACE_FLUX = 3, KERNEL_UPDATE = 4,
-    KERNEL_STATE_MOMENTS = 5
+    KERNEL_STATE_MOMENTS = 5, KERNEL_TANGENTIAL = 6
 };
 
 // first segment of DV chunk k of n
@@ -64,8 +64,12 @@ cudaError_t launch_init(const StepArgs& a, int precision, cudaStream_t s);
 cudaError_t launch_pass(const StepArgs& a, int precision, int which, cudaStream_t s);
 // face (or cell) macros and records from the sums in chunk 0
 cudaError_t launch_finish(const StepArgs& a, bool faces, cudaStream_t s);
-// DevMesh::upw, from the geometry and the DV set
-cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, cudaStream_t s);
+// kernel attributes on the current device
+cudaError_t configure_kernels(int D, int precision);
+// DevMesh::upw from the geometry and the DV set, with the number of tangential
+// (internal face, DV) pairs, and their list DevMesh::tang (counters start at 0)
+cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, unsigned long long* n_tang, cudaStream_t s);
+cudaError_t launch_list_tangential(const DevMesh& m, int2* list, unsigned long long* cursor, cudaStream_t s);
 // partial moments of all chunks summed into chunk 0 (n doubles per chunk)
 cudaError_t launch_sum_chunks(double* part, int chunks, size_t n, cudaStream_t s);
 // cell records and Maxwellian tables rebuilt from the cell macros

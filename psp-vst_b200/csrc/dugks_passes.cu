@@ -38,7 +38,9 @@ namespace {
 
 constexpr int kLanes = 32;      // entities per CTA of the reducing kernels
 constexpr int kParts = 4;       // warps per CTA of the reducing kernels: segments interleaved
-constexpr int kStream = 128;    // threads per CTA of k_half_step and k_face_flux
+constexpr int kStream = 128;    // threads per CTA of k_half_step
+constexpr int kFaces = 128;     // internal faces per CTA of k_face_moments and k_face_flux
+constexpr int kGroupDv = 8;     // DVs per stage of their rings
 constexpr int kCells = 256;     // threads per CTA of k_face_values: its L1 holds the block's ring
 constexpr int kFast = 6;        // neighbours and faces of a cell kept in registers (a hexahedron)
 
@@ -112,6 +114,36 @@ __device__ __forceinline__ void groups(int len, F&& f) {
         }
     }
     if (U > 1 && j < len) f(j, std::integral_constant<int, 1>{});
+}
+
+// Walks the segments s, s + step, ... below s1 in groups of U DVs, the loads
+// of a group issued one group ahead (into the next segment at a segment's
+// end), so that a warp's loads are in flight while it computes.  load(q, j, buf)
+// reads DVs j .. j + U - 1 of segment q, clamped to the segment; row(q) forms
+// what depends on the segment; body(q, j, buf) uses a group, DVs past the
+// segment's end excluded; fold(q) closes a segment.
+template <int U, bool GEN, typename Buf, class Load, class Row, class Body, class Fold>
+__device__ __forceinline__ void walk_dvs(const DevMesh& m, int s, int s1, int step, Load&& load, Row&& row, Body&& body,
+                                         Fold&& fold) {
+    if (s >= s1) return;
+    Seg q = seg_at<GEN>(m, s);
+    Buf cur, ahead;
+    load(q, 0, cur);
+    for (;;) {
+        const bool more = s + step < s1;
+        const Seg qn = more ? seg_at<GEN>(m, s + step) : q;
+        row(q);
+        for (int j = 0; j < q.len; j += U) {
+            if (j + U < q.len) load(q, j + U, ahead);
+            else if (more) load(qn, 0, ahead);
+            body(q, j, cur);
+            cur = ahead;
+        }
+        fold(q);
+        if (!more) return;
+        s += step;
+        q = qn;
+    }
 }
 
 // one-dimensional nodes and weights of the DV set in shared memory
@@ -219,7 +251,8 @@ struct SumsShared {
 };
 struct SumsRegs {
     double v[15];
-    __device__ __forceinline__ explicit SumsRegs(Finish&) {
+    __device__ __forceinline__ explicit SumsRegs(Finish&) : SumsRegs() {}
+    __device__ __forceinline__ SumsRegs() {
 #pragma unroll
         for (int j = 0; j < 15; ++j) v[j] = 0.0;
     }
@@ -288,15 +321,15 @@ template <int D, bool HZ, bool GEN>
 struct Relax {
     const double* rec;   // records and tables of all entities (stride n)
     const double* tab;
-    unsigned n8, e8;     // bytes of a row of them; the entity's offset in one
+    unsigned n8, t8, e8; // bytes of a row of the records, of the tables; the entity's offset in one
     double Ux, invRT, qx, RTh, r;
     double Cyz, Syz, eyzr;                  // rows
     double Uy, Uz, qy, qz, rA;              // DV lists
-    const double* ex;
-    __device__ __forceinline__ Relax(const double* rec_, const double* tab_, int n_, int e, double r_) {
+    __device__ __forceinline__ Relax(const double* rec_, const double* tab_, int n_, int tn, int e, double r_) {
         rec = rec_;
         tab = tab_;
         n8 = 8u * n_;
+        t8 = 8u * tn;
         e8 = 8u * e;
         Ux = field(REC_UX);
         invRT = field(REC_INVRT);
@@ -315,10 +348,10 @@ struct Relax {
     __device__ __forceinline__ void row(const DevMesh& m, const Seg& q, double Y, double Z) {
         if constexpr (!GEN) {
             const double cy = Y - field(REC_UY), vy = field(REC_QY);
-            const double ey = __ldg(at(row_of(tab, m.n1d + q.iy, n8), e8));
+            const double ey = __ldg(at(row_of(tab, m.n1d + q.iy, t8), e8));
             if constexpr (D == 3) {
                 const double cz = Z - field(REC_UZ), vz = field(REC_QZ);
-                const double ez = __ldg(at(row_of(tab, 2 * m.n1d + q.iz, n8), e8));
+                const double ez = __ldg(at(row_of(tab, 2 * m.n1d + q.iz, t8), e8));
                 Cyz = (cy * cy + cz * cz) * invRT;
                 Syz = cy * vy + cz * vz;
                 eyzr = r * ey * ez;
@@ -327,13 +360,12 @@ struct Relax {
                 Syz = cy * vy;
                 eyzr = r * ey;
             }
-            ex = row_of(tab, q.ix0, n8);
         }
     }
-    // the Maxwellian factor of DV j of the segment
-    __device__ __forceinline__ double factor(int j) const {
+    // the Maxwellian factor of DV j of a segment
+    __device__ __forceinline__ double factor(const Seg& q, int j) const {
         if constexpr (GEN) return 0.0;
-        else return __ldg(at(row_of(ex, j, n8), e8));
+        else return __ldg(at(row_of(tab, q.ix0 + j, t8), e8));
     }
     __device__ __forceinline__ void operator()(const Dv& v, double e, double g, double h, double K3D, double c0h,
                                                double& go, double& ho) const {
@@ -383,37 +415,45 @@ __global__ void __launch_bounds__(kStream) k_half_step(const __grid_constant__ S
     const size_t nC = static_cast<size_t>(m.nC);
     const unsigned cb = sizeof(Real) * c, rb = sizeof(Real) * m.nC;
     const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
-    Relax<D, HZ, GEN> rx(a.ds.cellrec, a.ds.ctab, m.nC, c, cell_r(a, c));
+    Relax<D, HZ, GEN> rx(a.ds.cellrec, a.ds.ctab, m.nC, m.nC, c, cell_r(a, c));
     const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
-    for (int s = s0; s < s1; ++s) {
-        const Seg q = seg_at<GEN>(m, s);
-        rx.row(m, q, x1[q.iy], x1[q.iz]);
-        const size_t base = static_cast<size_t>(q.d0) * nC;
-        const Real* __restrict__ gs = reinterpret_cast<const Real*>(a.ds.g) + base;
-        const Real* __restrict__ hs = reinterpret_cast<const Real*>(a.ds.h) + base;
-        Real* __restrict__ gd = reinterpret_cast<Real*>(a.ds.gbar) + base;
-        Real* __restrict__ hd = reinterpret_cast<Real*>(a.ds.hbar) + base;
-        groups<4>(q.len, [&](int j, auto uc) {
-            constexpr int U = decltype(uc)::value;
-            Real gi[U], hi[U];
-            double e[U];
+    const Real* __restrict__ g = reinterpret_cast<const Real*>(a.ds.g);
+    const Real* __restrict__ h = reinterpret_cast<const Real*>(a.ds.h);
+    Real* __restrict__ gb = reinterpret_cast<Real*>(a.ds.gbar);
+    Real* __restrict__ hb = reinterpret_cast<Real*>(a.ds.hbar);
+    constexpr int U = 4;
+    struct Buf {
+        Real g[U], h[U];
+        double e[U];
+    };
+    walk_dvs<U, GEN, Buf>(
+        m, s0, s1, 1,
+        [&](const Seg& q, int j, Buf& b) {
+            const Real *gs = g + q.d0 * nC, *hs = h + q.d0 * nC;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                gi[u] = __ldcs(at(row_of(gs, j + u, rb), cb));
-                if (!HZ) hi[u] = __ldcs(at(row_of(hs, j + u, rb), cb));
-                e[u] = rx.factor(j + u);
+                const int ju = min(j + u, q.len - 1);
+                b.g[u] = __ldcs(at(row_of(gs, ju, rb), cb));
+                if (!HZ) b.h[u] = __ldcs(at(row_of(hs, ju, rb), cb));
+                b.e[u] = rx.factor(q, ju);
             }
+        },
+        [&](const Seg& q) { rx.row(m, q, x1[q.iy], x1[q.iz]); },
+        [&](const Seg& q, int j, const Buf& b) {
+            Real *gd = gb + q.d0 * nC, *hd = hb + q.d0 * nC;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j + u), hr = dv_ref<Real, GEN>(m.href, q.d0 + j + u);
-                double go, ho;
-                rx(dv_at<D, GEN>(m, q, x1, j + u), e[u], double(gi[u]) + gr, HZ ? 0.0 : double(hi[u]) + hr, K3D, c0h, go,
-                   ho);
-                *at(row_of(gd, j + u, rb), cb) = Real(go - gr);
-                if (!HZ) *at(row_of(hd, j + u, rb), cb) = Real(ho - hr);
+                if (j + u < q.len) {
+                    const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j + u), hr = dv_ref<Real, GEN>(m.href, q.d0 + j + u);
+                    double go, ho;
+                    rx(dv_at<D, GEN>(m, q, x1, j + u), b.e[u], double(b.g[u]) + gr, HZ ? 0.0 : double(b.h[u]) + hr, K3D,
+                       c0h, go, ho);
+                    *at(row_of(gd, j + u, rb), cb) = Real(go - gr);
+                    if (!HZ) *at(row_of(hd, j + u, rb), cb) = Real(ho - hr);
+                }
             }
-        });
-    }
+        },
+        [](const Seg&) {});
 }
 
 // ---------------------------------------------------------------------
@@ -496,15 +536,16 @@ __device__ __forceinline__ Real recon_mem(const DevMesh& m, const Real* row, int
 // through L1: a CTA's cells are a compact block of the mesh) and the value of
 // every face it is upwind of (one bit per face and DV, DevMesh::upw).  The
 // gradient never leaves registers.  On an exactly tangential internal face
-// no side is upwind; k_face_moments averages both there.
+// no side is upwind; k_tangential averages both there.
 template <int D, typename Real, bool HZ, bool GEN, int NS>
 __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant__ StepArgs a) {
     const DevMesh& m = a.dm;
     __shared__ double x1[kMaxN1d], w1[kMaxN1d];
+    __shared__ Real dist_s[NS * D * kCells];
     load_nodes(m, x1, w1);
     const int c = blockIdx.x * kCells + threadIdx.x;
     if (c >= m.nC) return;
-    const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF);
+    const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF), pF = static_cast<size_t>(m.pF);
     const Real* __restrict__ gbar = reinterpret_cast<const Real*>(a.ds.gbar);
     const Real* __restrict__ hbar = reinterpret_cast<const Real*>(a.ds.hbar);
     Real* __restrict__ fvg = reinterpret_cast<Real*>(a.ds.fvg);
@@ -513,26 +554,27 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
     // FP64 folds the DV's part of v once per cell, gbar+ - G.xi dt/2; FP32
     // keeps the reference's order, one v per face
     constexpr bool kFold = sizeof(Real) == 8;
-    const unsigned cr = sizeof(Real) * m.nC, fr = sizeof(Real) * m.nF, own = sizeof(Real) * c;
+    // DVs whose loads are issued together, as the registers allow
+    constexpr int kGroup = sizeof(Real) == 4 ? 4 : HZ || D == 2 ? 2 : 1;
+    const unsigned cr = sizeof(Real) * m.nC, fr = sizeof(Real) * m.pF, own = sizeof(Real) * c;
     unsigned nb[NS], fo[NS];   // byte offsets in a row of cells, of faces
-    int code[NS];
-    Real ls[NS][D], dist[NS][D];
+    unsigned has = 0, side = 0, in_tile = 0;
+    Real ls[NS][D];
+    Real* dist = dist_s + threadIdx.x;   // Cf - C of slot k, dimension q: dist[(k D + q) kCells]
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
         nb[k] = sizeof(Real) * (k < m.nb_max ? chk(__ldg(m.nbr + k * nC + c), 0, m.nC, a.ds.err) : c);
-        code[k] = k < m.nf_max ? chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err) : -1;
+        const int code = k < m.nf_max ? chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err) : -1;
+        const int f = code < 0 ? 0 : code >> 2, sd = code < 0 ? 0 : code & 1;
+        fo[k] = sizeof(Real) * f;
+        has |= (code >= 0 ? 1u : 0u) << k;
+        side |= static_cast<unsigned>(sd) << k;
+        if (rounds_rows<D, Real, GEN>(m) && code >= 0) in_tile |= ((code >> 1) & 1u) << k;
 #pragma unroll
         for (int q = 0; q < D; ++q) {
             ls[k][q] = k < m.nb_max ? Real(__ldg(m.nbr_ls + (k * 3 + q) * nC + c)) : Real(0);
-            fo[k] = code[k] < 0 ? 0u : sizeof(Real) * (code[k] >> 2);
-            dist[k][q] = code[k] < 0 ? Real(0) : Real(__ldg(m.fgeo + (3 + 3 * (code[k] & 1) + q) * nF + (code[k] >> 2)));
+            dist[(k * D + q) * kCells] = Real(__ldg(m.fgeo + (3 + 3 * sd + q) * nF + f));
         }
-    }
-    unsigned in_tile = 0;
-    if (rounds_rows<D, Real, GEN>(m)) {
-#pragma unroll
-        for (int k = 0; k < NS; ++k)
-            if (code[k] >= 0 && (code[k] & 2)) in_tile |= 1u << k;
     }
     const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
     const bool more = m.nb_max > NS || m.nf_max > NS;
@@ -540,84 +582,91 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
         const Seg q = seg_at<GEN>(m, s);
         const double Y = x1[q.iy], Z = x1[q.iz];
         unsigned up[NS];   // the segment's upwind bits
+        const uint32_t* us = m.upw + s * nF * 2;
 #pragma unroll
         for (int k = 0; k < NS; ++k)
-            up[k] = code[k] < 0 ? 0u : __ldg(m.upw + (static_cast<size_t>(s) * nF + (code[k] >> 2)) * 2 + (code[k] & 1));
-        const Real *gr = gbar + static_cast<size_t>(q.d0) * nC, *hr = hbar + static_cast<size_t>(q.d0) * nC;
-        Real *fg = fvg + static_cast<size_t>(q.d0) * nF, *fh = fvh + static_cast<size_t>(q.d0) * nF;
-        groups<kFold && D == 3 && !HZ ? 1 : 2>(q.len, [&](int j0, auto uc) {
+            up[k] = (has >> k) & 1u ? __ldg(at(us, fo[k] * (8 / sizeof(Real)) + 4 * ((side >> k) & 1u))) : 0u;
+        const Real *gr = gbar + q.d0 * nC, *hr = hbar + q.d0 * nC;
+        Real *fg = fvg + q.d0 * pF, *fh = fvh + q.d0 * pF;
+        groups<kGroup>(q.len, [&](int j0, auto uc) {
             constexpr int U = decltype(uc)::value;
-            Real g0[U], h0[U], dg[U][NS], dh[U][NS];
+            Real g0[U], h0[U], G[U][D], H[U][D];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const Real *gj = row_of(gr, j0 + u, cr), *hj = row_of(hr, j0 + u, cr);
+                Real dg[NS], dh[NS];
                 g0[u] = __ldg(at(gj, own));
                 if (!HZ) h0[u] = __ldg(at(hj, own));
 #pragma unroll
                 for (int k = 0; k < NS; ++k) {
-                    dg[u][k] = __ldg(at(gj, nb[k]));
-                    if (!HZ) dh[u][k] = __ldg(at(hj, nb[k]));
+                    dg[k] = __ldg(at(gj, nb[k]));
+                    if (!HZ) dh[k] = __ldg(at(hj, nb[k]));
+                }
+#pragma unroll
+                for (int p = 0; p < D; ++p) G[u][p] = H[u][p] = Real(0);
+#pragma unroll
+                for (int k = 0; k < NS; ++k) {
+                    const Real x = dg[k] - g0[u];
+#pragma unroll
+                    for (int p = 0; p < D; ++p) G[u][p] = fma(ls[k][p], x, G[u][p]);
+                    if (!HZ) {
+                        const Real y = dh[k] - h0[u];
+#pragma unroll
+                        for (int p = 0; p < D; ++p) H[u][p] = fma(ls[k][p], y, H[u][p]);
+                    }
                 }
             }
+            Dv v[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int j = j0 + u;
-                Real G[D], H[D];
-#pragma unroll
-                for (int p = 0; p < D; ++p) G[p] = H[p] = Real(0);
-#pragma unroll
-                for (int k = 0; k < NS; ++k) {
-                    const Real x = dg[u][k] - g0[u];
-#pragma unroll
-                    for (int p = 0; p < D; ++p) G[p] = fma(ls[k][p], x, G[p]);
-                    if (!HZ) {
-                        const Real y = dh[u][k] - h0[u];
-#pragma unroll
-                        for (int p = 0; p < D; ++p) H[p] = fma(ls[k][p], y, H[p]);
-                    }
-                }
-                if (more) {
-                    grad_mem<D, Real>(m, gr + j * m.nC, c, G, NS, a.ds.err);
-                    if (!HZ) grad_mem<D, Real>(m, hr + j * m.nC, c, H, NS, a.ds.err);
-                }
-                Dv v = dv_at<D, GEN>(m, q, x1, j);
+                v[u] = dv_at<D, GEN>(m, q, x1, j);
                 if constexpr (!GEN) {
-                    v.y = Y;
-                    v.z = Z;
-                }
-                Real gc = g0[u], hc = HZ ? Real(0) : h0[u];
-                if constexpr (kFold) {
-                    const Real t[3] = {Real(-hdt * v.x), Real(-hdt * v.y), Real(-hdt * v.z)};
-                    gc = recon<D, Real>(gc, G, t);
-                    if (!HZ) hc = recon<D, Real>(hc, H, t);
-                }
-                Real *fgj = row_of(fg, j, fr), *fhj = row_of(fh, j, fr);
-#pragma unroll
-                for (int k = 0; k < NS; ++k) {
-                    if (up[k] & (1u << j)) {
-                        Real vk[D];
-                        if constexpr (kFold) {
-#pragma unroll
-                            for (int p = 0; p < D; ++p) vk[p] = dist[k][p];
-                        } else {
-                            half_dist<D, Real, GEN>(dist[k], hdt, v, q.ix0 + j, (in_tile >> k) & 1u, vk);
-                        }
-                        *at(fgj, fo[k]) = recon<D, Real>(gc, G, vk);
-                        if (!HZ) *at(fhj, fo[k]) = recon<D, Real>(hc, H, vk);
-                    }
+                    v[u].y = Y;
+                    v[u].z = Z;
                 }
                 if (more) {
+                    grad_mem<D, Real>(m, gr + j * nC, c, G[u], NS, a.ds.err);
+                    if (!HZ) grad_mem<D, Real>(m, hr + j * nC, c, H[u], NS, a.ds.err);
                     for (int k = NS; k < m.nf_max; ++k) {
                         const int cd = chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err);
                         if (cd < 0) break;
-                        const int f = cd >> 2, side = cd & 1;
-                        if ((__ldg(m.upw + (static_cast<size_t>(s) * nF + f) * 2 + side) >> j) & 1u) {
+                        const int f = cd >> 2, sd = cd & 1;
+                        if ((__ldg(us + 2 * f + sd) >> j) & 1u) {
                             Real dk[D], vk[D];
 #pragma unroll
-                            for (int p = 0; p < D; ++p) dk[p] = Real(__ldg(m.fgeo + (3 + 3 * side + p) * nF + f));
-                            half_dist<D, Real, GEN>(dk, hdt, v, q.ix0 + j, (cd & 2) && rounds_rows<D, Real, GEN>(m), vk);
-                            fgj[f] = recon<D, Real>(g0[u], G, vk);
-                            if (!HZ) fhj[f] = recon<D, Real>(h0[u], H, vk);
+                            for (int p = 0; p < D; ++p) dk[p] = Real(__ldg(m.fgeo + (3 + 3 * sd + p) * nF + f));
+                            half_dist<D, Real, GEN>(dk, hdt, v[u], q.ix0 + j, (cd & 2) && rounds_rows<D, Real, GEN>(m), vk);
+                            fg[j * pF + f] = recon<D, Real>(g0[u], G[u], vk);
+                            if (!HZ) fh[j * pF + f] = recon<D, Real>(h0[u], H[u], vk);
+                        }
+                    }
+                }
+                if constexpr (kFold) {
+                    const Real t[3] = {Real(-hdt * v[u].x), Real(-hdt * v[u].y), Real(-hdt * v[u].z)};
+                    g0[u] = recon<D, Real>(g0[u], G[u], t);
+                    if (!HZ) h0[u] = recon<D, Real>(h0[u], H[u], t);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < NS; ++k) {
+                const unsigned bits = up[k] >> j0;
+                if (bits & ((1u << U) - 1u)) {
+                    Real dk[D];
+#pragma unroll
+                    for (int p = 0; p < D; ++p) dk[p] = dist[(k * D + p) * kCells];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        if (bits & (1u << u)) {
+                            Real vk[D];
+                            if constexpr (kFold) {
+#pragma unroll
+                                for (int p = 0; p < D; ++p) vk[p] = dk[p];
+                            } else {
+                                half_dist<D, Real, GEN>(dk, hdt, v[u], q.ix0 + j0 + u, (in_tile >> k) & 1u, vk);
+                            }
+                            *at(row_of(fg, j0 + u, fr), fo[k]) = recon<D, Real>(g0[u], G[u], vk);
+                            if (!HZ) *at(row_of(fh, j0 + u, fr), fo[k]) = recon<D, Real>(h0[u], H[u], vk);
                         }
                     }
                 }
@@ -631,9 +680,10 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
 // face f from that side -- internal faces by the switch of fvDVM.C:829-863
 // (neither side on an exactly tangential face), boundary faces the outgoing
 // DVs (:916-923), symmetry faces the tangential ones too (:1013-1023);
-// zero-gradient faces take the cell's value for every DV instead.
+// zero-gradient faces take the cell's value for every DV instead.  Counts the
+// tangential (face, DV) pairs of internal faces into *n_tang.
 template <int D, bool GEN>
-__global__ void k_upwind_bits(const DevMesh m, uint32_t* upw) {
+__global__ void k_upwind_bits(const DevMesh m, uint32_t* upw, unsigned long long* n_tang) {
     __shared__ double x1[kMaxN1d], w1[kMaxN1d];
     load_nodes(m, x1, w1);
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -642,6 +692,7 @@ __global__ void k_upwind_bits(const DevMesh m, uint32_t* upw) {
     const double S[3] = {__ldg(m.fgeo + f), __ldg(m.fgeo + nF + f), __ldg(m.fgeo + 2 * nF + f)};
     const int pt = f < m.nIF ? 0 : __ldg(m.bface_ptype + f - m.nIF);
     const bool sym = pt == DUGKS_PATCH_SYMMETRY || pt == DUGKS_PATCH_DVM_SYMMETRY;
+    int tangential = 0;
     for (int s = blockIdx.y; s < m.n_seg; s += gridDim.y) {
         const Seg q = seg_at<GEN>(m, s);
         uint32_t own = 0, nei = 0;
@@ -657,12 +708,184 @@ __global__ void k_upwind_bits(const DevMesh m, uint32_t* upw) {
         uint32_t* w = upw + (static_cast<size_t>(s) * nF + f) * 2;
         w[0] = own;
         w[1] = nei;
+        if (pt == 0) tangential += q.len - __popc(own) - __popc(nei);
     }
+    if (tangential) atomicAdd(n_tang, static_cast<unsigned long long>(tangential));
+}
+
+// the list of those pairs (DevMesh::tang), pairs of one DV and consecutive
+// faces together
+template <bool GEN>
+__global__ void k_list_tangential(const DevMesh m, int2* list, unsigned long long* cursor) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t nF = static_cast<size_t>(m.nF);
+    for (int s = blockIdx.y; s < m.n_seg; s += gridDim.y) {
+        const Seg q = seg_at<GEN>(m, s);
+        unsigned t = 0;
+        if (f < m.nIF) {
+            const uint2 up = reinterpret_cast<const uint2*>(m.upw)[s * nF + f];
+            t = ~(up.x | up.y) & (q.len == 32 ? 0xffffffffu : (1u << q.len) - 1u);
+        }
+        if (!__any_sync(0xffffffffu, t != 0)) continue;
+        for (int j = 0; j < q.len; ++j) {
+            const unsigned who = __ballot_sync(0xffffffffu, (t >> j) & 1u);
+            if (!who) continue;
+            unsigned long long base = 0;
+            if (threadIdx.x % 32 == 0) base = atomicAdd(cursor, static_cast<unsigned long long>(__popc(who)));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if ((t >> j) & 1u) list[base + __popc(who & ((1u << (threadIdx.x % 32)) - 1u))] = make_int2(f, s * kSeg + j);
+        }
+    }
+}
+
+// Exactly tangential DVs of internal faces: both sides averaged
+// (fvDVM.C:847-863).  One thread per listed pair, each side's gradient formed
+// again from gbar+: pairs are few (a node at rest on an axis-aligned mesh: one
+// DV in n1d) but sit on few faces, where a face's own thread in
+// k_face_moments took 3.2 ms of a 110,592-cell ball's 4.5.
+template <int D, typename Real, bool HZ, bool GEN>
+__global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ StepArgs a) {
+    const DevMesh& m = a.dm;
+    __shared__ double x1[kMaxN1d], w1[kMaxN1d];
+    load_nodes(m, x1, w1);
+    const size_t nC = static_cast<size_t>(m.nC);
+    const double hdt = 0.5 * step_dt(a);
+    for (long long i = blockIdx.x * static_cast<long long>(kStream) + threadIdx.x; i < m.n_tang;
+         i += static_cast<long long>(gridDim.x) * kStream) {
+        const int2 t = __ldg(m.tang + i);
+        const int f = chk(t.x, 0, m.nIF, a.ds.err), s = chk(t.y / kSeg, 0, m.n_seg, a.ds.err), j = t.y % kSeg;
+        const Seg q = seg_at<GEN>(m, s);
+        const int o = chk(__ldg(m.fown + f), 0, m.nC, a.ds.err), n = chk(__ldg(m.fnei + f), 0, m.nC, a.ds.err);
+        bool in_tile = false;
+        if (rounds_rows<D, Real, GEN>(m))
+            for (int k = 0; k < m.nf_max; ++k) {
+                const int code = __ldg(m.cface + k * nC + o);
+                if (code >= 0 && (code >> 2) == f) in_tile = code & 2;
+            }
+        const Dv v = dv_at<D, GEN>(m, q, x1, j);
+        const size_t rc = (q.d0 + j) * nC, rf = static_cast<size_t>(q.d0 + j) * m.pF + f;
+        const Real* g = reinterpret_cast<const Real*>(a.ds.gbar) + rc;
+        reinterpret_cast<Real*>(a.ds.fvg)[rf] =
+            Real(0.5) * (recon_mem<D, Real, GEN>(m, g, f, 1, n, hdt, v, q.ix0 + j, in_tile, a.ds.err) +
+                         recon_mem<D, Real, GEN>(m, g, f, 0, o, hdt, v, q.ix0 + j, in_tile, a.ds.err));
+        if (!HZ) {
+            const Real* h = reinterpret_cast<const Real*>(a.ds.hbar) + rc;
+            reinterpret_cast<Real*>(a.ds.fvh)[rf] =
+                Real(0.5) * (recon_mem<D, Real, GEN>(m, h, f, 1, n, hdt, v, q.ix0 + j, in_tile, a.ds.err) +
+                             recon_mem<D, Real, GEN>(m, h, f, 0, o, hdt, v, q.ix0 + j, in_tile, a.ds.err));
+        }
+    }
+}
+
+// ---------------------------------------------------------------------
+// Rings of face rows in shared memory
+// ---------------------------------------------------------------------
+// The face kernels stream rows of kFaces consecutive faces: one thread copies
+// the rows of a group of DVs with bulk asynchronous copies (a row is
+// contiguous and, its pitch padded to 32, 16-byte aligned), kStages - 1 groups
+// ahead.  The loads need no registers and no address arithmetic in the other
+// threads, and stay in flight while a group is used.  Register prefetch at 24
+// warps per SM reached 4.5 TB/s in k_face_flux and 2.5 in k_face_moments.
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void mbar_init(uint64_t* b) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(b)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t* b, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
+}
+// waits for phase `parity` of b; false after about a second (the copy's
+// completion is the hardware's to signal: the limit only bounds the wait)
+__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity) {
+    const unsigned addr = smem_addr(b);
+    for (int k = 0; k < 1 << 20; ++k) {
+        unsigned ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok)
+            : "r"(addr), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* b) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_addr(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_addr(b))
+                 : "memory");
+}
+
+// Walks the groups of kGroupDv DVs of the segments s0 .. s1 - 1 through a ring
+// of stages.  src(q, j, u, dst row u of a stage, mbarrier) issues the copies of DV
+// j + u; use(q, j, n, stage, last) takes a group of n DVs.  Every thread of the
+// CTA calls this; the set-up before it is visible to all.  Returns false when
+// a wait ran out.
+template <bool GEN, int STAGES, class Issue, class Use>
+__device__ __forceinline__ bool ring_walk(const DevMesh& m, uint64_t* full, int s0, int s1, unsigned row_bytes, Issue&& issue,
+                                          Use&& use) {
+    int ps = s0, pj = 0;   // the producer's position
+    auto fill = [&](int stage) {
+        if (ps >= s1) return;
+        const Seg q = seg_at<GEN>(m, ps);
+        const int n = min(kGroupDv, q.len - pj);
+        if (threadIdx.x == 0) {
+            mbar_expect(full + stage, n * row_bytes);
+            for (int u = 0; u < n; ++u) issue(q, pj + u, stage, u, full + stage);
+        }
+        pj += kGroupDv;
+        if (pj >= q.len) {
+            pj = 0;
+            ++ps;
+        }
+    };
+    for (int i = 0; i < STAGES; ++i) fill(i);
+    int stage = 0;
+    unsigned parity = 0;
+    for (int s = s0; s < s1; ++s) {
+        const Seg q = seg_at<GEN>(m, s);
+        for (int j = 0; j < q.len; j += kGroupDv) {
+            const bool ok = mbar_wait(full + stage, parity);
+            if (ok) use(q, j, min(kGroupDv, q.len - j), stage);
+            if (!__syncthreads_and(ok)) {   // (the barrier that frees the stage)
+                // give up: let the copies in flight land, within the same limit, before the CTA ends
+                for (int i = 0; i < STAGES; ++i) {
+                    mbar_wait(full + stage, parity);
+                    if (++stage == STAGES) {
+                        stage = 0;
+                        parity ^= 1;
+                    }
+                }
+                return false;
+            }
+            fill(stage);
+            if (++stage == STAGES) {
+                stage = 0;
+                parity ^= 1;
+            }
+        }
+    }
+    return true;
 }
 
 // ---------------------------------------------------------------------
 // Reductions of the face and cell kernels
 // ---------------------------------------------------------------------
+// after this CTA's chunk sums went to memory: true in the CTA that completes
+// the entity block
+__device__ __forceinline__ bool last_chunk(int* done, int& last) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int k = gridDim.y > 1 ? atomicAdd(done, 1) : 0;
+        last = k == static_cast<int>(gridDim.y) - 1;
+        if (last && gridDim.y > 1) *done = 0;   // for the next launch
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    return true;
+}
+
 // this CTA's chunk, from its warps' sums in f.red, into part [chunk][kNM][n];
 // true in the CTA that completes the entity block
 __device__ __forceinline__ bool reduce_chunk(Finish& f, double* part, size_t n, int e0, int count, int* done, bool fused) {
@@ -673,18 +896,7 @@ __device__ __forceinline__ bool reduce_chunk(Finish& f, double* part, size_t n, 
         for (int p = 1; p < kParts; ++p) v += f.red[p][j][lane];
         if (lane < count) part[(static_cast<size_t>(blockIdx.y) * kNM + j) * n + e0 + lane] = v;
     }
-    if (!fused) return false;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int k = gridDim.y > 1 ? atomicAdd(done, 1) : 0;
-        f.last = k == static_cast<int>(gridDim.y) - 1;
-        if (f.last && gridDim.y > 1) *done = 0;   // for the next launch
-    }
-    __syncthreads();
-    if (!f.last) return false;
-    __threadfence();
-    return true;
+    return fused && last_chunk(done, f.last);
 }
 
 // chunk sums of the block's entities, added in chunk order, into f.tot
@@ -715,70 +927,85 @@ __device__ __forceinline__ void write_tables(const Finish& f, const DevMesh& m, 
     }
 }
 
-// Face macros and relaxation coefficients of the block's faces from the
-// chunk sums (updateMaxwellWallRho fvDVM.C:1032-1052,
-// calculatedMaxwellFvPatchField.C:140-164, updateMacroSurf :1248-1300).
-__device__ __noinline__ void finish_faces(Finish& sm, const StepArgs& a, const Consts& kc, int f0, int count, int chunks) {
+// chunk sums of one entity, added in chunk order
+__device__ __forceinline__ void sum_chunks_of(double* s, const double* part, size_t n, int e, int chunks) {
+#pragma unroll
+    for (int j = 0; j < 15; ++j) s[j] = 0.0;
+#pragma unroll 2
+    for (int ch = 0; ch < chunks; ++ch) {
+        const double* p = part + static_cast<size_t>(ch) * kNM * n + e;
+#pragma unroll
+        for (int j = 0; j < 15; ++j) s[j] += __ldcg(p + j * n);
+    }
+}
+
+// Face macros, relaxation coefficients and Maxwellian tables of one face from
+// its chunk sums (updateMaxwellWallRho fvDVM.C:1032-1052,
+// calculatedMaxwellFvPatchField.C:140-164, updateMacroSurf :1248-1300), and
+// the warp's Courant numbers.  Whole warps call it; f < 0: no face.
+__device__ __noinline__ void finish_face(const StepArgs& a, const Consts& kc, int f, int chunks) {
     const DevMesh& m = a.dm;
     const size_t nF = static_cast<size_t>(m.nF);
-    sum_chunks(sm, a.ds.partF, nF, f0, count, chunks);
-    const int lane = threadIdx.x % kLanes;
-    if (threadIdx.x < kLanes) {
-        double co = 0.0;
-        if (lane < count) {
-            const int f = f0 + lane;
-            const double dt = step_dt(a);
-            double s[15];
-            for (int j = 0; j < 15; ++j) s[j] = sm.tot[j][lane];
-            if (f >= m.nIF && __ldg(m.bface_ptype + f - m.nIF) == DUGKS_PATCH_MAXWELL_WALL) {
-                // rho_w = outGoing / |inComingByRho|; the incoming wall DFs enter through it
-                BRec* br = a.ds.brec + (f - m.nIF);
-                const double rho_w = s[MOM_OUT] / fabs(br->inByRho);
-                br->rho_in = rho_w;
-                const double* mi = a.ds.bmom_in + static_cast<size_t>(f - m.nIF) * kNM;
-                for (int j = 0; j < 14; ++j) s[j] += rho_w * mi[j];
-            }
-            double rho, U[3], T, q[3], tau;
-            macros_from_moments(s, kc, rho, U, T, q, tau);
-            const double fac = 2.0 * tau / (2.0 * tau + 0.5 * dt * kc.Pr);  // fvDVM.C:1300
-            for (int i = 0; i < 3; ++i) q[i] *= fac;
-            const int fo = __ldg(m.forig + f);
-            double* fm = a.ds.fm + static_cast<size_t>(fo) * 9;
-            fm[0] = rho;
-            fm[4] = T;
-            fm[8] = tau;
-            const double RT = kc.R * T, A = rho * inv_norm(RT, kc.D);
-            const double qs = kc.Pr1 / (5.0 * rho * RT * RT);
-            double* fr = a.ds.facerec + f;
-            for (int i = 0; i < 3; ++i) {
-                fm[1 + i] = U[i];
-                fm[5 + i] = q[i];
-                fr[(REC_UX + i) * nF] = U[i];
-                fr[(REC_QX + i) * nF] = q[i] * qs;
-                sm.mac[i][lane] = U[i];
-            }
-            fr[REC_INVRT * nF] = 1.0 / RT;
-            fr[REC_A * nF] = A;
-            fr[REC_R * nF] = 0.5 * dt / (2.0 * tau + 0.5 * dt);
-            fr[REC_RTH * nF] = RT;
-            sm.mac[3][lane] = 1.0 / RT;
-            sm.mac[4][lane] = A;
-            if (f < m.nIF)  // getCoNum, fvDVM.C:2180-2182
-                co = __ldg(m.dc + fo) * (sqrt(U[0] * U[0] + U[1] * U[1] + U[2] * U[2]) + m.xi_max_co);
+    double co = 0.0;
+    if (f >= 0) {
+        const double dt = step_dt(a);
+        double s[15];
+        sum_chunks_of(s, a.ds.partF, nF, f, chunks);
+        if (f >= m.nIF && __ldg(m.bface_ptype + f - m.nIF) == DUGKS_PATCH_MAXWELL_WALL) {
+            // rho_w = outGoing / |inComingByRho|; the incoming wall DFs enter through it
+            BRec* br = a.ds.brec + (f - m.nIF);
+            const double rho_w = s[MOM_OUT] / fabs(br->inByRho);
+            br->rho_in = rho_w;
+            const double* mi = a.ds.bmom_in + static_cast<size_t>(f - m.nIF) * kNM;
+            for (int j = 0; j < 14; ++j) s[j] += rho_w * mi[j];
         }
-        double vmax = co, vsum = co;
-        for (int o = 16; o > 0; o >>= 1) {
-            vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
-            vsum += __shfl_xor_sync(0xffffffffu, vsum, o);
+        double rho, U[3], T, q[3], tau;
+        macros_from_moments(s, kc, rho, U, T, q, tau);
+        const double fac = 2.0 * tau / (2.0 * tau + 0.5 * dt * kc.Pr);  // fvDVM.C:1300
+        for (int i = 0; i < 3; ++i) q[i] *= fac;
+        const int fo = __ldg(m.forig + f);
+        double* fm = a.ds.fm + static_cast<size_t>(fo) * 9;
+        fm[0] = rho;
+        fm[4] = T;
+        fm[8] = tau;
+        const double RT = kc.R * T, A = rho * inv_norm(RT, kc.D), invRT = 1.0 / RT;
+        const double qs = kc.Pr1 / (5.0 * rho * RT * RT);
+        double* fr = a.ds.facerec + f;
+        for (int i = 0; i < 3; ++i) {
+            fm[1 + i] = U[i];
+            fm[5 + i] = q[i];
+            fr[(REC_UX + i) * nF] = U[i];
+            fr[(REC_QX + i) * nF] = q[i] * qs;
         }
-        if (lane == 0) {
-            // non-negative doubles order like their bit patterns
-            atomicMax(reinterpret_cast<unsigned long long*>(a.ds.co), static_cast<unsigned long long>(__double_as_longlong(vmax)));
-            atomicAdd(a.ds.co + 1, vsum);
+        fr[REC_INVRT * nF] = invRT;
+        fr[REC_A * nF] = A;
+        fr[REC_R * nF] = 0.5 * dt / (2.0 * tau + 0.5 * dt);
+        fr[REC_RTH * nF] = RT;
+        if (f < m.nIF)  // getCoNum, fvDVM.C:2180-2182
+            co = __ldg(m.dc + fo) * (sqrt(U[0] * U[0] + U[1] * U[1] + U[2] * U[2]) + m.xi_max_co);
+        if (!m.general_dv) {
+            // one-dimensional Maxwellian factors (layout in dugks_internal.h)
+            for (int k = 0; k < m.D; ++k) {
+                const double Uk = k == 0 ? U[0] : k == 1 ? U[1] : U[2], Ak = k == 0 ? A : 1.0;
+                double* tab = a.ds.ftab + static_cast<size_t>(k) * m.n1d * m.pF + f;
+#pragma unroll 4
+                for (int i = 0; i < m.n1d; ++i) {
+                    const double x = __ldg(m.X1 + i) - Uk;
+                    tab[static_cast<size_t>(i) * m.pF] = exp(-0.5 * x * x * invRT) * Ak;
+                }
+            }
         }
     }
-    __syncthreads();
-    if (!m.general_dv) write_tables(sm, m, a.ds.ftab, nF, f0, count);
+    double vmax = co, vsum = co;
+    for (int o = 16; o > 0; o >>= 1) {
+        vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+        vsum += __shfl_xor_sync(0xffffffffu, vsum, o);
+    }
+    if (threadIdx.x % kLanes == 0) {
+        // non-negative doubles order like their bit patterns
+        atomicMax(reinterpret_cast<unsigned long long*>(a.ds.co), static_cast<unsigned long long>(__double_as_longlong(vmax)));
+        atomicAdd(a.ds.co + 1, vsum);
+    }
 }
 
 // the coefficient record of the next half step
@@ -1002,9 +1229,22 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
     for (int s = s0 + w; s < s1; s += kParts) {
         const Seg q = seg_at<GEN>(m, s);
         RowSums rs;
+        Real g4[4] = {0, 0, 0, 0}, h4[4] = {0, 0, 0, 0};
         for (int j = 0; j < q.len; ++j) {
             const int d = q.d0 + j;
-            const size_t o = static_cast<size_t>(d) * nF;
+            const size_t o = static_cast<size_t>(d) * m.pF;
+            if ((j & 3) == 0) {
+                // the stored values of four DVs at a time (those of incoming DVs are not used)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const size_t ou = static_cast<size_t>(min(d + u, q.d0 + q.len - 1)) * m.pF;
+                    g4[u] = fg[ou];
+                    if (!HZ) h4[u] = fh[ou];
+                }
+            }
+            const Real gv = g4[0], hv = h4[0];
+            g4[0] = g4[1], g4[1] = g4[2], g4[2] = g4[3];
+            h4[0] = h4[1], h4[1] = h4[2], h4[2] = h4[3];
             const Dv v = dv_at<D, GEN>(m, q, x1, j);
             const double xs = xs_dv(v, S);
             const double gr = dv_ref<Real, GEN>(m.gref, d), hr = dv_ref<Real, GEN>(m.href, d);
@@ -1012,13 +1252,13 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
             if (zero_grad) {
                 // every DV: the owner cell's gbar+ (fvDVM.C:887-891)
                 const size_t oc = static_cast<size_t>(d) * nC + own;
-                const Real gv = reinterpret_cast<const Real*>(a.ds.gbar)[oc];
-                fg[o] = gv;
-                g = double(gv) + gr;
+                const Real gc = reinterpret_cast<const Real*>(a.ds.gbar)[oc];
+                fg[o] = gc;
+                g = double(gc) + gr;
                 if (!HZ) {
-                    const Real hv = reinterpret_cast<const Real*>(a.ds.hbar)[oc];
-                    fh[o] = hv;
-                    h = double(hv) + hr;
+                    const Real hc = reinterpret_cast<const Real*>(a.ds.hbar)[oc];
+                    fh[o] = hc;
+                    h = double(hc) + hr;
                 }
             } else if (sym) {
                 // incoming through the patch's first face (updateGHbarSurfSymmetryIn,
@@ -1036,7 +1276,7 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
                             Dv vt = v;
                             (axis == 0 ? vt.x : axis == 1 ? vt.y : vt.z) = x1[n - 1 - i];
                             if (xs_dv(vt, S0) > 0 || t > d) {
-                                const size_t ot = static_cast<size_t>(t) * nF;
+                                const size_t ot = static_cast<size_t>(t) * m.pF;
                                 const double grt = dv_ref<Real, GEN>(m.gref, t), hrt = dv_ref<Real, GEN>(m.href, t);
                                 fg[o] = Real((double(fg[ot]) + grt) - gr);
                                 if (!HZ) fh[o] = Real((double(fh[ot]) + hrt) - hr);
@@ -1049,8 +1289,8 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
                 if (!HZ) h = double(fh[o]) + hr;
             } else if (xs > 0) {
                 // outgoing: upwind from the owner (fvDVM.C:916-923, :950-961)
-                g = double(fg[o]) + gr;
-                if (!HZ) h = double(fh[o]) + hr;
+                g = double(gv) + gr;
+                if (!HZ) h = double(hv) + hr;
             } else if (wall) {
                 continue;   // incoming wall DFs enter through rho_w
             } else {
@@ -1070,94 +1310,98 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
     acc.put(sm);
 }
 
+constexpr int kStagesM = 4;   // ring stages of k_face_moments
+constexpr int kStagesF = 3;   // and of k_face_flux, whose stages hold e_x too
+
+template <typename Real, bool HZ>
+constexpr size_t ring_moments() {
+    const size_t ring = static_cast<size_t>(kStagesM) * (HZ ? 1 : 2) * kGroupDv * kFaces * sizeof(Real);
+    return ring > sizeof(Finish) ? ring : sizeof(Finish);   // boundary blocks hold their sums there
+}
+
+// Internal faces: reads each face value once (8 B per face, DV and FP64
+// field) and adds seven FP64 operations.  Boundary faces: 32 per CTA, the
+// segments split over its warps, as incoming DFs cost an exponential each.
 template <int D, typename Real, bool HZ, bool GEN>
-__global__ void __launch_bounds__(kLanes* kParts, 8) k_face_moments(const __grid_constant__ StepArgs a,
-                                                                 const __grid_constant__ Consts kc) {
+__global__ void __launch_bounds__(kFaces, 5) k_face_moments(const __grid_constant__ StepArgs a,
+                                                            const __grid_constant__ Consts kc) {
+    static_assert(kFaces == kLanes * kParts, "one CTA size for internal and boundary blocks");
     const DevMesh& m = a.dm;
+    extern __shared__ __align__(128) unsigned char ring_raw[];
     __shared__ double x1[kMaxN1d], w1[kMaxN1d];
-    __shared__ Finish sm;
+    __shared__ __align__(8) uint64_t full[kStagesM];
+    __shared__ int last;
+    if (threadIdx.x < kStagesM) mbar_init(full + threadIdx.x);
     load_nodes(m, x1, w1);
-    // boundary face blocks first: they evaluate exponentials and take longest
-    const int nbB = (m.nBF + kLanes - 1) / kLanes, bx = blockIdx.x;
-    const bool bnd = bx < nbB;
-    const int f0 = bnd ? m.nIF + bx * kLanes : (bx - nbB) * kLanes;
-    const int count = min(kLanes, (bnd ? m.nF : m.nIF) - f0);
-    const int lane = threadIdx.x % kLanes, f = f0 + lane;
-    const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF);
+    const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF), pF = static_cast<size_t>(m.pF);
     const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
-    const int w = warp_id();
-    Sums<GEN> acc(sm);
-    if (bnd) {
-        if (lane < count) boundary_moments<D, Real, HZ, GEN>(a, x1, w1, f, s0, s1, w, sm);
-    } else {
-        if (lane < count) {
-            Real* fg = reinterpret_cast<Real*>(a.ds.fvg);
-            Real* fh = reinterpret_cast<Real*>(a.ds.fvh);
-            const unsigned fb = sizeof(Real) * f, fr = sizeof(Real) * m.nF;
-            for (int s = s0 + w; s < s1; s += kParts) {
-                const Seg q = seg_at<GEN>(m, s);
-                const uint2 up = __ldg(reinterpret_cast<const uint2*>(m.upw) + static_cast<size_t>(s) * nF + f);
-                unsigned tang = ~(up.x | up.y) & (q.len == 32 ? 0xffffffffu : (1u << q.len) - 1u);
-                while (tang) {
-                    // exactly tangential: both sides averaged (fvDVM.C:847-863)
-                    const int j = __ffs(tang) - 1;
-                    tang &= tang - 1;
-                    const int o = chk(__ldg(m.fown + f), 0, m.nC, a.ds.err), n = chk(__ldg(m.fnei + f), 0, m.nC, a.ds.err);
-                    const double hdt = 0.5 * step_dt(a);
-                    const Dv v = dv_at<D, GEN>(m, q, x1, j);
-                    bool in_tile = false;
-                    if (rounds_rows<D, Real, GEN>(m))
-                        for (int k = 0; k < m.nf_max; ++k) {
-                            const int code = __ldg(m.cface + k * nC + o);
-                            if (code >= 0 && (code >> 2) == f) in_tile = code & 2;
-                        }
-                    const size_t rc = static_cast<size_t>(q.d0 + j) * nC, rf = static_cast<size_t>(q.d0 + j) * nF + f;
-                    const Real* g = reinterpret_cast<const Real*>(a.ds.gbar) + rc;
-                    fg[rf] = Real(0.5) * (recon_mem<D, Real, GEN>(m, g, f, 1, n, hdt, v, q.ix0 + j, in_tile, a.ds.err) +
-                                          recon_mem<D, Real, GEN>(m, g, f, 0, o, hdt, v, q.ix0 + j, in_tile, a.ds.err));
-                    if (!HZ) {
-                        const Real* h = reinterpret_cast<const Real*>(a.ds.hbar) + rc;
-                        fh[rf] = Real(0.5) * (recon_mem<D, Real, GEN>(m, h, f, 1, n, hdt, v, q.ix0 + j, in_tile, a.ds.err) +
-                                              recon_mem<D, Real, GEN>(m, h, f, 0, o, hdt, v, q.ix0 + j, in_tile, a.ds.err));
-                    }
-                }
-                RowSums rs;
-                const Real *gs = fg + static_cast<size_t>(q.d0) * nF, *hs = fh + static_cast<size_t>(q.d0) * nF;
-                // FP32 storage: the deviations only; the reference part is added once below
-                groups<HZ ? 8 : 4>(q.len, [&](int j, auto uc) {
-                    constexpr int U = decltype(uc)::value;
-                    Real gi[U], hi[U];
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        gi[u] = *at(row_of(gs, j + u, fr), fb);
-                        if (!HZ) hi[u] = *at(row_of(hs, j + u, fr), fb);
-                    }
-#pragma unroll
-                    for (int u = 0; u < U; ++u)
-                        add_dv<D, HZ, GEN>(acc, rs, w1, q, dv_at<D, GEN>(m, q, x1, j + u), j + u, double(gi[u]),
-                                           HZ ? 0.0 : double(hi[u]));
-                });
-                if constexpr (!GEN) row_fold<D>(acc, rs, row_const<D>(x1, w1, q));
-            }
-            if constexpr (sizeof(Real) == 4 && !GEN) {
-                // an internal face counts every DV in full: the reference's moments once
-                if (blockIdx.y == 0 && threadIdx.x < kLanes)
-                    for (int j = 0; j < 14; ++j) acc[j] += __ldg(a.ds.refmom + j);
-            }
-        }
-        acc.put(sm);
+    // boundary face blocks first: they take longest
+    const int nbB = (m.nBF + kLanes - 1) / kLanes, bx = blockIdx.x;
+    if (bx < nbB) {
+        const int f0 = m.nIF + bx * kLanes, count = min(kLanes, m.nF - f0), lane = threadIdx.x % kLanes;
+        const int w = warp_id();
+        Finish& sm = *reinterpret_cast<Finish*>(ring_raw);
+        if (lane < count) boundary_moments<D, Real, HZ, GEN>(a, x1, w1, f0 + lane, s0, s1, w, sm);
+        if (reduce_chunk(sm, a.ds.partF, nF, f0, count, a.ds.done + bx, a.fused != 0) && w == 0)
+            finish_face(a, kc, lane < count ? f0 + lane : -1, gridDim.y);
+        return;
     }
-    if (reduce_chunk(sm, a.ds.partF, nF, f0, count, a.ds.done + bx, a.fused != 0))
-        finish_faces(sm, a, kc, f0, count, gridDim.y);
+    const int f0 = (bx - nbB) * kFaces, f = f0 + threadIdx.x;
+    const bool active = f < m.nIF;
+    Real* fg = reinterpret_cast<Real*>(a.ds.fvg);
+    Real* fh = reinterpret_cast<Real*>(a.ds.fvh);
+    // the copies see the barriers' set-up
+    asm volatile("fence.proxy.async;" ::: "memory");
+    __syncthreads();
+    SumsRegs acc;
+    RowSums rs;
+    constexpr int NH = HZ ? 1 : 2;
+    Real* ring = reinterpret_cast<Real*>(ring_raw);
+    const unsigned row = sizeof(Real) * min(kFaces, m.pF - f0);
+    const bool ok = ring_walk<GEN, kStagesM>(
+        m, full, s0, s1, NH * row,
+        [&](const Seg& q, int j, int stage, int u, uint64_t* bar) {
+            Real* dst = ring + (stage * NH * kGroupDv + u) * kFaces;
+            bulk_load(dst, fg + (q.d0 + j) * pF + f0, row, bar);
+            if (!HZ) bulk_load(dst + kGroupDv * kFaces, fh + (q.d0 + j) * pF + f0, row, bar);
+        },
+        [&](const Seg& q, int j, int n, int stage) {
+            const Real* st = ring + stage * NH * kGroupDv * kFaces + threadIdx.x;
+            // FP32 storage: the deviations only; the reference part is added once below
+            groups<kGroupDv>(n, [&](int i, auto uc) {
+                constexpr int U = decltype(uc)::value;
+                const Real* su = st + i * kFaces;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    add_dv<D, HZ, GEN>(acc, rs, w1, q, dv_at<D, GEN>(m, q, x1, j + i + u), j + i + u,
+                                       double(su[u * kFaces]), HZ ? 0.0 : double(su[(kGroupDv + u) * kFaces]));
+            });
+            if constexpr (!GEN) {
+                if (j + kGroupDv >= q.len) {
+                    row_fold<D>(acc, rs, row_const<D>(x1, w1, q));
+                    rs = RowSums();
+                }
+            }
+        });
+    if (!ok) atomicOr(a.ds.err, 2);
+    if constexpr (sizeof(Real) == 4 && !GEN) {
+        // an internal face counts every DV in full: the reference's moments once
+        if (blockIdx.y == 0)
+            for (int j = 0; j < 14; ++j) acc[j] += __ldg(a.ds.refmom + j);
+    }
+    if (active) {
+#pragma unroll
+        for (int j = 0; j < 15; ++j) a.ds.partF[(static_cast<size_t>(blockIdx.y) * kNM + j) * nF + f] = acc[j];
+    }
+    if (a.fused && last_chunk(a.ds.done + bx, last)) finish_face(a, kc, active ? f : -1, gridDim.y);
 }
 
 // the finishing part alone, for sharded handles: the chunk sums of all
 // shards have been added into chunk 0
-__global__ void __launch_bounds__(kLanes* kParts) k_finish_faces(const __grid_constant__ StepArgs a,
-                                                                 const __grid_constant__ Consts kc) {
-    __shared__ Finish sm;
-    const int f0 = blockIdx.x * kLanes;
-    finish_faces(sm, a, kc, f0, min(kLanes, a.dm.nF - f0), 1);
+__global__ void __launch_bounds__(kFaces) k_finish_faces(const __grid_constant__ StepArgs a,
+                                                         const __grid_constant__ Consts kc) {
+    const int f = blockIdx.x * kFaces + threadIdx.x;
+    finish_face(a, kc, f < a.dm.nF ? f : -1, 1);
 }
 __global__ void __launch_bounds__(kLanes* kParts) k_finish_cells(const __grid_constant__ StepArgs a,
                                                                  const __grid_constant__ Consts kc) {
@@ -1170,103 +1414,146 @@ __global__ void __launch_bounds__(kLanes* kParts) k_finish_cells(const __grid_co
 // k_face_flux
 // ---------------------------------------------------------------------
 // Reads a face value, relaxes it and writes the flux xi.S g_f in its place:
-// 16 B per (face, DV) and FP64 field, bound by HBM; the face's e_x column
-// is read back through L1 once per row.  FP32 storage keeps the flux of the
-// deviation: the reference's cancels over a closed cell (sum of +-Sf = 0).
-template <int D, typename Real, bool HZ, bool GEN, bool BND>
-__device__ __forceinline__ void face_flux(const StepArgs& a, const double* x1, int f) {
+// 16 B per (face, DV) and FP64 field.  The ring's stages carry the faces' e_x
+// rows too (from L2).  FP32 storage keeps the flux of the deviation: the
+// reference's cancels over a closed cell (sum of +-Sf = 0).
+//
+// Boundary faces, by patch type.  Outgoing DFs are relaxed, h with the
+// internal-face T at the patch-local index (fvDVM.C:1367, :1413, :1429-1444).
+// Incoming ones are not: wall rho_w M(U_w, T_w) (fvDVM.C:1079-1092), far field
+// and pressure rho_b M(U_owner, T_b) (fvDVM.C:926-938) and mixed
+// rho_b M(U_b, T_b); zero-gradient and symmetry ones are stored.
+// DVMsymmetry relaxes every DV once more (fvDVM.C:1445-1453).
+template <int D, typename Real, bool HZ, bool GEN>
+__device__ __noinline__ void boundary_flux(const StepArgs& a, const double* x1, int f, int s0, int s1, int step) {
     const DevMesh& m = a.dm;
-    const int n = m.nF;
-    const size_t nF = static_cast<size_t>(n);
-    Real* fg = reinterpret_cast<Real*>(a.ds.fvg);
-    Real* fh = reinterpret_cast<Real*>(a.ds.fvh);
-    const unsigned fb = sizeof(Real) * f, fr = sizeof(Real) * n;
+    const size_t nF = static_cast<size_t>(m.nF);
     const double S[3] = {__ldg(m.fgeo + f), __ldg(m.fgeo + nF + f), __ldg(m.fgeo + 2 * nF + f)};
     const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
-    Relax<D, HZ, GEN> rx(a.ds.facerec, a.ds.ftab, n, f, __ldg(a.ds.facerec + REC_R * nF + f));
-    // boundary faces, by patch type.  Outgoing DFs are relaxed, h with the
-    // internal-face T at the patch-local index (fvDVM.C:1367, :1413,
-    // :1429-1444).  Incoming ones are not: wall rho_w M(U_w, T_w)
-    // (fvDVM.C:1079-1092), far field and pressure rho_b M(U_owner, T_b)
-    // (fvDVM.C:926-938) and mixed rho_b M(U_b, T_b); zero-gradient and
-    // symmetry ones are stored.  DVMsymmetry relaxes every DV once more
-    // (fvDVM.C:1445-1453).
+    Relax<D, HZ, GEN> rx(a.ds.facerec, a.ds.ftab, m.nF, m.pF, f, __ldg(a.ds.facerec + REC_R * nF + f));
+    const int b = f - m.nIF, pt = __ldg(m.bface_ptype + b);
+    const int li = chk(__ldg(m.bface_patch_local + b), 0, m.nIF, a.ds.err);
+    rx.RTh = m.R * a.ds.fm[static_cast<size_t>(li) * 9 + 4];
+    const bool stored = pt == DUGKS_PATCH_ZERO_GRADIENT || pt == DUGKS_PATCH_SYMMETRY || pt == DUGKS_PATCH_DVM_SYMMETRY;
+    const bool again = pt == DUGKS_PATCH_DVM_SYMMETRY;
     Incoming in{};
-    bool stored = false, again = false;
-    if constexpr (BND) {
-        const int b = f - m.nIF, pt = __ldg(m.bface_ptype + b);
-        const int li = chk(__ldg(m.bface_patch_local + b), 0, m.nIF, a.ds.err);
-        rx.RTh = m.R * a.ds.fm[static_cast<size_t>(li) * 9 + 4];
-        stored = pt == DUGKS_PATCH_ZERO_GRADIENT || pt == DUGKS_PATCH_SYMMETRY || pt == DUGKS_PATCH_DVM_SYMMETRY;
-        again = pt == DUGKS_PATCH_DVM_SYMMETRY;
-        if (!stored) in = load_incoming(a, b, pt);
-    }
-    const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
-    for (int s = s0; s < s1; ++s) {
+    if (!stored) in = load_incoming(a, b, pt);
+    for (int s = s0; s < s1; s += step) {
         const Seg q = seg_at<GEN>(m, s);
-        const double Y = x1[q.iy], Z = x1[q.iz];
-        rx.row(m, q, Y, Z);
-        const double p2 = __dmul_rn(Y, S[1]), p3 = D == 3 ? __dmul_rn(Z, S[2]) : 0.0;
-        Real *gs = fg + static_cast<size_t>(q.d0) * nF, *hs = fh + static_cast<size_t>(q.d0) * nF;
-        groups<4>(q.len, [&](int j, auto uc) {
-            constexpr int U = decltype(uc)::value;
-            Real gi[U], hi[U];
-            double e[U];
+        rx.row(m, q, x1[q.iy], x1[q.iz]);
+        Real g4[4] = {0, 0, 0, 0}, h4[4] = {0, 0, 0, 0};
+        for (int j = 0; j < q.len; ++j) {
+            const Dv v = dv_at<D, GEN>(m, q, x1, j);
+            const size_t o = static_cast<size_t>(q.d0 + j) * m.pF + f;
+            Real* pg = reinterpret_cast<Real*>(a.ds.fvg) + o;
+            Real* ph = reinterpret_cast<Real*>(a.ds.fvh) + o;
+            if ((j & 3) == 0) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                gi[u] = __ldcs(at(row_of(gs, j + u, fr), fb));
-                if (!HZ) hi[u] = __ldcs(at(row_of(hs, j + u, fr), fb));
-                e[u] = rx.factor(j + u);
+                for (int u = 0; u < 4; ++u) {
+                    const size_t ou = static_cast<size_t>(min(u, q.len - 1 - j)) * m.pF;
+                    g4[u] = pg[ou];
+                    if (!HZ) h4[u] = ph[ou];
+                }
             }
+            const Real gv = g4[0], hv = h4[0];
+            g4[0] = g4[1], g4[1] = g4[2], g4[2] = g4[3];
+            h4[0] = h4[1], h4[1] = h4[2], h4[2] = h4[3];
+            const double xs = xs_dv(v, S), e = rx.factor(q, j);
+            const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j), hr = dv_ref<Real, GEN>(m.href, q.d0 + j);
+            double gf = double(gv) + gr, hf = HZ ? 0.0 : double(hv) + hr;
+            if (xs > 0) {
+                rx(v, e, gf, hf, K3D, c0h, gf, hf);
+            } else if (!stored) {
+                in.at<D>(v, gf, hf);
+                gf = double(Real(gf - gr)) + gr;
+                hf = double(Real(hf - hr)) + hr;
+            }
+            if (again) rx(v, e, gf, hf, K3D, c0h, gf, hf);
+            *pg = Real(xs * (gf - gr));
+            if (!HZ) *ph = Real(xs * (hf - hr));
+        }
+    }
+}
+
+template <typename Real, bool HZ, bool GEN>
+constexpr size_t ring_flux() {
+    return static_cast<size_t>(kStagesF) * kGroupDv * kFaces * ((HZ ? 1 : 2) * sizeof(Real) + (GEN ? 0 : sizeof(double)));
+}
+
+template <int D, typename Real, bool HZ, bool GEN>
+__global__ void __launch_bounds__(kFaces, 4) k_face_flux(const __grid_constant__ StepArgs a) {
+    const DevMesh& m = a.dm;
+    extern __shared__ __align__(128) unsigned char ring_raw[];
+    __shared__ double x1[kMaxN1d], w1[kMaxN1d];
+    __shared__ __align__(8) uint64_t full[kStagesF];
+    if (threadIdx.x < kStagesF) mbar_init(full + threadIdx.x);
+    load_nodes(m, x1, w1);
+    asm volatile("fence.proxy.async;" ::: "memory");
+    __syncthreads();
+    const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
+    // boundary face blocks first, as in k_face_moments
+    const int nbB = (m.nBF + kLanes - 1) / kLanes, bx = blockIdx.x;
+    if (bx < nbB) {
+        const int f = m.nIF + bx * kLanes + threadIdx.x % kLanes;
+        if (f < m.nF) boundary_flux<D, Real, HZ, GEN>(a, x1, f, s0 + threadIdx.x / kLanes, s1, kParts);
+        return;
+    }
+    const int f0 = (bx - nbB) * kFaces;
+    const bool active = f0 + threadIdx.x < m.nIF;
+    const int f = active ? f0 + threadIdx.x : f0;
+    const size_t nF = static_cast<size_t>(m.nF), pF = static_cast<size_t>(m.pF);
+    const unsigned fb = sizeof(Real) * f, fr = sizeof(Real) * m.pF;
+    Real* fg = reinterpret_cast<Real*>(a.ds.fvg);
+    Real* fh = reinterpret_cast<Real*>(a.ds.fvh);
+    const double S[3] = {__ldg(m.fgeo + f), __ldg(m.fgeo + nF + f), __ldg(m.fgeo + 2 * nF + f)};
+    const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
+    Relax<D, HZ, GEN> rx(a.ds.facerec, a.ds.ftab, m.nF, m.pF, f, __ldg(a.ds.facerec + REC_R * nF + f));
+    double p2 = 0, p3 = 0;
+    constexpr int NH = HZ ? 1 : 2;
+    Real* ring = reinterpret_cast<Real*>(ring_raw);
+    double* ring_e = reinterpret_cast<double*>(ring + kStagesF * NH * kGroupDv * kFaces);
+    const unsigned cnt = min(kFaces, m.pF - f0), row = sizeof(Real) * cnt;
+    const bool ok = ring_walk<GEN, kStagesF>(
+        m, full, s0, s1, NH * row + (GEN ? 0 : 8 * cnt),
+        [&](const Seg& q, int j, int stage, int u, uint64_t* bar) {
+            Real* dst = ring + (stage * NH * kGroupDv + u) * kFaces;
+            bulk_load(dst, fg + (q.d0 + j) * pF + f0, row, bar);
+            if (!HZ) bulk_load(dst + kGroupDv * kFaces, fh + (q.d0 + j) * pF + f0, row, bar);
+            if (!GEN) bulk_load(ring_e + (stage * kGroupDv + u) * kFaces, a.ds.ftab + (q.ix0 + j) * pF + f0, 8 * cnt, bar);
+        },
+        [&](const Seg& q, int j, int n, int stage) {
+            if constexpr (!GEN) {
+                if (j == 0) {
+                    const double Y = x1[q.iy], Z = x1[q.iz];
+                    rx.row(m, q, Y, Z);
+                    p2 = __dmul_rn(Y, S[1]);
+                    p3 = D == 3 ? __dmul_rn(Z, S[2]) : 0.0;
+                }
+            }
+            const Real* st = ring + stage * NH * kGroupDv * kFaces + threadIdx.x;
+            const double* se = ring_e + stage * kGroupDv * kFaces + threadIdx.x;
+            Real *gs = fg + (q.d0 + j) * pF, *hs = fh + (q.d0 + j) * pF;
+            groups<HZ ? kGroupDv : 4>(n, [&](int i, auto uc) {
+                constexpr int U = decltype(uc)::value;
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const Dv v = dv_at<D, GEN>(m, q, x1, j + u);
-                double xs;
-                if constexpr (GEN) xs = xs_dv(v, S);
-                else xs = __dadd_rn(__dadd_rn(__dmul_rn(v.x, S[0]), p2), p3);
-                const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j + u), hr = dv_ref<Real, GEN>(m.href, q.d0 + j + u);
-                double gf = double(gi[u]) + gr, hf = HZ ? 0.0 : double(hi[u]) + hr;
-                if (!BND || xs > 0) {
-                    rx(v, e[u], gf, hf, K3D, c0h, gf, hf);
-                } else if (!stored) {
-                    if constexpr (BND) {
-                        Dv w = v;
-                        if constexpr (!GEN) {
-                            w.y = Y;
-                            w.z = D == 3 ? Z : 0.0;
-                        }
-                        in.at<D>(w, gf, hf);
-                        gf = double(Real(gf - gr)) + gr;
-                        hf = double(Real(hf - hr)) + hr;
+                for (int u = 0; u < U; ++u) {
+                    const Dv v = dv_at<D, GEN>(m, q, x1, j + i + u);
+                    double xs;
+                    if constexpr (GEN) xs = xs_dv(v, S);
+                    else xs = __dadd_rn(__dadd_rn(__dmul_rn(v.x, S[0]), p2), p3);
+                    const int d = q.d0 + j + i + u;
+                    const double gr = dv_ref<Real, GEN>(m.gref, d), hr = dv_ref<Real, GEN>(m.href, d);
+                    double gf, hf;
+                    rx(v, GEN ? 0.0 : se[(i + u) * kFaces], double(st[(i + u) * kFaces]) + gr,
+                       HZ ? 0.0 : double(st[(kGroupDv + i + u) * kFaces]) + hr, K3D, c0h, gf, hf);
+                    if (active) {
+                        *at(row_of(gs, i + u, fr), fb) = Real(xs * (gf - gr));
+                        if (!HZ) *at(row_of(hs, i + u, fr), fb) = Real(xs * (hf - hr));
                     }
                 }
-                if (BND && again) rx(v, e[u], gf, hf, K3D, c0h, gf, hf);
-                *at(row_of(gs, j + u, fr), fb) = Real(xs * (gf - gr));
-                if (!HZ) *at(row_of(hs, j + u, fr), fb) = Real(xs * (hf - hr));
-            }
+            });
         });
-    }
-}
-
-template <int D, typename Real, bool HZ, bool GEN>
-__device__ __noinline__ void boundary_flux(const StepArgs& a, const double* x1, int f) {
-    face_flux<D, Real, HZ, GEN, true>(a, x1, f);
-}
-
-template <int D, typename Real, bool HZ, bool GEN>
-__global__ void __launch_bounds__(kStream, 6) k_face_flux(const __grid_constant__ StepArgs a) {
-    const DevMesh& m = a.dm;
-    __shared__ double x1[kMaxN1d], w1[kMaxN1d];
-    load_nodes(m, x1, w1);
-    // boundary face blocks first, as in k_face_moments
-    const int nbB = (m.nBF + kStream - 1) / kStream, bx = blockIdx.x;
-    if (bx < nbB) {
-        const int f = m.nIF + bx * kStream + threadIdx.x;
-        if (f < m.nF) boundary_flux<D, Real, HZ, GEN>(a, x1, f);
-    } else {
-        const int f = (bx - nbB) * kStream + threadIdx.x;
-        if (f < m.nIF) face_flux<D, Real, HZ, GEN, false>(a, x1, f);
-    }
+    if (!ok) atomicOr(a.ds.err, 2);
 }
 
 // ---------------------------------------------------------------------
@@ -1276,7 +1563,7 @@ __global__ void __launch_bounds__(kStream, 6) k_face_flux(const __grid_constant_
 // (owner side: outflow, negated), updates g~ in place and sums the cell's
 // moments.  A flux is read by the two cells of its face; the second read hits L2.
 template <int D, typename Real, bool HZ, bool GEN, int NS>
-__global__ void __launch_bounds__(kLanes* kParts, 5) k_update(const __grid_constant__ StepArgs a,
+__global__ void __launch_bounds__(kLanes* kParts, 4) k_update(const __grid_constant__ StepArgs a,
                                                            const __grid_constant__ Consts kc) {
     const DevMesh& m = a.dm;
     __shared__ double x1[kMaxN1d], w1[kMaxN1d];
@@ -1284,7 +1571,7 @@ __global__ void __launch_bounds__(kLanes* kParts, 5) k_update(const __grid_const
     load_nodes(m, x1, w1);
     const int c0 = blockIdx.x * kLanes, count = min(kLanes, m.nC - c0);
     const int lane = threadIdx.x % kLanes, c = c0 + lane;
-    const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF);
+    const size_t nC = static_cast<size_t>(m.nC), pF = static_cast<size_t>(m.pF);
     const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
     const int w = warp_id();
     Sums<GEN> acc(sm);
@@ -1296,12 +1583,12 @@ __global__ void __launch_bounds__(kLanes* kParts, 5) k_update(const __grid_const
     if (lane < count) {
         Real* g = reinterpret_cast<Real*>(a.ds.g);
         Real* h = reinterpret_cast<Real*>(a.ds.h);
-        const unsigned cb = sizeof(Real) * c, cr = sizeof(Real) * m.nC, fr = sizeof(Real) * m.nF;
+        const unsigned cb = sizeof(Real) * c, cr = sizeof(Real) * m.nC, fr = sizeof(Real) * m.pF;
         const Real* __restrict__ fvg = reinterpret_cast<const Real*>(a.ds.fvg);
         const Real* __restrict__ fvh = reinterpret_cast<const Real*>(a.ds.fvh);
         const double dtV = step_dt(a) * __ldg(m.invV + c);
         const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
-        Relax<D, HZ, GEN> rx(a.ds.cellrec, a.ds.ctab, m.nC, c, cell_r(a, c));
+        Relax<D, HZ, GEN> rx(a.ds.cellrec, a.ds.ctab, m.nC, m.nC, c, cell_r(a, c));
         // faces with their sign (owner side: outflow, -1); an absent slot
         // repeats the first face with sign 0
         unsigned fc[NS];
@@ -1312,75 +1599,88 @@ __global__ void __launch_bounds__(kLanes* kParts, 5) k_update(const __grid_const
             fc[k] = code < 0 ? fc[0] : sizeof(Real) * (code >> 2);
             sign[k] = code < 0 ? Real(0) : (code & 1) ? Real(1) : Real(-1);
         }
-        for (int s = s0 + w; s < s1; s += kParts) {
-            const Seg q = seg_at<GEN>(m, s);
-            rx.row(m, q, x1[q.iy], x1[q.iz]);
-            RowSums rs;
-            Real *gs = g + static_cast<size_t>(q.d0) * nC, *hs = h + static_cast<size_t>(q.d0) * nC;
-            const Real *fgs = fvg + static_cast<size_t>(q.d0) * nF, *fhs = fvh + static_cast<size_t>(q.d0) * nF;
-            groups<2>(q.len, [&](int j, auto uc) {
-                constexpr int U = decltype(uc)::value;
-                Real gi[U], hi[U], fg[U][NS], fh[U][NS];
-                double e[U];
+        RowSums rs;
+        constexpr int U = HZ || sizeof(Real) == 4 ? 2 : 1;
+        struct Buf {
+            Real g[U], h[U], fg[U][NS], fh[U][NS];
+            double e[U];
+        };
+        walk_dvs<U, GEN, Buf>(
+            m, s0 + w, s1, kParts,
+            [&](const Seg& q, int j, Buf& b) {
+                const Real *gs = g + q.d0 * nC, *hs = h + q.d0 * nC, *fgs = fvg + q.d0 * pF, *fhs = fvh + q.d0 * pF;
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    gi[u] = *at(row_of(gs, j + u, cr), cb);
-                    if (!HZ) hi[u] = *at(row_of(hs, j + u, cr), cb);
-                    e[u] = rx.factor(j + u);
-                    const Real *fgj = row_of(fgs, j + u, fr), *fhj = row_of(fhs, j + u, fr);
+                    const int ju = min(j + u, q.len - 1);
+                    b.g[u] = *at(row_of(gs, ju, cr), cb);
+                    if (!HZ) b.h[u] = *at(row_of(hs, ju, cr), cb);
+                    b.e[u] = rx.factor(q, ju);
+                    const Real *fgj = row_of(fgs, ju, fr), *fhj = row_of(fhs, ju, fr);
 #pragma unroll
                     for (int k = 0; k < NS; ++k) {
-                        fg[u][k] = __ldg(at(fgj, fc[k]));
-                        if (!HZ) fh[u][k] = __ldg(at(fhj, fc[k]));
+                        b.fg[u][k] = __ldg(at(fgj, fc[k]));
+                        if (!HZ) b.fh[u][k] = __ldg(at(fhj, fc[k]));
                     }
                 }
+            },
+            [&](const Seg& q) {
+                rx.row(m, q, x1[q.iy], x1[q.iz]);
+                rs = RowSums();
+            },
+            [&](const Seg& q, int j, const Buf& b) {
+                Real *gs = g + q.d0 * nC, *hs = h + q.d0 * nC;
+                const Real *fgs = fvg + q.d0 * pF, *fhs = fvh + q.d0 * pF;
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const Dv v = dv_at<D, GEN>(m, q, x1, j + u);
-                    const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j + u), hr = dv_ref<Real, GEN>(m.href, q.d0 + j + u);
-                    double gb, hb;
-                    rx(v, e[u], double(gi[u]) + gr, HZ ? 0.0 : double(hi[u]) + hr, K3D, c0h, gb, hb);
-                    // (a product with +-1 is exact: the sum in slot order)
-                    Real sg = 0, sh = 0;
-#pragma unroll
-                    for (int k = 0; k < NS; ++k) {
-                        sg = fma(sign[k], fg[u][k], sg);
-                        if (!HZ) sh = fma(sign[k], fh[u][k], sh);
-                    }
-                    if (m.nf_max > NS) {
-                        for (int k = NS; k < m.nf_max; ++k) {
-                            const int code = chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err);
-                            if (code < 0) break;
-                            const int of = (j + u) * m.nF + (code >> 2);
-                            const Real sk = (code & 1) ? Real(1) : Real(-1);
-                            sg = fma(sk, __ldg(fgs + of), sg);
-                            if (!HZ) sh = fma(sk, __ldg(fhs + of), sh);
+                    if (j + u < q.len) {
+                        const Dv v = dv_at<D, GEN>(m, q, x1, j + u);
+                        const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j + u),
+                                     hr = dv_ref<Real, GEN>(m.href, q.d0 + j + u);
+                        double gb, hb;
+                        rx(v, b.e[u], double(b.g[u]) + gr, HZ ? 0.0 : double(b.h[u]) + hr, K3D, c0h, gb, hb);
+                        // (a product with +-1 is exact: the sum in slot order)
+                        Real sg = 0, sh = 0;
+    #pragma unroll
+                        for (int k = 0; k < NS; ++k) {
+                            sg = fma(sign[k], b.fg[u][k], sg);
+                            if (!HZ) sh = fma(sign[k], b.fh[u][k], sh);
                         }
-                    }
-                    // the update in FP64, one rounding to the storage type; with a
-                    // reference, -g/3 + 4/3 gbar+ - ref = -(g - ref)/3 + 4/3 (gbar+ - ref)
-                    const Real gn = Real(fma(-1.0 / 3, double(gi[u]), fma(4.0 / 3, gb - gr, double(sg) * dtV)));
-                    *at(row_of(gs, j + u, cr), cb) = gn;
-                    Real hn = 0;
-                    if (!HZ) {
-                        hn = Real(fma(-1.0 / 3, double(hi[u]), fma(4.0 / 3, hb - hr, double(sh) * dtV)));
-                        *at(row_of(hs, j + u, cr), cb) = hn;
-                    }
-                    add_dv<D, HZ, GEN>(acc, rs, w1, q, v, j + u, double(gn), double(hn));
-                    if constexpr (GEN) {
-                        if (fx) {
-                            const double fgd = double(sg) * dtV, fhd = double(sh) * dtV, aw = v.w * fgd;
-                            accx[0] += aw;
-                            accx[1] += aw * v.x;
-                            accx[2] += aw * v.y;
-                            accx[3] += aw * v.z;
-                            accx[4] += 0.5 * v.w * (fgd * (v.x * v.x + v.y * v.y + v.z * v.z) + fhd);
+                        if (m.nf_max > NS) {
+                            for (int k = NS; k < m.nf_max; ++k) {
+                                const int code = chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err);
+                                if (code < 0) break;
+                                const int of = (j + u) * m.pF + (code >> 2);
+                                const Real sk = (code & 1) ? Real(1) : Real(-1);
+                                sg = fma(sk, __ldg(fgs + of), sg);
+                                if (!HZ) sh = fma(sk, __ldg(fhs + of), sh);
+                            }
+                        }
+                        // the update in FP64, one rounding to the storage type; with a
+                        // reference, -g/3 + 4/3 gbar+ - ref = -(g - ref)/3 + 4/3 (gbar+ - ref)
+                        const Real gn = Real(fma(-1.0 / 3, double(b.g[u]), fma(4.0 / 3, gb - gr, double(sg) * dtV)));
+                        *at(row_of(gs, j + u, cr), cb) = gn;
+                        Real hn = 0;
+                        if (!HZ) {
+                            hn = Real(fma(-1.0 / 3, double(b.h[u]), fma(4.0 / 3, hb - hr, double(sh) * dtV)));
+                            *at(row_of(hs, j + u, cr), cb) = hn;
+                        }
+                        add_dv<D, HZ, GEN>(acc, rs, w1, q, v, j + u, double(gn), double(hn));
+                        if constexpr (GEN) {
+                            if (fx) {
+                                const double fgd = double(sg) * dtV, fhd = double(sh) * dtV, aw = v.w * fgd;
+                                accx[0] += aw;
+                                accx[1] += aw * v.x;
+                                accx[2] += aw * v.y;
+                                accx[3] += aw * v.z;
+                                accx[4] += 0.5 * v.w * (fgd * (v.x * v.x + v.y * v.y + v.z * v.z) + fhd);
+                            }
                         }
                     }
                 }
+            },
+            [&](const Seg& q) {
+                if constexpr (!GEN) row_fold<D>(acc, rs, row_const<D>(x1, w1, q));
             });
-            if constexpr (!GEN) row_fold<D>(acc, rs, row_const<D>(x1, w1, q));
-        }
         if constexpr (sizeof(Real) == 4 && !GEN) {
             // FP32 storage: the reference's moments once
             if (blockIdx.y == 0 && threadIdx.x < kLanes)
@@ -1454,7 +1754,7 @@ template <int D, typename Real, bool HZ, bool GEN>
 cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
     const DevMesh& m = a.dm;
     const Consts k = make_consts(m, a.dt);
-    const int nbI = blocks(m.nIF, kLanes), nbB = blocks(m.nBF, kLanes);
+    const int nbF = blocks(m.nIF, kFaces) + blocks(m.nBF, kLanes);
     const bool quad = m.nb_max <= 4 && m.nf_max <= 4;   // quadrilaterals, tetrahedra: shorter face lists
     switch (which) {
         case KERNEL_HALF_STEP: {
@@ -1469,12 +1769,18 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
             else k_face_values<D, Real, HZ, GEN, kFast><<<grid, kCells, 0, s>>>(a);
             break;
         }
+        case KERNEL_TANGENTIAL: {
+            const long long nb = (m.n_tang + kStream - 1) / kStream;
+            k_tangential<D, Real, HZ, GEN><<<static_cast<int>(std::min<long long>(nb, 148 * 64)), kStream, 0, s>>>(a);
+            break;
+        }
         case KERNEL_FACE_MOMENTS:
-            k_face_moments<D, Real, HZ, GEN><<<dim3(nbI + nbB, a.chunks_f), kLanes * kParts, 0, s>>>(a, k);
+            k_face_moments<D, Real, HZ, GEN>
+                <<<dim3(nbF, a.chunks_f), kFaces, ring_moments<Real, HZ>(), s>>>(a, k);
             break;
         case KERNEL_FACE_FLUX: {
-            const int nb = blocks(m.nIF, kStream) + blocks(m.nBF, kStream);
-            k_face_flux<D, Real, HZ, GEN><<<dim3(nb, stream_chunks(m, nb)), kStream, 0, s>>>(a);
+            k_face_flux<D, Real, HZ, GEN>
+                <<<dim3(nbF, stream_chunks(m, nbF)), kFaces, ring_flux<Real, HZ, GEN>(), s>>>(a);
             break;
         }
         case KERNEL_UPDATE: {
@@ -1490,6 +1796,16 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
             return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
+}
+
+// dynamic shared memory of the rings (above the default limit)
+template <int D, typename Real, bool HZ, bool GEN>
+cudaError_t allow_rings() {
+    cudaError_t e = cudaFuncSetAttribute(k_face_moments<D, Real, HZ, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(ring_moments<Real, HZ>()));
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(k_face_flux<D, Real, HZ, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   static_cast<int>(ring_flux<Real, HZ, GEN>()));
 }
 
 template <int D, typename Real>
@@ -1508,9 +1824,24 @@ cudaError_t launch_pass(const StepArgs& a, int precision, int which, cudaStream_
     return a.dm.D == 3 ? launch_d<3, float>(a, which, s) : launch_d<2, float>(a, which, s);
 }
 
+template <int D, typename Real>
+static cudaError_t configure_d() {
+    cudaError_t e = allow_rings<D, Real, false, false>();
+    if (e == cudaSuccess) e = allow_rings<D, Real, false, true>();
+    if constexpr (D == 3) {
+        if (e == cudaSuccess) e = allow_rings<D, Real, true, false>();
+    }
+    return e;
+}
+
+cudaError_t configure_kernels(int D, int precision) {
+    if (precision == DUGKS_FP64) return D == 3 ? configure_d<3, double>() : configure_d<2, double>();
+    return D == 3 ? configure_d<3, float>() : configure_d<2, float>();
+}
+
 cudaError_t launch_finish(const StepArgs& a, bool faces, cudaStream_t s) {
     const Consts k = make_consts(a.dm, a.dt);
-    if (faces) k_finish_faces<<<blocks(a.dm.nF, kLanes), kLanes * kParts, 0, s>>>(a, k);
+    if (faces) k_finish_faces<<<blocks(a.dm.nF, kFaces), kFaces, 0, s>>>(a, k);
     else k_finish_cells<<<blocks(a.dm.nC, kLanes), kLanes * kParts, 0, s>>>(a, k);
     return cudaGetLastError();
 }
@@ -1520,16 +1851,24 @@ cudaError_t launch_cell_records(const StepArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, cudaStream_t s) {
+cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, unsigned long long* n_tang, cudaStream_t s) {
     const int nb = blocks(m.nF, 128);
     const dim3 grid(nb, std::min(m.n_seg, std::max(1, 148 * 32 / std::max(nb, 1))));
     if (m.general_dv) {
-        if (m.D == 3) k_upwind_bits<3, true><<<grid, 128, 0, s>>>(m, upw);
-        else k_upwind_bits<2, true><<<grid, 128, 0, s>>>(m, upw);
+        if (m.D == 3) k_upwind_bits<3, true><<<grid, 128, 0, s>>>(m, upw, n_tang);
+        else k_upwind_bits<2, true><<<grid, 128, 0, s>>>(m, upw, n_tang);
     } else {
-        if (m.D == 3) k_upwind_bits<3, false><<<grid, 128, 0, s>>>(m, upw);
-        else k_upwind_bits<2, false><<<grid, 128, 0, s>>>(m, upw);
+        if (m.D == 3) k_upwind_bits<3, false><<<grid, 128, 0, s>>>(m, upw, n_tang);
+        else k_upwind_bits<2, false><<<grid, 128, 0, s>>>(m, upw, n_tang);
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_list_tangential(const DevMesh& m, int2* list, unsigned long long* cursor, cudaStream_t s) {
+    const int nb = blocks(m.nIF, 128);
+    const dim3 grid(nb, std::min(m.n_seg, std::max(1, 148 * 32 / std::max(nb, 1))));
+    if (m.general_dv) k_list_tangential<true><<<grid, 128, 0, s>>>(m, list, cursor);
+    else k_list_tangential<false><<<grid, 128, 0, s>>>(m, list, cursor);
     return cudaGetLastError();
 }
 
