@@ -148,7 +148,8 @@ static bool can_skip_h(const dugks_handle* h) { return h->D == 3 && h->gas.K_inn
 static int alloc_h(dugks_handle* h) {
     if (h->ds.hbar) return DUGKS_OK;
     const size_t rs = real_size(h);
-    const size_t nvc = static_cast<size_t>(h->dm.nv_loc) * h->nC, nfv = static_cast<size_t>(h->dm.nv_loc) * h->dm.pF;
+    const size_t nvc = static_cast<size_t>(h->dm.nv_loc) * h->dm.pC + dugks::kSlack,
+                 nfv = static_cast<size_t>(h->dm.nv_loc) * h->dm.pF + dugks::kSlack;
     unsigned char *b = nullptr, *f = nullptr;
     if (int st = dev_alloc(h, &b, nvc * rs)) return st;
     if (int st = dev_alloc(h, &f, nfv * rs)) return st;
@@ -404,6 +405,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dm.n1d = h->n1d;
     dm.general_dv = dvl ? 1 : 0;
     dm.nF = nF;
+    dm.pC = (nC + 31) / 32 * 32;
     dm.pF = (nF + 31) / 32 * 32;
     dm.n_seg = n_seg;
     dm.xi_max_co = std::sqrt(static_cast<double>(h->D)) * h->xi_max;
@@ -515,8 +517,8 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dm.bS = d_bS;
     dugks::DevState& ds = h->ds;
     const size_t rs = real_size(h);
-    const size_t nvc = static_cast<size_t>(dm.nv_loc) * nC;
-    const size_t nfv = static_cast<size_t>(dm.nv_loc) * dm.pF;
+    const size_t nvc = static_cast<size_t>(dm.nv_loc) * dm.pC + dugks::kSlack;
+    const size_t nfv = static_cast<size_t>(dm.nv_loc) * dm.pF + dugks::kSlack;
     unsigned char* p;
     // One state buffer: the update runs in place, as k_update reads each
     // (DV, cell) entry once and then writes it and no kernel of a step reads
@@ -544,10 +546,10 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         (dvl && opt.macro_flux && (st = dev_alloc(h, &ds.partX, static_cast<size_t>(h->chunks) * nC * dugks::kFX))) ||
         (dvl && opt.macro_flux && shard &&
          (st = dev_alloc(h, &ds.redC, static_cast<size_t>(nC) * (dugks::kNM + dugks::kFX)))) ||
-        (st = dev_alloc(h, &ds.cellrec, static_cast<size_t>(dugks::REC_N) * nC)) ||
-        (st = dev_alloc(h, &ds.facerec, static_cast<size_t>(dugks::REC_N) * nF)) ||
-        (st = dev_alloc(h, &ds.ctab, static_cast<size_t>(h->D) * h->n1d * nC)) ||
-        (st = dev_alloc(h, &ds.ftab, static_cast<size_t>(h->D) * h->n1d * dm.pF)) ||
+        (st = dev_alloc(h, &ds.cellrec, static_cast<size_t>(dugks::REC_N) * dm.pC)) ||
+        (st = dev_alloc(h, &ds.facerec, static_cast<size_t>(dugks::REC_N) * dm.pF)) ||
+        (st = dev_alloc(h, &ds.ctab, static_cast<size_t>(h->D) * h->n1d * dm.pC + dugks::kSlack)) ||
+        (st = dev_alloc(h, &ds.ftab, static_cast<size_t>(h->D) * h->n1d * dm.pF + dugks::kSlack)) ||
         (st = dev_alloc(h, &ds.brec, nBF)) || (st = dev_alloc(h, &ds.bmom_in, static_cast<size_t>(nBF) * dugks::kNM)) ||
         (st = dev_alloc(h, &ds.cm, static_cast<size_t>(nC) * 9)) ||
         (st = dev_alloc(h, &ds.fm, static_cast<size_t>(nF) * 9)) || (st = dev_alloc(h, &ds.co, 2)) ||
@@ -1323,9 +1325,10 @@ int dugks_get_df(dugks_handle* h, const int32_t* cells, int32_t n, double* g_out
             double* dst = which == 0 ? g_out : h_out;
             if (!dst) continue;
             const unsigned char* src =
-                static_cast<const unsigned char*>(which == 0 ? h->ds.g : h->ds.h) + c * rs;
-            CUDA_TRY(h, cudaMemcpy2DAsync(col.data(), rs, src, static_cast<size_t>(h->nC) * rs, rs, h->dm.nv_loc,
-                                          cudaMemcpyDeviceToHost, h->stream));
+                static_cast<const unsigned char*>(which == 0 ? h->ds.g : h->ds.h) +
+                (static_cast<size_t>(c / 32) * h->dm.nv_loc * 32 + c % 32) * rs;
+            CUDA_TRY(h, cudaMemcpy2DAsync(col.data(), rs, src, 32 * rs, rs, h->dm.nv_loc, cudaMemcpyDeviceToHost,
+                                          h->stream));
             CUDA_TRY(h, cudaStreamSynchronize(h->stream));
             for (int d = 0; d < h->dm.nv_loc; ++d) {
                 double v;
@@ -1347,7 +1350,7 @@ static int state_io(dugks_handle* h, double* g, double* hh, const double* gi, co
     if (!h) return DUGKS_ERR_ARG;
     if (!h->initialised) return set_error(h, DUGKS_ERR_STATE, "state access before dugks_set_macros");
     const size_t rs = real_size(h);
-    const size_t nvc = static_cast<size_t>(h->dm.nv_loc) * h->nC;
+    const size_t nvc = static_cast<size_t>(h->dm.nv_loc) * h->dm.pC;
     std::vector<unsigned char> buf(nvc * rs);
     const std::vector<int32_t>& perm = h->tiling.perm;
     for (int which = 0; which < 2; ++which) {
@@ -1359,7 +1362,7 @@ static int state_io(dugks_handle* h, double* g, double* hh, const double* gi, co
             CUDA_TRY(h, cudaMemcpy(buf.data(), dev, nvc * rs, cudaMemcpyDeviceToHost));
             for (int d = 0; d < h->dm.nv_loc; ++d)
                 for (int c = 0; c < h->nC; ++c) {
-                    const size_t s = static_cast<size_t>(d) * h->nC + c;
+                    const size_t s = (static_cast<size_t>(c / 32) * h->dm.nv_loc + d) * 32 + c % 32;
                     const size_t o = static_cast<size_t>(d) * h->nC + perm[c];
                     if (rs == sizeof(double)) std::memcpy(&dst[o], &buf[s * rs], sizeof(double));
                     else {
@@ -1373,7 +1376,7 @@ static int state_io(dugks_handle* h, double* g, double* hh, const double* gi, co
             if (!src) return set_error(h, DUGKS_ERR_ARG, "dugks_set_state: null array");
             for (int d = 0; d < h->dm.nv_loc; ++d)
                 for (int c = 0; c < h->nC; ++c) {
-                    const size_t s = static_cast<size_t>(d) * h->nC + c;
+                    const size_t s = (static_cast<size_t>(c / 32) * h->dm.nv_loc + d) * 32 + c % 32;
                     const size_t o = static_cast<size_t>(d) * h->nC + perm[c];
                     if (rs == sizeof(double)) std::memcpy(&buf[s * rs], &src[o], sizeof(double));
                     else {

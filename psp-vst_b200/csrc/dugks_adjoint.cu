@@ -186,7 +186,7 @@ int prepare(dugks_handle* h, const dugks_objective* obj, const char* who, Arena&
     ADJ_TRY(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
 
     const int nC = h->nC, nIF = h->nIF, nBF = h->nBF, nF = nIF + nBF, nv = h->nv;
-    const size_t nvc = static_cast<size_t>(nv) * nC, nvf = static_cast<size_t>(nv) * h->dm.pF;
+    const size_t nvc = static_cast<size_t>(nv) * h->dm.pC, nvf = static_cast<size_t>(nv) * h->dm.pF;
     // mesh tables in the handle's cell numbering
     const std::vector<int32_t>& perm = h->tiling.perm;
     const std::vector<int32_t>&own = h->tiling.fown, &nei = h->tiling.fnei, &forig = h->tiling.forig;
@@ -221,7 +221,7 @@ int prepare(dugks_handle* h, const dugks_objective* obj, const char* who, Arena&
     v.nIF = nIF;
     v.nBF = nBF;
     v.nF = nF;
-    v.pF = h->dm.pF;
+    v.pC = h->dm.pC;
     v.nv = nv;
     v.D = h->D;
     v.K = h->gas.K_inner;
@@ -309,7 +309,7 @@ extern "C" int dugks_adjoint_run(dugks_handle* h, const dugks_objective* obj, do
     int sms = 0, st;
     if ((st = prepare(h, obj, "dugks_adjoint_run", ar, v, sms, true, lam))) return st;
     const int nC = h->nC, nBF = h->nBF, nF = v.nF;
-    const size_t nvc = static_cast<size_t>(h->nv) * nC;
+    const size_t nvc = static_cast<size_t>(h->nv) * h->dm.pC;
 
     HandleOps ops;
     ops.h = h;

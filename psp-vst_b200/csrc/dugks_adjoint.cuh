@@ -28,8 +28,8 @@
 // run by an executor (a grid-stride CUDA launch in the library).  Sums over
 // DVs are split into DV chunks written to per-chunk partials and added in
 // chunk order by a combine functor, so results are reproducible run to run.
-// Layouts: DV-major [dv][entity] for per-(entity, DV) arrays, entity-major
-// [entity][k] for per-entity records, [chunk][entity][kP] for partials.
+// Layouts: [block of 32 entities][dv][32] for per-(entity, DV) arrays, as the
+// step's, entity-major [entity][k] for per-entity records, [chunk][entity][kP] for partials.
 #pragma once
 
 #include <algorithm>
@@ -63,7 +63,7 @@ enum {
 enum { CO_AL = 0, CO_BE = 1, CO_GA = 4, CO_AQ = 5, CO_U = 8 };
 
 struct View {
-    int nC, nIF, nBF, nF, pF, nv, D, K, nchF, nchC;   // pF: pitch of the face rows
+    int nC, nIF, nBF, nF, pC, nv, D, K, nchF, nchC;   // pC: nC padded to a multiple of 32
     double R, Pr, omega, Tref, mu, dt;
     // mesh (cells and faces in the handle's numbering; faces internal then boundary)
     const int32_t* own;     // [nF]
@@ -94,7 +94,7 @@ struct View {
     // forward record of the step: the handle's face-value buffers, faces in
     // the order of the step's arrays, and the raw moments k_face_moments sums
     // of them ([nchM][16][nF]) with the incoming wall DFs' per unit rho_w
-    double* fg;             // [nv][pF] face values before the relaxation
+    double* fg;             // faces: face values before the relaxation
     double* fh;
     const double* fmom;
     int nchM;
@@ -106,13 +106,13 @@ struct View {
     double* fmac;           // [nF][kMac]
     double* cmac;           // [nC][kMac] macros of the state, from its moments
     // adjoint of the step
-    const double* lg;       // [nv][nC] adjoint of the state after the step
+    const double* lg;       // cells: adjoint of the state after the step
     const double* lh;
-    double* og;             // [nv][nC] adjoint of the state before the step (output)
+    double* og;             // cells: adjoint of the state before the step (output)
     double* oh;
-    double* ag;             // [nv][pF] adjoint of the face values before the relaxation
+    double* ag;             // faces: adjoint of the face values before the relaxation
     double* ah;
-    double* aGg;            // [3][nv][nC] adjoint of the gradients
+    double* aGg;            // [3] cells: adjoint of the gradients
     double* aGh;
     double* fco;            // [nF][kCo]
     double* cco;            // [nC][kCo]
@@ -162,7 +162,8 @@ ADJ_HD double xs_of(const double* xi, const double* S) {
     return (xi[0] * S[0] + xi[1] * S[1]) + xi[2] * S[2];
 #endif
 }
-ADJ_HD size_t at(int i, int n, int e) { return static_cast<size_t>(i) * n + e; }
+// element of DV i of cell or face e ([block of 32][dv][32])
+ADJ_HD size_t at(int i, int nv, int e) { return (static_cast<size_t>(e >> 5) * nv + i) * 32 + (e & 31); }
 ADJ_HD int chunk_lo(int nv, int nch, int ch) { return static_cast<int>(static_cast<int64_t>(nv) * ch / nch); }
 
 // fvDVM::updateTau (fvDVM.C:1823-1832)
@@ -448,8 +449,8 @@ struct FIncoming {
         const double Tb = v.bT[b];
         const double gi = wall ? v.rhow[b] * eq_by_rho(v, xi, v.bU + 3 * b, Tb)
                                : v.brho[b] * eq_by_rho(v, xi, v.cm + 9 * static_cast<size_t>(v.own[f]) + 1, Tb);
-        v.fg[at(i, v.pF, f)] = gi;
-        v.fh[at(i, v.pF, f)] = gi * (v.R * Tb) * static_cast<double>(v.K + 3 - v.D);
+        v.fg[at(i, v.nv, f)] = gi;
+        v.fh[at(i, v.nv, f)] = gi * (v.R * Tb) * static_cast<double>(v.K + 3 - v.D);
     }
 };
 
@@ -461,7 +462,7 @@ struct FCellMom {
         const int ch = static_cast<int>(idx / v.nC), c = static_cast<int>(idx % v.nC);
         double m[14] = {0};
         for (int i = chunk_lo(v.nv, v.nchC, ch); i < chunk_lo(v.nv, v.nchC, ch + 1); ++i)
-            add_moments(v.xi + 3 * i, v.w[i], v.g[at(i, v.nC, c)], v.h[at(i, v.nC, c)], m);
+            add_moments(v.xi + 3 * i, v.w[i], v.g[at(i, v.nv, c)], v.h[at(i, v.nv, c)], m);
         double* p = v.pc + (static_cast<size_t>(ch) * v.nC + c) * kP;
         for (int k = 0; k < 14; ++k) p[k] = m[k];
     }
@@ -482,7 +483,7 @@ struct FCellMac {
 ADJ_HD bool relaxed_value(const View& v, int i, int f, double& gr, double& hr, double& gEq, double& hEq,
                           double& r) {
     const double* xi = v.xi + 3 * i;
-    const size_t id = at(i, v.pF, f);
+    const size_t id = at(i, v.nv, f);
     gr = v.fg[id];
     hr = v.fh[id];
     if (f >= v.nIF && !(xs_of(xi, v.S + 3 * f) > 0)) return false;
@@ -569,9 +570,9 @@ struct RRelax {
         for (int i = chunk_lo(v.nv, v.nchF, ch); i < chunk_lo(v.nv, v.nchF, ch + 1); ++i) {
             const double* xi = v.xi + 3 * i;
             const double xs = xs_of(xi, S);
-            const size_t id = at(i, v.pF, f);
-            const double lgo = ro(v.lg + at(i, v.nC, ow)), lho = ro(v.lh + at(i, v.nC, ow));
-            const double lgn = ro(v.lg + at(i, v.nC, ne)), lhn = ro(v.lh + at(i, v.nC, ne));
+            const size_t id = at(i, v.nv, f);
+            const double lgo = ro(v.lg + at(i, v.nv, ow)), lho = ro(v.lh + at(i, v.nv, ow));
+            const double lgn = ro(v.lg + at(i, v.nv, ne)), lhn = ro(v.lh + at(i, v.nv, ne));
             const double pg = ro(v.fg + id), ph = ro(v.fh + id);
             double a_g = xs * (dtVn * lgn - dtVo * lgo);
             double a_h = xs * (dtVn * lhn - dtVo * lho);
@@ -648,7 +649,7 @@ struct RFaceMom {
         double s[5] = {0, 0, 0, 0, 0};
         for (int i = chunk_lo(v.nv, v.nchF, ch); i < chunk_lo(v.nv, v.nchF, ch + 1); ++i) {
             const double* xi = v.xi + 3 * i;
-            const size_t id = at(i, v.pF, f);
+            const size_t id = at(i, v.nv, f);
             double a_g, a_h;
             moment_adjoint(co, xi, v.w[i], a_g, a_h);
             a_g += v.ag[id];
@@ -708,7 +709,7 @@ struct RWallOut {
         if (v.btype[b] != 1) return;
         const int f = v.nIF + b;
         const double xs = xs_of(v.xi + 3 * i, v.S + 3 * f);
-        if (xs > 0) v.ag[at(i, v.pF, f)] += v.aout[b] * v.w[i] * xs;
+        if (xs > 0) v.ag[at(i, v.nv, f)] += v.aout[b] * v.w[i] * xs;
     }
 };
 
@@ -719,9 +720,10 @@ struct RGradAdj {
     View v;
     ADJ_HD void operator()(int64_t idx) const {
         const int i = static_cast<int>(idx / v.nC), c = static_cast<int>(idx % v.nC);
+        const size_t ic = at(i, v.nv, c);
         const double* xi = v.xi + 3 * i;
         double Gg[3] = {0, 0, 0}, Gh[3] = {0, 0, 0};
-        double dg = 4.0 / 3 * v.lg[idx], dh = 4.0 / 3 * v.lh[idx];
+        double dg = 4.0 / 3 * v.lg[ic], dh = 4.0 / 3 * v.lh[ic];
         for (int e = v.cf_off[c]; e < v.cf_off[c + 1]; ++e) {
             const int f = v.cf_ent[e] >> 1;
             const bool is_nei = v.cf_ent[e] & 1;
@@ -732,7 +734,7 @@ struct RGradAdj {
             else if (xs < -kVSmall) share = is_nei ? 1.0 : 0.0;
             else share = 0.5;
             if (share == 0.0) continue;
-            const size_t id = at(i, v.pF, f);
+            const size_t id = at(i, v.nv, f);
             const double a_g = share * v.ag[id], a_h = share * v.ah[id];
             double d[3];
             recon_vec(v, f, c, xi, d);
@@ -743,13 +745,13 @@ struct RGradAdj {
                 Gh[k] += a_h * d[k];
             }
         }
-        const size_t n = static_cast<size_t>(v.nv) * v.nC;
+        const size_t n = static_cast<size_t>(v.nv) * v.pC;
         for (int k = 0; k < 3; ++k) {
-            v.aGg[k * n + idx] = Gg[k];
-            v.aGh[k * n + idx] = Gh[k];
+            v.aGg[k * n + ic] = Gg[k];
+            v.aGh[k * n + ic] = Gh[k];
         }
-        v.og[idx] = dg;
-        v.oh[idx] = dh;
+        v.og[ic] = dg;
+        v.oh[ic] = dh;
     }
 };
 
@@ -764,9 +766,8 @@ struct RHalf {
     View v;
     static constexpr int kRegF = 6;
     static constexpr int kMinCtas = 2;  // 16 warps per SM: at most 128 registers
-    ADJ_HD void face_add(size_t cb, size_t n, int f, int o, bool is_nei, const double* gc, const double* hc,
+    ADJ_HD void face_add(size_t io, size_t n, int f, bool is_nei, const double* gc, const double* hc,
                          double& abg, double& abh) const {
-        const size_t io = cb + o;
         const double go[3] = {ro(v.aGg + io), ro(v.aGg + n + io), ro(v.aGg + 2 * n + io)};
         const double ho[3] = {ro(v.aGh + io), ro(v.aGh + n + io), ro(v.aGh + 2 * n + io)};
         const double P[3] = {ro(v.lsP + 3 * f), ro(v.lsP + 3 * f + 1), ro(v.lsP + 3 * f + 2)};
@@ -786,7 +787,7 @@ struct RHalf {
         const double tau = tau_of(v, m[4], m[0]);
         const double r = 1.5 * v.dt / (2.0 * tau + v.dt);
         const ShkEntity e(v, m + 1, m[4], m[0], m + 5, m[4]);
-        const size_t n = static_cast<size_t>(v.nv) * v.nC;
+        const size_t n = static_cast<size_t>(v.nv) * v.pC;
         const int e0 = v.cf_off[c], e1 = v.cf_off[c + 1];
         // the internal faces lead the cell's list
         int nf = 0;
@@ -807,19 +808,19 @@ struct RHalf {
         }
         double s[9] = {0};
         for (int i = chunk_lo(v.nv, v.nchC, ch); i < chunk_lo(v.nv, v.nchC, ch + 1); ++i) {
-            const size_t cb = at(i, v.nC, 0), id = cb + c;
+            const size_t id = at(i, v.nv, c);
             double abg = v.og[id], abh = v.oh[id];
             const double gc[3] = {ro(v.aGg + id), ro(v.aGg + n + id), ro(v.aGg + 2 * n + id)};
             const double hc[3] = {ro(v.aGh + id), ro(v.aGh + n + id), ro(v.aGh + 2 * n + id)};
             if (reg) {
 #pragma unroll
                 for (int q = 0; q < kRegF; ++q)
-                    if (q < nf) face_add(cb, n, rf[q], oc[q], (rn >> q) & 1u, gc, hc, abg, abh);
+                    if (q < nf) face_add(at(i, v.nv, oc[q]), n, rf[q], (rn >> q) & 1u, gc, hc, abg, abh);
             } else {
                 for (int en = e0; en < e0 + nf; ++en) {
                     const int ent = ro(v.cf_ent + en);
                     const int f = ent >> 1;
-                    face_add(cb, n, f, (ent & 1) ? ro(v.own + f) : ro(v.nei + f), ent & 1, gc, hc, abg, abh);
+                    face_add(at(i, v.nv, (ent & 1) ? ro(v.own + f) : ro(v.nei + f)), n, f, ent & 1, gc, hc, abg, abh);
                 }
             }
             const ShkEntity::DV d = e.at(v.xi + 3 * i);
@@ -876,8 +877,9 @@ struct RCellMom {
         const int i = static_cast<int>(idx / v.nC), c = static_cast<int>(idx % v.nC);
         double a_g, a_h;
         moment_adjoint(v.cco + kCo * static_cast<size_t>(c), v.xi + 3 * i, v.w[i], a_g, a_h);
-        v.og[idx] += a_g;
-        v.oh[idx] += a_h;
+        const size_t ic = at(i, v.nv, c);
+        v.og[ic] += a_g;
+        v.oh[ic] += a_h;
     }
 };
 

@@ -16,6 +16,7 @@ constexpr int kMaxTile = 128;      // cells per tile at most
 constexpr int kMaxLocal = 256;     // cells of a tile with its ring of neighbours at most
 constexpr int kMaxItems = 511;     // faces of a tile's cells at most
 constexpr int kSeg = 32;           // DVs per segment at most (one bit each in DevMesh::upw)
+constexpr int kSlack = 1024;       // elements to spare behind the (entity, DV) arrays (group loads read past a segment)
 constexpr int kMaxN1d = 64;        // DV nodes per dimension at most
 constexpr int kNM = 16;            // stride of a partial-moment record (doubles)
 constexpr int kFX = 8;             // stride of a flux-moment record: M0, M1[3], W/2
@@ -31,10 +32,9 @@ enum {
     MOM_M0 = 0, MOM_M1 = 1, MOM_W = 4, MOM_V3 = 5, MOM_M2 = 8, MOM_OUT = 14
 };
 
-// Record fields of the structure-of-arrays coefficient tables.  Cell
-// records (gbar+ half step, fvDVM.C:668-679) and face records (face
-// relaxation, fvDVM.C:1374-1444) share the layout: field k of entity e is
-// rec[k * n + e].
+// Fields of the coefficient records.  Cell records (gbar+ half step,
+// fvDVM.C:668-679) and face records (face relaxation, fvDVM.C:1374-1444)
+// share them.
 enum {
     REC_UX = 0, REC_UY = 1, REC_UZ = 2,
     REC_INVRT = 3,   // 1/(R T)
@@ -64,7 +64,10 @@ struct DevMesh {
     int D, K;
     double R, Pr, omega, Tref, muRef;
     int nC, nIF, nBF, nF, nv;
-    int pF;                // pitch of the face-value rows and of ftab: nF padded to a multiple of 32
+    // (entity, DV) arrays hold blocks of 32 cells or faces, [block][dv][32]:
+    // entity e, DV d is element ((e / 32) nv_loc + d) 32 + e % 32.  Records
+    // and Maxwellian tables alike: [block][field][32].  pC, pF: nC, nF padded
+    int pC, pF;
     // DVs this device holds: global DVs dv_base .. dv_base + nv_loc - 1, the
     // DV rows row_base ..; the state and face-value arrays are [nv_loc][..]
     int nv_loc, dv_base, row_base;
@@ -122,11 +125,11 @@ struct DevMesh {
 
 // Mutable device state
 struct DevState {
-    void* g;           // state g~ [nv][nC] (Real), updated in place
+    void* g;           // state g~ (cells, Real), updated in place
     void* h;
-    void* gbar;        // gbar+ of the step [nv][nC] (Real)
+    void* gbar;        // gbar+ of the step (cells, Real)
     void* hbar;        // (null while h is identically zero)
-    // face values [nv][pF] (Real): the upwind reconstruction at the half step,
+    // face values (faces, Real): the upwind reconstruction at the half step,
     // then, relaxed and multiplied by xi.S, the flux
     void* fvg;
     void* fvh;         // (null while h is identically zero)
@@ -135,15 +138,15 @@ struct DevState {
     double* partX;     // [chunks][kFX][nC] DV-list macroFlux: moments of the flux term (else null)
     double* redC;      // sharded DV-list macroFlux: [kNM][nC] cell moments then [kFX][nC] flux moments, reduced together
     int* done;         // chunks finished per face block, then per cell block; zero between launches
-    double* cellrec;   // [REC_N][nC]
-    double* facerec;   // [REC_N][nF]
+    double* cellrec;   // cells, REC_N fields
+    double* facerec;   // faces, REC_N fields
     // one-dimensional Maxwellian factors, FP64 for both precisions (the
     // equilibrium and the relaxation are evaluated in FP64, so that the FP32
     // path injects no rounding bias into the conserved moments): table k of
-    // entity e at node i is tab[(k * n1d + i) * n + e] = exp(-(X_i - U_k)^2 /
+    // entity e at node i is field k * n1d + i of D n1d: exp(-(X_i - U_k)^2 /
     // (2 R T)), the x table multiplied by A = rho (2 pi R T)^(-D/2)
-    double* ctab;      // [D][n1d][nC]
-    double* ftab;      // [D][n1d][pF]
+    double* ctab;
+    double* ftab;
     BRec* brec;        // [nBF]
     double* bmom_in;   // [nBF][kNM] incoming wall moments per unit rho_w
     double* cm;        // cell macros [nC][9]: rho U(3) T q(3) tau (renumbered)

@@ -4,8 +4,8 @@
 // One fvDVM::evolution() (src/fvDVM/fvDVM/fvDVM.C:2128-2174) is
 //   pass A  half step, face values, face moments and macros (dugks_passes.cu)
 //   pass B  face fluxes, update, cell moments and macros
-// The state g~, h~ is DV-major [dv][cell], the cells renumbered by recursive
-// coordinate bisection.
+// The state g~, h~ is laid out [block of 32 cells][dv][32], the cells
+// renumbered by recursive coordinate bisection.
 #include <algorithm>
 
 #include "dugks_device.cuh"
@@ -14,15 +14,18 @@ namespace dugks {
 
 namespace {
 
-// initial Maxwellian state (fvDVM.C:414-426), DV-major
+// initial Maxwellian state (fvDVM.C:414-426)
 template <typename Real>
 __global__ void k_init_state(const StepArgs a) {
     const DevMesh& m = a.dm;
-    const size_t n = static_cast<size_t>(m.nv_loc) * m.nC;
+    const size_t n = static_cast<size_t>(m.nv_loc) * m.pC;
     const double K3D = m.K + 3.0 - m.D;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const int d = m.dv_base + static_cast<int>(i / m.nC), c = static_cast<int>(i % m.nC);
+        const unsigned row = static_cast<unsigned>(i / 32), blk = row / m.nv_loc;   // [block][dv][32]
+        const int dl = static_cast<int>(row - blk * m.nv_loc), d = m.dv_base + dl;
+        const int c = static_cast<int>(blk * 32 + i % 32);
+        if (c >= m.nC) continue;
         const double* cm = a.ds.cm + static_cast<size_t>(c) * 9;
         const double RT = m.R * cm[4];
         const double cx = cm[1] - m.xi[3 * d], cy = cm[2] - m.xi[3 * d + 1], cz = cm[3] - m.xi[3 * d + 2];
@@ -30,7 +33,6 @@ __global__ void k_init_state(const StepArgs a) {
         const double he = K3D * ge * RT;
         if (sizeof(Real) == 4 && m.gref) {
             // FP32 storage of a tensor DV set: the deviation from the reference
-            const int dl = static_cast<int>(i / m.nC);
             reinterpret_cast<Real*>(a.ds.g)[i] = Real(ge - m.gref[dl]);
             reinterpret_cast<Real*>(a.ds.h)[i] = Real(he - m.href[dl]);
         } else {

@@ -1,9 +1,10 @@
 // The kernels of one DUGKS step over (DV, cell) and (DV, face) arrays (sm_100a).
 //
-// Every array of the step is DV-major, [dv][cell] or [dv][face], so that a
-// warp of consecutive cells or faces reads and writes contiguously; a thread
-// keeps one cell's or face's geometry and coefficients in registers and walks
-// DVs.  DVs are walked in segments (DevMesh::n_seg): up to 32 consecutive DVs
+// Every (entity, DV) array of the step is laid out [block of 32 cells or
+// faces][dv][32] (DevMesh): a warp's 32 entities read and write contiguously,
+// a thread, which keeps one entity's geometry and coefficients in registers and
+// walks DVs, finds the next DV a constant 32 elements on, so that a group of
+// DVs shares one address, and a group's rows of a warp are one contiguous copy.  DVs are walked in segments (DevMesh::n_seg): up to 32 consecutive DVs
 // of one row of the tensor product (the n1d DVs along x at fixed y and z), or
 // of the DV list.  Within a row xi = (x_j, Y, Z) varies in x only, so xi.S, the
 // Shakhov exponent and the raw moments split into a part computed once per
@@ -80,20 +81,13 @@ __device__ __forceinline__ Seg seg_at(const DevMesh& m, int s) {
     return q;
 }
 
-// p + off bytes: with p uniform over the warp the offset is part of the load
-template <typename T>
-__device__ __forceinline__ T* at(T* p, unsigned off) {
-    return reinterpret_cast<T*>(reinterpret_cast<char*>(const_cast<std::remove_const_t<T>*>(p)) + off);
-}
-
-// row j of an array of rows of n bytes each
-template <typename T>
-__device__ __forceinline__ T* row_of(T* p, int j, unsigned n) {
-    return at(p, static_cast<unsigned>(j) * n);
-}
-
 // this thread's warp in its CTA, known to be uniform
 __device__ __forceinline__ int warp_id() { return __shfl_sync(0xffffffffu, threadIdx.x / kLanes, 0); }
+
+// element of entity e, DV 0, in an (entity, DV) array of nd DVs; DV d is 32 d on
+__device__ __forceinline__ size_t slot(int e, int nd) {
+    return static_cast<size_t>(e >> 5) * nd * 32 + (e & 31);
+}
 
 // calls f(j, U) for groups of U consecutive DVs of a segment, then narrower
 // groups for the rest: the loads of a group are issued together
@@ -119,7 +113,8 @@ __device__ __forceinline__ void groups(int len, F&& f) {
 // Walks the segments s, s + step, ... below s1 in groups of U DVs, the loads
 // of a group issued one group ahead (into the next segment at a segment's
 // end), so that a warp's loads are in flight while it computes.  load(q, j, buf)
-// reads DVs j .. j + U - 1 of segment q, clamped to the segment; row(q) forms
+// reads DVs j .. j + U - 1 of segment q (past its end what follows: the arrays
+// are allocated with kSlack elements to spare); row(q) forms
 // what depends on the segment; body(q, j, buf) uses a group, DVs past the
 // segment's end excluded; fold(q) closes a segment.
 template <int U, bool GEN, typename Buf, class Load, class Row, class Body, class Fold>
@@ -319,18 +314,14 @@ __device__ __forceinline__ double xs_dv(const Dv& v, const double* S) {
 // memory (it stays in L1), so that a thread holds five numbers per entity.
 template <int D, bool HZ, bool GEN>
 struct Relax {
-    const double* rec;   // records and tables of all entities (stride n)
+    const double* rec;   // the entity's record and tables: fields and nodes are 32 apart
     const double* tab;
-    unsigned n8, t8, e8; // bytes of a row of the records, of the tables; the entity's offset in one
     double Ux, invRT, qx, RTh, r;
     double Cyz, Syz, eyzr;                  // rows
     double Uy, Uz, qy, qz, rA;              // DV lists
-    __device__ __forceinline__ Relax(const double* rec_, const double* tab_, int n_, int tn, int e, double r_) {
-        rec = rec_;
-        tab = tab_;
-        n8 = 8u * n_;
-        t8 = 8u * tn;
-        e8 = 8u * e;
+    __device__ __forceinline__ Relax(const double* rec_, const double* tab_, int n1d, int e, double r_) {
+        rec = rec_ + slot(e, REC_N);
+        tab = tab_ + slot(e, D * n1d);
         Ux = field(REC_UX);
         invRT = field(REC_INVRT);
         qx = field(REC_QX);
@@ -344,14 +335,14 @@ struct Relax {
             rA = r * field(REC_A);
         }
     }
-    __device__ __forceinline__ double field(int k) const { return __ldg(at(row_of(rec, k, n8), e8)); }
+    __device__ __forceinline__ double field(int k) const { return __ldg(rec + 32 * k); }
     __device__ __forceinline__ void row(const DevMesh& m, const Seg& q, double Y, double Z) {
         if constexpr (!GEN) {
             const double cy = Y - field(REC_UY), vy = field(REC_QY);
-            const double ey = __ldg(at(row_of(tab, m.n1d + q.iy, t8), e8));
+            const double ey = __ldg(tab + 32 * (m.n1d + q.iy));
             if constexpr (D == 3) {
                 const double cz = Z - field(REC_UZ), vz = field(REC_QZ);
-                const double ez = __ldg(at(row_of(tab, 2 * m.n1d + q.iz, t8), e8));
+                const double ez = __ldg(tab + 32 * (2 * m.n1d + q.iz));
                 Cyz = (cy * cy + cz * cz) * invRT;
                 Syz = cy * vy + cz * vz;
                 eyzr = r * ey * ez;
@@ -365,7 +356,7 @@ struct Relax {
     // the Maxwellian factor of DV j of a segment
     __device__ __forceinline__ double factor(const Seg& q, int j) const {
         if constexpr (GEN) return 0.0;
-        else return __ldg(at(row_of(tab, q.ix0 + j, t8), e8));
+        else return __ldg(tab + 32 * (q.ix0 + j));
     }
     __device__ __forceinline__ void operator()(const Dv& v, double e, double g, double h, double K3D, double c0h,
                                                double& go, double& ho) const {
@@ -396,7 +387,7 @@ __device__ __forceinline__ double c0h_of(const DevMesh& m) { return -(D * (m.K +
 
 // a cell's relax factor of this step (fvDVM.C:668); its record holds tau
 __device__ __forceinline__ double cell_r(const StepArgs& a, int c) {
-    const double dt = step_dt(a), tau = __ldg(a.ds.cellrec + REC_R * static_cast<size_t>(a.dm.nC) + c);
+    const double dt = step_dt(a), tau = __ldg(a.ds.cellrec + slot(c, REC_N) + 32 * REC_R);
     return 1.5 * dt / (2.0 * tau + dt);
 }
 
@@ -412,15 +403,14 @@ __global__ void __launch_bounds__(kStream) k_half_step(const __grid_constant__ S
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2 && !a.keep_co) a.ds.co[threadIdx.x] = 0.0;
     const int c = blockIdx.x * kStream + threadIdx.x;
     if (c >= m.nC) return;
-    const size_t nC = static_cast<size_t>(m.nC);
-    const unsigned cb = sizeof(Real) * c, rb = sizeof(Real) * m.nC;
+    const size_t at = slot(c, m.nv_loc);
     const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
-    Relax<D, HZ, GEN> rx(a.ds.cellrec, a.ds.ctab, m.nC, m.nC, c, cell_r(a, c));
+    Relax<D, HZ, GEN> rx(a.ds.cellrec, a.ds.ctab, m.n1d, c, cell_r(a, c));
     const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
-    const Real* __restrict__ g = reinterpret_cast<const Real*>(a.ds.g);
-    const Real* __restrict__ h = reinterpret_cast<const Real*>(a.ds.h);
-    Real* __restrict__ gb = reinterpret_cast<Real*>(a.ds.gbar);
-    Real* __restrict__ hb = reinterpret_cast<Real*>(a.ds.hbar);
+    const Real* __restrict__ g = reinterpret_cast<const Real*>(a.ds.g) + at;
+    const Real* __restrict__ h = reinterpret_cast<const Real*>(a.ds.h) + at;
+    Real* __restrict__ gb = reinterpret_cast<Real*>(a.ds.gbar) + at;
+    Real* __restrict__ hb = reinterpret_cast<Real*>(a.ds.hbar) + at;
     constexpr int U = 4;
     struct Buf {
         Real g[U], h[U];
@@ -429,18 +419,17 @@ __global__ void __launch_bounds__(kStream) k_half_step(const __grid_constant__ S
     walk_dvs<U, GEN, Buf>(
         m, s0, s1, 1,
         [&](const Seg& q, int j, Buf& b) {
-            const Real *gs = g + q.d0 * nC, *hs = h + q.d0 * nC;
+            const Real *gs = g + 32 * static_cast<size_t>(q.d0 + j), *hs = h + 32 * static_cast<size_t>(q.d0 + j);
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int ju = min(j + u, q.len - 1);
-                b.g[u] = __ldcs(at(row_of(gs, ju, rb), cb));
-                if (!HZ) b.h[u] = __ldcs(at(row_of(hs, ju, rb), cb));
-                b.e[u] = rx.factor(q, ju);
+                b.g[u] = __ldcs(gs + 32 * u);
+                if (!HZ) b.h[u] = __ldcs(hs + 32 * u);
+                b.e[u] = rx.factor(q, j + u);
             }
         },
         [&](const Seg& q) { rx.row(m, q, x1[q.iy], x1[q.iz]); },
         [&](const Seg& q, int j, const Buf& b) {
-            Real *gd = gb + q.d0 * nC, *hd = hb + q.d0 * nC;
+            Real *gd = gb + 32 * static_cast<size_t>(q.d0 + j), *hd = hb + 32 * static_cast<size_t>(q.d0 + j);
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 if (j + u < q.len) {
@@ -448,8 +437,8 @@ __global__ void __launch_bounds__(kStream) k_half_step(const __grid_constant__ S
                     double go, ho;
                     rx(dv_at<D, GEN>(m, q, x1, j + u), b.e[u], double(b.g[u]) + gr, HZ ? 0.0 : double(b.h[u]) + hr, K3D,
                        c0h, go, ho);
-                    *at(row_of(gd, j + u, rb), cb) = Real(go - gr);
-                    if (!HZ) *at(row_of(hd, j + u, rb), cb) = Real(ho - hr);
+                    gd[32 * u] = Real(go - gr);
+                    if (!HZ) hd[32 * u] = Real(ho - hr);
                 }
             }
         },
@@ -502,15 +491,15 @@ __device__ __forceinline__ void half_dist(const Real* d, double hdt, const Dv& v
     }
 }
 
-// gradient of cell c's gbar+ (field f of DV row pointer) from the tables in
+// gradient of cell c's gbar+ (f: the field's element of cell 0 and one DV) from the tables in
 // memory: cells with more than kFast neighbours, and tangential faces
 template <int D, typename Real>
 __device__ __forceinline__ void grad_mem(const DevMesh& m, const Real* f, int c, Real* G, int k0, int* err) {
     const size_t nC = static_cast<size_t>(m.nC);
-    const Real f0 = f[c];
+    const Real f0 = f[slot(c, m.nv_loc)];
     for (int k = k0; k < m.nb_max; ++k) {
         const int n = chk(__ldg(m.nbr + k * nC + c), 0, m.nC, err);
-        const Real df = f[n] - f0;
+        const Real df = f[slot(n, m.nv_loc)] - f0;
 #pragma unroll
         for (int q = 0; q < D; ++q) G[q] = fma(Real(__ldg(m.nbr_ls + (k * 3 + q) * nC + c)), df, G[q]);
     }
@@ -529,7 +518,7 @@ __device__ __forceinline__ Real recon_mem(const DevMesh& m, const Real* row, int
 #pragma unroll
     for (int q = 0; q < D; ++q) d[q] = Real(__ldg(m.fgeo + (3 + 3 * side + q) * nF + f));
     half_dist<D, Real, GEN>(d, hdt, v, ix, in_tile, r);
-    return recon<D, Real>(row[c], G, r);
+    return recon<D, Real>(row[slot(c, m.nv_loc)], G, r);
 }
 
 // One thread per cell: the gradient from its neighbours' gbar+ (gathered
@@ -537,7 +526,8 @@ __device__ __forceinline__ Real recon_mem(const DevMesh& m, const Real* row, int
 // every face it is upwind of (one bit per face and DV, DevMesh::upw).  The
 // gradient never leaves registers.  On an exactly tangential internal face
 // no side is upwind; k_tangential averages both there.
-template <int D, typename Real, bool HZ, bool GEN, int NS>
+// Off: 32-bit element offsets wherever the arrays have fewer than 2^32 elements.
+template <int D, typename Real, bool HZ, bool GEN, int NS, typename Off>
 __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant__ StepArgs a) {
     const DevMesh& m = a.dm;
     __shared__ double x1[kMaxN1d], w1[kMaxN1d];
@@ -545,7 +535,7 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
     load_nodes(m, x1, w1);
     const int c = blockIdx.x * kCells + threadIdx.x;
     if (c >= m.nC) return;
-    const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF), pF = static_cast<size_t>(m.pF);
+    const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF);
     const Real* __restrict__ gbar = reinterpret_cast<const Real*>(a.ds.gbar);
     const Real* __restrict__ hbar = reinterpret_cast<const Real*>(a.ds.hbar);
     Real* __restrict__ fvg = reinterpret_cast<Real*>(a.ds.fvg);
@@ -556,19 +546,20 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
     constexpr bool kFold = sizeof(Real) == 8;
     // DVs whose loads are issued together, as the registers allow
     constexpr int kGroup = sizeof(Real) == 4 ? 4 : HZ || D == 2 ? 2 : 1;
-    const unsigned cr = sizeof(Real) * m.nC, fr = sizeof(Real) * m.pF, own = sizeof(Real) * c;
-    unsigned nb[NS], fo[NS];   // byte offsets in a row of cells, of faces
-    unsigned has = 0, side = 0, in_tile = 0;
+    const Off own = static_cast<Off>(slot(c, m.nv_loc));
+    Off nb[NS], fo[NS];   // the neighbours' and faces' elements
+    unsigned uo[NS];      // the faces' upwind words in a segment's row
+    unsigned has = 0, in_tile = 0;
     Real ls[NS][D];
     Real* dist = dist_s + threadIdx.x;   // Cf - C of slot k, dimension q: dist[(k D + q) kCells]
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
-        nb[k] = sizeof(Real) * (k < m.nb_max ? chk(__ldg(m.nbr + k * nC + c), 0, m.nC, a.ds.err) : c);
+        nb[k] = static_cast<Off>(slot(k < m.nb_max ? chk(__ldg(m.nbr + k * nC + c), 0, m.nC, a.ds.err) : c, m.nv_loc));
         const int code = k < m.nf_max ? chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err) : -1;
         const int f = code < 0 ? 0 : code >> 2, sd = code < 0 ? 0 : code & 1;
-        fo[k] = sizeof(Real) * f;
+        fo[k] = static_cast<Off>(slot(f, m.nv_loc));
+        uo[k] = 2u * f + sd;
         has |= (code >= 0 ? 1u : 0u) << k;
-        side |= static_cast<unsigned>(sd) << k;
         if (rounds_rows<D, Real, GEN>(m) && code >= 0) in_tile |= ((code >> 1) & 1u) << k;
 #pragma unroll
         for (int q = 0; q < D; ++q) {
@@ -585,22 +576,22 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
         const uint32_t* us = m.upw + s * nF * 2;
 #pragma unroll
         for (int k = 0; k < NS; ++k)
-            up[k] = (has >> k) & 1u ? __ldg(at(us, fo[k] * (8 / sizeof(Real)) + 4 * ((side >> k) & 1u))) : 0u;
-        const Real *gr = gbar + q.d0 * nC, *hr = hbar + q.d0 * nC;
-        Real *fg = fvg + q.d0 * pF, *fh = fvh + q.d0 * pF;
+            up[k] = (has >> k) & 1u ? __ldg(us + uo[k]) : 0u;
+        const Real *gr = gbar + 32 * static_cast<size_t>(q.d0), *hr = hbar + 32 * static_cast<size_t>(q.d0);
+        Real *fg = fvg + 32 * static_cast<size_t>(q.d0), *fh = fvh + 32 * static_cast<size_t>(q.d0);
         groups<kGroup>(q.len, [&](int j0, auto uc) {
             constexpr int U = decltype(uc)::value;
             Real g0[U], h0[U], G[U][D], H[U][D];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const Real *gj = row_of(gr, j0 + u, cr), *hj = row_of(hr, j0 + u, cr);
+                const Real *gj = gr + 32 * j0, *hj = hr + 32 * j0;
                 Real dg[NS], dh[NS];
-                g0[u] = __ldg(at(gj, own));
-                if (!HZ) h0[u] = __ldg(at(hj, own));
+                g0[u] = __ldg(gj + own + 32 * u);
+                if (!HZ) h0[u] = __ldg(hj + own + 32 * u);
 #pragma unroll
                 for (int k = 0; k < NS; ++k) {
-                    dg[k] = __ldg(at(gj, nb[k]));
-                    if (!HZ) dh[k] = __ldg(at(hj, nb[k]));
+                    dg[k] = __ldg(gj + nb[k] + 32 * u);
+                    if (!HZ) dh[k] = __ldg(hj + nb[k] + 32 * u);
                 }
 #pragma unroll
                 for (int p = 0; p < D; ++p) G[u][p] = H[u][p] = Real(0);
@@ -626,8 +617,8 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
                     v[u].z = Z;
                 }
                 if (more) {
-                    grad_mem<D, Real>(m, gr + j * nC, c, G[u], NS, a.ds.err);
-                    if (!HZ) grad_mem<D, Real>(m, hr + j * nC, c, H[u], NS, a.ds.err);
+                    grad_mem<D, Real>(m, gr + 32 * j, c, G[u], NS, a.ds.err);
+                    if (!HZ) grad_mem<D, Real>(m, hr + 32 * j, c, H[u], NS, a.ds.err);
                     for (int k = NS; k < m.nf_max; ++k) {
                         const int cd = chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err);
                         if (cd < 0) break;
@@ -637,8 +628,8 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
 #pragma unroll
                             for (int p = 0; p < D; ++p) dk[p] = Real(__ldg(m.fgeo + (3 + 3 * sd + p) * nF + f));
                             half_dist<D, Real, GEN>(dk, hdt, v[u], q.ix0 + j, (cd & 2) && rounds_rows<D, Real, GEN>(m), vk);
-                            fg[j * pF + f] = recon<D, Real>(g0[u], G[u], vk);
-                            if (!HZ) fh[j * pF + f] = recon<D, Real>(h0[u], H[u], vk);
+                            fg[slot(f, m.nv_loc) + 32 * j] = recon<D, Real>(g0[u], G[u], vk);
+                            if (!HZ) fh[slot(f, m.nv_loc) + 32 * j] = recon<D, Real>(h0[u], H[u], vk);
                         }
                     }
                 }
@@ -665,8 +656,8 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
                             } else {
                                 half_dist<D, Real, GEN>(dk, hdt, v[u], q.ix0 + j0 + u, (in_tile >> k) & 1u, vk);
                             }
-                            *at(row_of(fg, j0 + u, fr), fo[k]) = recon<D, Real>(g0[u], G[u], vk);
-                            if (!HZ) *at(row_of(fh, j0 + u, fr), fo[k]) = recon<D, Real>(h0[u], H[u], vk);
+                            (fg + 32 * j0 + fo[k])[32 * u] = recon<D, Real>(g0[u], G[u], vk);
+                            if (!HZ) (fh + 32 * j0 + fo[k])[32 * u] = recon<D, Real>(h0[u], H[u], vk);
                         }
                     }
                 }
@@ -763,7 +754,7 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
                 if (code >= 0 && (code >> 2) == f) in_tile = code & 2;
             }
         const Dv v = dv_at<D, GEN>(m, q, x1, j);
-        const size_t rc = (q.d0 + j) * nC, rf = static_cast<size_t>(q.d0 + j) * m.pF + f;
+        const size_t rc = 32 * static_cast<size_t>(q.d0 + j), rf = slot(f, m.nv_loc) + rc;
         const Real* g = reinterpret_cast<const Real*>(a.ds.gbar) + rc;
         reinterpret_cast<Real*>(a.ds.fvg)[rf] =
             Real(0.5) * (recon_mem<D, Real, GEN>(m, g, f, 1, n, hdt, v, q.ix0 + j, in_tile, a.ds.err) +
@@ -780,12 +771,12 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
 // ---------------------------------------------------------------------
 // Rings of face rows in shared memory
 // ---------------------------------------------------------------------
-// The face kernels stream rows of kFaces consecutive faces: one thread copies
-// the rows of a group of DVs with bulk asynchronous copies (a row is
-// contiguous and, its pitch padded to 32, 16-byte aligned), kStages - 1 groups
-// ahead.  The loads need no registers and no address arithmetic in the other
-// threads, and stay in flight while a group is used.  Register prefetch at 24
-// warps per SM reached 4.5 TB/s in k_face_flux and 2.5 in k_face_moments.
+// The face kernels stream their faces' values: a warp's group of DVs is one
+// contiguous run (32 faces x kGroupDv DVs), which one lane copies with a bulk
+// asynchronous copy into the warp's own ring, kStages groups ahead.  The loads
+// need no registers and no address arithmetic in the other lanes, stay in flight
+// while a group is used, and no barrier joins the warps.  Register prefetch at
+// 24 warps per SM reached 4.5 TB/s in k_face_flux and 2.5 in k_face_moments.
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(uint64_t* b) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(b)) : "memory");
@@ -815,22 +806,21 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
                  : "memory");
 }
 
-// Walks the groups of kGroupDv DVs of the segments s0 .. s1 - 1 through a ring
-// of stages.  src(q, j, u, dst row u of a stage, mbarrier) issues the copies of DV
-// j + u; use(q, j, n, stage, last) takes a group of n DVs.  Every thread of the
-// CTA calls this; the set-up before it is visible to all.  Returns false when
-// a wait ran out.
+// Walks the groups of kGroupDv DVs of the segments s0 .. s1 - 1 through the
+// warp's ring.  issue(q, j, n, stage, barrier) copies n DVs from j on, n * dv_bytes in
+// all; use(q, j, n, stage) takes them.  Whole warps call it, the barriers
+// initialised and visible.  Returns false when a wait ran out.
 template <bool GEN, int STAGES, class Issue, class Use>
-__device__ __forceinline__ bool ring_walk(const DevMesh& m, uint64_t* full, int s0, int s1, unsigned row_bytes, Issue&& issue,
+__device__ __forceinline__ bool ring_walk(const DevMesh& m, uint64_t* full, int s0, int s1, unsigned dv_bytes, Issue&& issue,
                                           Use&& use) {
     int ps = s0, pj = 0;   // the producer's position
     auto fill = [&](int stage) {
         if (ps >= s1) return;
         const Seg q = seg_at<GEN>(m, ps);
         const int n = min(kGroupDv, q.len - pj);
-        if (threadIdx.x == 0) {
-            mbar_expect(full + stage, n * row_bytes);
-            for (int u = 0; u < n; ++u) issue(q, pj + u, stage, u, full + stage);
+        if (threadIdx.x % 32 == 0) {
+            mbar_expect(full + stage, n * dv_bytes);
+            issue(q, pj, n, stage, full + stage);
         }
         pj += kGroupDv;
         if (pj >= q.len) {
@@ -844,9 +834,7 @@ __device__ __forceinline__ bool ring_walk(const DevMesh& m, uint64_t* full, int 
     for (int s = s0; s < s1; ++s) {
         const Seg q = seg_at<GEN>(m, s);
         for (int j = 0; j < q.len; j += kGroupDv) {
-            const bool ok = mbar_wait(full + stage, parity);
-            if (ok) use(q, j, min(kGroupDv, q.len - j), stage);
-            if (!__syncthreads_and(ok)) {   // (the barrier that frees the stage)
+            if (!__all_sync(0xffffffffu, mbar_wait(full + stage, parity))) {
                 // give up: let the copies in flight land, within the same limit, before the CTA ends
                 for (int i = 0; i < STAGES; ++i) {
                     mbar_wait(full + stage, parity);
@@ -857,6 +845,8 @@ __device__ __forceinline__ bool ring_walk(const DevMesh& m, uint64_t* full, int 
                 }
                 return false;
             }
+            use(q, j, min(kGroupDv, q.len - j), stage);
+            __syncwarp();   // the stage is free
             fill(stage);
             if (++stage == STAGES) {
                 stage = 0;
@@ -915,7 +905,7 @@ __device__ __forceinline__ void sum_chunks(Finish& f, const double* part, size_t
 
 // one-dimensional Maxwellian factors of the block's entities (layout in
 // dugks_internal.h): D * n1d exponentials each, shared by the CTA's warps
-__device__ __forceinline__ void write_tables(const Finish& f, const DevMesh& m, double* tab, size_t n, int e0, int count) {
+__device__ __forceinline__ void write_tables(const Finish& f, const DevMesh& m, double* tab, int e0, int count) {
     const int lane = threadIdx.x % kLanes, w = threadIdx.x / kLanes;
     if (lane >= count) return;
     for (int i = w; i < m.D * m.n1d; i += kParts) {
@@ -923,7 +913,7 @@ __device__ __forceinline__ void write_tables(const Finish& f, const DevMesh& m, 
         const double x = __ldg(m.X1 + i - k * m.n1d) - f.mac[k][lane];
         double v = exp(-0.5 * x * x * f.mac[3][lane]);
         if (k == 0) v *= f.mac[4][lane];
-        tab[static_cast<size_t>(i) * n + e0 + lane] = v;
+        tab[slot(e0 + lane, m.D * m.n1d) + 32 * i] = v;
     }
 }
 
@@ -970,28 +960,28 @@ __device__ __noinline__ void finish_face(const StepArgs& a, const Consts& kc, in
         fm[8] = tau;
         const double RT = kc.R * T, A = rho * inv_norm(RT, kc.D), invRT = 1.0 / RT;
         const double qs = kc.Pr1 / (5.0 * rho * RT * RT);
-        double* fr = a.ds.facerec + f;
+        double* fr = a.ds.facerec + slot(f, REC_N);
         for (int i = 0; i < 3; ++i) {
             fm[1 + i] = U[i];
             fm[5 + i] = q[i];
-            fr[(REC_UX + i) * nF] = U[i];
-            fr[(REC_QX + i) * nF] = q[i] * qs;
+            fr[(REC_UX + i) * 32] = U[i];
+            fr[(REC_QX + i) * 32] = q[i] * qs;
         }
-        fr[REC_INVRT * nF] = invRT;
-        fr[REC_A * nF] = A;
-        fr[REC_R * nF] = 0.5 * dt / (2.0 * tau + 0.5 * dt);
-        fr[REC_RTH * nF] = RT;
+        fr[REC_INVRT * 32] = invRT;
+        fr[REC_A * 32] = A;
+        fr[REC_R * 32] = 0.5 * dt / (2.0 * tau + 0.5 * dt);
+        fr[REC_RTH * 32] = RT;
         if (f < m.nIF)  // getCoNum, fvDVM.C:2180-2182
             co = __ldg(m.dc + fo) * (sqrt(U[0] * U[0] + U[1] * U[1] + U[2] * U[2]) + m.xi_max_co);
         if (!m.general_dv) {
             // one-dimensional Maxwellian factors (layout in dugks_internal.h)
             for (int k = 0; k < m.D; ++k) {
                 const double Uk = k == 0 ? U[0] : k == 1 ? U[1] : U[2], Ak = k == 0 ? A : 1.0;
-                double* tab = a.ds.ftab + static_cast<size_t>(k) * m.n1d * m.pF + f;
+                double* tab = a.ds.ftab + slot(f, m.D * m.n1d) + 32 * k * m.n1d;
 #pragma unroll 4
                 for (int i = 0; i < m.n1d; ++i) {
                     const double x = __ldg(m.X1 + i) - Uk;
-                    tab[static_cast<size_t>(i) * m.pF] = exp(-0.5 * x * x * invRT) * Ak;
+                    tab[32 * i] = exp(-0.5 * x * x * invRT) * Ak;
                 }
             }
         }
@@ -1013,16 +1003,15 @@ __device__ __noinline__ void write_cellrec(const StepArgs& a, const Consts& k, i
                                            double T, const double* q, double tau) {
     const double RT = k.R * T;
     const double qs = k.Pr1 / (5.0 * rho * RT * RT);
-    const size_t n = static_cast<size_t>(a.dm.nC);
-    double* cr = a.ds.cellrec + c;
+    double* cr = a.ds.cellrec + slot(c, REC_N);
     for (int i = 0; i < 3; ++i) {
-        cr[(REC_UX + i) * n] = U[i];
-        cr[(REC_QX + i) * n] = q[i] * qs;
+        cr[(REC_UX + i) * 32] = U[i];
+        cr[(REC_QX + i) * 32] = q[i] * qs;
     }
-    cr[REC_INVRT * n] = 1.0 / RT;
-    cr[REC_A * n] = rho * inv_norm(RT, k.D);
-    cr[REC_R * n] = tau;
-    cr[REC_RTH * n] = RT;
+    cr[REC_INVRT * 32] = 1.0 / RT;
+    cr[REC_A * 32] = rho * inv_norm(RT, k.D);
+    cr[REC_R * 32] = tau;
+    cr[REC_RTH * 32] = RT;
 }
 
 // macroFlux yes (fvDVM.C:1523-1526, :1613-1679): the cell's old rho, rho U,
@@ -1133,16 +1122,15 @@ __device__ __noinline__ void cell_macros(const StepArgs& a, const Consts& k, int
 
 // record factors of the block's cells for their tables
 __device__ __forceinline__ void tables_of_records(Finish& sm, const StepArgs& a, int c0, int count) {
-    const size_t nC = static_cast<size_t>(a.dm.nC);
     const int lane = threadIdx.x % kLanes;
     if (threadIdx.x < kLanes && lane < count) {
-        const double* cr = a.ds.cellrec + c0 + lane;
-        for (int i = 0; i < 3; ++i) sm.mac[i][lane] = cr[(REC_UX + i) * nC];
-        sm.mac[3][lane] = cr[REC_INVRT * nC];
-        sm.mac[4][lane] = cr[REC_A * nC];
+        const double* cr = a.ds.cellrec + slot(c0 + lane, REC_N);
+        for (int i = 0; i < 3; ++i) sm.mac[i][lane] = cr[(REC_UX + i) * 32];
+        sm.mac[3][lane] = cr[REC_INVRT * 32];
+        sm.mac[4][lane] = cr[REC_A * 32];
     }
     __syncthreads();
-    if (!a.dm.general_dv) write_tables(sm, a.dm, a.ds.ctab, nC, c0, count);
+    if (!a.dm.general_dv) write_tables(sm, a.dm, a.ds.ctab, c0, count);
 }
 
 // Cell macros (updateMacroVol, fvDVM.C:1682-1742) and the coefficient
@@ -1197,9 +1185,8 @@ __device__ __forceinline__ Incoming load_incoming(const StepArgs& a, int b, int 
     if (pt == DUGKS_PATCH_MAXWELL_WALL || pt == DUGKS_PATCH_MIXED) {
         for (int i = 0; i < 3; ++i) t.U[i] = br->U[i];
     } else {
-        const size_t nC = static_cast<size_t>(a.dm.nC);
         const int own = chk(__ldg(a.dm.bface_owner + b), 0, a.dm.nC, a.ds.err);
-        for (int i = 0; i < 3; ++i) t.U[i] = a.ds.cellrec[(REC_UX + i) * nC + own];
+        for (int i = 0; i < 3; ++i) t.U[i] = a.ds.cellrec[slot(own, REC_N) + 32 * (REC_UX + i)];
     }
     return t;
 }
@@ -1210,9 +1197,9 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
                                               int s1, int w, Finish& sm) {
     const DevMesh& m = a.dm;
     Sums<GEN> acc(sm);
-    const size_t nF = static_cast<size_t>(m.nF), nC = static_cast<size_t>(m.nC);
-    Real* fg = reinterpret_cast<Real*>(a.ds.fvg) + f;
-    Real* fh = reinterpret_cast<Real*>(a.ds.fvh) + f;
+    const size_t nF = static_cast<size_t>(m.nF);
+    Real* fg = reinterpret_cast<Real*>(a.ds.fvg) + slot(f, m.nv_loc);
+    Real* fh = reinterpret_cast<Real*>(a.ds.fvh) + slot(f, m.nv_loc);
     const int b = f - m.nIF, pt = __ldg(m.bface_ptype + b);
     const bool wall = pt == DUGKS_PATCH_MAXWELL_WALL, zero_grad = pt == DUGKS_PATCH_ZERO_GRADIENT;
     const bool sym = pt == DUGKS_PATCH_SYMMETRY || pt == DUGKS_PATCH_DVM_SYMMETRY;
@@ -1232,12 +1219,12 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
         Real g4[4] = {0, 0, 0, 0}, h4[4] = {0, 0, 0, 0};
         for (int j = 0; j < q.len; ++j) {
             const int d = q.d0 + j;
-            const size_t o = static_cast<size_t>(d) * m.pF;
+            const size_t o = 32 * static_cast<size_t>(d);
             if ((j & 3) == 0) {
                 // the stored values of four DVs at a time (those of incoming DVs are not used)
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const size_t ou = static_cast<size_t>(min(d + u, q.d0 + q.len - 1)) * m.pF;
+                    const size_t ou = o + 32 * u;
                     g4[u] = fg[ou];
                     if (!HZ) h4[u] = fh[ou];
                 }
@@ -1251,7 +1238,7 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
             double g, h = 0.0;
             if (zero_grad) {
                 // every DV: the owner cell's gbar+ (fvDVM.C:887-891)
-                const size_t oc = static_cast<size_t>(d) * nC + own;
+                const size_t oc = slot(own, m.nv_loc) + o;
                 const Real gc = reinterpret_cast<const Real*>(a.ds.gbar)[oc];
                 fg[o] = gc;
                 g = double(gc) + gr;
@@ -1276,7 +1263,7 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
                             Dv vt = v;
                             (axis == 0 ? vt.x : axis == 1 ? vt.y : vt.z) = x1[n - 1 - i];
                             if (xs_dv(vt, S0) > 0 || t > d) {
-                                const size_t ot = static_cast<size_t>(t) * m.pF;
+                                const size_t ot = 32 * static_cast<size_t>(t);
                                 const double grt = dv_ref<Real, GEN>(m.gref, t), hrt = dv_ref<Real, GEN>(m.href, t);
                                 fg[o] = Real((double(fg[ot]) + grt) - gr);
                                 if (!HZ) fh[o] = Real((double(fh[ot]) + hrt) - hr);
@@ -1329,11 +1316,11 @@ __global__ void __launch_bounds__(kFaces, 5) k_face_moments(const __grid_constan
     const DevMesh& m = a.dm;
     extern __shared__ __align__(128) unsigned char ring_raw[];
     __shared__ double x1[kMaxN1d], w1[kMaxN1d];
-    __shared__ __align__(8) uint64_t full[kStagesM];
+    __shared__ __align__(8) uint64_t full[kParts * kStagesM];
     __shared__ int last;
-    if (threadIdx.x < kStagesM) mbar_init(full + threadIdx.x);
+    if (threadIdx.x < kParts * kStagesM) mbar_init(full + threadIdx.x);
     load_nodes(m, x1, w1);
-    const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF), pF = static_cast<size_t>(m.pF);
+    const size_t nF = static_cast<size_t>(m.nF);
     const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
     // boundary face blocks first: they take longest
     const int nbB = (m.nBF + kLanes - 1) / kLanes, bx = blockIdx.x;
@@ -1355,26 +1342,30 @@ __global__ void __launch_bounds__(kFaces, 5) k_face_moments(const __grid_constan
     __syncthreads();
     SumsRegs acc;
     RowSums rs;
+    // the warp's 32 faces and ring
     constexpr int NH = HZ ? 1 : 2;
-    Real* ring = reinterpret_cast<Real*>(ring_raw);
-    const unsigned row = sizeof(Real) * min(kFaces, m.pF - f0);
+    const int w = warp_id(), wf0 = f0 + w * kLanes;
+    Real* ring = reinterpret_cast<Real*>(ring_raw) + w * kStagesM * NH * kGroupDv * kLanes;
+    const Real* wg = fg + slot(wf0, m.nv_loc);
+    const Real* wh = fh + slot(wf0, m.nv_loc);
     const bool ok = ring_walk<GEN, kStagesM>(
-        m, full, s0, s1, NH * row,
-        [&](const Seg& q, int j, int stage, int u, uint64_t* bar) {
-            Real* dst = ring + (stage * NH * kGroupDv + u) * kFaces;
-            bulk_load(dst, fg + (q.d0 + j) * pF + f0, row, bar);
-            if (!HZ) bulk_load(dst + kGroupDv * kFaces, fh + (q.d0 + j) * pF + f0, row, bar);
+        m, full + w * kStagesM, s0, wf0 < m.nIF ? s1 : s0, NH * kLanes * sizeof(Real),
+        [&](const Seg& q, int j, int n, int stage, uint64_t* bar) {
+            Real* dst = ring + stage * NH * kGroupDv * kLanes;
+            const size_t o = kLanes * static_cast<size_t>(q.d0 + j);
+            bulk_load(dst, wg + o, n * kLanes * sizeof(Real), bar);
+            if (!HZ) bulk_load(dst + kGroupDv * kLanes, wh + o, n * kLanes * sizeof(Real), bar);
         },
         [&](const Seg& q, int j, int n, int stage) {
-            const Real* st = ring + stage * NH * kGroupDv * kFaces + threadIdx.x;
+            const Real* st = ring + stage * NH * kGroupDv * kLanes + threadIdx.x % kLanes;
             // FP32 storage: the deviations only; the reference part is added once below
             groups<kGroupDv>(n, [&](int i, auto uc) {
                 constexpr int U = decltype(uc)::value;
-                const Real* su = st + i * kFaces;
+                const Real* su = st + i * kLanes;
 #pragma unroll
                 for (int u = 0; u < U; ++u)
                     add_dv<D, HZ, GEN>(acc, rs, w1, q, dv_at<D, GEN>(m, q, x1, j + i + u), j + i + u,
-                                       double(su[u * kFaces]), HZ ? 0.0 : double(su[(kGroupDv + u) * kFaces]));
+                                       double(su[u * kLanes]), HZ ? 0.0 : double(su[(kGroupDv + u) * kLanes]));
             });
             if constexpr (!GEN) {
                 if (j + kGroupDv >= q.len) {
@@ -1430,7 +1421,7 @@ __device__ __noinline__ void boundary_flux(const StepArgs& a, const double* x1, 
     const size_t nF = static_cast<size_t>(m.nF);
     const double S[3] = {__ldg(m.fgeo + f), __ldg(m.fgeo + nF + f), __ldg(m.fgeo + 2 * nF + f)};
     const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
-    Relax<D, HZ, GEN> rx(a.ds.facerec, a.ds.ftab, m.nF, m.pF, f, __ldg(a.ds.facerec + REC_R * nF + f));
+    Relax<D, HZ, GEN> rx(a.ds.facerec, a.ds.ftab, m.n1d, f, __ldg(a.ds.facerec + slot(f, REC_N) + 32 * REC_R));
     const int b = f - m.nIF, pt = __ldg(m.bface_ptype + b);
     const int li = chk(__ldg(m.bface_patch_local + b), 0, m.nIF, a.ds.err);
     rx.RTh = m.R * a.ds.fm[static_cast<size_t>(li) * 9 + 4];
@@ -1444,15 +1435,14 @@ __device__ __noinline__ void boundary_flux(const StepArgs& a, const double* x1, 
         Real g4[4] = {0, 0, 0, 0}, h4[4] = {0, 0, 0, 0};
         for (int j = 0; j < q.len; ++j) {
             const Dv v = dv_at<D, GEN>(m, q, x1, j);
-            const size_t o = static_cast<size_t>(q.d0 + j) * m.pF + f;
+            const size_t o = slot(f, m.nv_loc) + 32 * static_cast<size_t>(q.d0 + j);
             Real* pg = reinterpret_cast<Real*>(a.ds.fvg) + o;
             Real* ph = reinterpret_cast<Real*>(a.ds.fvh) + o;
             if ((j & 3) == 0) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const size_t ou = static_cast<size_t>(min(u, q.len - 1 - j)) * m.pF;
-                    g4[u] = pg[ou];
-                    if (!HZ) h4[u] = ph[ou];
+                    g4[u] = pg[32 * u];
+                    if (!HZ) h4[u] = ph[32 * u];
                 }
             }
             const Real gv = g4[0], hv = h4[0];
@@ -1485,8 +1475,8 @@ __global__ void __launch_bounds__(kFaces, 4) k_face_flux(const __grid_constant__
     const DevMesh& m = a.dm;
     extern __shared__ __align__(128) unsigned char ring_raw[];
     __shared__ double x1[kMaxN1d], w1[kMaxN1d];
-    __shared__ __align__(8) uint64_t full[kStagesF];
-    if (threadIdx.x < kStagesF) mbar_init(full + threadIdx.x);
+    __shared__ __align__(8) uint64_t full[kParts * kStagesF];
+    if (threadIdx.x < kParts * kStagesF) mbar_init(full + threadIdx.x);
     load_nodes(m, x1, w1);
     asm volatile("fence.proxy.async;" ::: "memory");
     __syncthreads();
@@ -1501,25 +1491,31 @@ __global__ void __launch_bounds__(kFaces, 4) k_face_flux(const __grid_constant__
     const int f0 = (bx - nbB) * kFaces;
     const bool active = f0 + threadIdx.x < m.nIF;
     const int f = active ? f0 + threadIdx.x : f0;
-    const size_t nF = static_cast<size_t>(m.nF), pF = static_cast<size_t>(m.pF);
-    const unsigned fb = sizeof(Real) * f, fr = sizeof(Real) * m.pF;
-    Real* fg = reinterpret_cast<Real*>(a.ds.fvg);
-    Real* fh = reinterpret_cast<Real*>(a.ds.fvh);
+    const size_t nF = static_cast<size_t>(m.nF);
+    Real* fg = reinterpret_cast<Real*>(a.ds.fvg) + slot(f, m.nv_loc);
+    Real* fh = reinterpret_cast<Real*>(a.ds.fvh) + slot(f, m.nv_loc);
     const double S[3] = {__ldg(m.fgeo + f), __ldg(m.fgeo + nF + f), __ldg(m.fgeo + 2 * nF + f)};
     const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
-    Relax<D, HZ, GEN> rx(a.ds.facerec, a.ds.ftab, m.nF, m.pF, f, __ldg(a.ds.facerec + REC_R * nF + f));
+    Relax<D, HZ, GEN> rx(a.ds.facerec, a.ds.ftab, m.n1d, f, __ldg(a.ds.facerec + slot(f, REC_N) + 32 * REC_R));
     double p2 = 0, p3 = 0;
+    // the warp's 32 faces and ring
     constexpr int NH = HZ ? 1 : 2;
-    Real* ring = reinterpret_cast<Real*>(ring_raw);
-    double* ring_e = reinterpret_cast<double*>(ring + kStagesF * NH * kGroupDv * kFaces);
-    const unsigned cnt = min(kFaces, m.pF - f0), row = sizeof(Real) * cnt;
+    const int w = warp_id(), wf0 = f0 + w * kLanes;
+    Real* ring = reinterpret_cast<Real*>(ring_raw) + w * kStagesF * NH * kGroupDv * kLanes;
+    double* ring_e = reinterpret_cast<double*>(reinterpret_cast<Real*>(ring_raw) + kStagesF * NH * kGroupDv * kFaces) +
+                     w * kStagesF * kGroupDv * kLanes;
+    const Real* wg = reinterpret_cast<const Real*>(a.ds.fvg) + slot(wf0, m.nv_loc);
+    const Real* wh = reinterpret_cast<const Real*>(a.ds.fvh) + slot(wf0, m.nv_loc);
+    const double* we = a.ds.ftab + slot(wf0, D * m.n1d);
     const bool ok = ring_walk<GEN, kStagesF>(
-        m, full, s0, s1, NH * row + (GEN ? 0 : 8 * cnt),
-        [&](const Seg& q, int j, int stage, int u, uint64_t* bar) {
-            Real* dst = ring + (stage * NH * kGroupDv + u) * kFaces;
-            bulk_load(dst, fg + (q.d0 + j) * pF + f0, row, bar);
-            if (!HZ) bulk_load(dst + kGroupDv * kFaces, fh + (q.d0 + j) * pF + f0, row, bar);
-            if (!GEN) bulk_load(ring_e + (stage * kGroupDv + u) * kFaces, a.ds.ftab + (q.ix0 + j) * pF + f0, 8 * cnt, bar);
+        m, full + w * kStagesF, s0, wf0 < m.nIF ? s1 : s0, kLanes * (NH * sizeof(Real) + (GEN ? 0 : sizeof(double))),
+        [&](const Seg& q, int j, int n, int stage, uint64_t* bar) {
+            Real* dst = ring + stage * NH * kGroupDv * kLanes;
+            const size_t o = kLanes * static_cast<size_t>(q.d0 + j);
+            bulk_load(dst, wg + o, n * kLanes * sizeof(Real), bar);
+            if (!HZ) bulk_load(dst + kGroupDv * kLanes, wh + o, n * kLanes * sizeof(Real), bar);
+            if (!GEN)
+                bulk_load(ring_e + stage * kGroupDv * kLanes, we + kLanes * (q.ix0 + j), n * kLanes * sizeof(double), bar);
         },
         [&](const Seg& q, int j, int n, int stage) {
             if constexpr (!GEN) {
@@ -1530,9 +1526,9 @@ __global__ void __launch_bounds__(kFaces, 4) k_face_flux(const __grid_constant__
                     p3 = D == 3 ? __dmul_rn(Z, S[2]) : 0.0;
                 }
             }
-            const Real* st = ring + stage * NH * kGroupDv * kFaces + threadIdx.x;
-            const double* se = ring_e + stage * kGroupDv * kFaces + threadIdx.x;
-            Real *gs = fg + (q.d0 + j) * pF, *hs = fh + (q.d0 + j) * pF;
+            const Real* st = ring + stage * NH * kGroupDv * kLanes + threadIdx.x % kLanes;
+            const double* se = ring_e + stage * kGroupDv * kLanes + threadIdx.x % kLanes;
+            Real *gs = fg + 32 * static_cast<size_t>(q.d0 + j), *hs = fh + 32 * static_cast<size_t>(q.d0 + j);
             groups<HZ ? kGroupDv : 4>(n, [&](int i, auto uc) {
                 constexpr int U = decltype(uc)::value;
 #pragma unroll
@@ -1544,11 +1540,12 @@ __global__ void __launch_bounds__(kFaces, 4) k_face_flux(const __grid_constant__
                     const int d = q.d0 + j + i + u;
                     const double gr = dv_ref<Real, GEN>(m.gref, d), hr = dv_ref<Real, GEN>(m.href, d);
                     double gf, hf;
-                    rx(v, GEN ? 0.0 : se[(i + u) * kFaces], double(st[(i + u) * kFaces]) + gr,
-                       HZ ? 0.0 : double(st[(kGroupDv + i + u) * kFaces]) + hr, K3D, c0h, gf, hf);
+                    const Real* su = st + i * kLanes;
+                    rx(v, GEN ? 0.0 : (se + i * kLanes)[u * kLanes], double(su[u * kLanes]) + gr,
+                       HZ ? 0.0 : double(su[(kGroupDv + u) * kLanes]) + hr, K3D, c0h, gf, hf);
                     if (active) {
-                        *at(row_of(gs, i + u, fr), fb) = Real(xs * (gf - gr));
-                        if (!HZ) *at(row_of(hs, i + u, fr), fb) = Real(xs * (hf - hr));
+                        (gs + 32 * i)[32 * u] = Real(xs * (gf - gr));
+                        if (!HZ) (hs + 32 * i)[32 * u] = Real(xs * (hf - hr));
                     }
                 }
             });
@@ -1562,7 +1559,7 @@ __global__ void __launch_bounds__(kFaces, 4) k_face_flux(const __grid_constant__
 // One thread per cell and DV segment: gathers the fluxes of the cell's faces
 // (owner side: outflow, negated), updates g~ in place and sums the cell's
 // moments.  A flux is read by the two cells of its face; the second read hits L2.
-template <int D, typename Real, bool HZ, bool GEN, int NS>
+template <int D, typename Real, bool HZ, bool GEN, int NS, typename Off>
 __global__ void __launch_bounds__(kLanes* kParts, 4) k_update(const __grid_constant__ StepArgs a,
                                                            const __grid_constant__ Consts kc) {
     const DevMesh& m = a.dm;
@@ -1571,7 +1568,7 @@ __global__ void __launch_bounds__(kLanes* kParts, 4) k_update(const __grid_const
     load_nodes(m, x1, w1);
     const int c0 = blockIdx.x * kLanes, count = min(kLanes, m.nC - c0);
     const int lane = threadIdx.x % kLanes, c = c0 + lane;
-    const size_t nC = static_cast<size_t>(m.nC), pF = static_cast<size_t>(m.pF);
+    const size_t nC = static_cast<size_t>(m.nC);
     const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
     const int w = warp_id();
     Sums<GEN> acc(sm);
@@ -1581,22 +1578,21 @@ __global__ void __launch_bounds__(kLanes* kParts, 4) k_update(const __grid_const
     double accx[5] = {0, 0, 0, 0, 0};
     const bool fx = GEN && m.macro_flux;
     if (lane < count) {
-        Real* g = reinterpret_cast<Real*>(a.ds.g);
-        Real* h = reinterpret_cast<Real*>(a.ds.h);
-        const unsigned cb = sizeof(Real) * c, cr = sizeof(Real) * m.nC, fr = sizeof(Real) * m.pF;
+        Real* g = reinterpret_cast<Real*>(a.ds.g) + slot(c, m.nv_loc);
+        Real* h = reinterpret_cast<Real*>(a.ds.h) + slot(c, m.nv_loc);
         const Real* __restrict__ fvg = reinterpret_cast<const Real*>(a.ds.fvg);
         const Real* __restrict__ fvh = reinterpret_cast<const Real*>(a.ds.fvh);
         const double dtV = step_dt(a) * __ldg(m.invV + c);
         const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
-        Relax<D, HZ, GEN> rx(a.ds.cellrec, a.ds.ctab, m.nC, m.nC, c, cell_r(a, c));
+        Relax<D, HZ, GEN> rx(a.ds.cellrec, a.ds.ctab, m.n1d, c, cell_r(a, c));
         // faces with their sign (owner side: outflow, -1); an absent slot
         // repeats the first face with sign 0
-        unsigned fc[NS];
+        Off fc[NS];
         Real sign[NS];
 #pragma unroll
         for (int k = 0; k < NS; ++k) {
             const int code = k < m.nf_max ? chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err) : -1;
-            fc[k] = code < 0 ? fc[0] : sizeof(Real) * (code >> 2);
+            fc[k] = code < 0 ? fc[0] : static_cast<Off>(slot(code >> 2, m.nv_loc));
             sign[k] = code < 0 ? Real(0) : (code & 1) ? Real(1) : Real(-1);
         }
         RowSums rs;
@@ -1608,18 +1604,17 @@ __global__ void __launch_bounds__(kLanes* kParts, 4) k_update(const __grid_const
         walk_dvs<U, GEN, Buf>(
             m, s0 + w, s1, kParts,
             [&](const Seg& q, int j, Buf& b) {
-                const Real *gs = g + q.d0 * nC, *hs = h + q.d0 * nC, *fgs = fvg + q.d0 * pF, *fhs = fvh + q.d0 * pF;
+                const size_t d = 32 * static_cast<size_t>(q.d0 + j);
+                const Real *gs = g + d, *hs = h + d, *fgs = fvg + d, *fhs = fvh + d;
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int ju = min(j + u, q.len - 1);
-                    b.g[u] = *at(row_of(gs, ju, cr), cb);
-                    if (!HZ) b.h[u] = *at(row_of(hs, ju, cr), cb);
-                    b.e[u] = rx.factor(q, ju);
-                    const Real *fgj = row_of(fgs, ju, fr), *fhj = row_of(fhs, ju, fr);
+                    b.g[u] = gs[32 * u];
+                    if (!HZ) b.h[u] = hs[32 * u];
+                    b.e[u] = rx.factor(q, j + u);
 #pragma unroll
                     for (int k = 0; k < NS; ++k) {
-                        b.fg[u][k] = __ldg(at(fgj, fc[k]));
-                        if (!HZ) b.fh[u][k] = __ldg(at(fhj, fc[k]));
+                        b.fg[u][k] = __ldg(fgs + fc[k] + 32 * u);
+                        if (!HZ) b.fh[u][k] = __ldg(fhs + fc[k] + 32 * u);
                     }
                 }
             },
@@ -1628,8 +1623,9 @@ __global__ void __launch_bounds__(kLanes* kParts, 4) k_update(const __grid_const
                 rs = RowSums();
             },
             [&](const Seg& q, int j, const Buf& b) {
-                Real *gs = g + q.d0 * nC, *hs = h + q.d0 * nC;
-                const Real *fgs = fvg + q.d0 * pF, *fhs = fvh + q.d0 * pF;
+                const size_t dj = 32 * static_cast<size_t>(q.d0 + j);
+                Real *gs = g + dj, *hs = h + dj;
+                const Real *fgs = fvg + dj, *fhs = fvh + dj;
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     if (j + u < q.len) {
@@ -1649,7 +1645,7 @@ __global__ void __launch_bounds__(kLanes* kParts, 4) k_update(const __grid_const
                             for (int k = NS; k < m.nf_max; ++k) {
                                 const int code = chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err);
                                 if (code < 0) break;
-                                const int of = (j + u) * m.pF + (code >> 2);
+                                const size_t of = slot(code >> 2, m.nv_loc) + 32 * u;
                                 const Real sk = (code & 1) ? Real(1) : Real(-1);
                                 sg = fma(sk, __ldg(fgs + of), sg);
                                 if (!HZ) sh = fma(sk, __ldg(fhs + of), sh);
@@ -1658,11 +1654,11 @@ __global__ void __launch_bounds__(kLanes* kParts, 4) k_update(const __grid_const
                         // the update in FP64, one rounding to the storage type; with a
                         // reference, -g/3 + 4/3 gbar+ - ref = -(g - ref)/3 + 4/3 (gbar+ - ref)
                         const Real gn = Real(fma(-1.0 / 3, double(b.g[u]), fma(4.0 / 3, gb - gr, double(sg) * dtV)));
-                        *at(row_of(gs, j + u, cr), cb) = gn;
+                        gs[32 * u] = gn;
                         Real hn = 0;
                         if (!HZ) {
                             hn = Real(fma(-1.0 / 3, double(b.h[u]), fma(4.0 / 3, hb - hr, double(sh) * dtV)));
-                            *at(row_of(hs, j + u, cr), cb) = hn;
+                            hs[32 * u] = hn;
                         }
                         add_dv<D, HZ, GEN>(acc, rs, w1, q, v, j + u, double(gn), double(hn));
                         if constexpr (GEN) {
@@ -1720,14 +1716,14 @@ __global__ void __launch_bounds__(kLanes* kParts) k_state_moments(const __grid_c
     const int w = warp_id();
     Sums<GEN> acc(sm);
     if (lane < count) {
-        const Real* __restrict__ g = reinterpret_cast<const Real*>(a.ds.g) + c;
-        const Real* __restrict__ h = reinterpret_cast<const Real*>(a.ds.h) + c;
+        const Real* __restrict__ g = reinterpret_cast<const Real*>(a.ds.g) + slot(c, m.nv_loc);
+        const Real* __restrict__ h = reinterpret_cast<const Real*>(a.ds.h) + slot(c, m.nv_loc);
         for (int s = s0 + w; s < s1; s += kParts) {
             const Seg q = seg_at<GEN>(m, s);
             RowSums rs;
 #pragma unroll 4
             for (int j = 0; j < q.len; ++j) {
-                const size_t o = static_cast<size_t>(q.d0 + j) * nC;
+                const size_t o = 32 * static_cast<size_t>(q.d0 + j);
                 const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j), hr = dv_ref<Real, GEN>(m.href, q.d0 + j);
                 add_dv<D, false, GEN>(acc, rs, w1, q, dv_at<D, GEN>(m, q, x1, j), j, double(__ldg(g + o)) + gr,
                                       double(__ldg(h + o)) + hr);
@@ -1756,6 +1752,8 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
     const Consts k = make_consts(m, a.dt);
     const int nbF = blocks(m.nIF, kFaces) + blocks(m.nBF, kLanes);
     const bool quad = m.nb_max <= 4 && m.nf_max <= 4;   // quadrilaterals, tetrahedra: shorter face lists
+    // (with room for the constant offsets of a group)
+    const bool wide = static_cast<unsigned long long>(m.nv_loc) * m.pF + kSlack >= 1ull << 32;
     switch (which) {
         case KERNEL_HALF_STEP: {
             const int nb = blocks(m.nC, kStream);
@@ -1765,8 +1763,9 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
         case KERNEL_FACE_VALUES: {
             const int nb = blocks(m.nC, kCells);
             const dim3 grid(nb, stream_chunks(m, nb));
-            if (quad) k_face_values<D, Real, HZ, GEN, 4><<<grid, kCells, 0, s>>>(a);
-            else k_face_values<D, Real, HZ, GEN, kFast><<<grid, kCells, 0, s>>>(a);
+            if (wide) k_face_values<D, Real, HZ, GEN, kFast, size_t><<<grid, kCells, 0, s>>>(a);
+            else if (quad) k_face_values<D, Real, HZ, GEN, 4, unsigned><<<grid, kCells, 0, s>>>(a);
+            else k_face_values<D, Real, HZ, GEN, kFast, unsigned><<<grid, kCells, 0, s>>>(a);
             break;
         }
         case KERNEL_TANGENTIAL: {
@@ -1785,8 +1784,9 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
         }
         case KERNEL_UPDATE: {
             const dim3 grid(blocks(m.nC, kLanes), a.chunks);
-            if (quad) k_update<D, Real, HZ, GEN, 4><<<grid, kLanes * kParts, 0, s>>>(a, k);
-            else k_update<D, Real, HZ, GEN, kFast><<<grid, kLanes * kParts, 0, s>>>(a, k);
+            if (wide) k_update<D, Real, HZ, GEN, kFast, size_t><<<grid, kLanes * kParts, 0, s>>>(a, k);
+            else if (quad) k_update<D, Real, HZ, GEN, 4, unsigned><<<grid, kLanes * kParts, 0, s>>>(a, k);
+            else k_update<D, Real, HZ, GEN, kFast, unsigned><<<grid, kLanes * kParts, 0, s>>>(a, k);
             break;
         }
         case KERNEL_STATE_MOMENTS:
