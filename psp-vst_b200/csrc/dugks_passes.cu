@@ -521,6 +521,16 @@ __device__ __forceinline__ Real recon_mem(const DevMesh& m, const Real* row, int
     return recon<D, Real>(row[slot(c, m.nv_loc)], G, r);
 }
 
+// *p = v where cond is not 0, as one predicated store
+__device__ __forceinline__ void store_if(double* p, double v, unsigned cond) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q st.global.f64 [%0], %1;\n}\n" ::"l"(p), "d"(v), "r"(cond)
+                 : "memory");
+}
+__device__ __forceinline__ void store_if(float* p, float v, unsigned cond) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q st.global.f32 [%0], %1;\n}\n" ::"l"(p), "f"(v), "r"(cond)
+                 : "memory");
+}
+
 // One thread per cell: the gradient from its neighbours' gbar+ (gathered
 // through L1: a CTA's cells are a compact block of the mesh) and the value of
 // every face it is upwind of (one bit per face and DV, DevMesh::upw).  The
@@ -531,7 +541,9 @@ template <int D, typename Real, bool HZ, bool GEN, int NS, typename Off>
 __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant__ StepArgs a) {
     const DevMesh& m = a.dm;
     __shared__ double x1[kMaxN1d], w1[kMaxN1d];
+    constexpr bool kRowDist = sizeof(Real) == 4 && !GEN;   // v's y and z components formed once per row
     __shared__ Real dist_s[NS * D * kCells];
+    __shared__ Real row_s[kRowDist ? NS * (D - 1) * kCells : 1];
     load_nodes(m, x1, w1);
     const int c = blockIdx.x * kCells + threadIdx.x;
     if (c >= m.nC) return;
@@ -577,6 +589,14 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
 #pragma unroll
         for (int k = 0; k < NS; ++k)
             up[k] = (has >> k) & 1u ? __ldg(us + uo[k]) : 0u;
+        Real* rowd = row_s + (kRowDist ? threadIdx.x : 0);
+        if constexpr (kRowDist) {
+#pragma unroll
+            for (int k = 0; k < NS; ++k) {
+                rowd[k * (D - 1) * kCells] = rounded_dist<Real>(dist[(k * D + 1) * kCells], Real(hdt), Y);
+                if (D == 3) rowd[(k * (D - 1) + 1) * kCells] = rounded_dist<Real>(dist[(k * D + D - 1) * kCells], Real(hdt), Z);
+            }
+        }
         const Real *gr = gbar + 32 * static_cast<size_t>(q.d0), *hr = hbar + 32 * static_cast<size_t>(q.d0);
         Real *fg = fvg + 32 * static_cast<size_t>(q.d0), *fh = fvh + 32 * static_cast<size_t>(q.d0);
         groups<kGroup>(q.len, [&](int j0, auto uc) {
@@ -639,27 +659,34 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
                     if (!HZ) h0[u] = recon<D, Real>(h0[u], H[u], t);
                 }
             }
+            // every face's value, stored where the cell is upwind: without
+            // branches, which cost more than the values not needed
 #pragma unroll
             for (int k = 0; k < NS; ++k) {
                 const unsigned bits = up[k] >> j0;
-                if (bits & ((1u << U) - 1u)) {
-                    Real dk[D];
+                Real* pg = fg + 32 * j0 + fo[k];
+                Real* ph = fh + 32 * j0 + fo[k];
+                Real dk[D];
 #pragma unroll
-                    for (int p = 0; p < D; ++p) dk[p] = dist[(k * D + p) * kCells];
+                for (int p = 0; p < D; ++p)
+                    dk[p] = kRowDist && p > 0 ? rowd[(k * (D - 1) + p - 1) * kCells] : dist[(k * D + p) * kCells];
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        if (bits & (1u << u)) {
-                            Real vk[D];
-                            if constexpr (kFold) {
+                for (int u = 0; u < U; ++u) {
+                    Real vk[D];
+                    if constexpr (kFold) {
 #pragma unroll
-                                for (int p = 0; p < D; ++p) vk[p] = dk[p];
-                            } else {
-                                half_dist<D, Real, GEN>(dk, hdt, v[u], q.ix0 + j0 + u, (in_tile >> k) & 1u, vk);
-                            }
-                            (fg + 32 * j0 + fo[k])[32 * u] = recon<D, Real>(g0[u], G[u], vk);
-                            if (!HZ) (fh + 32 * j0 + fo[k])[32 * u] = recon<D, Real>(h0[u], H[u], vk);
-                        }
+                        for (int p = 0; p < D; ++p) vk[p] = dk[p];
+                    } else if constexpr (kRowDist) {
+                        vk[0] = ((in_tile >> k) & 1u) && ((q.ix0 + j0 + u + 1) & 6) == 0
+                                    ? rounded_dist<Real>(dk[0], Real(hdt), v[u].x)
+                                    : fused_dist<Real>(dk[0], Real(hdt), v[u].x);
+#pragma unroll
+                        for (int p = 1; p < D; ++p) vk[p] = dk[p];
+                    } else {
+                        half_dist<D, Real, GEN>(dk, hdt, v[u], q.ix0 + j0 + u, (in_tile >> k) & 1u, vk);
                     }
+                    store_if(pg + 32 * u, recon<D, Real>(g0[u], G[u], vk), bits & (1u << u));
+                    if (!HZ) store_if(ph + 32 * u, recon<D, Real>(h0[u], H[u], vk), bits & (1u << u));
                 }
             }
         });
@@ -1596,16 +1623,19 @@ __global__ void __launch_bounds__(kLanes* kParts, 4) k_update(const __grid_const
             sign[k] = code < 0 ? Real(0) : (code & 1) ? Real(1) : Real(-1);
         }
         RowSums rs;
-        constexpr int U = HZ || sizeof(Real) == 4 ? 2 : 1;
-        struct Buf {
-            Real g[U], h[U], fg[U][NS], fh[U][NS];
-            double e[U];
-        };
-        walk_dvs<U, GEN, Buf>(
-            m, s0 + w, s1, kParts,
-            [&](const Seg& q, int j, Buf& b) {
-                const size_t d = 32 * static_cast<size_t>(q.d0 + j);
-                const Real *gs = g + d, *hs = h + d, *fgs = fvg + d, *fhs = fvh + d;
+        for (int s = s0 + w; s < s1; s += kParts) {
+            const Seg q = seg_at<GEN>(m, s);
+            rx.row(m, q, x1[q.iy], x1[q.iz]);
+            rs = RowSums();
+            groups<HZ || sizeof(Real) == 4 ? 4 : 2>(q.len, [&](int j, auto uc) {
+                constexpr int U = decltype(uc)::value;
+                struct {
+                    Real g[U], h[U], fg[U][NS], fh[U][NS];
+                    double e[U];
+                } b;
+                const size_t dj = 32 * static_cast<size_t>(q.d0 + j);
+                Real *gs = g + dj, *hs = h + dj;
+                const Real *fgs = fvg + dj, *fhs = fvh + dj;
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     b.g[u] = gs[32 * u];
@@ -1617,18 +1647,9 @@ __global__ void __launch_bounds__(kLanes* kParts, 4) k_update(const __grid_const
                         if (!HZ) b.fh[u][k] = __ldg(fhs + fc[k] + 32 * u);
                     }
                 }
-            },
-            [&](const Seg& q) {
-                rx.row(m, q, x1[q.iy], x1[q.iz]);
-                rs = RowSums();
-            },
-            [&](const Seg& q, int j, const Buf& b) {
-                const size_t dj = 32 * static_cast<size_t>(q.d0 + j);
-                Real *gs = g + dj, *hs = h + dj;
-                const Real *fgs = fvg + dj, *fhs = fvh + dj;
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    if (j + u < q.len) {
+                    {
                         const Dv v = dv_at<D, GEN>(m, q, x1, j + u);
                         const double gr = dv_ref<Real, GEN>(m.gref, q.d0 + j + u),
                                      hr = dv_ref<Real, GEN>(m.href, q.d0 + j + u);
@@ -1673,10 +1694,9 @@ __global__ void __launch_bounds__(kLanes* kParts, 4) k_update(const __grid_const
                         }
                     }
                 }
-            },
-            [&](const Seg& q) {
-                if constexpr (!GEN) row_fold<D>(acc, rs, row_const<D>(x1, w1, q));
             });
+            if constexpr (!GEN) row_fold<D>(acc, rs, row_const<D>(x1, w1, q));
+        }
         if constexpr (sizeof(Real) == 4 && !GEN) {
             // FP32 storage: the reference's moments once
             if (blockIdx.y == 0 && threadIdx.x < kLanes)
