@@ -471,21 +471,21 @@ __device__ __forceinline__ Real rounded_dist(Real d, Real hdt, double x) {
     if constexpr (sizeof(Real) == 4) return __fsub_rn(d, __fmul_rn(hdt, Real(x)));
     else return fma(-hdt, x, d);
 }
-// (2-D rows that do not split into eights round the x product too at the
-// first and last of every eight nodes, on faces inside a tile: in_tile)
+// (2-D rows round the x product too at the first and last of every eight
+// nodes, on faces inside a tile)
 template <int D, typename Real, bool GEN>
-__device__ __forceinline__ bool rounds_rows(const DevMesh& m) {
-    return D == 2 && sizeof(Real) == 4 && !GEN && (m.n1d & 7) != 0;
-}
+constexpr bool kRoundsRows = D == 2 && sizeof(Real) == 4 && !GEN;
+__device__ __forceinline__ bool rounds_node(int ix) { return ((ix + 1) & 6) == 0; }
+// rounded: the x product is rounded first
 template <int D, typename Real, bool GEN>
-__device__ __forceinline__ void half_dist(const Real* d, double hdt, const Dv& v, int ix, bool in_tile, Real* r) {
+__device__ __forceinline__ void half_dist(const Real* d, double hdt, const Dv& v, bool rounded, Real* r) {
     if constexpr (GEN && sizeof(Real) == 4) {
         r[0] = d[0] - Real(hdt * v.x);
         r[1] = d[1] - Real(hdt * v.y);
         if (D == 3) r[D - 1] = d[D - 1] - Real(hdt * v.z);
     } else {
         const Real h = Real(hdt);
-        r[0] = in_tile && ((ix + 1) & 6) == 0 ? rounded_dist<Real>(d[0], h, v.x) : fused_dist<Real>(d[0], h, v.x);
+        r[0] = rounded ? rounded_dist<Real>(d[0], h, v.x) : fused_dist<Real>(d[0], h, v.x);
         r[1] = rounded_dist<Real>(d[1], h, v.y);
         if (D == 3) r[D - 1] = rounded_dist<Real>(d[D - 1], h, v.z);
     }
@@ -508,7 +508,7 @@ __device__ __forceinline__ void grad_mem(const DevMesh& m, const Real* f, int c,
 // the reconstruction from one side of face f, everything from memory
 template <int D, typename Real, bool GEN>
 __device__ __forceinline__ Real recon_mem(const DevMesh& m, const Real* row, int f, int side, int c, double hdt,
-                                          const Dv& v, int ix, bool in_tile, int* err) {
+                                          const Dv& v, bool rounded, int* err) {
     const size_t nF = static_cast<size_t>(m.nF);
     Real G[D];
 #pragma unroll
@@ -517,7 +517,7 @@ __device__ __forceinline__ Real recon_mem(const DevMesh& m, const Real* row, int
     Real d[D], r[D];
 #pragma unroll
     for (int q = 0; q < D; ++q) d[q] = Real(__ldg(m.fgeo + (3 + 3 * side + q) * nF + f));
-    half_dist<D, Real, GEN>(d, hdt, v, ix, in_tile, r);
+    half_dist<D, Real, GEN>(d, hdt, v, rounded, r);
     return recon<D, Real>(row[slot(c, m.nv_loc)], G, r);
 }
 
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
         fo[k] = static_cast<Off>(slot(f, m.nv_loc));
         uo[k] = 2u * f + sd;
         has |= (code >= 0 ? 1u : 0u) << k;
-        if (rounds_rows<D, Real, GEN>(m) && code >= 0) in_tile |= ((code >> 1) & 1u) << k;
+        if (kRoundsRows<D, Real, GEN> && code >= 0) in_tile |= ((code >> 1) & 1u) << k;
 #pragma unroll
         for (int q = 0; q < D; ++q) {
             ls[k][q] = k < m.nb_max ? Real(__ldg(m.nbr_ls + (k * 3 + q) * nC + c)) : Real(0);
@@ -647,7 +647,8 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
                             Real dk[D], vk[D];
 #pragma unroll
                             for (int p = 0; p < D; ++p) dk[p] = Real(__ldg(m.fgeo + (3 + 3 * sd + p) * nF + f));
-                            half_dist<D, Real, GEN>(dk, hdt, v[u], q.ix0 + j, (cd & 2) && rounds_rows<D, Real, GEN>(m), vk);
+                            half_dist<D, Real, GEN>(dk, hdt, v[u], kRoundsRows<D, Real, GEN> && (cd & 2) && rounds_node(q.ix0 + j),
+                                                     vk);
                             fg[slot(f, m.nv_loc) + 32 * j] = recon<D, Real>(g0[u], G[u], vk);
                             if (!HZ) fh[slot(f, m.nv_loc) + 32 * j] = recon<D, Real>(h0[u], H[u], vk);
                         }
@@ -677,13 +678,13 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
 #pragma unroll
                         for (int p = 0; p < D; ++p) vk[p] = dk[p];
                     } else if constexpr (kRowDist) {
-                        vk[0] = ((in_tile >> k) & 1u) && ((q.ix0 + j0 + u + 1) & 6) == 0
+                        vk[0] = ((in_tile >> k) & 1u) && rounds_node(q.ix0 + j0 + u)
                                     ? rounded_dist<Real>(dk[0], Real(hdt), v[u].x)
                                     : fused_dist<Real>(dk[0], Real(hdt), v[u].x);
 #pragma unroll
                         for (int p = 1; p < D; ++p) vk[p] = dk[p];
                     } else {
-                        half_dist<D, Real, GEN>(dk, hdt, v[u], q.ix0 + j0 + u, (in_tile >> k) & 1u, vk);
+                        half_dist<D, Real, GEN>(dk, hdt, v[u], false, vk);
                     }
                     store_if(pg + 32 * u, recon<D, Real>(g0[u], G[u], vk), bits & (1u << u));
                     if (!HZ) store_if(ph + 32 * u, recon<D, Real>(h0[u], H[u], vk), bits & (1u << u));
@@ -774,23 +775,23 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
         const int f = chk(t.x, 0, m.nIF, a.ds.err), s = chk(t.y / kSeg, 0, m.n_seg, a.ds.err), j = t.y % kSeg;
         const Seg q = seg_at<GEN>(m, s);
         const int o = chk(__ldg(m.fown + f), 0, m.nC, a.ds.err), n = chk(__ldg(m.fnei + f), 0, m.nC, a.ds.err);
-        bool in_tile = false;
-        if (rounds_rows<D, Real, GEN>(m))
+        bool rounded = false;
+        if (kRoundsRows<D, Real, GEN> && rounds_node(q.ix0 + j))
             for (int k = 0; k < m.nf_max; ++k) {
                 const int code = __ldg(m.cface + k * nC + o);
-                if (code >= 0 && (code >> 2) == f) in_tile = code & 2;
+                if (code >= 0 && (code >> 2) == f) rounded = code & 2;
             }
         const Dv v = dv_at<D, GEN>(m, q, x1, j);
         const size_t rc = 32 * static_cast<size_t>(q.d0 + j), rf = slot(f, m.nv_loc) + rc;
         const Real* g = reinterpret_cast<const Real*>(a.ds.gbar) + rc;
         reinterpret_cast<Real*>(a.ds.fvg)[rf] =
-            Real(0.5) * (recon_mem<D, Real, GEN>(m, g, f, 1, n, hdt, v, q.ix0 + j, in_tile, a.ds.err) +
-                         recon_mem<D, Real, GEN>(m, g, f, 0, o, hdt, v, q.ix0 + j, in_tile, a.ds.err));
+            Real(0.5) * (recon_mem<D, Real, GEN>(m, g, f, 1, n, hdt, v, rounded, a.ds.err) +
+                         recon_mem<D, Real, GEN>(m, g, f, 0, o, hdt, v, rounded, a.ds.err));
         if (!HZ) {
             const Real* h = reinterpret_cast<const Real*>(a.ds.hbar) + rc;
             reinterpret_cast<Real*>(a.ds.fvh)[rf] =
-                Real(0.5) * (recon_mem<D, Real, GEN>(m, h, f, 1, n, hdt, v, q.ix0 + j, in_tile, a.ds.err) +
-                             recon_mem<D, Real, GEN>(m, h, f, 0, o, hdt, v, q.ix0 + j, in_tile, a.ds.err));
+                Real(0.5) * (recon_mem<D, Real, GEN>(m, h, f, 1, n, hdt, v, rounded, a.ds.err) +
+                             recon_mem<D, Real, GEN>(m, h, f, 0, o, hdt, v, rounded, a.ds.err));
         }
     }
 }
