@@ -471,6 +471,8 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dm.tang = nullptr;
     dm.n_tang = 0;
     dm.bface_patch_local = d_bpl;
+    dm.tang_at = nullptr;
+    dm.tang_seg = nullptr;
     dm.bface_ptype = d_bpt;
     dm.bface_owner = d_bown;
     dm.bface_mirror = d_bmir;
@@ -585,7 +587,17 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     if (ce == cudaSuccess && n_tang > 0) {
         int2* d_tang = nullptr;
         if ((st = dev_alloc(h, &d_tang, n_tang))) return *out = h, st;
-        ce = dugks::launch_list_tangential(dm, d_tang, d_count + 1, h->stream);
+        uint2* at = nullptr;
+        unsigned* seg = nullptr;
+        if (h->precision == DUGKS_FP32C && !dvl && n_tang < (1ull << 32)) {
+            if ((st = dev_alloc(h, &at, static_cast<size_t>(dm.pF / 32) * dm.nv_loc)) ||
+                (st = dev_alloc(h, &seg, static_cast<size_t>(dm.pF / 32) * n_seg)) ||
+                (st = dev_alloc(h, &ds.tang_res, 2 * n_tang)))
+                return *out = h, st;
+            dm.tang_at = at;
+            dm.tang_seg = seg;
+        }
+        ce = dugks::launch_list_tangential(dm, d_tang, d_count + 1, at, seg, h->stream);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);
         dm.tang = d_tang;
         dm.n_tang = static_cast<long long>(n_tang);

@@ -69,11 +69,16 @@ cudaError_t configure_kernels(int D, int precision);
 // DevMesh::upw from the geometry and the DV set, with the number of tangential
 // (internal face, DV) pairs, and their list DevMesh::tang (counters start at 0)
 cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, unsigned long long* n_tang, cudaStream_t s);
-cudaError_t launch_list_tangential(const DevMesh& m, int2* list, unsigned long long* cursor, cudaStream_t s);
+cudaError_t launch_list_tangential(const DevMesh& m, int2* list, unsigned long long* cursor, uint2* at, unsigned* seg,
+                                   cudaStream_t s);
 // partial moments of all chunks summed into chunk 0 (n doubles per chunk)
 cudaError_t launch_sum_chunks(double* part, int chunks, size_t n, cudaStream_t s);
 // cell records and Maxwellian tables rebuilt from the cell macros
 cudaError_t launch_cell_records(const StepArgs& a, cudaStream_t s);
+// entries first .. first + n - 1 of the caller's [dv][cell] array of g~ (or
+// h~) at buf, from the state (get) or into it
+cudaError_t launch_state_order(const StepArgs& a, int precision, bool second, bool get, const int32_t* iperm, double* buf,
+                               size_t first, size_t n, cudaStream_t s);
 // the next time step of an adaptive run from the Courant maximum (in ds.co)
 // and dt_in, as src/setDeltaTvar.H:34-48 adjusts it; also stored to *hist
 // when hist is not null

@@ -735,7 +735,7 @@ __global__ void k_upwind_bits(const DevMesh m, uint32_t* upw, unsigned long long
 // the list of those pairs (DevMesh::tang), pairs of one DV and consecutive
 // faces together
 template <bool GEN>
-__global__ void k_list_tangential(const DevMesh m, int2* list, unsigned long long* cursor) {
+__global__ void k_list_tangential(const DevMesh m, int2* list, unsigned long long* cursor, uint2* at, unsigned* seg) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     const size_t nF = static_cast<size_t>(m.nF);
     for (int s = blockIdx.y; s < m.n_seg; s += gridDim.y) {
@@ -745,13 +745,17 @@ __global__ void k_list_tangential(const DevMesh m, int2* list, unsigned long lon
             const uint2 up = reinterpret_cast<const uint2*>(m.upw)[s * nF + f];
             t = ~(up.x | up.y) & (q.len == 32 ? 0xffffffffu : (1u << q.len) - 1u);
         }
-        if (!__any_sync(0xffffffffu, t != 0)) continue;
+        const unsigned any = __reduce_or_sync(0xffffffffu, t);
+        const bool first = threadIdx.x % 32 == 0 && f < m.nIF;
+        if (seg && first) seg[(f / 32) * static_cast<size_t>(m.n_seg) + s] = any;
+        if (!any) continue;
         for (int j = 0; j < q.len; ++j) {
             const unsigned who = __ballot_sync(0xffffffffu, (t >> j) & 1u);
             if (!who) continue;
             unsigned long long base = 0;
             if (threadIdx.x % 32 == 0) base = atomicAdd(cursor, static_cast<unsigned long long>(__popc(who)));
             base = __shfl_sync(0xffffffffu, base, 0);
+            if (at && first) at[(f / 32) * static_cast<size_t>(m.nv_loc) + q.d0 + j] = make_uint2(who, static_cast<unsigned>(base));
             if ((t >> j) & 1u) list[base + __popc(who & ((1u << (threadIdx.x % 32)) - 1u))] = make_int2(f, s * kSeg + j);
         }
     }
@@ -775,24 +779,27 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
         const int f = chk(t.x, 0, m.nIF, a.ds.err), s = chk(t.y / kSeg, 0, m.n_seg, a.ds.err), j = t.y % kSeg;
         const Seg q = seg_at<GEN>(m, s);
         const int o = chk(__ldg(m.fown + f), 0, m.nC, a.ds.err), n = chk(__ldg(m.fnei + f), 0, m.nC, a.ds.err);
-        bool rounded = false;
-        if (kRoundsRows<D, Real, GEN> && rounds_node(q.ix0 + j))
+        bool in_tile = false;
+        if constexpr (sizeof(Real) == 4 && !GEN)
             for (int k = 0; k < m.nf_max; ++k) {
                 const int code = __ldg(m.cface + k * nC + o);
-                if (code >= 0 && (code >> 2) == f) rounded = code & 2;
+                if (code >= 0 && (code >> 2) == f) in_tile = code & 2;
             }
+        const bool rounded = kRoundsRows<D, Real, GEN> && in_tile && rounds_node(q.ix0 + j);
         const Dv v = dv_at<D, GEN>(m, q, x1, j);
         const size_t rc = 32 * static_cast<size_t>(q.d0 + j), rf = slot(f, m.nv_loc) + rc;
-        const Real* g = reinterpret_cast<const Real*>(a.ds.gbar) + rc;
-        reinterpret_cast<Real*>(a.ds.fvg)[rf] =
-            Real(0.5) * (recon_mem<D, Real, GEN>(m, g, f, 1, n, hdt, v, rounded, a.ds.err) +
-                         recon_mem<D, Real, GEN>(m, g, f, 0, o, hdt, v, rounded, a.ds.err));
-        if (!HZ) {
-            const Real* h = reinterpret_cast<const Real*>(a.ds.hbar) + rc;
-            reinterpret_cast<Real*>(a.ds.fvh)[rf] =
-                Real(0.5) * (recon_mem<D, Real, GEN>(m, h, f, 1, n, hdt, v, rounded, a.ds.err) +
-                             recon_mem<D, Real, GEN>(m, h, f, 0, o, hdt, v, rounded, a.ds.err));
-        }
+        auto average = [&](const void* bar, void* fv, float* res) {
+            const Real* b = reinterpret_cast<const Real*>(bar) + rc;
+            const Real vn = recon_mem<D, Real, GEN>(m, b, f, 1, n, hdt, v, rounded, a.ds.err);
+            const Real vo = recon_mem<D, Real, GEN>(m, b, f, 0, o, hdt, v, rounded, a.ds.err);
+            const Real mean = Real(0.5) * (vn + vo);
+            reinterpret_cast<Real*>(fv)[rf] = mean;
+            // what the moments of a face between tiles add: its two halves, not their rounded sum
+            if constexpr (sizeof(Real) == 4)
+                if (res) res[i] = in_tile ? 0.f : float(0.5 * double(vo) + 0.5 * double(vn) - double(mean));
+        };
+        average(a.ds.gbar, a.ds.fvg, a.ds.tang_res);
+        if (!HZ) average(a.ds.hbar, a.ds.fvh, a.ds.tang_res ? a.ds.tang_res + m.n_tang : nullptr);
     }
 }
 
@@ -1376,6 +1383,16 @@ __global__ void __launch_bounds__(kFaces, 5) k_face_moments(const __grid_constan
     Real* ring = reinterpret_cast<Real*>(ring_raw) + w * kStagesM * NH * kGroupDv * kLanes;
     const Real* wg = fg + slot(wf0, m.nv_loc);
     const Real* wh = fh + slot(wf0, m.nv_loc);
+    // FP32 storage: what rounding took from the mean of tangential pairs
+    unsigned tang = 0;   // the segment's DVs with such pairs among the warp's faces
+    auto tang_rest = [&](int d, double& g, double& h) {
+        const uint2 t = __ldg(m.tang_at + static_cast<size_t>(wf0 / kLanes) * m.nv_loc + d);
+        const unsigned bit = 1u << (threadIdx.x % kLanes);
+        if (!(t.x & bit)) return;
+        const size_t i = t.y + static_cast<unsigned>(__popc(t.x & (bit - 1)));
+        g += double(a.ds.tang_res[i]);
+        if (!HZ) h += double(a.ds.tang_res[m.n_tang + i]);
+    };
     const bool ok = ring_walk<GEN, kStagesM>(
         m, full + w * kStagesM, s0, wf0 < m.nIF ? s1 : s0, NH * kLanes * sizeof(Real),
         [&](const Seg& q, int j, int n, int stage, uint64_t* bar) {
@@ -1386,14 +1403,23 @@ __global__ void __launch_bounds__(kFaces, 5) k_face_moments(const __grid_constan
         },
         [&](const Seg& q, int j, int n, int stage) {
             const Real* st = ring + stage * NH * kGroupDv * kLanes + threadIdx.x % kLanes;
+            if constexpr (sizeof(Real) == 4 && !GEN) {
+                if (m.tang_at && j == 0)
+                    tang = __ldg(m.tang_seg + static_cast<size_t>(wf0 / kLanes) * m.n_seg +
+                                 ((q.d0 - q.ix0) / m.n1d << (m.n1d > kSeg)) + q.ix0 / kSeg);
+            }
             // FP32 storage: the deviations only; the reference part is added once below
             groups<kGroupDv>(n, [&](int i, auto uc) {
                 constexpr int U = decltype(uc)::value;
                 const Real* su = st + i * kLanes;
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    add_dv<D, HZ, GEN>(acc, rs, w1, q, dv_at<D, GEN>(m, q, x1, j + i + u), j + i + u,
-                                       double(su[u * kLanes]), HZ ? 0.0 : double(su[(kGroupDv + u) * kLanes]));
+                for (int u = 0; u < U; ++u) {
+                    double g = double(su[u * kLanes]), h = HZ ? 0.0 : double(su[(kGroupDv + u) * kLanes]);
+                    if constexpr (sizeof(Real) == 4 && !GEN) {
+                        if ((tang >> (j + i + u)) & 1u) tang_rest(q.d0 + j + i + u, g, h);
+                    }
+                    add_dv<D, HZ, GEN>(acc, rs, w1, q, dv_at<D, GEN>(m, q, x1, j + i + u), j + i + u, g, h);
+                }
             });
             if constexpr (!GEN) {
                 if (j + kGroupDv >= q.len) {
@@ -1885,11 +1911,12 @@ cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, unsigned long lo
     return cudaGetLastError();
 }
 
-cudaError_t launch_list_tangential(const DevMesh& m, int2* list, unsigned long long* cursor, cudaStream_t s) {
+cudaError_t launch_list_tangential(const DevMesh& m, int2* list, unsigned long long* cursor, uint2* at, unsigned* seg,
+                                   cudaStream_t s) {
     const int nb = blocks(m.nIF, 128);
     const dim3 grid(nb, std::min(m.n_seg, std::max(1, 148 * 32 / std::max(nb, 1))));
-    if (m.general_dv) k_list_tangential<true><<<grid, 128, 0, s>>>(m, list, cursor);
-    else k_list_tangential<false><<<grid, 128, 0, s>>>(m, list, cursor);
+    if (m.general_dv) k_list_tangential<true><<<grid, 128, 0, s>>>(m, list, cursor, at, seg);
+    else k_list_tangential<false><<<grid, 128, 0, s>>>(m, list, cursor, at, seg);
     return cudaGetLastError();
 }
 
