@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -44,7 +45,7 @@ template <typename T>
 int upload(dugks_handle* h, T** p, const std::vector<T>& v) {
     int st = dev_alloc(h, p, v.size());
     if (st) return st;
-    if (!v.empty()) CUDA_TRY(h, cudaMemcpy(*p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    if (!v.empty()) CUDA_TRY(h, cudaMemcpyAsync(*p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, h->stream));
     return DUGKS_OK;
 }
 
@@ -153,7 +154,7 @@ static int alloc_h(dugks_handle* h) {
     unsigned char *b = nullptr, *f = nullptr;
     if (int st = dev_alloc(h, &b, nvc * rs)) return st;
     if (int st = dev_alloc(h, &f, nfv * rs)) return st;
-    CUDA_TRY(h, cudaMemset(f, 0, nfv * rs));
+    CUDA_TRY(h, cudaMemsetAsync(f, 0, nfv * rs, h->stream));
     h->ds.hbar = b;
     h->ds.fvh = f;
     return DUGKS_OK;
@@ -442,7 +443,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     double *d_X1, *d_W1;
     if ((st = upload(h, &d_X1, h->X1)) || (st = upload(h, &d_W1, h->W1)) ||
         (st = upload(h, &d_row_yz, row_yz)) || (st = upload(h, &d_xi, h->xi)) || (st = upload(h, &d_w, h->w)) ||
-        (st = upload(h, &d_nbr, t.nbr)) ||
+        (st = upload(h, &d_nbr, t.nbr)) || (st = upload(h, &h->d_iperm, t.iperm)) ||
         (st = upload(h, &d_nls, t.nbr_ls)) || (st = upload(h, &d_cf, t.cface)) || (st = upload(h, &d_geo, t.fgeo)) ||
         (st = upload(h, &d_fo, t.fown)) || (st = upload(h, &d_fn, t.fnei)) || (st = upload(h, &d_for, t.forig)) ||
         (st = upload(h, &d_invV, invV)) || (st = upload(h, &d_bpl, h->bface_patch_local)) ||
@@ -470,9 +471,9 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dm.upw = d_upw;
     dm.tang = nullptr;
     dm.n_tang = 0;
-    dm.bface_patch_local = d_bpl;
     dm.tang_at = nullptr;
     dm.tang_seg = nullptr;
+    dm.bface_patch_local = d_bpl;
     dm.bface_ptype = d_bpt;
     dm.bface_owner = d_bown;
     dm.bface_mirror = d_bmir;
@@ -535,7 +536,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     ds.fvg = p;
     // face values start at zero: the slots of incoming boundary DVs are read
     // (and not used) before any kernel writes them
-    if (cudaMemset(ds.fvg, 0, nfv * rs) != cudaSuccess) return fail(DUGKS_ERR_CUDA, "cudaMemset of the face values");
+    if (cudaMemsetAsync(ds.fvg, 0, nfv * rs, h->stream) != cudaSuccess) return fail(DUGKS_ERR_CUDA, "cudaMemset of the face values");
     // where h stays identically zero its step arrays are left out until a
     // nonzero h~ is loaded (alloc_h)
     if (!can_skip_h(h) && (st = alloc_h(h))) return *out = h, st;
@@ -572,9 +573,9 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         dm.gref = dm.href = nullptr;
         ds.refmom = nullptr;
     }
-    ce = cudaMemset(ds.err, 0, 4 * sizeof(int));
+    ce = cudaMemsetAsync(ds.err, 0, 4 * sizeof(int), h->stream);
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, cudaGetErrorString(ce));
-    ce = cudaMemset(ds.done, 0, n_done * sizeof(int));
+    ce = cudaMemsetAsync(ds.done, 0, n_done * sizeof(int), h->stream);
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, cudaGetErrorString(ce));
     ce = dugks::configure_kernels(h->D, h->precision);
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, std::string("configure kernels: ") + cudaGetErrorString(ce));
@@ -1358,47 +1359,37 @@ int dugks_get_df(dugks_handle* h, const int32_t* cells, int32_t n, double* g_out
     return DUGKS_OK;
 }
 
+// g~ and h~ in the caller's [dv][cell] order of doubles, from the state (get)
+// or into it.  The copies go straight between the caller's arrays and gbar+'s
+// buffer, which holds nothing between steps, in as many parts as its size
+// asks for (one in FP64), and k_state_order puts each part in order.
 static int state_io(dugks_handle* h, double* g, double* hh, const double* gi, const double* hi, bool get) {
     if (!h) return DUGKS_ERR_ARG;
     if (!h->initialised) return set_error(h, DUGKS_ERR_STATE, "state access before dugks_set_macros");
-    const size_t rs = real_size(h);
-    const size_t nvc = static_cast<size_t>(h->dm.nv_loc) * h->dm.pC;
-    std::vector<unsigned char> buf(nvc * rs);
-    const std::vector<int32_t>& perm = h->tiling.perm;
+    const size_t n = static_cast<size_t>(h->dm.nv_loc) * h->nC;
+    const size_t part = (static_cast<size_t>(h->dm.nv_loc) * h->dm.pC + dugks::kSlack) * real_size(h) / sizeof(double);
+    const dugks::StepArgs a = make_args(h, 0.0);
+    double* buf = static_cast<double*>(h->ds.gbar);
+    // (a step whose phases the caller drives may be half done: gbar+ is kept)
+    std::unique_ptr<void, cudaError_t (*)(void*)> own(nullptr, cudaFree);
+    if (h->shard_phase_next != 0) {
+        CUDA_TRY(h, cudaMalloc(&buf, part * sizeof(double)));
+        own.reset(buf);
+    }
     for (int which = 0; which < 2; ++which) {
-        void* dev = which == 0 ? h->ds.g : h->ds.h;
-        const std::vector<double>& ref = which == 0 ? h->gref : h->href;
-        if (get) {
-            double* dst = which == 0 ? g : hh;
-            if (!dst) continue;
-            CUDA_TRY(h, cudaMemcpy(buf.data(), dev, nvc * rs, cudaMemcpyDeviceToHost));
-            for (int d = 0; d < h->dm.nv_loc; ++d)
-                for (int c = 0; c < h->nC; ++c) {
-                    const size_t s = (static_cast<size_t>(c / 32) * h->dm.nv_loc + d) * 32 + c % 32;
-                    const size_t o = static_cast<size_t>(d) * h->nC + perm[c];
-                    if (rs == sizeof(double)) std::memcpy(&dst[o], &buf[s * rs], sizeof(double));
-                    else {
-                        float fv;
-                        std::memcpy(&fv, &buf[s * rs], sizeof fv);
-                        dst[o] = ref.empty() ? fv : fv + ref[d];
-                    }
-                }
-        } else {
-            const double* src = which == 0 ? gi : hi;
-            if (!src) return set_error(h, DUGKS_ERR_ARG, "dugks_set_state: null array");
-            for (int d = 0; d < h->dm.nv_loc; ++d)
-                for (int c = 0; c < h->nC; ++c) {
-                    const size_t s = (static_cast<size_t>(c / 32) * h->dm.nv_loc + d) * 32 + c % 32;
-                    const size_t o = static_cast<size_t>(d) * h->nC + perm[c];
-                    if (rs == sizeof(double)) std::memcpy(&buf[s * rs], &src[o], sizeof(double));
-                    else {
-                        const float fv = static_cast<float>(ref.empty() ? src[o] : src[o] - ref[d]);
-                        std::memcpy(&buf[s * rs], &fv, sizeof fv);
-                    }
-                }
-            CUDA_TRY(h, cudaMemcpy(dev, buf.data(), nvc * rs, cudaMemcpyHostToDevice));
+        double* dst = which == 0 ? g : hh;
+        const double* src = which == 0 ? gi : hi;
+        if (get && !dst) continue;
+        if (!get && !src) return set_error(h, DUGKS_ERR_ARG, "dugks_set_state: null array");
+        for (size_t i = 0; i < n; i += part) {
+            const size_t k = std::min(part, n - i);
+            if (!get) CUDA_TRY(h, cudaMemcpyAsync(buf, src + i, k * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+            CUDA_TRY(h, dugks::launch_state_order(a, h->precision, which == 1, get, h->d_iperm, buf, i, k, h->stream));
+            h->launches += 1;
+            if (get) CUDA_TRY(h, cudaMemcpyAsync(dst + i, buf, k * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
         }
     }
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     return DUGKS_OK;
 }
 

@@ -215,6 +215,7 @@ struct dugks_handle {
     dugks::DevMesh dm{};
     dugks::DevState ds{};
     std::vector<void*> allocations;
+    int32_t* d_iperm = nullptr;     // Tiling::iperm
     double* d_dt = nullptr;         // [2] device time steps of adaptive stepping (ping-pong)
     double* d_hist = nullptr;       // time steps of the last adaptive call
     int32_t hist_cap = 0;

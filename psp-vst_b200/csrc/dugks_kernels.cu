@@ -42,6 +42,25 @@ __global__ void k_init_state(const StepArgs a) {
     }
 }
 
+// The caller's [dv][cell] order of doubles and the state's blocks of 32 cells,
+// an FP32 state with its reference taken off or added.  The caller's side is
+// contiguous, the state's in runs of a mesh row inside a bisection block.  The
+// host did this entry by entry before (46 of the 54 ms of a 3,721-cell,
+// 784-DV state set, stepped twice and read back).
+template <typename Real, bool GET>
+__global__ void k_state_order(const int nC, const int nv, const int32_t* __restrict__ iperm, Real* __restrict__ state,
+                              const double* __restrict__ ref, double* __restrict__ buf, const size_t first, const size_t n) {
+    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
+         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+        const size_t d = (first + i) / nC;
+        const int c = iperm[first + i - d * nC];
+        Real* s = state + (static_cast<size_t>(c / 32) * nv + d) * 32 + c % 32;
+        const double r = sizeof(Real) == 4 && ref ? ref[d] : 0.0;
+        if (GET) buf[i] = sizeof(Real) == 4 && ref ? double(*s) + r : double(*s);
+        else *s = sizeof(Real) == 4 && ref ? Real(buf[i] - r) : Real(buf[i]);
+    }
+}
+
 // wall: inComingByRho_f = sum_{xi.S<0} -w (xi.S) M/rho (fvDVM.C:598-617) and
 // the raw moments of the incoming wall DFs per unit rho_w
 // (xi.S <= 0, fvDVM.C:1079-1092)
@@ -217,6 +236,24 @@ cudaError_t launch_init(const StepArgs& a, int precision, cudaStream_t s) {
     else k_init_state<float><<<1184, 256, 0, s>>>(a);
     if (cudaError_t e = launch_cell_records(a, s)) return e;
     if (a.dm.nBF > 0) k_init_wall<<<a.dm.nBF, 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_state_order(const StepArgs& a, int precision, bool second, bool get, const int32_t* iperm, double* buf,
+                               size_t first, size_t n, cudaStream_t s) {
+    const DevMesh& m = a.dm;
+    void* st = second ? a.ds.h : a.ds.g;
+    const double* ref = second ? m.href : m.gref;
+    const unsigned nb = static_cast<unsigned>(std::min<size_t>((n + 255) / 256, 1u << 16));
+    if (precision == DUGKS_FP64) {
+        double* p = static_cast<double*>(st);
+        if (get) k_state_order<double, true><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n);
+        else k_state_order<double, false><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n);
+    } else {
+        float* p = static_cast<float*>(st);
+        if (get) k_state_order<float, true><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n);
+        else k_state_order<float, false><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n);
+    }
     return cudaGetLastError();
 }
 
