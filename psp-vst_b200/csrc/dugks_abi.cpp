@@ -368,19 +368,38 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         row1 = static_cast<int>(static_cast<int64_t>(rows) * (shard->rank + 1) / shard->world);
     }
     const int rows_loc = row1 - row0;
-    // DV segments, and DV chunks of the face and cell reductions: about three
-    // waves of 128-thread CTAs (four per SM), a chunk at least one segment per
-    // warp of its CTA; a given dv_chunks is taken as far as there are segments
+    // DV segments, and DV chunks of the face and cell reductions; a given
+    // dv_chunks is taken as far as there are segments
     const int seg_per_row = dvl ? 1 : (h->n1d + dugks::kSeg - 1) / dugks::kSeg;
     const int n_seg = dvl ? (rows_loc + dugks::kSeg - 1) / dugks::kSeg : rows_loc * seg_per_row;
+    // A chunk costs a write of its partial sums and a term of the finishing
+    // sum, so there are at most as many as a chunk has segments.  Up to that,
+    // cells: one wave of CTAs (4 an SM) where it leaves a warp eight segments
+    // or less, else the fewest chunks that fill the last of at most four waves
+    // best.  (28x28 DVs, 3,721 cells: 5 chunks 253 us a step, 7, a wave and a
+    // third, 261 and 16 290; 14,400 cells: 1 chunk 627 us, 4 658; 12,096 cells,
+    // 1,331 listed DVs: 3 and 6 chunks 1,450 us, 5 1,506 and 8 1,590.)
+    const int cap = std::max(1, static_cast<int>(std::sqrt(static_cast<double>(n_seg))));
     auto chunks_for = [&](int entities) {
-        const int nb = (entities + 31) / 32, want = (148 * 4 * 3 + nb - 1) / nb;
-        return opt.dv_chunks > 0 ? std::min(opt.dv_chunks, n_seg) : std::max(1, std::min(want, n_seg / 4));
+        if (opt.dv_chunks > 0) return std::min(opt.dv_chunks, n_seg);
+        const long long nb = (entities + 31) / 32, slots = 148 * 4;
+        const int one = static_cast<int>(std::min<long long>(slots / nb, cap));
+        if (one > 0 && n_seg <= 8 * 4 * one) return one;
+        int best = 1;
+        double fill = 0;
+        for (int c = 1; c <= cap && (c == 1 || nb * c <= 4 * slots); ++c) {
+            const long long waves = (nb * c + slots - 1) / slots;
+            const double f = static_cast<double>(nb * c) / (waves * slots);
+            if (f > 1.01 * fill) best = c, fill = f;
+        }
+        return best;
     };
-    // (the face reduction: one thread per internal face)
+    // the face reduction, one thread per internal face: four waves (3,721
+    // cells: 28 chunks 260 us a step, 5 234; 1,728 cells, 10^3 DVs: 46 chunks 222 us, 10 171)
     auto chunks_f_for = [&](int entities) {
+        if (opt.dv_chunks > 0) return std::min(opt.dv_chunks, n_seg);
         const int nb = (entities + 127) / 128, want = (148 * 5 * 4 + nb - 1) / nb;
-        return opt.dv_chunks > 0 ? std::min(opt.dv_chunks, n_seg) : std::max(1, std::min(want, n_seg));
+        return std::max(1, std::min(want, cap));
     };
     h->chunks = chunks_for(nC);
     h->chunks_f = chunks_f_for(nF);

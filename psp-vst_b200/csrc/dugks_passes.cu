@@ -1786,10 +1786,12 @@ __global__ void __launch_bounds__(kLanes* kParts) k_state_moments(const __grid_c
 int blocks(int n, int per) { return (n + per - 1) / per; }
 
 // CTAs along the DV segments for the kernels without a reduction: about
-// eight CTAs of 128 threads on each of 148 SMs, four times over, so that the
-// last wave is short
-int stream_chunks(const DevMesh& m, int nb) {
-    const int target = 148 * 8 * 4;
+// eight CTAs of 128 threads on each of 148 SMs, `waves` times over, so that the
+// last wave is short.  (Two for k_face_flux, whose rings and boundary records
+// each CTA sets up: 1,728 cells and 10^3 DVs 147 us a step, four 159; the
+// others are level from two to eight.)
+int stream_chunks(const DevMesh& m, int nb, int waves = 4) {
+    const int target = 148 * 8 * waves;
     return std::max(1, std::min({m.n_seg, (target + nb - 1) / std::max(nb, 1), 65535}));
 }
 
@@ -1826,7 +1828,7 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
             break;
         case KERNEL_FACE_FLUX: {
             k_face_flux<D, Real, HZ, GEN>
-                <<<dim3(nbF, stream_chunks(m, nbF)), kFaces, ring_flux<Real, HZ, GEN>(), s>>>(a);
+                <<<dim3(nbF, stream_chunks(m, nbF, 2)), kFaces, ring_flux<Real, HZ, GEN>(), s>>>(a);
             break;
         }
         case KERNEL_UPDATE: {
