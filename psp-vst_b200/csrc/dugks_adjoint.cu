@@ -339,9 +339,9 @@ extern "C" int dugks_adjoint_run(dugks_handle* h, const dugks_objective* obj, do
     ADJ_TRY(h, cudaEventCreate(&t0));
     ADJ_TRY(h, cudaEventCreate(&t1));
     ADJ_TRY(h, cudaEventRecord(t0, h->stream));
-    if ((st = ops.ex.run(nBF, adj::FInBy{v}))) return st;
+    if ((st = adj::in_by(ops.ex, v))) return st;
     if ((st = adj::revolve_run(ops, obj->n_steps, n_slots))) return st;
-    if ((st = ops.ex.run(nBF, adj::RInBy{v}))) return st;
+    if ((st = adj::reverse_in_by(ops.ex, v))) return st;
     ADJ_TRY(h, cudaEventRecord(t1, h->stream));
     std::vector<double> Jb(nBF), gT(nBF), gU(3 * static_cast<size_t>(nBF)), mF(nF), mC(nC);
     ADJ_TRY(h, cudaMemcpyAsync(Jb.data(), v.Jb, nBF * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -421,7 +421,7 @@ extern "C" int dugks_boundary_fluxes(dugks_handle* h, double dt, double* flux) {
     v.g = static_cast<const double*>(h->ds.g);
     v.h = static_cast<const double*>(h->ds.h);
     v.cm = h->ds.cm;
-    if ((st = ex.run(nBF, adj::FInBy{v}))) return st;
+    if ((st = adj::in_by(ex, v))) return st;
     if ((st = adj::record_step(ex, v))) return st;
     if ((st = ex.run(nBF, adj::FBoundaryFlux{v, d_out}))) return st;
     ADJ_TRY(h, cudaMemcpyAsync(flux, d_out, 5 * static_cast<size_t>(nBF) * sizeof(double), cudaMemcpyDeviceToHost,
@@ -444,7 +444,7 @@ extern "C" int dugks_objective_run(dugks_handle* h, const dugks_objective* obj, 
     ADJ_TRY(h, cudaEventCreate(&t0));
     ADJ_TRY(h, cudaEventCreate(&t1));
     ADJ_TRY(h, cudaEventRecord(t0, h->stream));
-    if ((st = ex.run(nBF, adj::FInBy{v}))) return st;
+    if ((st = adj::in_by(ex, v))) return st;
     if (obj->window_start > 0) {
         std::vector<double> dts(obj->window_start, dt);
         if ((st = dugks_step(h, obj->window_start, dts.data()))) return st;

@@ -99,8 +99,8 @@ struct View {
     const double* fmom;
     int nchM;
     const double* bmom_in;  // [nBF][16]
-    double* pf;             // [nchF][nF][kP]
-    double* pc;             // [nchC][nC][kP]
+    double* pf;             // [nchF][kP][nF] partial sums by DV chunk
+    double* pc;             // [nchC][kP][nC]
     double* rhow;           // [nBF]
     double* inby;           // [nBF] inComingByRho of the patch values
     double* fmac;           // [nF][kMac]
@@ -165,6 +165,8 @@ ADJ_HD double xs_of(const double* xi, const double* S) {
 // element of DV i of cell or face e ([block of 32][dv][32])
 ADJ_HD size_t at(int i, int nv, int e) { return (static_cast<size_t>(e >> 5) * nv + i) * 32 + (e & 31); }
 ADJ_HD int chunk_lo(int nv, int nch, int ch) { return static_cast<int>(static_cast<int64_t>(nv) * ch / nch); }
+// field 0 of chunk ch and entity e (of n) in the partial sums; field k is k n on
+ADJ_HD size_t part_at(int ch, int n, int e) { return static_cast<size_t>(ch) * kP * n + e; }
 
 // fvDVM::updateTau (fvDVM.C:1823-1832)
 ADJ_HD double tau_of(const View& v, double T, double rho) {
@@ -400,19 +402,43 @@ struct ShkEntity {
 // ---------------------------------------------------------------- forward
 
 // inComingByRho of the wall faces (fvDVM.C:578-624)
-struct FInBy {
+struct FInByPart {
     View v;
-    ADJ_HD void operator()(int64_t b) const {
+    ADJ_HD void operator()(int64_t idx) const {
+        const int ch = static_cast<int>(idx / v.nBF), b = static_cast<int>(idx % v.nBF);
         double acc = 0;
         if (v.btype[b] == 1) {
             const double* S = v.S + 3 * (v.nIF + b);
-            for (int i = 0; i < v.nv; ++i) {
+            for (int i = chunk_lo(v.nv, v.nchF, ch); i < chunk_lo(v.nv, v.nchF, ch + 1); ++i) {
                 const double* xi = v.xi + 3 * i;
                 const double xs = xs_of(xi, S);
                 if (xs < 0) acc += -v.w[i] * xs * eq_by_rho(v, xi, v.bU + 3 * b, v.bT[b]);
             }
         }
-        v.inby[b] = acc;
+        v.pf[part_at(ch, v.nF, v.nIF + b)] = acc;
+    }
+};
+struct FInBy {
+    View v;
+    ADJ_HD void operator()(int64_t b) const { v.inby[b] = v.pf[v.nIF + b]; }
+};
+
+// Fields 0..K-1 of the partial sums of entities e0.. (n of the n_all), summed
+// over the chunks into the first one.  A thread per entity that reads all
+// fields of all chunks has too few loads in flight: with 4,096 cells and 64
+// chunks of [cell][field] sums it took 122 us for the cell macros; this and
+// the macros from one chunk take a fifth of it.
+struct SumParts {
+    double* p;
+    int n_all, e0, n, nch;
+    ADJ_HD void operator()(int64_t idx) const {
+        const int k = static_cast<int>(idx / n), e = e0 + static_cast<int>(idx % n);
+        double a = 0;
+#ifdef __CUDACC__
+#pragma unroll 8
+#endif
+        for (int ch = 0; ch < nch; ++ch) a += p[part_at(ch, n_all, e) + static_cast<size_t>(k) * n_all];
+        p[static_cast<size_t>(k) * n_all + e] = a;
     }
 };
 
@@ -463,18 +489,15 @@ struct FCellMom {
         double m[14] = {0};
         for (int i = chunk_lo(v.nv, v.nchC, ch); i < chunk_lo(v.nv, v.nchC, ch + 1); ++i)
             add_moments(v.xi + 3 * i, v.w[i], v.g[at(i, v.nv, c)], v.h[at(i, v.nv, c)], m);
-        double* p = v.pc + (static_cast<size_t>(ch) * v.nC + c) * kP;
-        for (int k = 0; k < 14; ++k) p[k] = m[k];
+        double* p = v.pc + part_at(ch, v.nC, c);
+        for (int k = 0; k < 14; ++k) p[static_cast<size_t>(k) * v.nC] = m[k];
     }
 };
 struct FCellMac {
     View v;
     ADJ_HD void operator()(int64_t c) const {
-        double m[14] = {0};
-        for (int ch = 0; ch < v.nchC; ++ch) {
-            const double* p = v.pc + (static_cast<size_t>(ch) * v.nC + c) * kP;
-            for (int k = 0; k < 14; ++k) m[k] += p[k];
-        }
+        double m[14];
+        for (int k = 0; k < 14; ++k) m[k] = v.pc[static_cast<size_t>(k) * v.nC + c];
         macros_from_moments(v, m, v.dt * v.Pr, v.cmac + kMac * static_cast<size_t>(c));
     }
 };
@@ -602,8 +625,8 @@ struct RRelax {
                 v.ah[id] = a_h;
             }
         }
-        double* p = v.pf + (static_cast<size_t>(ch) * v.nF + f) * kP;
-        for (int k = 0; k < 11; ++k) p[k] = s[k];
+        double* p = v.pf + part_at(ch, v.nF, f);
+        for (int k = 0; k < 11; ++k) p[static_cast<size_t>(k) * v.nF] = s[k];
     }
 };
 
@@ -612,11 +635,7 @@ struct RRelax {
 // objective are accumulated
 struct RFaceMac {
     View v;
-    ADJ_HD double psum(int f, int k) const {
-        double a = 0;
-        for (int ch = 0; ch < v.nchF; ++ch) a += v.pf[(static_cast<size_t>(ch) * v.nF + f) * kP + k];
-        return a;
-    }
+    ADJ_HD double psum(int f, int k) const { return v.pf[static_cast<size_t>(k) * v.nF + f]; }
     ADJ_HD void operator()(int64_t fi) const {
         const int f = static_cast<int>(fi);
         const double* m = v.fmac + kMac * static_cast<size_t>(f);
@@ -670,8 +689,8 @@ struct RFaceMom {
             for (int k = 0; k < 3; ++k) s[2 + k] += agt * rin * dEU[k];
         }
         if (bnd) {
-            double* p = v.pf + (static_cast<size_t>(ch) * v.nF + f) * kP;
-            for (int k = 0; k < 5; ++k) p[k] = s[k];
+            double* p = v.pf + part_at(ch, v.nF, f);
+            for (int k = 0; k < 5; ++k) p[static_cast<size_t>(k) * v.nF] = s[k];
         }
     }
 };
@@ -682,9 +701,8 @@ struct RBoundary {
     View v;
     ADJ_HD void operator()(int64_t bi) const {
         const int b = static_cast<int>(bi), f = v.nIF + b;
-        double s[5] = {0, 0, 0, 0, 0};
-        for (int ch = 0; ch < v.nchF; ++ch)
-            for (int k = 0; k < 5; ++k) s[k] += v.pf[(static_cast<size_t>(ch) * v.nF + f) * kP + k];
+        double s[5];
+        for (int k = 0; k < 5; ++k) s[k] = v.pf[static_cast<size_t>(k) * v.nF + f];
         v.gTb[b] += s[1];
         if (v.btype[b] == 1) {
             const double I = v.inby[b];
@@ -833,8 +851,8 @@ struct RHalf {
             v.og[id] = -1.0 / 3 * ro(v.lg + id) + (1.0 - r) * abg;
             v.oh[id] = -1.0 / 3 * ro(v.lh + id) + (1.0 - r) * abh;
         }
-        double* p = v.pc + (static_cast<size_t>(ch) * v.nC + c) * kP;
-        for (int k = 0; k < 9; ++k) p[k] = s[k];
+        double* p = v.pc + part_at(ch, v.nC, c);
+        for (int k = 0; k < 9; ++k) p[static_cast<size_t>(k) * v.nC] = s[k];
     }
 };
 
@@ -846,9 +864,8 @@ struct RCellMac {
     ADJ_HD void operator()(int64_t ci) const {
         const int c = static_cast<int>(ci);
         const double* m = v.cm + 9 * static_cast<size_t>(c);
-        double s[9] = {0};
-        for (int ch = 0; ch < v.nchC; ++ch)
-            for (int k = 0; k < 9; ++k) s[k] += v.pc[(static_cast<size_t>(ch) * v.nC + c) * kP + k];
+        double s[9];
+        for (int k = 0; k < 9; ++k) s[k] = v.pc[static_cast<size_t>(k) * v.nC + c];
         double aM[9];
         for (int k = 0; k < 8; ++k) aM[k] = s[1 + k];
         for (int e = v.cf_off[c]; e < v.cf_off[c + 1]; ++e) {
@@ -884,31 +901,69 @@ struct RCellMom {
 };
 
 // the parameters' adjoint through inComingByRho (wall faces), at the end
+struct RInByPart {
+    View v;
+    ADJ_HD void operator()(int64_t idx) const {
+        const int ch = static_cast<int>(idx / v.nBF), b = static_cast<int>(idx % v.nBF);
+        double s[4] = {0, 0, 0, 0};
+        if (v.btype[b] == 1) {
+            const double* S = v.S + 3 * (v.nIF + b);
+            for (int i = chunk_lo(v.nv, v.nchF, ch); i < chunk_lo(v.nv, v.nchF, ch + 1); ++i) {
+                const double* xi = v.xi + 3 * i;
+                const double xs = xs_of(xi, S);
+                if (!(xs < 0)) continue;
+                const double E = eq_by_rho(v, xi, v.bU + 3 * b, v.bT[b]);
+                double dET, dEU[3];
+                eq_by_rho_d(v, xi, v.bU + 3 * b, v.bT[b], E, dET, dEU);
+                s[0] += -v.w[i] * xs * dET;
+                for (int k = 0; k < 3; ++k) s[1 + k] += -v.w[i] * xs * dEU[k];
+            }
+        }
+        double* p = v.pf + part_at(ch, v.nF, v.nIF + b);
+        for (int k = 0; k < 4; ++k) p[static_cast<size_t>(k) * v.nF] = s[k];
+    }
+};
 struct RInBy {
     View v;
     ADJ_HD void operator()(int64_t bi) const {
         const int b = static_cast<int>(bi);
         if (v.btype[b] != 1) return;
-        const double* S = v.S + 3 * (v.nIF + b);
-        double sT = 0, sU[3] = {0, 0, 0};
-        for (int i = 0; i < v.nv; ++i) {
-            const double* xi = v.xi + 3 * i;
-            const double xs = xs_of(xi, S);
-            if (!(xs < 0)) continue;
-            const double E = eq_by_rho(v, xi, v.bU + 3 * b, v.bT[b]);
-            double dET, dEU[3];
-            eq_by_rho_d(v, xi, v.bU + 3 * b, v.bT[b], E, dET, dEU);
-            sT += -v.w[i] * xs * dET;
-            for (int k = 0; k < 3; ++k) sU[k] += -v.w[i] * xs * dEU[k];
-        }
-        v.gTb[b] += v.aI[b] * sT;
-        for (int k = 0; k < 3; ++k) v.gUb[3 * b + k] += v.aI[b] * sU[k];
+        const double* p = v.pf + v.nIF + b;
+        v.gTb[b] += v.aI[b] * p[0];
+        for (int k = 0; k < 3; ++k) v.gUb[3 * b + k] += v.aI[b] * p[static_cast<size_t>(1 + k) * v.nF];
     }
 };
 
 // ---------------------------------------------------------------- sequences
 
 // Ex: run(n, functor) applies the functor to 0..n-1 (in any order).
+template <class Ex>
+int sum_faces(Ex& ex, const View& v, int fields, bool boundary_only) {
+    const int e0 = boundary_only ? v.nIF : 0, n = v.nF - e0;
+    return ex.run(static_cast<int64_t>(fields) * n, SumParts{v.pf, v.nF, e0, n, v.nchF});
+}
+template <class Ex>
+int sum_cells(Ex& ex, const View& v, int fields) {
+    return ex.run(static_cast<int64_t>(fields) * v.nC, SumParts{v.pc, v.nC, 0, v.nC, v.nchC});
+}
+
+// inComingByRho of the walls (1,024 DVs and 256 wall faces: one thread a face
+// took 760 us, and the reverse 1,290), and its reverse
+template <class Ex>
+int in_by(Ex& ex, const View& v) {
+    int st;
+    if ((st = ex.run(static_cast<int64_t>(v.nchF) * v.nBF, FInByPart{v}))) return st;
+    if ((st = sum_faces(ex, v, 1, true))) return st;
+    return ex.run(v.nBF, FInBy{v});
+}
+template <class Ex>
+int reverse_in_by(Ex& ex, const View& v) {
+    int st;
+    if ((st = ex.run(static_cast<int64_t>(v.nchF) * v.nBF, RInByPart{v}))) return st;
+    if ((st = sum_faces(ex, v, 4, true))) return st;
+    return ex.run(v.nBF, RInBy{v});
+}
+
 template <class Ex>
 int record_step(Ex& ex, const View& v) {
     int st;
@@ -924,17 +979,21 @@ int reverse_step(Ex& ex, const View& v) {
     int st;
     if (v.fold) {
         if ((st = ex.run(static_cast<int64_t>(v.nchC) * v.nC, FCellMom{v}))) return st;
+        if ((st = sum_cells(ex, v, 14))) return st;
         if ((st = ex.run(v.nC, FCellMac{v}))) return st;
     }
     if ((st = ex.run(static_cast<int64_t>(v.nchF) * v.nF, RRelax{v}))) return st;
+    if ((st = sum_faces(ex, v, 11, false))) return st;
     if ((st = ex.run(v.nF, RFaceMac{v}))) return st;
     if ((st = ex.run(static_cast<int64_t>(v.nchF) * v.nF, RFaceMom{v}))) return st;
     if (v.nBF > 0) {
+        if ((st = sum_faces(ex, v, 5, true))) return st;
         if ((st = ex.run(v.nBF, RBoundary{v}))) return st;
         if ((st = ex.run(static_cast<int64_t>(v.nv) * v.nBF, RWallOut{v}))) return st;
     }
     if ((st = ex.run(static_cast<int64_t>(v.nv) * v.nC, RGradAdj{v}))) return st;
     if ((st = ex.run(static_cast<int64_t>(v.nchC) * v.nC, RHalf{v}))) return st;
+    if ((st = sum_cells(ex, v, 9))) return st;
     if ((st = ex.run(v.nC, RCellMac{v}))) return st;
     if (v.fold) return ex.run(static_cast<int64_t>(v.nv) * v.nC, RCellMom{v});
     return 0;
