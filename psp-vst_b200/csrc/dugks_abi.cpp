@@ -33,6 +33,11 @@ int dev_alloc(dugks_handle* h, T** p, size_t count) {
     void* q = nullptr;
     const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
     cudaError_t e = cudaMalloc(&q, bytes);
+    if (e == cudaErrorMemoryAllocation && !h->kept.empty()) {
+        cudaGetLastError();
+        dugks::free_kept(h);
+        e = cudaMalloc(&q, bytes);
+    }
     if (e != cudaSuccess)
         return set_error(h, e == cudaErrorMemoryAllocation ? DUGKS_ERR_OOM : DUGKS_ERR_CUDA,
                          "cudaMalloc of " + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e));
@@ -1469,6 +1474,7 @@ void dugks_destroy(dugks_handle* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->nccl_comm) nccl_api().comm_destroy(static_cast<ncclComm_t>(h->nccl_comm));
     for (void* p : h->allocations) cudaFree(p);
+    dugks::free_kept(h);
     if (h->host_cm) cudaFreeHost(h->host_cm);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
@@ -1479,6 +1485,11 @@ void dugks_destroy(dugks_handle* h) {
 }  // extern "C"
 
 namespace dugks {
+
+void free_kept(dugks_handle* h) {
+    for (auto& k : h->kept) cudaFree(k.first);
+    h->kept.clear();
+}
 
 // Rebuilds the cell records and Maxwellian tables from the cell macros in
 // ds.cm, as dugks_set_step_record does after restoring them.

@@ -64,24 +64,53 @@ struct GpuEx {
     int face_values(const adj::View& v) { return dugks::record_face_values(h, v.dt); }
 };
 
-// device allocations of one run, freed together
+// Device memory of one run.  It goes back to the handle, which keeps up to
+// kKeep bytes of it for its next run: mapping and unmapping the 950 MB of a
+// 12-step run with 4,096 cells and 1,024 DVs takes as long as its kernels.  What
+// the handle keeps is the last run's, is used on the handle's stream alone, and
+// is given back when the handle is destroyed or an allocation of it fails.
+constexpr size_t kKeep = size_t(2) << 30;
 struct Arena {
-    std::vector<void*> p;
+    dugks_handle* h;
+    std::vector<std::pair<void*, size_t>> p;
     double bytes = 0;
+    explicit Arena(dugks_handle* h) : h(h) {}
+    Arena(const Arena&) = delete;
     ~Arena() {
-        for (void* q : p) cudaFree(q);
+        dugks::free_kept(h);
+        size_t kept = 0;
+        for (auto& q : p) {
+            if (kept + q.second > kKeep) {
+                cudaFree(q.first);
+                continue;
+            }
+            kept += q.second;
+            h->kept.push_back(q);
+        }
     }
     template <class T>
     int get(dugks_handle* h, T** out, size_t n) {
-        void* q = nullptr;
         const size_t b = std::max<size_t>(n, 1) * sizeof(T);
+        bytes += static_cast<double>(b);
+        for (size_t i = 0; i < h->kept.size(); ++i)
+            if (h->kept[i].second == b) {
+                p.push_back(h->kept[i]);
+                h->kept.erase(h->kept.begin() + i);
+                *out = static_cast<T*>(p.back().first);
+                return DUGKS_OK;
+            }
+        void* q = nullptr;
         cudaError_t e = cudaMalloc(&q, b);
+        if (e == cudaErrorMemoryAllocation && !h->kept.empty()) {
+            cudaGetLastError();
+            dugks::free_kept(h);
+            e = cudaMalloc(&q, b);
+        }
         if (e != cudaSuccess)
             return set_error(h, e == cudaErrorMemoryAllocation ? DUGKS_ERR_OOM : DUGKS_ERR_CUDA,
                              "dugks_adjoint_run: cudaMalloc of " + std::to_string(b) + " bytes: " +
                                  cudaGetErrorString(e));
-        p.push_back(q);
-        bytes += static_cast<double>(b);
+        p.emplace_back(q, b);
         *out = static_cast<T*>(q);
         return DUGKS_OK;
     }
@@ -303,7 +332,7 @@ double host_sum(const std::vector<double>& a) {
 extern "C" int dugks_adjoint_run(dugks_handle* h, const dugks_objective* obj, double* J, double* dJ_dT_b,
                                  double* dJ_dU_b, double* dJ_dmu_ref, dugks_adjoint_stats* stats) {
     if (!h) return DUGKS_ERR_ARG;
-    Arena ar;
+    Arena ar(h);
     adj::View v;
     double* lam[4] = {};
     int sms = 0, st;
@@ -409,7 +438,7 @@ extern "C" int dugks_boundary_fluxes(dugks_handle* h, double dt, double* flux) {
     obj.n_steps = 1;
     obj.dt = dt;
     obj.max_snapshots = 1;
-    Arena ar;
+    Arena ar(h);
     adj::View v;
     int sms = 0, st;
     if ((st = prepare(h, &obj, "dugks_boundary_fluxes", ar, v, sms, false, nullptr))) return st;
@@ -433,7 +462,7 @@ extern "C" int dugks_boundary_fluxes(dugks_handle* h, double dt, double* flux) {
 extern "C" int dugks_objective_run(dugks_handle* h, const dugks_objective* obj, double* J,
                                    dugks_adjoint_stats* stats) {
     if (!h) return DUGKS_ERR_ARG;
-    Arena ar;
+    Arena ar(h);
     adj::View v;
     int sms = 0, st;
     if ((st = prepare(h, obj, "dugks_objective_run", ar, v, sms, false, nullptr))) return st;
