@@ -48,6 +48,7 @@ constexpr int kNoAllocMaxCells = 131072;
 constexpr int kNoAllocMom = 15;                        // raw moments per cell (layout in dugks_internal.h)
 constexpr size_t kNoAllocScratch = static_cast<size_t>(kNoAllocMaxCells) * 16;  // doubles (16 MiB)
 constexpr int kNoAllocThreads = 128;
+constexpr int kNoAllocGroup = 4;                       // DVs whose loads are issued together
 constexpr int kNoAllocTargetBlocks = 1184;             // 8 CTAs per SM on 148 SMs
 constexpr int kNoAllocMaxDevices = 64;
 
@@ -107,9 +108,12 @@ bool has_room(const void* p, size_t bytes) {
 }
 
 // raw moments of the DVs [d0, d1) of chunk blockIdx.y, one thread per cell;
-// rows of g, h are contiguous in cells, so a warp reads coalesced
+// rows of g, h are contiguous in cells, so a warp reads coalesced.  Bound by
+// HBM (16 B per cell and DV) once the loads of kNoAllocGroup DVs are in flight
+// together: 65,536 cells and 784 DVs (822 MB) 169 us a call, 4.9 TB/s, against
+// 241 us with one DV's loads at a time.
 template <int D>
-__global__ void __launch_bounds__(kNoAllocThreads) k_noalloc_partials(const double* __restrict__ xi,
+__global__ void __launch_bounds__(kNoAllocThreads, 8) k_noalloc_partials(const double* __restrict__ xi,
                                                                       const double* __restrict__ w,
                                                                       const double* __restrict__ g,
                                                                       const double* __restrict__ hh, int nC, int nv,
@@ -121,12 +125,26 @@ __global__ void __launch_bounds__(kNoAllocThreads) k_noalloc_partials(const doub
     const int d1 = static_cast<int>(static_cast<long long>(nv) * (ch + 1) / chunks);
     double acc[kNoAllocMom];
     for (int j = 0; j < kNoAllocMom; ++j) acc[j] = 0.0;
-    for (int d = d0; d < d1; ++d) {
+    const double *pg = g + static_cast<size_t>(d0) * nC + c, *ph = hh + static_cast<size_t>(d0) * nC + c;
+    auto add = [&](int d, double gv, double hv) {
         const double x[3] = {__ldg(xi + 3 * d), __ldg(xi + 3 * d + 1), D == 3 ? __ldg(xi + 3 * d + 2) : 0.0};
         const double x2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        const size_t idx = static_cast<size_t>(d) * nC + c;
-        accum<D>(acc, __ldg(w + d), x, x2, __ldg(g + idx), __ldg(hh + idx));
+        accum<D>(acc, __ldg(w + d), x, x2, gv, hv);
+    };
+    int d = d0;
+    for (; d + kNoAllocGroup <= d1; d += kNoAllocGroup) {
+        double gv[kNoAllocGroup], hv[kNoAllocGroup];
+#pragma unroll
+        for (int u = 0; u < kNoAllocGroup; ++u) {
+            gv[u] = __ldg(pg);
+            hv[u] = __ldg(ph);
+            pg += nC;
+            ph += nC;
+        }
+#pragma unroll
+        for (int u = 0; u < kNoAllocGroup; ++u) add(d + u, gv[u], hv[u]);
     }
+    for (; d < d1; ++d, pg += nC, ph += nC) add(d, __ldg(pg), __ldg(ph));
     for (int j = 0; j < kNoAllocMom; ++j)
         scratch[(static_cast<size_t>(ch) * kNoAllocMom + j) * nC + c] = acc[j];
 }
