@@ -119,17 +119,16 @@ def run_config(cfg, precision, world, shard, nv_loc, nc):
                 l2="inputs larger than L2 (state %.2f GB per GPU)" % (2 * rs * nc * nv_loc / 1e9))
 
 
-def profiled_traffic(kernel: str, precision: str):
-    """DRAM bytes per cell.DV update of a pass kernel, from the committed
-    ncu summary of the same kernel with the same 16^3 DV set on a smaller
+def profiled_traffic(which: str, precision: str):
+    """DRAM bytes per cell.DV update of a pass's kernels, from the committed
+    ncu summary of the same kernels with the same 16^3 DV set on a smaller
     cubed sphere (6 x 16^3 = 24,576 cells; the full launch is too large to
-    capture; traffic per update is set by the tile layout, alike on both
-    meshes), or None."""
-    path = os.path.join(ROOT, "profiles", f"{kernel}_ball24576_dv4096_{precision}.md")
+    capture; the kernels stream whole arrays, alike on both meshes), or None."""
+    path = os.path.join(ROOT, "profiles", f"step_kernels_ball24576_dv4096_{precision}.md")
     try:
         with open(path) as f:
             for ln in f:
-                if ln.startswith("traffic_bytes_per_update:"):
+                if ln.startswith(f"traffic_bytes_per_update {which}:"):
                     return float(ln.split(":")[1])
     except OSError:
         pass
@@ -753,11 +752,11 @@ def main():
     a_ms, b_ms = stage[0] / K, stage[2] / K
     # per-launch figures of this rank's kernels (its DV block)
     if b_ms >= a_ms:
-        kname, kbytes, kms = "pass B (face relaxation, flux, update, cell moments)", 2 * arr * rs * nc * nv_loc, b_ms
-        tpu = profiled_traffic("k_pass_b", args.precision) if args.workload == "ball" else None
+        kname, kbytes, kms = "pass B (face flux; update and cell moments)", 2 * arr * rs * nc * nv_loc, b_ms
+        tpu = profiled_traffic("pass_b", args.precision) if args.workload == "ball" else None
     else:
-        kname, kbytes, kms = "pass A (reconstruction, face moments)", arr * rs * nc * nv_loc, a_ms
-        tpu = profiled_traffic("k_pass_a", args.precision) if args.workload == "ball" else None
+        kname, kbytes, kms = "pass A (half step, face values, face moments)", arr * rs * nc * nv_loc, a_ms
+        tpu = profiled_traffic("pass_a", args.precision) if args.workload == "ball" else None
     achieved = kbytes / (kms / 1e3) / 1e9
     traffic = tpu * nc * nv_loc if tpu is not None else None
     step_bytes = 3 * arr * rs * nc * nv_loc
@@ -772,7 +771,7 @@ def main():
         "roofline": {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind, "traffic": traffic,
                      "algorithmic_bytes_per_launch": kbytes,
-                     "traffic_source": "ncu DRAM read+write per update of the same kernel on a 6x16^3 cubed "
+                     "traffic_source": "ncu DRAM read+write per update of the same kernels on a 6x16^3 cubed "
                                        "sphere with the same DV set, times this launch's updates"
                      if traffic is not None else None},
         "step_roofline": {"bytes_per_update": 3 * arr * rs, "h_identically_zero": arr == 1,

@@ -432,9 +432,10 @@ int32_t dugks_n_dv(const dugks_handle* h);
 int dugks_last_step_ms(dugks_handle* h, double* ms);
 
 /* dugks_step with CUDA events around every kernel stage on the handle's
- * stream; stage_ms[0..4] receive the summed milliseconds of pass A (face
- * reconstruction and moments), the face combine, pass B (relaxation, flux,
- * update, cell moments), the cell combine, and the whole call. */
+ * stream; stage_ms[0..4] receive the summed milliseconds of pass A (half step,
+ * face values, face moments and macros), 0 or the face sums of a sharded
+ * handle, pass B (flux, update, cell moments and macros), 0 or the cell sums
+ * of a sharded handle, and the whole call. */
 int dugks_step_timed(dugks_handle* h, int32_t n_steps, const double* dt, double* stage_ms);
 
 /* Number of kernels this handle has launched so far. */
