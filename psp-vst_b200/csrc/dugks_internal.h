@@ -101,8 +101,8 @@ struct DevMesh {
     const int2* tang;              // [n_tang] exactly tangential pairs: internal face, segment * kSeg + DV in it
     long long n_tang;
     // FP32 storage of a tensor DV set: where the pairs are in the list, by
-    // face block (null without pairs): the faces of one DV that have one (a bit
-    // each) and the first one's place; and the DVs of a segment that have any
+    // face block (null without pairs): the faces between tiles that have one at
+    // a DV (a bit each) and the first one's place; and the DVs of a segment with any
     const uint2* tang_at;          // [pF/32][nv_loc]
     const unsigned* tang_seg;      // [pF/32][n_seg]
     int done_cells;                // first cell-block counter in DevState::done (face blocks before it)

@@ -736,12 +736,23 @@ __global__ void k_upwind_bits(const DevMesh m, uint32_t* upw, unsigned long long
     if (tangential) atomicAdd(n_tang, static_cast<unsigned long long>(tangential));
 }
 
+// whether internal face f of owner o lies inside a tile (cell face code, bit 1)
+__device__ __forceinline__ bool in_tile_face(const DevMesh& m, int f, int o) {
+    for (int k = 0; k < m.nf_max; ++k) {
+        const int code = __ldg(m.cface + static_cast<size_t>(k) * m.nC + o);
+        if (code >= 0 && (code >> 2) == f) return code & 2;
+    }
+    return false;
+}
+
 // the list of those pairs (DevMesh::tang), pairs of one DV and consecutive
 // faces together
 template <bool GEN>
 __global__ void k_list_tangential(const DevMesh m, int2* list, unsigned long long* cursor, uint2* at, unsigned* seg) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     const size_t nF = static_cast<size_t>(m.nF);
+    const bool between = f < m.nIF && !in_tile_face(m, f, __ldg(m.fown + f));
+    const unsigned tiles = __ballot_sync(0xffffffffu, between);
     for (int s = blockIdx.y; s < m.n_seg; s += gridDim.y) {
         const Seg q = seg_at<GEN>(m, s);
         unsigned t = 0;
@@ -749,18 +760,22 @@ __global__ void k_list_tangential(const DevMesh m, int2* list, unsigned long lon
             const uint2 up = reinterpret_cast<const uint2*>(m.upw)[s * nF + f];
             t = ~(up.x | up.y) & (q.len == 32 ? 0xffffffffu : (1u << q.len) - 1u);
         }
-        const unsigned any = __reduce_or_sync(0xffffffffu, t);
+        const unsigned rest = __reduce_or_sync(0xffffffffu, between ? t : 0u);
         const bool first = threadIdx.x % 32 == 0 && f < m.nIF;
-        if (seg && first) seg[(f / 32) * static_cast<size_t>(m.n_seg) + s] = any;
-        if (!any) continue;
+        if (seg && first) seg[(f / 32) * static_cast<size_t>(m.n_seg) + s] = rest;
+        if (!__any_sync(0xffffffffu, t != 0)) continue;
         for (int j = 0; j < q.len; ++j) {
             const unsigned who = __ballot_sync(0xffffffffu, (t >> j) & 1u);
             if (!who) continue;
             unsigned long long base = 0;
             if (threadIdx.x % 32 == 0) base = atomicAdd(cursor, static_cast<unsigned long long>(__popc(who)));
             base = __shfl_sync(0xffffffffu, base, 0);
-            if (at && first) at[(f / 32) * static_cast<size_t>(m.nv_loc) + q.d0 + j] = make_uint2(who, static_cast<unsigned>(base));
-            if ((t >> j) & 1u) list[base + __popc(who & ((1u << (threadIdx.x % 32)) - 1u))] = make_int2(f, s * kSeg + j);
+            // a warp's pairs between tiles first
+            const unsigned lt = (1u << (threadIdx.x % 32)) - 1u, inter = who & tiles;
+            if (at && first) at[(f / 32) * static_cast<size_t>(m.nv_loc) + q.d0 + j] = make_uint2(inter, static_cast<unsigned>(base));
+            if ((t >> j) & 1u)
+                list[base + (between ? __popc(inter & lt) : __popc(inter) + __popc(who & ~inter & lt))] =
+                    make_int2(f, s * kSeg + j);
         }
     }
 }
@@ -775,7 +790,6 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
     const DevMesh& m = a.dm;
     __shared__ double x1[kMaxN1d], w1[kMaxN1d];
     load_nodes(m, x1, w1);
-    const size_t nC = static_cast<size_t>(m.nC);
     const double hdt = 0.5 * step_dt(a);
     for (long long i = blockIdx.x * static_cast<long long>(kStream) + threadIdx.x; i < m.n_tang;
          i += static_cast<long long>(gridDim.x) * kStream) {
@@ -785,10 +799,7 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
         const int o = chk(__ldg(m.fown + f), 0, m.nC, a.ds.err), n = chk(__ldg(m.fnei + f), 0, m.nC, a.ds.err);
         bool in_tile = false;
         if constexpr (sizeof(Real) == 4 && !GEN)
-            for (int k = 0; k < m.nf_max; ++k) {
-                const int code = __ldg(m.cface + k * nC + o);
-                if (code >= 0 && (code >> 2) == f) in_tile = code & 2;
-            }
+            in_tile = in_tile_face(m, f, o);
         const bool rounded = kRoundsRows<D, Real, GEN> && in_tile && rounds_node(q.ix0 + j);
         const Dv v = dv_at<D, GEN>(m, q, x1, j);
         const size_t rc = 32 * static_cast<size_t>(q.d0 + j), rf = slot(f, m.nv_loc) + rc;
@@ -1405,7 +1416,9 @@ __global__ void __launch_bounds__(kFaces, 5) k_face_moments(const __grid_constan
     Real* ring = reinterpret_cast<Real*>(ring_raw) + w * kStagesM * NH * kGroupDv * kLanes;
     const Real* wg = fg + slot(wf0, m.nv_loc);
     const Real* wh = fh + slot(wf0, m.nv_loc);
-    // FP32 storage: what rounding took from the mean of tangential pairs
+    // FP32 storage: what rounding took from the mean of tangential pairs on
+    // faces between tiles, added after a group (a test in the group's loop cost
+    // every case 2 % of its step)
     unsigned tang = 0;   // the segment's DVs with such pairs among the warp's faces
     auto tang_rest = [&](int d, double& g, double& h) {
         const uint2 t = __ldg(m.tang_at + static_cast<size_t>(wf0 / kLanes) * m.nv_loc + d);
@@ -1435,14 +1448,18 @@ __global__ void __launch_bounds__(kFaces, 5) k_face_moments(const __grid_constan
                 constexpr int U = decltype(uc)::value;
                 const Real* su = st + i * kLanes;
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    double g = double(su[u * kLanes]), h = HZ ? 0.0 : double(su[(kGroupDv + u) * kLanes]);
-                    if constexpr (sizeof(Real) == 4 && !GEN) {
-                        if ((tang >> (j + i + u)) & 1u) tang_rest(q.d0 + j + i + u, g, h);
-                    }
-                    add_dv<D, HZ, GEN>(acc, rs, w1, q, dv_at<D, GEN>(m, q, x1, j + i + u), j + i + u, g, h);
-                }
+                for (int u = 0; u < U; ++u)
+                    add_dv<D, HZ, GEN>(acc, rs, w1, q, dv_at<D, GEN>(m, q, x1, j + i + u), j + i + u,
+                                       double(su[u * kLanes]), HZ ? 0.0 : double(su[(kGroupDv + u) * kLanes]));
             });
+            if constexpr (sizeof(Real) == 4 && !GEN) {
+                for (unsigned b = tang & (0xffu << j); b; b &= b - 1) {
+                    const int i = __ffs(b) - 1;
+                    double g = 0.0, h = 0.0;
+                    tang_rest(q.d0 + i, g, h);
+                    add_dv<D, HZ, GEN>(acc, rs, w1, q, dv_at<D, GEN>(m, q, x1, i), i, g, h);
+                }
+            }
             if constexpr (!GEN) {
                 if (j + kGroupDv >= q.len) {
                     row_fold<D>(acc, rs, row_const<D>(x1, w1, q));
