@@ -529,6 +529,9 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
             *out = h;
             return st;
         }
+        // (the vectors of this block end here)
+        if ((ce = cudaStreamSynchronize(h->stream)) != cudaSuccess)
+            return fail(DUGKS_ERR_CUDA, std::string("tables: ") + cudaGetErrorString(ce));
         dm.mf_off = d_mo;
         dm.mf_ent = d_me;
         dm.mf_Sf = d_ms;
