@@ -1314,8 +1314,13 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
             } else if (sym) {
                 // incoming through the patch's first face (updateGHbarSurfSymmetryIn,
                 // fvDVM.C:1100-1179, discreteVelocity.C:691-773): the face value of the
-                // mirror DV along the patch's axis; a DV that is its own mirror stays
-                bool counted = xs > -kVSmall;
+                // mirror DV along the patch's axis; a DV that is its own mirror stays.
+                // Values reconstructed this step are those outgoing or tangential here;
+                // on a face tilted against the first others stay without one: zero, not
+                // the last step's flux that their slot holds
+                const bool here = xs > -kVSmall;
+                bool counted = here, mirrored = false;
+                Real gn = here ? gv : Real(0), hn = here && !HZ ? hv : Real(0);
                 if constexpr (!GEN) {
                     if (!(xs_dv(v, S0) > 0)) {
                         const int n = m.n1d, st = axis == 0 ? 1 : axis == 1 ? n : n * n;
@@ -1326,18 +1331,24 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
                             // of two mirrors that are both incoming the later one keeps its value
                             Dv vt = v;
                             (axis == 0 ? vt.x : axis == 1 ? vt.y : vt.z) = x1[n - 1 - i];
-                            if (xs_dv(vt, S0) > 0 || t > d) {
+                            mirrored = xs_dv(vt, S0) > 0 || t > d;
+                            if (mirrored) {
+                                const bool there = xs_dv(vt, S) > -kVSmall;
                                 const size_t ot = 32 * static_cast<size_t>(t);
                                 const double grt = dv_ref<Real, GEN>(m.gref, t), hrt = dv_ref<Real, GEN>(m.href, t);
-                                fg[o] = Real((double(fg[ot]) + grt) - gr);
-                                if (!HZ) fh[o] = Real((double(fh[ot]) + hrt) - hr);
+                                gn = Real((double(there ? fg[ot] : Real(0)) + grt) - gr);
+                                if (!HZ) hn = Real((double(there ? fh[ot] : Real(0)) + hrt) - hr);
                             }
                         }
                     }
                 }
+                if (mirrored || !here) {
+                    fg[o] = gn;
+                    if (!HZ) fh[o] = hn;
+                }
                 if (!counted) continue;
-                g = double(fg[o]) + gr;
-                if (!HZ) h = double(fh[o]) + hr;
+                g = double(gn) + gr;
+                if (!HZ) h = double(hn) + hr;
             } else if (xs > 0) {
                 // outgoing: upwind from the owner (fvDVM.C:916-923, :950-961)
                 g = double(gv) + gr;
