@@ -297,11 +297,12 @@ int prepare(dugks_handle* h, const dugks_objective* obj, const char* who, Arena&
     v.ha = d_ha;
     v.fw = d_fw;
     v.fg = static_cast<double*>(h->ds.fvg);
-    v.fh = static_cast<double*>(h->ds.fvh);
+    // with h identically zero the step writes no face values of it; its array
+    // may be absent, or hold those of an earlier run that carried h
+    v.fh = h->h_zero ? nullptr : static_cast<double*>(h->ds.fvh);
     v.fmom = h->ds.partF;
     v.nchM = h->chunks_f;
     v.bmom_in = h->ds.bmom_in;
-    // with h identically zero the step keeps no face values of it
     if ((!v.fh && (st = ar.zeros(h, &v.fh, nvf))) ||
         (st = ar.get(h, &v.pf, static_cast<size_t>(v.nchF) * nF * adj::kP)) || (st = ar.get(h, &v.rhow, nBF)) ||
         (st = ar.get(h, &v.inby, nBF)) || (st = ar.get(h, &v.fmac, static_cast<size_t>(nF) * adj::kMac)) ||
