@@ -122,6 +122,19 @@ int shard_allreduce(dugks_handle* h, double* buf, size_t n) {
     return DUGKS_OK;
 }
 
+// a device current in a scope, the caller's own again after it
+struct OnDevice {
+    int before = -1;
+    cudaError_t status;
+    explicit OnDevice(int device) : status(cudaGetDevice(&before)) {
+        if (status == cudaSuccess) status = cudaSetDevice(device);
+    }
+    OnDevice(const OnDevice&) = delete;
+    ~OnDevice() {
+        if (before >= 0) cudaSetDevice(before);
+    }
+};
+
 int check_device_errors(dugks_handle* h) {
     int err[4] = {0, 0, 0, 0};
     CUDA_TRY(h, cudaMemcpyAsync(err, h->ds.err, sizeof err, cudaMemcpyDeviceToHost, h->stream));
@@ -1395,6 +1408,8 @@ static int state_io(dugks_handle* h, double* g, double* hh, const double* gi, co
     if (!h->initialised) return set_error(h, DUGKS_ERR_STATE, "state access before dugks_set_macros");
     const size_t n = static_cast<size_t>(h->dm.nv_loc) * h->nC;
     const size_t part = (static_cast<size_t>(h->dm.nv_loc) * h->dm.pC + dugks::kSlack) * real_size(h) / sizeof(double);
+    const OnDevice on(h->device);
+    CUDA_TRY(h, on.status);
     const dugks::StepArgs a = make_args(h, 0.0);
     double* buf = static_cast<double*>(h->ds.gbar);
     // (a step whose phases the caller drives may be half done: gbar+ is kept)
@@ -1425,6 +1440,8 @@ int dugks_get_state(dugks_handle* h, double* g, double* hh) { return state_io(h,
 int dugks_set_state(dugks_handle* h, const double* g, const double* hh, double dt_prev) {
     if (!h) return DUGKS_ERR_ARG;
     if (int st = require_internal_reduction(h, "dugks_set_state")) return st;
+    const OnDevice on(h->device);
+    CUDA_TRY(h, on.status);
     int st = state_io(h, nullptr, nullptr, g, hh, false);
     if (st) return st;
     if (!(dt_prev > 0)) return set_error(h, DUGKS_ERR_ARG, "dugks_set_state: dt_prev must be > 0");

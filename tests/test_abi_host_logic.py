@@ -1,0 +1,46 @@
+"""The C ABI's host code on a CUDA runtime that runs on the host
+(fake_device.cpp): which device a call works on, what it allocates and what a
+call that runs out of device memory leaves behind."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from dugks_b200 import case as cs
+from dugks_b200 import lib as dl
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "libdugks_fake.so")
+    csrc = os.path.join(ROOT, "psp-vst_b200", "csrc")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-w", "-I", csrc, "-I", os.path.join(ROOT, "include"),
+                    "-I", "/usr/local/cuda/include", "-o", so, os.path.join(ROOT, "tests", "fake_device.cpp"),
+                    os.path.join(csrc, "dugks_abi.cpp"), os.path.join(csrc, "dugks_host.cpp"), "-Wl,-Bsymbolic", "-ldl"],
+                   check=True)
+    lib = dl.load(so)
+    lib.path = so
+    lib.fake_used.restype = C.c_size_t
+    lib.fake_capacity.argtypes = [C.c_int, C.c_size_t]
+    return lib
+
+
+@pytest.fixture
+def memory(fake):
+    yield fake
+    for d in (0, 1):
+        fake.fake_capacity(d, 1 << 40)
+
+
+def test_a_handles_state_is_read_whatever_device_is_current(memory):
+    s = dl.Solver(cs.cavity_case(4, 6), device=1, lib_path=memory.path)
+    memory.fake_current(0)
+    g, h = s.state()
+    assert np.all(g == 1.0) and not np.any(h)
+    assert memory.fake_device() == 0
+    s.set_state(2.0 * g, h, 1e-6)
+    assert memory.fake_device() == 0 and np.all(s.state()[0] == 2.0)
