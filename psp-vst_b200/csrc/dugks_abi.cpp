@@ -46,6 +46,11 @@ int dev_alloc(dugks_handle* h, T** p, size_t count) {
     return DUGKS_OK;
 }
 
+void dev_free(dugks_handle* h, void* p) {
+    h->allocations.erase(std::find(h->allocations.begin(), h->allocations.end(), p));
+    cudaFree(p);
+}
+
 template <typename T>
 int upload(dugks_handle* h, T** p, const std::vector<T>& v) {
     int st = dev_alloc(h, p, v.size());
@@ -171,7 +176,10 @@ static int alloc_h(dugks_handle* h) {
                  nfv = static_cast<size_t>(h->dm.nv_loc) * h->dm.pF + dugks::kSlack;
     unsigned char *b = nullptr, *f = nullptr;
     if (int st = dev_alloc(h, &b, nvc * rs)) return st;
-    if (int st = dev_alloc(h, &f, nfv * rs)) return st;
+    if (int st = dev_alloc(h, &f, nfv * rs)) {
+        dev_free(h, b);
+        return st;
+    }
     CUDA_TRY(h, cudaMemsetAsync(f, 0, nfv * rs, h->stream));
     h->ds.hbar = b;
     h->ds.fvh = f;
@@ -1442,10 +1450,12 @@ int dugks_set_state(dugks_handle* h, const double* g, const double* hh, double d
     if (int st = require_internal_reduction(h, "dugks_set_state")) return st;
     const OnDevice on(h->device);
     CUDA_TRY(h, on.status);
-    int st = state_io(h, nullptr, nullptr, g, hh, false);
-    if (st) return st;
+    if (!h->initialised) return set_error(h, DUGKS_ERR_STATE, "state access before dugks_set_macros");
+    if (!g || !hh) return set_error(h, DUGKS_ERR_ARG, "dugks_set_state: null array");
     if (!(dt_prev > 0)) return set_error(h, DUGKS_ERR_ARG, "dugks_set_state: dt_prev must be > 0");
-    // a nonzero h~ ends the g-only passes for this handle
+    // a nonzero h~ ends the g-only passes for this handle; what it needs is
+    // there before anything of the old state is replaced
+    int st;
     if (h->h_zero) {
         const size_t nvc = static_cast<size_t>(h->dm.nv_loc) * h->nC;
         bool zero = true;
@@ -1453,6 +1463,7 @@ int dugks_set_state(dugks_handle* h, const double* g, const double* hh, double d
         if (!zero && (st = alloc_h(h))) return st;
         h->h_zero = zero;
     }
+    if ((st = state_io(h, nullptr, nullptr, g, hh, false))) return st;
     dugks::StepArgs a = make_args(h, dt_prev);
     a.dm.macro_flux = 0;   // the macros of given DFs are their moments (macroFlux yes: restore the step record)
     // a new state replaces a poisoned one: its own check starts clear

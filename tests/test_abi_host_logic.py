@@ -44,3 +44,31 @@ def test_a_handles_state_is_read_whatever_device_is_current(memory):
     assert memory.fake_device() == 0
     s.set_state(2.0 * g, h, 1e-6)
     assert memory.fake_device() == 0 and np.all(s.state()[0] == 2.0)
+
+
+def test_a_set_state_that_finds_no_memory_changes_nothing(memory):
+    # 3-D, KInner 0: the first nonzero h~ needs two more arrays, one at a time
+    c = cs.cube_case(3, 6)
+    s = dl.Solver(c, lib_path=memory.path)
+    g, h = s.state()
+    used = memory.fake_used(0)
+    s.step(1, c.dt)
+    assert memory.fake_last_hzero() == 1
+    for spare in (0, 8 * 32 * 216 + 20000):      # neither array fits, only the first does
+        memory.fake_capacity(0, used + spare)
+        passes = memory.fake_passes()
+        with pytest.raises(dl.DugksError) as e:
+            s.set_state(2.0 * g, h + 1.0, c.dt)
+        assert e.value.code == 3
+        g1, h1 = s.state()
+        assert np.array_equal(g1, g) and np.array_equal(h1, h)
+        assert memory.fake_used(0) == used and memory.fake_passes() == passes
+        s.step(1, c.dt)
+        assert memory.fake_last_hzero() == 1
+    memory.fake_capacity(0, 1 << 40)
+    with pytest.raises(dl.DugksError) as e:
+        s.set_state(2.0 * g, h, 0.0)             # dt_prev 0
+    assert e.value.code == 1 and np.array_equal(s.state()[0], g)
+    s.set_state(2.0 * g, h + 1.0, c.dt)
+    s.step(1, c.dt)
+    assert memory.fake_last_hzero() == 0 and np.all(s.state()[1] == 1.0)
