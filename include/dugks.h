@@ -172,7 +172,8 @@ typedef struct dugks_options {
     int32_t ls_weighting;           /* dugks_ls_weighting */
     int32_t device;                 /* CUDA device ordinal */
     int32_t tile_cells;             /* cells per tile; 0 = automatic */
-    int32_t dv_chunks;              /* DV chunks per tile; 0 = automatic */
+    int32_t dv_chunks;              /* DV chunks of the cell sums, the face sums' by the same
+                                       factor; 0 = automatic */
     int32_t macro_flux;             /* fvDVMparas macroFlux: 0 "no" (cell macros from the
                                        DF moments), 1 "yes" (cell rho, rho U, rho E advance by
                                        the face macro fluxes, fvDVM.C:1613-1679; the

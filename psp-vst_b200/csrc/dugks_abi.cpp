@@ -394,8 +394,10 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         row1 = static_cast<int>(static_cast<int64_t>(rows) * (shard->rank + 1) / shard->world);
     }
     const int rows_loc = row1 - row0;
-    // DV segments, and DV chunks of the face and cell reductions; a given
-    // dv_chunks is taken as far as there are segments
+    // DV segments, and DV chunks of the face and cell reductions.  A given
+    // dv_chunks is that of the cells, as far as there are segments; the faces'
+    // moves from its automatic count by the same factor, so that the count
+    // dugks_layout reports gives the handle it was read from
     const int seg_per_row = dvl ? 1 : (h->n1d + dugks::kSeg - 1) / dugks::kSeg;
     const int n_seg = dvl ? (rows_loc + dugks::kSeg - 1) / dugks::kSeg : rows_loc * seg_per_row;
     // A chunk costs a write of its partial sums and a term of the finishing
@@ -407,7 +409,6 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     // 1,331 listed DVs: 3 and 6 chunks 1,450 us, 5 1,506 and 8 1,590.)
     const int cap = std::max(1, static_cast<int>(std::sqrt(static_cast<double>(n_seg))));
     auto chunks_for = [&](int entities) {
-        if (opt.dv_chunks > 0) return std::min(opt.dv_chunks, n_seg);
         const long long nb = (entities + 31) / 32, slots = 148 * 4;
         const int one = static_cast<int>(std::min<long long>(slots / nb, cap));
         if (one > 0 && n_seg <= 8 * 4 * one) return one;
@@ -423,12 +424,17 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     // the face reduction, one thread per internal face: four waves (3,721
     // cells: 28 chunks 260 us a step, 5 234; 1,728 cells, 10^3 DVs: 46 chunks 222 us, 10 171)
     auto chunks_f_for = [&](int entities) {
-        if (opt.dv_chunks > 0) return std::min(opt.dv_chunks, n_seg);
         const int nb = (entities + 127) / 128, want = (148 * 5 * 4 + nb - 1) / nb;
         return std::max(1, std::min(want, cap));
     };
     h->chunks = chunks_for(nC);
     h->chunks_f = chunks_f_for(nF);
+    if (opt.dv_chunks > 0) {
+        const int given = std::min(opt.dv_chunks, n_seg);
+        const long long f = (static_cast<long long>(h->chunks_f) * given + h->chunks / 2) / h->chunks;
+        h->chunks_f = static_cast<int>(std::max(1LL, std::min<long long>(f, n_seg)));
+        h->chunks = given;
+    }
 
     // ---- device layout ----
     const dugks::Tiling& t = h->tiling;

@@ -21,7 +21,7 @@ std::map<void*, Block> blocks;
 size_t capacity[2] = {size_t(1) << 40, size_t(1) << 40}, used[2];
 thread_local int current = 0;
 thread_local cudaError_t last = cudaSuccess;
-int last_hzero = -1, passes = 0;
+int last_hzero = -1, last_chunks[2], passes = 0;
 
 int device_of(cudaStream_t s) { return *reinterpret_cast<int*>(s); }
 cudaError_t launch(cudaStream_t s) { return device_of(s) == current ? cudaSuccess : cudaErrorInvalidResourceHandle; }
@@ -35,6 +35,7 @@ size_t fake_used(int device) { return used[device]; }
 void fake_current(int device) { current = device; }
 int fake_device() { return current; }
 int fake_last_hzero() { return last_hzero; }
+int fake_last_chunks(int faces) { return last_chunks[faces]; }
 int fake_passes() { return passes; }
 
 cudaError_t cudaMalloc(void** p, size_t n) {
@@ -122,6 +123,8 @@ namespace dugks {
 
 cudaError_t launch_stage(const StepArgs& a, int, int, cudaStream_t s, int*) {
     last_hzero = a.hzero;
+    last_chunks[0] = a.chunks;
+    last_chunks[1] = a.chunks_f;
     return launch(s);
 }
 cudaError_t launch_init(const StepArgs& a, int, cudaStream_t s) {

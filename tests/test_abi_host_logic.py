@@ -72,3 +72,21 @@ def test_a_set_state_that_finds_no_memory_changes_nothing(memory):
     s.set_state(2.0 * g, h + 1.0, c.dt)
     s.step(1, c.dt)
     assert memory.fake_last_hzero() == 0 and np.all(s.state()[1] == 1.0)
+
+
+@pytest.mark.parametrize("n,n_dv,scale", [(120, 12, 1), (120, 12, 2), (40, 20, 1), (40, 20, 3), (4, 6, 1)])
+def test_reported_chunks_give_the_handle_they_were_read_from(fake, n, n_dv, scale):
+    c = cs.cavity_case(n, n_dv)
+
+    def chunks(dv_chunks):
+        s = dl.Solver(c, dv_chunks=dv_chunks, lib_path=fake.path)
+        s.step(1, c.dt)
+        return s.layout()["dv_chunks"], fake.fake_last_chunks(0), fake.fake_last_chunks(1)
+
+    auto = chunks(0)
+    assert auto[0] == auto[1]
+    got = chunks(scale * auto[0])
+    assert got[0] == got[1] == min(scale * auto[0], n_dv)
+    assert got == chunks(got[0])
+    if scale == 1:
+        assert got == auto
