@@ -399,6 +399,13 @@ typedef struct dugks_adjoint_stats {
 int dugks_adjoint_run(dugks_handle* h, const dugks_objective* obj, double* J, double* dJ_dT_b, double* dJ_dU_b,
                       double* dJ_dmu_ref, dugks_adjoint_stats* stats);
 
+/* dugks_adjoint_run, dugks_objective_run and dugks_boundary_fluxes keep up to
+ * 2 GiB of device memory a device for the next such run of any handle there.
+ * It goes back by itself before an allocation of this library fails and with
+ * the device's last handle; this call gives it back at once, for a program
+ * that needs all of the device for allocations of its own. */
+int dugks_release_memory(int32_t device);
+
 /* The objective alone: a forward run of obj->n_steps steps (the handle
  * advances by n_steps) that evaluates J as dugks_adjoint_run defines it;
  * max_snapshots is not used.  For finite-difference checks and line

@@ -12,6 +12,7 @@
 #include <string>
 
 #include "dugks_internal.h"
+#include "dugks_arena.h"
 #include "dugks_kernels.cuh"
 
 using dugks::set_error;
@@ -28,16 +29,47 @@ constexpr double kPi = 3.14159265358979323846;
                              std::string(#call) + ": " + cudaGetErrorString(e_));                       \
     } while (0)
 
+// memory kept between runs (dugks_arena.h), the oldest first, and the handles
+// of every device
+struct Kept {
+    void* p;
+    size_t bytes;
+    int device;
+};
+std::mutex kept_lock;
+std::vector<Kept> kept;
+std::vector<int> device_handles;
+
+// whether there was any to give back
+bool release_kept(int device) {
+    std::lock_guard<std::mutex> g(kept_lock);
+    const auto mine = std::stable_partition(kept.begin(), kept.end(), [&](const Kept& k) { return k.device != device; });
+    const bool any = mine != kept.end();
+    for (auto k = mine; k != kept.end(); ++k) cudaFree(k->p);
+    kept.erase(mine, kept.end());
+    return any;
+}
+
+void enter_device(dugks_handle* h) {
+    std::lock_guard<std::mutex> g(kept_lock);
+    if (device_handles.size() <= static_cast<size_t>(h->device)) device_handles.resize(h->device + 1, 0);
+    ++device_handles[h->device];
+    h->counted = true;
+}
+
+void leave_device(int device) {
+    {
+        std::lock_guard<std::mutex> g(kept_lock);
+        if (--device_handles[device] > 0) return;
+    }
+    release_kept(device);
+}
+
 template <typename T>
 int dev_alloc(dugks_handle* h, T** p, size_t count) {
     void* q = nullptr;
     const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-    cudaError_t e = cudaMalloc(&q, bytes);
-    if (e == cudaErrorMemoryAllocation && !h->kept.empty()) {
-        cudaGetLastError();
-        dugks::free_kept(h);
-        e = cudaMalloc(&q, bytes);
-    }
+    const cudaError_t e = dugks::device_malloc(&q, bytes);
     if (e != cudaSuccess)
         return set_error(h, e == cudaErrorMemoryAllocation ? DUGKS_ERR_OOM : DUGKS_ERR_CUDA,
                          "cudaMalloc of " + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e));
@@ -380,6 +412,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     if (h->device < 0 || h->device >= dev_count) return fail(DUGKS_ERR_ARG, "dugks_create: bad device ordinal");
     cudaError_t ce = cudaSetDevice(h->device);
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(ce));
+    enter_device(h);
     const int rows = h->nv / h->n1d;
     // velocity-space shard: this device's block of DV rows
     int row0 = 0, row1 = rows;
@@ -1429,7 +1462,7 @@ static int state_io(dugks_handle* h, double* g, double* hh, const double* gi, co
     // (a step whose phases the caller drives may be half done: gbar+ is kept)
     std::unique_ptr<void, cudaError_t (*)(void*)> own(nullptr, cudaFree);
     if (h->shard_phase_next != 0) {
-        CUDA_TRY(h, cudaMalloc(&buf, part * sizeof(double)));
+        CUDA_TRY(h, dugks::device_malloc(reinterpret_cast<void**>(&buf), part * sizeof(double)));
         own.reset(buf);
     }
     for (int which = 0; which < 2; ++which) {
@@ -1505,13 +1538,19 @@ int dugks_last_step_ms(dugks_handle* h, double* ms) {
 
 const char* dugks_last_error(const dugks_handle* h) { return h ? h->last_error.c_str() : "null handle"; }
 
+int dugks_release_memory(int32_t device) {
+    if (device < 0) return DUGKS_ERR_ARG;
+    release_kept(device);
+    return DUGKS_OK;
+}
+
 void dugks_destroy(dugks_handle* h) {
     if (!h) return;
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->nccl_comm) nccl_api().comm_destroy(static_cast<ncclComm_t>(h->nccl_comm));
     for (void* p : h->allocations) cudaFree(p);
-    dugks::free_kept(h);
+    if (h->counted) leave_device(h->device);
     if (h->host_cm) cudaFreeHost(h->host_cm);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
@@ -1523,9 +1562,40 @@ void dugks_destroy(dugks_handle* h) {
 
 namespace dugks {
 
-void free_kept(dugks_handle* h) {
-    for (auto& k : h->kept) cudaFree(k.first);
-    h->kept.clear();
+void* take_kept(int device, size_t bytes) {
+    std::lock_guard<std::mutex> g(kept_lock);
+    for (size_t i = 0; i < kept.size(); ++i)
+        if (kept[i].device == device && kept[i].bytes == bytes) {
+            void* p = kept[i].p;
+            kept.erase(kept.begin() + i);
+            return p;
+        }
+    return nullptr;
+}
+
+void keep(int device, void* p, size_t bytes) {
+    std::lock_guard<std::mutex> g(kept_lock);
+    kept.push_back({p, bytes, device});
+    size_t total = 0;
+    for (const Kept& k : kept) total += k.device == device ? k.bytes : 0;
+    for (size_t i = 0; total > kKeep; ++i) {
+        if (kept[i].device != device) continue;
+        cudaFree(kept[i].p);
+        total -= kept[i].bytes;
+        kept.erase(kept.begin() + i--);
+    }
+}
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        int device = 0;
+        cudaGetLastError();
+        cudaGetDevice(&device);
+        if (release_kept(device)) e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 // Rebuilds the cell records and Maxwellian tables from the cell macros in

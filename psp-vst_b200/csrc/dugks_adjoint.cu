@@ -12,10 +12,11 @@
 #include <vector>
 
 #include "dugks_adjoint.cuh"
-#include "dugks_internal.h"
+#include "dugks_arena.h"
 
 namespace {
 
+using dugks::Arena;
 using dugks::set_error;
 namespace adj = dugks::adj;
 
@@ -62,71 +63,6 @@ struct GpuEx {
     }
     // face values and their moments of the recorded step, into the handle's buffers
     int face_values(const adj::View& v) { return dugks::record_face_values(h, v.dt); }
-};
-
-// Device memory of one run.  It goes back to the handle, which keeps up to
-// kKeep bytes of it for its next run: mapping and unmapping the 950 MB of a
-// 12-step run with 4,096 cells and 1,024 DVs takes as long as its kernels.  What
-// the handle keeps is the last run's, is used on the handle's stream alone, and
-// is given back when the handle is destroyed or an allocation of it fails.
-constexpr size_t kKeep = size_t(2) << 30;
-struct Arena {
-    dugks_handle* h;
-    std::vector<std::pair<void*, size_t>> p;
-    double bytes = 0;
-    explicit Arena(dugks_handle* h) : h(h) {}
-    Arena(const Arena&) = delete;
-    ~Arena() {
-        dugks::free_kept(h);
-        size_t kept = 0;
-        for (auto& q : p) {
-            if (kept + q.second > kKeep) {
-                cudaFree(q.first);
-                continue;
-            }
-            kept += q.second;
-            h->kept.push_back(q);
-        }
-    }
-    template <class T>
-    int get(dugks_handle* h, T** out, size_t n) {
-        const size_t b = std::max<size_t>(n, 1) * sizeof(T);
-        bytes += static_cast<double>(b);
-        for (size_t i = 0; i < h->kept.size(); ++i)
-            if (h->kept[i].second == b) {
-                p.push_back(h->kept[i]);
-                h->kept.erase(h->kept.begin() + i);
-                *out = static_cast<T*>(p.back().first);
-                return DUGKS_OK;
-            }
-        void* q = nullptr;
-        cudaError_t e = cudaMalloc(&q, b);
-        if (e == cudaErrorMemoryAllocation && !h->kept.empty()) {
-            cudaGetLastError();
-            dugks::free_kept(h);
-            e = cudaMalloc(&q, b);
-        }
-        if (e != cudaSuccess)
-            return set_error(h, e == cudaErrorMemoryAllocation ? DUGKS_ERR_OOM : DUGKS_ERR_CUDA,
-                             "dugks_adjoint_run: cudaMalloc of " + std::to_string(b) + " bytes: " +
-                                 cudaGetErrorString(e));
-        p.emplace_back(q, b);
-        *out = static_cast<T*>(q);
-        return DUGKS_OK;
-    }
-    template <class T>
-    int put(dugks_handle* h, T** out, const std::vector<T>& v) {
-        if (int st = get(h, out, v.size())) return st;
-        if (!v.empty()) ADJ_TRY(h, cudaMemcpyAsync(*out, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice,
-                                                   h->stream));
-        return DUGKS_OK;
-    }
-    template <class T>
-    int zeros(dugks_handle* h, T** out, size_t n) {
-        if (int st = get(h, out, n)) return st;
-        ADJ_TRY(h, cudaMemsetAsync(*out, 0, std::max<size_t>(n, 1) * sizeof(T), h->stream));
-        return DUGKS_OK;
-    }
 };
 
 // checkpoint operations on the handle (revolve's Ops)

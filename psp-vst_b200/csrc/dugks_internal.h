@@ -6,7 +6,6 @@
 
 #include <cstdint>
 #include <string>
-#include <utility>
 #include <vector>
 
 #include "dugks.h"
@@ -216,7 +215,7 @@ struct dugks_handle {
     dugks::DevMesh dm{};
     dugks::DevState ds{};
     std::vector<void*> allocations;
-    std::vector<std::pair<void*, size_t>> kept;   // adjoint memory between runs: block, bytes
+    bool counted = false;           // among its device's handles (dugks_arena.h)
     int32_t* d_iperm = nullptr;     // Tiling::iperm
     double* d_dt = nullptr;         // [2] device time steps of adaptive stepping (ping-pong)
     double* d_hist = nullptr;       // time steps of the last adaptive call
@@ -238,8 +237,6 @@ namespace dugks {
 void compute_weights_and_ls(dugks_handle* h, int weighting);
 void build_tiling(dugks_handle* h, int tile_cells);
 int set_error(dugks_handle* h, int code, const std::string& msg);
-// gives back the adjoint memory kept between runs
-void free_kept(dugks_handle* h);
 // ABI helpers (dugks_abi.cpp): cell records and tables from ds.cm
 int rebuild_cell_records(dugks_handle* h);
 // the step's face values at the half step (DevState::fvg, fvh) and their raw

@@ -150,6 +150,7 @@ SIGNATURES = {
     "dugks_get_step_record": (C.c_int, [C.c_void_p, _dp]),
     "dugks_set_step_record": (C.c_int, [C.c_void_p, _dp]),
     "dugks_adjoint_run": (C.c_int, [C.c_void_p, C.POINTER(Objective), _dp, _dp, _dp, _dp, C.POINTER(AdjointStats)]),
+    "dugks_release_memory": (C.c_int, [C.c_int32]),
     "dugks_objective_run": (C.c_int, [C.c_void_p, C.POINTER(Objective), _dp, C.POINTER(AdjointStats)]),
     "dugks_boundary_fluxes": (C.c_int, [C.c_void_p, C.c_double, _dp]),
     "dugks_checkpoint_forward_steps": (C.c_int64, [C.c_int32, C.c_int32]),

@@ -8,6 +8,7 @@
 #include <mutex>
 #include <vector>
 
+#include "dugks_arena.h"
 #include "dugks_kernels.cuh"
 
 namespace {
@@ -24,7 +25,11 @@ thread_local cudaError_t last = cudaSuccess;
 int last_hzero = -1, last_chunks[2], passes = 0;
 
 int device_of(cudaStream_t s) { return *reinterpret_cast<int*>(s); }
-cudaError_t launch(cudaStream_t s) { return device_of(s) == current ? cudaSuccess : cudaErrorInvalidResourceHandle; }
+// (a launch reports what cudaGetLastError finds, an error before it included)
+cudaError_t launch(cudaStream_t s) {
+    const cudaError_t e = device_of(s) == current ? last : cudaErrorInvalidResourceHandle;
+    return last = cudaSuccess, e;
+}
 
 }  // namespace
 
@@ -37,6 +42,16 @@ int fake_device() { return current; }
 int fake_last_hzero() { return last_hzero; }
 int fake_last_chunks(int faces) { return last_chunks[faces]; }
 int fake_passes() { return passes; }
+// a run that takes n blocks of these bytes
+int fake_run(dugks_handle* h, const size_t* bytes, int n) {
+    cudaSetDevice(h->device);
+    dugks::Arena ar(h);
+    for (int i = 0; i < n; ++i) {
+        unsigned char* p;
+        if (int st = ar.get(h, &p, bytes[i])) return st;
+    }
+    return DUGKS_OK;
+}
 
 cudaError_t cudaMalloc(void** p, size_t n) {
     std::lock_guard<std::mutex> g(lock);

@@ -90,3 +90,46 @@ def test_reported_chunks_give_the_handle_they_were_read_from(fake, n, n_dv, scal
     assert got == chunks(got[0])
     if scale == 1:
         assert got == auto
+
+
+def _run(fake, s, *mib):
+    sizes = (C.c_size_t * len(mib))(*[m << 20 for m in mib])
+    return fake.fake_run(s.h, sizes, len(mib))
+
+
+def test_memory_kept_between_runs_is_bounded_and_given_back(memory):
+    c = cs.cavity_case(4, 6)
+    a, b = (dl.Solver(c, lib_path=memory.path) for _ in range(2))
+    other = dl.Solver(c, device=1, lib_path=memory.path)
+    bare = memory.fake_used(0)
+    kept = lambda: (memory.fake_used(0) - bare) >> 20   # noqa: E731
+    assert _run(memory, a, 500, 300) == 0 and kept() == 800
+    # a small run in between, another handle's run and another device's: the
+    # blocks are there for the next run
+    assert _run(memory, a, 1) == 0 and _run(memory, b, 500, 300) == 0 and kept() == 801
+    assert _run(memory, other, 7) == 0 and kept() == 801
+    # 2 GiB a device at most, over all handles
+    for m in (600, 700, 900, 3000):
+        assert _run(memory, b, m) == 0 and kept() <= 2048
+    # no allocation of any handle fails while memory is kept
+    assert _run(memory, a, 1000, 900) == 0
+    memory.fake_capacity(0, memory.fake_used(0))
+    d = dl.Solver(cs.cavity_case(40, 20), lib_path=memory.path)
+    assert kept() < 100
+    d.close()
+    memory.fake_capacity(0, bare + (500 << 20))
+    assert _run(memory, a, 400) == 0 and kept() == 400
+    assert _run(memory, b, 450) == 0 and kept() == 450
+    assert _run(memory, b, 600) == 3
+    a.step(1, c.dt)                                      # the failure leaves no error behind
+    memory.fake_capacity(0, 1 << 40)
+    # a call for it, and the last handle of the device
+    assert _run(memory, a, 300) == 0 and kept() == 300
+    assert memory.dugks_release_memory(0) == 0 and kept() == 0 and memory.dugks_release_memory(-1) == 1
+    assert _run(memory, a, 300) == 0
+    a.close()
+    assert kept() >= 299
+    b.close()
+    assert memory.fake_used(0) == 0 and memory.fake_used(1) > 7 << 20
+    other.close()
+    assert memory.fake_used(1) == 0
