@@ -109,6 +109,7 @@ dugks::StepArgs make_args(const dugks_handle* h, double dt) {
     a.chunks_f = h->chunks_f;
     a.hzero = h->h_zero ? 1 : 0;
     a.fused = sharded(h) ? 0 : 1;
+    a.seg1 = h->dm.n_seg;
     return a;
 }
 
@@ -200,21 +201,63 @@ void dugks_default_options(dugks_options* opt) {
 // (DV lists carry it all the same)
 static bool can_skip_h(const dugks_handle* h) { return h->D == 3 && h->gas.K_inner == 0 && !h->dm.general_dv; }
 
-// the step arrays of h
+// gbar+ (g) and hbar+ (hh) for all DVs, or as many at a time as memory allows:
+// pass A fills and uses them, so it can walk the DVs in parts.  Whole, they are
+// a quarter of the step's memory where h is carried in 2-D (8 reals a cell and
+// DV, 6 without them), and the largest case a device holds would be a fifth
+// smaller.  Arrays over kWholeBars take a quarter of the free memory at most.
+constexpr size_t kWholeBars = size_t(1) << 28;
+static int alloc_bars(dugks_handle* h, bool g, bool hh) {
+    dugks::DevMesh& dm = h->dm;
+    const int unit = !dm.general_dv && dm.n1d > dugks::kSeg ? 2 : 1, arrays = g + hh;   // whole rows
+    auto dvs = [&](int per) { return per < dm.n_seg ? dugks::seg_dv(dm, per) : dm.nv_loc; };
+    auto bytes = [&](int per) { return (static_cast<size_t>(dvs(per)) * dm.pC + dugks::kSlack) * real_size(h); };
+    int per = g ? dm.n_seg : dm.seg_bar;
+    size_t most = arrays * bytes(per), total = 0;
+    if (most > kWholeBars) {
+        CUDA_TRY(h, cudaMemGetInfo(&most, &total));
+        most /= 4;
+    }
+    for (;; per = std::max(unit, (per / 2 + unit - 1) / unit * unit)) {
+        if (per > unit && arrays * bytes(per) > most) continue;
+        void* p[2] = {nullptr, nullptr};
+        cudaError_t e = g ? dugks::device_malloc(&p[0], bytes(per)) : cudaSuccess;
+        if (hh && e == cudaSuccess) e = dugks::device_malloc(&p[1], bytes(per));
+        if (e == cudaSuccess) {
+            for (void* q : p)
+                if (q) h->allocations.push_back(q);
+            if (g) h->ds.gbar = p[0];
+            if (hh) h->ds.hbar = p[1];
+            dm.seg_bar = per;
+            dm.nv_bar = dvs(per);
+            return DUGKS_OK;
+        }
+        if (p[0]) cudaFree(p[0]);
+        if (e != cudaErrorMemoryAllocation || per == unit)
+            return set_error(h, e == cudaErrorMemoryAllocation ? DUGKS_ERR_OOM : DUGKS_ERR_CUDA,
+                             "cudaMalloc of " + std::to_string(bytes(per)) + " bytes: " + cudaGetErrorString(e));
+    }
+}
+
+// h's face values, zero
+static int alloc_fvh(dugks_handle* h) {
+    const size_t bytes = (static_cast<size_t>(h->dm.nv_loc) * h->dm.pF + dugks::kSlack) * real_size(h);
+    unsigned char* f = nullptr;
+    if (int st = dev_alloc(h, &f, bytes)) return st;
+    CUDA_TRY(h, cudaMemsetAsync(f, 0, bytes, h->stream));
+    h->ds.fvh = f;
+    return DUGKS_OK;
+}
+
+// the step arrays of h, for a handle that was created without them
 static int alloc_h(dugks_handle* h) {
     if (h->ds.hbar) return DUGKS_OK;
-    const size_t rs = real_size(h);
-    const size_t nvc = static_cast<size_t>(h->dm.nv_loc) * h->dm.pC + dugks::kSlack,
-                 nfv = static_cast<size_t>(h->dm.nv_loc) * h->dm.pF + dugks::kSlack;
-    unsigned char *b = nullptr, *f = nullptr;
-    if (int st = dev_alloc(h, &b, nvc * rs)) return st;
-    if (int st = dev_alloc(h, &f, nfv * rs)) {
-        dev_free(h, b);
+    if (int st = alloc_fvh(h)) return st;
+    if (int st = alloc_bars(h, false, true)) {
+        dev_free(h, h->ds.fvh);
+        h->ds.fvh = nullptr;
         return st;
     }
-    CUDA_TRY(h, cudaMemsetAsync(f, 0, nfv * rs, h->stream));
-    h->ds.hbar = b;
-    h->ds.fvh = f;
     return DUGKS_OK;
 }
 
@@ -617,8 +660,6 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     ds.g = p;
     if ((st = dev_alloc(h, &p, nvc * rs))) return *out = h, st;
     ds.h = p;
-    if ((st = dev_alloc(h, &p, nvc * rs))) return *out = h, st;
-    ds.gbar = p;
     if ((st = dev_alloc(h, &p, nfv * rs))) return *out = h, st;
     ds.fvg = p;
     // face values start at zero: the slots of incoming boundary DVs are read
@@ -626,7 +667,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     if (cudaMemsetAsync(ds.fvg, 0, nfv * rs, h->stream) != cudaSuccess) return fail(DUGKS_ERR_CUDA, "cudaMemset of the face values");
     // where h stays identically zero its step arrays are left out until a
     // nonzero h~ is loaded (alloc_h)
-    if (!can_skip_h(h) && (st = alloc_h(h))) return *out = h, st;
+    if (!can_skip_h(h) && (st = alloc_fvh(h))) return *out = h, st;
     const int nbl = (nIF + 127) / 128 + (nBF + 31) / 32;
     dm.done_cells = nbl;
     const size_t n_done = static_cast<size_t>(nbl) + (nC + 31) / 32;
@@ -691,6 +732,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         dm.n_tang = static_cast<long long>(n_tang);
     }
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, std::string("upwind bits: ") + cudaGetErrorString(ce));
+    if ((st = alloc_bars(h, true, !can_skip_h(h)))) return *out = h, st;
     if (shard && shard->use_nccl) {
         // collective: every rank of the shard set makes this call
         const NcclApi& api = nccl_api();
@@ -1449,12 +1491,12 @@ int dugks_get_df(dugks_handle* h, const int32_t* cells, int32_t n, double* g_out
 // g~ and h~ in the caller's [dv][cell] order of doubles, from the state (get)
 // or into it.  The copies go straight between the caller's arrays and gbar+'s
 // buffer, which holds nothing between steps, in as many parts as its size
-// asks for (one in FP64), and k_state_order puts each part in order.
+// asks for (one in FP64 where gbar+ is whole), and k_state_order puts each part in order.
 static int state_io(dugks_handle* h, double* g, double* hh, const double* gi, const double* hi, bool get) {
     if (!h) return DUGKS_ERR_ARG;
     if (!h->initialised) return set_error(h, DUGKS_ERR_STATE, "state access before dugks_set_macros");
     const size_t n = static_cast<size_t>(h->dm.nv_loc) * h->nC;
-    const size_t part = (static_cast<size_t>(h->dm.nv_loc) * h->dm.pC + dugks::kSlack) * real_size(h) / sizeof(double);
+    const size_t part = (static_cast<size_t>(h->dm.nv_bar) * h->dm.pC + dugks::kSlack) * real_size(h) / sizeof(double);
     const OnDevice on(h->device);
     CUDA_TRY(h, on.status);
     const dugks::StepArgs a = make_args(h, 0.0);

@@ -82,6 +82,9 @@ struct DevMesh {
     // DV segments: up to kSeg consecutive DVs of one row (of the list); the
     // kernels walk DVs by segments and DV chunks are runs of segments
     int n_seg;
+    // gbar+ and hbar+ hold nv_bar DVs at a time, those of seg_bar segments: all
+    // of them, or as many as memory allowed; pass A then walks the DVs in parts
+    int seg_bar, nv_bar;
     const int2* row_yz;            // y and z index of every row of this device
     // Cells in the renumbered order.  Faces in the order of the step's arrays:
     // internal faces grouped by blocks of 32 cells, first faces of a block's
@@ -132,7 +135,7 @@ struct DevMesh {
 struct DevState {
     void* g;           // state g~ (cells, Real), updated in place
     void* h;
-    void* gbar;        // gbar+ of the step (cells, Real)
+    void* gbar;        // gbar+ of the step (cells, Real, nv_bar DVs)
     void* hbar;        // (null while h is identically zero)
     // face values (faces, Real): the upwind reconstruction at the half step,
     // then, relaxed and multiplied by xi.S, the flux

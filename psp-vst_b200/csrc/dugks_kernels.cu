@@ -178,16 +178,23 @@ __global__ void k_sum_chunks(double* part, int chunks, size_t n) {
 cudaError_t launch_stage(const StepArgs& a, int precision, int stage, cudaStream_t s, int* launches) {
     int n = 0;
     cudaError_t e = cudaSuccess;
-    auto pass = [&](int which) {
-        if (e == cudaSuccess) e = launch_pass(a, precision, which, s);
+    auto pass = [&](int which, const StepArgs& b) {
+        if (e == cudaSuccess) e = launch_pass(b, precision, which, s);
         ++n;
     };
     switch (stage) {
         case STAGE_PASS_A:
-            pass(KERNEL_HALF_STEP);
-            pass(KERNEL_FACE_VALUES);
-            if (a.dm.n_tang > 0) pass(KERNEL_TANGENTIAL);
-            pass(KERNEL_FACE_MOMENTS);
+            for (int seg = 0; seg < a.dm.n_seg; seg += a.dm.seg_bar) {
+                StepArgs b = a;
+                b.seg0 = seg;
+                b.seg1 = std::min(seg + a.dm.seg_bar, a.dm.n_seg);
+                b.d_bar = seg_dv(a.dm, seg);
+                pass(KERNEL_HALF_STEP, b);
+                pass(KERNEL_FACE_VALUES, b);
+                if (a.dm.n_tang > 0) pass(KERNEL_TANGENTIAL, b);
+                if (a.dm.seg_bar < a.dm.n_seg) pass(KERNEL_ZERO_GRADIENT, b);
+            }
+            pass(KERNEL_FACE_MOMENTS, a);
             break;
         case STAGE_FACE_COMBINE:
             if (!a.fused) {
@@ -196,8 +203,8 @@ cudaError_t launch_stage(const StepArgs& a, int precision, int stage, cudaStream
             }
             break;
         case STAGE_PASS_B:
-            pass(KERNEL_FACE_FLUX);
-            pass(KERNEL_UPDATE);
+            pass(KERNEL_FACE_FLUX, a);
+            pass(KERNEL_UPDATE, a);
             break;
         case STAGE_CELL_COMBINE:
             if (!a.fused) {

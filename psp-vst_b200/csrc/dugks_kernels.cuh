@@ -20,6 +20,9 @@ struct StepArgs {
     // done; 0: they leave the chunk sums (sharded handles reduce them first)
     int fused;
     int keep_co;                 // 1: leave the Courant sums of the last step
+    // the part of pass A whose gbar+ is held: segments seg0 .. seg1 - 1, the
+    // first at local DV d_bar (all segments but where DevMesh::seg_bar is less)
+    int seg0, seg1, d_bar;
 };
 
 enum { STAGE_PASS_A = 0, STAGE_FACE_COMBINE = 1, STAGE_PASS_B = 2, STAGE_CELL_COMBINE = 3 };
@@ -27,12 +30,19 @@ enum { STAGE_PASS_A = 0, STAGE_FACE_COMBINE = 1, STAGE_PASS_B = 2, STAGE_CELL_CO
 // kernels of dugks_passes.cu
 enum {
     KERNEL_HALF_STEP = 0, KERNEL_FACE_VALUES = 1, KERNEL_FACE_MOMENTS = 2, KERNEL_FACE_FLUX = 3, KERNEL_UPDATE = 4,
-    KERNEL_STATE_MOMENTS = 5, KERNEL_TANGENTIAL = 6
+    KERNEL_STATE_MOMENTS = 5, KERNEL_TANGENTIAL = 6, KERNEL_ZERO_GRADIENT = 7
 };
 
 // first segment of DV chunk k of n
 __host__ __device__ __forceinline__ int seg_begin(int n_seg, int k, int n) {
     return static_cast<int>(static_cast<long long>(n_seg) * k / n);
+}
+
+// first local DV of segment s
+__host__ __device__ __forceinline__ int seg_dv(const DevMesh& m, int s) {
+    if (m.general_dv) return s * kSeg;
+    const int two = m.n1d > kSeg;   // n1d <= 64: one or two segments a row
+    return (s >> two) * m.n1d + (s & two) * kSeg;
 }
 
 // Bounds-checked build (-DDUGKS_CHECK, libdugks_b200_check.so): every index

@@ -75,7 +75,7 @@ __device__ __forceinline__ Seg seg_at(const DevMesh& m, int s) {
     } else {
         const int two = m.n1d > kSeg, row = s >> two, k = s & two;   // n1d <= 64: one or two segments a row
         q.ix0 = k * kSeg;
-        q.d0 = row * m.n1d + q.ix0;
+        q.d0 = row * m.n1d + q.ix0;   // as seg_dv
         q.len = min(kSeg, m.n1d - q.ix0);
         const int2 t = __ldg(m.row_yz + row);
         q.iy = t.x;
@@ -90,6 +90,11 @@ __device__ __forceinline__ int warp_id() { return __shfl_sync(0xffffffffu, threa
 // element of entity e, DV 0, in an (entity, DV) array of nd DVs; DV d is 32 d on
 __device__ __forceinline__ size_t slot(int e, int nd) {
     return static_cast<size_t>(e >> 5) * nd * 32 + (e & 31);
+}
+
+// the same in gbar+ and hbar+, whose first DV held is a.d_bar
+__device__ __forceinline__ ptrdiff_t bar_slot(const StepArgs& a, int c) {
+    return static_cast<ptrdiff_t>(slot(c, a.dm.nv_bar)) - 32 * static_cast<ptrdiff_t>(a.d_bar);
 }
 
 // calls f(j, U) for groups of U consecutive DVs of a segment, then narrower
@@ -410,11 +415,12 @@ __global__ void __launch_bounds__(kStream) k_half_step(const __grid_constant__ S
     const size_t at = slot(c, m.nv_loc);
     const double K3D = k3d<D>(m), c0h = c0h_of<D>(m);
     Relax<D, HZ, GEN> rx(a.ds.cellrec, a.ds.ctab, m.n1d, c, cell_r(a, c));
-    const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
+    const int ns = a.seg1 - a.seg0;
+    const int s0 = a.seg0 + seg_begin(ns, blockIdx.y, gridDim.y), s1 = a.seg0 + seg_begin(ns, blockIdx.y + 1, gridDim.y);
     const Real* __restrict__ g = reinterpret_cast<const Real*>(a.ds.g) + at;
     const Real* __restrict__ h = reinterpret_cast<const Real*>(a.ds.h) + at;
-    Real* __restrict__ gb = reinterpret_cast<Real*>(a.ds.gbar) + at;
-    Real* __restrict__ hb = reinterpret_cast<Real*>(a.ds.hbar) + at;
+    Real* __restrict__ gb = reinterpret_cast<Real*>(a.ds.gbar) + bar_slot(a, c);
+    Real* __restrict__ hb = reinterpret_cast<Real*>(a.ds.hbar) + bar_slot(a, c);
     constexpr int U = 4;
     struct Buf {
         Real g[U], h[U];
@@ -500,10 +506,10 @@ __device__ __forceinline__ void half_dist(const Real* d, double hdt, const Dv& v
 template <int D, typename Real>
 __device__ __forceinline__ void grad_mem(const DevMesh& m, const Real* f, int c, Real* G, int k0, int* err) {
     const size_t nC = static_cast<size_t>(m.nC);
-    const Real f0 = f[slot(c, m.nv_loc)];
+    const Real f0 = f[slot(c, m.nv_bar)];
     for (int k = k0; k < m.nb_max; ++k) {
         const int n = chk(__ldg(m.nbr + k * nC + c), 0, m.nC, err);
-        const Real df = f[slot(n, m.nv_loc)] - f0;
+        const Real df = f[slot(n, m.nv_bar)] - f0;
 #pragma unroll
         for (int q = 0; q < D; ++q) G[q] = fma(Real(__ldg(m.nbr_ls + (k * 3 + q) * nC + c)), df, G[q]);
     }
@@ -522,7 +528,7 @@ __device__ __forceinline__ Real recon_mem(const DevMesh& m, const Real* row, int
 #pragma unroll
     for (int q = 0; q < D; ++q) d[q] = Real(__ldg(m.fgeo + (3 + 3 * side + q) * nF + f));
     half_dist<D, Real, GEN>(d, hdt, v, rounded, r);
-    return recon<D, Real>(row[slot(c, m.nv_loc)], G, r);
+    return recon<D, Real>(row[slot(c, m.nv_bar)], G, r);
 }
 
 // *p = v where cond is not 0, as one predicated store
@@ -552,8 +558,8 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
     const int c = blockIdx.x * kCells + threadIdx.x;
     if (c >= m.nC) return;
     const size_t nC = static_cast<size_t>(m.nC), nF = static_cast<size_t>(m.nF);
-    const Real* __restrict__ gbar = reinterpret_cast<const Real*>(a.ds.gbar);
-    const Real* __restrict__ hbar = reinterpret_cast<const Real*>(a.ds.hbar);
+    const Real* __restrict__ gbar = reinterpret_cast<const Real*>(a.ds.gbar) - 32 * static_cast<ptrdiff_t>(a.d_bar);
+    const Real* __restrict__ hbar = reinterpret_cast<const Real*>(a.ds.hbar) - 32 * static_cast<ptrdiff_t>(a.d_bar);
     Real* __restrict__ fvg = reinterpret_cast<Real*>(a.ds.fvg);
     Real* __restrict__ fvh = reinterpret_cast<Real*>(a.ds.fvh);
     const double hdt = 0.5 * step_dt(a);
@@ -562,7 +568,7 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
     constexpr bool kFold = sizeof(Real) == 8;
     // DVs whose loads are issued together, as the registers allow
     constexpr int kGroup = sizeof(Real) == 4 ? 4 : HZ || D == 2 ? 2 : 1;
-    const Off own = static_cast<Off>(slot(c, m.nv_loc));
+    const Off own = static_cast<Off>(slot(c, m.nv_bar));
     Off nb[NS], fo[NS];   // the neighbours' and faces' elements
     unsigned uo[NS];      // the faces' upwind words in a segment's row
     unsigned has = 0, in_tile = 0;
@@ -570,7 +576,7 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
     Real* dist = dist_s + threadIdx.x;   // Cf - C of slot k, dimension q: dist[(k D + q) kCells]
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
-        nb[k] = static_cast<Off>(slot(k < m.nb_max ? chk(__ldg(m.nbr + k * nC + c), 0, m.nC, a.ds.err) : c, m.nv_loc));
+        nb[k] = static_cast<Off>(slot(k < m.nb_max ? chk(__ldg(m.nbr + k * nC + c), 0, m.nC, a.ds.err) : c, m.nv_bar));
         const int code = k < m.nf_max ? chk(__ldg(m.cface + k * nC + c), -1, 4 * m.nF, a.ds.err) : -1;
         const int f = code < 0 ? 0 : code >> 2, sd = code < 0 ? 0 : code & 1;
         fo[k] = static_cast<Off>(slot(f, m.nv_loc));
@@ -583,7 +589,8 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
             dist[(k * D + q) * kCells] = Real(__ldg(m.fgeo + (3 + 3 * sd + q) * nF + f));
         }
     }
-    const int s0 = seg_begin(m.n_seg, blockIdx.y, gridDim.y), s1 = seg_begin(m.n_seg, blockIdx.y + 1, gridDim.y);
+    const int ns = a.seg1 - a.seg0;
+    const int s0 = a.seg0 + seg_begin(ns, blockIdx.y, gridDim.y), s1 = a.seg0 + seg_begin(ns, blockIdx.y + 1, gridDim.y);
     const bool more = m.nb_max > NS || m.nf_max > NS;
     for (int s = s0; s < s1; ++s) {
         const Seg q = seg_at<GEN>(m, s);
@@ -795,6 +802,7 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
          i += static_cast<long long>(gridDim.x) * kStream) {
         const int2 t = __ldg(m.tang + i);
         const int f = chk(t.x, 0, m.nIF, a.ds.err), s = chk(t.y / kSeg, 0, m.n_seg, a.ds.err), j = t.y % kSeg;
+        if (s < a.seg0 || s >= a.seg1) continue;
         const Seg q = seg_at<GEN>(m, s);
         const int o = chk(__ldg(m.fown + f), 0, m.nC, a.ds.err), n = chk(__ldg(m.fnei + f), 0, m.nC, a.ds.err);
         bool in_tile = false;
@@ -804,7 +812,7 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
         const Dv v = dv_at<D, GEN>(m, q, x1, j);
         const size_t rc = 32 * static_cast<size_t>(q.d0 + j), rf = slot(f, m.nv_loc) + rc;
         auto average = [&](const void* bar, void* fv, float* res) {
-            const Real* b = reinterpret_cast<const Real*>(bar) + rc;
+            const Real* b = reinterpret_cast<const Real*>(bar) + (rc - 32 * static_cast<size_t>(a.d_bar));
             const Real vn = recon_mem<D, Real, GEN>(m, b, f, 1, n, hdt, v, rounded, a.ds.err);
             const Real vo = recon_mem<D, Real, GEN>(m, b, f, 0, o, hdt, v, rounded, a.ds.err);
             const Real mean = Real(0.5) * (vn + vo);
@@ -815,6 +823,25 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
         };
         average(a.ds.gbar, a.ds.fvg, a.ds.tang_res);
         if (!HZ) average(a.ds.hbar, a.ds.fvh, a.ds.tang_res ? a.ds.tang_res + m.n_tang : nullptr);
+    }
+}
+
+// Zero-gradient faces of a part of pass A: the owner's gbar+, which the face
+// moments cannot read once the next part has taken its place.  Launched where
+// gbar+ is held in parts; otherwise k_face_moments reads it.
+template <typename Real>
+__global__ void __launch_bounds__(kStream) k_zero_gradient(const __grid_constant__ StepArgs a) {
+    const DevMesh& m = a.dm;
+    const int b = blockIdx.x * kLanes + threadIdx.x % kLanes;
+    if (b >= m.nBF || __ldg(m.bface_ptype + b) != DUGKS_PATCH_ZERO_GRADIENT) return;
+    const ptrdiff_t own = bar_slot(a, chk(__ldg(m.bface_owner + b), 0, m.nC, a.ds.err));
+    const size_t f = slot(m.nIF + b, m.nv_loc);
+    const int d1 = min(a.d_bar + m.nv_bar, m.nv_loc);
+    for (int d = a.d_bar + threadIdx.x / kLanes; d < d1; d += kStream / kLanes) {
+        const size_t o = 32 * static_cast<size_t>(d);
+        reinterpret_cast<Real*>(a.ds.fvg)[f + o] = reinterpret_cast<const Real*>(a.ds.gbar)[own + static_cast<ptrdiff_t>(o)];
+        if (!a.hzero)
+            reinterpret_cast<Real*>(a.ds.fvh)[f + o] = reinterpret_cast<const Real*>(a.ds.hbar)[own + static_cast<ptrdiff_t>(o)];
     }
 }
 
@@ -1301,13 +1328,15 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
             const double gr = dv_ref<Real, GEN>(m.gref, d), hr = dv_ref<Real, GEN>(m.href, d);
             double g, h = 0.0;
             if (zero_grad) {
-                // every DV: the owner cell's gbar+ (fvDVM.C:887-891)
+                // every DV: the owner cell's gbar+ (fvDVM.C:887-891), which
+                // k_zero_gradient has stored already where it is held in parts
+                const bool there = m.nv_bar < m.nv_loc;
                 const size_t oc = slot(own, m.nv_loc) + o;
-                const Real gc = reinterpret_cast<const Real*>(a.ds.gbar)[oc];
+                const Real gc = there ? gv : reinterpret_cast<const Real*>(a.ds.gbar)[oc];
                 fg[o] = gc;
                 g = double(gc) + gr;
                 if (!HZ) {
-                    const Real hc = reinterpret_cast<const Real*>(a.ds.hbar)[oc];
+                    const Real hc = there ? hv : reinterpret_cast<const Real*>(a.ds.hbar)[oc];
                     fh[o] = hc;
                     h = double(hc) + hr;
                 }
@@ -1840,9 +1869,9 @@ int blocks(int n, int per) { return (n + per - 1) / per; }
 // last wave is short.  (Two for k_face_flux, whose rings and boundary records
 // each CTA sets up: 1,728 cells and 10^3 DVs 147 us a step, four 159; the
 // others are level from two to eight.)
-int stream_chunks(const DevMesh& m, int nb, int waves = 4) {
+int stream_chunks(int n_seg, int nb, int waves = 4) {
     const int target = 148 * 8 * waves;
-    return std::max(1, std::min({m.n_seg, (target + nb - 1) / std::max(nb, 1), 65535}));
+    return std::max(1, std::min({n_seg, (target + nb - 1) / std::max(nb, 1), 65535}));
 }
 
 template <int D, typename Real, bool HZ, bool GEN>
@@ -1856,12 +1885,12 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
     switch (which) {
         case KERNEL_HALF_STEP: {
             const int nb = blocks(m.nC, kStream);
-            k_half_step<D, Real, HZ, GEN><<<dim3(nb, stream_chunks(m, nb)), kStream, 0, s>>>(a);
+            k_half_step<D, Real, HZ, GEN><<<dim3(nb, stream_chunks(a.seg1 - a.seg0, nb)), kStream, 0, s>>>(a);
             break;
         }
         case KERNEL_FACE_VALUES: {
             const int nb = blocks(m.nC, kCells);
-            const dim3 grid(nb, stream_chunks(m, nb));
+            const dim3 grid(nb, stream_chunks(a.seg1 - a.seg0, nb));
             if (wide) k_face_values<D, Real, HZ, GEN, kFast, size_t><<<grid, kCells, 0, s>>>(a);
             else if (quad) k_face_values<D, Real, HZ, GEN, 4, unsigned><<<grid, kCells, 0, s>>>(a);
             else k_face_values<D, Real, HZ, GEN, kFast, unsigned><<<grid, kCells, 0, s>>>(a);
@@ -1872,13 +1901,16 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
             k_tangential<D, Real, HZ, GEN><<<static_cast<int>(std::min<long long>(nb, 148 * 64)), kStream, 0, s>>>(a);
             break;
         }
+        case KERNEL_ZERO_GRADIENT:
+            if (m.nBF > 0) k_zero_gradient<Real><<<blocks(m.nBF, kLanes), kStream, 0, s>>>(a);
+            break;
         case KERNEL_FACE_MOMENTS:
             k_face_moments<D, Real, HZ, GEN>
                 <<<dim3(nbF, a.chunks_f), kFaces, ring_moments<Real, HZ>(), s>>>(a, k);
             break;
         case KERNEL_FACE_FLUX: {
             k_face_flux<D, Real, HZ, GEN>
-                <<<dim3(nbF, stream_chunks(m, nbF, 2)), kFaces, ring_flux<Real, HZ, GEN>(), s>>>(a);
+                <<<dim3(nbF, stream_chunks(m.n_seg, nbF, 2)), kFaces, ring_flux<Real, HZ, GEN>(), s>>>(a);
             break;
         }
         case KERNEL_UPDATE: {

@@ -133,3 +133,45 @@ def test_memory_kept_between_runs_is_bounded_and_given_back(memory):
     assert memory.fake_used(0) == 0 and memory.fake_used(1) > 7 << 20
     other.close()
     assert memory.fake_used(1) == 0
+
+
+def _with_nodes(c, n_dv):
+    c.xis, c.weights, c.xi_max = np.linspace(-1600.0, 1600.0, n_dv), np.full(n_dv, 3200.0 / n_dv), 1600.0
+    return c
+
+
+@pytest.mark.parametrize("n_dv", [8, 40])
+def test_the_half_steps_arrays_take_what_memory_is_left(memory, n_dv):
+    # 2-D: gbar+ and hbar+ are two of eight reals a cell and DV; with a
+    # quarter of them (whole rows of DVs at least) a handle still fits
+    c = _with_nodes(cs.cavity_case(24, 6), n_dv)
+    s = dl.Solver(c, lib_path=memory.path)
+    whole = memory.fake_used(0)
+    bars = 2 * 8 * 576 * n_dv * n_dv
+    s.close()
+    assert memory.fake_used(0) == 0
+    memory.fake_capacity(0, whole - bars * 3 // 4 + 20000)
+    s = dl.Solver(c, lib_path=memory.path)
+    assert memory.fake_used(0) <= whole - bars * 3 // 4 + 20000
+    g, h = s.state()
+    s.set_state(g + np.arange(g.size).reshape(g.shape), h + 2.0, 1e-6)     # in parts of gbar+'s size
+    assert np.array_equal(s.state()[0], 1.0 + np.arange(g.size).reshape(g.shape)) and np.all(s.state()[1] == 2.0)
+    s.close()
+    memory.fake_capacity(0, whole - bars)
+    with pytest.raises(dl.DugksError) as e:
+        dl.Solver(c, lib_path=memory.path)
+    assert e.value.code == 3 and memory.fake_used(0) == 0
+
+
+def test_large_half_step_arrays_leave_memory_free(memory):
+    # 2 x 284 MB of gbar+ and hbar+: whole on a large device, cut where they are
+    # more than a quarter of what is free
+    c = _with_nodes(cs.cavity_case(150, 6), 40)
+    s = dl.Solver(c, lib_path=memory.path)
+    whole = memory.fake_used(0)
+    s.close()
+    bars = 2 * 8 * 22528 * 1600
+    memory.fake_capacity(0, whole + bars)
+    s = dl.Solver(c, lib_path=memory.path)
+    assert memory.fake_used(0) <= whole - bars // 2 + 40000
+    s.close()
