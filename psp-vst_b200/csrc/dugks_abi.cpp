@@ -470,6 +470,8 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         row1 = static_cast<int>(static_cast<int64_t>(rows) * (shard->rank + 1) / shard->world);
     }
     const int rows_loc = row1 - row0;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
     // DV segments, and DV chunks of the face and cell reductions.  A given
     // dv_chunks is that of the cells, as far as there are segments; the faces'
     // moves from its automatic count by the same factor, so that the count
@@ -485,7 +487,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     // 1,331 listed DVs: 3 and 6 chunks 1,450 us, 5 1,506 and 8 1,590.)
     const int cap = std::max(1, static_cast<int>(std::sqrt(static_cast<double>(n_seg))));
     auto chunks_for = [&](int entities) {
-        const long long nb = (entities + 31) / 32, slots = 148 * 4;
+        const long long nb = (entities + 31) / 32, slots = sms * 4;
         const int one = static_cast<int>(std::min<long long>(slots / nb, cap));
         if (one > 0 && n_seg <= 8 * 4 * one) return one;
         int best = 1;
@@ -500,7 +502,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     // the face reduction, one thread per internal face: four waves (3,721
     // cells: 28 chunks 260 us a step, 5 234; 1,728 cells, 10^3 DVs: 46 chunks 222 us, 10 171)
     auto chunks_f_for = [&](int entities) {
-        const int nb = (entities + 127) / 128, want = (148 * 5 * 4 + nb - 1) / nb;
+        const int nb = (entities + 127) / 128, want = (sms * 5 * 4 + nb - 1) / nb;
         return std::max(1, std::min(want, cap));
     };
     h->chunks = chunks_for(nC);
@@ -536,6 +538,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dm.pC = (nC + 31) / 32 * 32;
     dm.pF = (nF + 31) / 32 * 32;
     dm.n_seg = n_seg;
+    dm.sms = sms;
     dm.xi_max_co = std::sqrt(static_cast<double>(h->D)) * h->xi_max;
     int st;
     ce = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);

@@ -1865,12 +1865,12 @@ __global__ void __launch_bounds__(kLanes* kParts) k_state_moments(const __grid_c
 int blocks(int n, int per) { return (n + per - 1) / per; }
 
 // CTAs along the DV segments for the kernels without a reduction: about
-// eight CTAs of 128 threads on each of 148 SMs, `waves` times over, so that the
+// eight CTAs of 128 threads on each SM, `waves` times over, so that the
 // last wave is short.  (Two for k_face_flux, whose rings and boundary records
 // each CTA sets up: 1,728 cells and 10^3 DVs 147 us a step, four 159; the
 // others are level from two to eight.)
-int stream_chunks(int n_seg, int nb, int waves = 4) {
-    const int target = 148 * 8 * waves;
+int stream_chunks(const DevMesh& m, int n_seg, int nb, int waves = 4) {
+    const int target = m.sms * 8 * waves;
     return std::max(1, std::min({n_seg, (target + nb - 1) / std::max(nb, 1), 65535}));
 }
 
@@ -1885,12 +1885,12 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
     switch (which) {
         case KERNEL_HALF_STEP: {
             const int nb = blocks(m.nC, kStream);
-            k_half_step<D, Real, HZ, GEN><<<dim3(nb, stream_chunks(a.seg1 - a.seg0, nb)), kStream, 0, s>>>(a);
+            k_half_step<D, Real, HZ, GEN><<<dim3(nb, stream_chunks(m, a.seg1 - a.seg0, nb)), kStream, 0, s>>>(a);
             break;
         }
         case KERNEL_FACE_VALUES: {
             const int nb = blocks(m.nC, kCells);
-            const dim3 grid(nb, stream_chunks(a.seg1 - a.seg0, nb));
+            const dim3 grid(nb, stream_chunks(m, a.seg1 - a.seg0, nb));
             if (wide) k_face_values<D, Real, HZ, GEN, kFast, size_t><<<grid, kCells, 0, s>>>(a);
             else if (quad) k_face_values<D, Real, HZ, GEN, 4, unsigned><<<grid, kCells, 0, s>>>(a);
             else k_face_values<D, Real, HZ, GEN, kFast, unsigned><<<grid, kCells, 0, s>>>(a);
@@ -1898,7 +1898,7 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
         }
         case KERNEL_TANGENTIAL: {
             const long long nb = (m.n_tang + kStream - 1) / kStream;
-            k_tangential<D, Real, HZ, GEN><<<static_cast<int>(std::min<long long>(nb, 148 * 64)), kStream, 0, s>>>(a);
+            k_tangential<D, Real, HZ, GEN><<<static_cast<int>(std::min<long long>(nb, m.sms * 64)), kStream, 0, s>>>(a);
             break;
         }
         case KERNEL_ZERO_GRADIENT:
@@ -1910,7 +1910,7 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
             break;
         case KERNEL_FACE_FLUX: {
             k_face_flux<D, Real, HZ, GEN>
-                <<<dim3(nbF, stream_chunks(m.n_seg, nbF, 2)), kFaces, ring_flux<Real, HZ, GEN>(), s>>>(a);
+                <<<dim3(nbF, stream_chunks(m, m.n_seg, nbF, 2)), kFaces, ring_flux<Real, HZ, GEN>(), s>>>(a);
             break;
         }
         case KERNEL_UPDATE: {
@@ -1984,7 +1984,7 @@ cudaError_t launch_cell_records(const StepArgs& a, cudaStream_t s) {
 
 cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, unsigned long long* n_tang, cudaStream_t s) {
     const int nb = blocks(m.nF, 128);
-    const dim3 grid(nb, std::min(m.n_seg, std::max(1, 148 * 32 / std::max(nb, 1))));
+    const dim3 grid(nb, std::min(m.n_seg, std::max(1, m.sms * 32 / std::max(nb, 1))));
     if (m.general_dv) {
         if (m.D == 3) k_upwind_bits<3, true><<<grid, 128, 0, s>>>(m, upw, n_tang);
         else k_upwind_bits<2, true><<<grid, 128, 0, s>>>(m, upw, n_tang);
@@ -1998,7 +1998,7 @@ cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, unsigned long lo
 cudaError_t launch_list_tangential(const DevMesh& m, int2* list, unsigned long long* cursor, uint2* at, unsigned* seg,
                                    cudaStream_t s) {
     const int nb = blocks(m.nIF, 128);
-    const dim3 grid(nb, std::min(m.n_seg, std::max(1, 148 * 32 / std::max(nb, 1))));
+    const dim3 grid(nb, std::min(m.n_seg, std::max(1, m.sms * 32 / std::max(nb, 1))));
     if (m.general_dv) k_list_tangential<true><<<grid, 128, 0, s>>>(m, list, cursor, at, seg);
     else k_list_tangential<false><<<grid, 128, 0, s>>>(m, list, cursor, at, seg);
     return cudaGetLastError();

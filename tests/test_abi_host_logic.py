@@ -175,3 +175,10 @@ def test_large_half_step_arrays_leave_memory_free(memory):
     s = dl.Solver(c, lib_path=memory.path)
     assert memory.fake_used(0) <= whole - bars // 2 + 40000
     s.close()
+
+
+def test_chunks_follow_the_devices_multiprocessors(fake):
+    # 3,721 cells, 28 x 28 DVs: one wave of CTAs is 5 chunks on 148
+    # multiprocessors (device 0) and 2 on 74 (device 1)
+    c = cs.cavity_case(61, 28)
+    assert [dl.Solver(c, device=d, lib_path=fake.path).layout()["dv_chunks"] for d in (0, 1)] == [5, 2]
