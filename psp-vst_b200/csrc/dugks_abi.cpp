@@ -704,6 +704,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         dm.gref = dm.href = nullptr;
         ds.refmom = nullptr;
     }
+    dm.err = ds.err;
     ce = cudaMemsetAsync(ds.err, 0, 4 * sizeof(int), h->stream);
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, cudaGetErrorString(ce));
     ce = cudaMemsetAsync(ds.done, 0, n_done * sizeof(int), h->stream);

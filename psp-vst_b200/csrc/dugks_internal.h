@@ -69,6 +69,7 @@ struct DevMesh {
     // and Maxwellian tables alike: [block][field][32].  pC, pF: nC, nF padded
     int pC, pF;
     int sms;               // multiprocessors of the device
+    int* err;              // DevState::err, for the bounds-checked build
     // DVs this device holds: global DVs dv_base .. dv_base + nv_loc - 1, the
     // DV rows row_base ..; the state and face-value arrays are [nv_loc][..]
     int nv_loc, dv_base, row_base;

@@ -49,11 +49,12 @@ __global__ void k_init_state(const StepArgs a) {
 // 784-DV state set, stepped twice and read back).
 template <typename Real, bool GET>
 __global__ void k_state_order(const int nC, const int nv, const int32_t* __restrict__ iperm, Real* __restrict__ state,
-                              const double* __restrict__ ref, double* __restrict__ buf, const size_t first, const size_t n) {
+                              const double* __restrict__ ref, double* __restrict__ buf, const size_t first, const size_t n,
+                              int* err) {
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         const size_t d = (first + i) / nC;
-        const int c = iperm[first + i - d * nC];
+        const int c = chk(iperm[first + i - d * nC], 0, nC, err);
         Real* s = state + (static_cast<size_t>(c / 32) * nv + d) * 32 + c % 32;
         const double r = sizeof(Real) == 4 && ref ? ref[d] : 0.0;
         if (GET) buf[i] = sizeof(Real) == 4 && ref ? double(*s) + r : double(*s);
@@ -254,12 +255,12 @@ cudaError_t launch_state_order(const StepArgs& a, int precision, bool second, bo
     const unsigned nb = static_cast<unsigned>(std::min<size_t>((n + 255) / 256, 1u << 16));
     if (precision == DUGKS_FP64) {
         double* p = static_cast<double*>(st);
-        if (get) k_state_order<double, true><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n);
-        else k_state_order<double, false><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n);
+        if (get) k_state_order<double, true><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n, m.err);
+        else k_state_order<double, false><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n, m.err);
     } else {
         float* p = static_cast<float*>(st);
-        if (get) k_state_order<float, true><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n);
-        else k_state_order<float, false><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n);
+        if (get) k_state_order<float, true><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n, m.err);
+        else k_state_order<float, false><<<nb, 256, 0, s>>>(m.nC, m.nv_loc, iperm, p, ref, buf, first, n, m.err);
     }
     return cudaGetLastError();
 }

@@ -58,8 +58,17 @@ __device__ __forceinline__ int chk(int i, int lo, int hi, int* err) {
     }
     return i;
 }
+// place i of a list of n
+__device__ __forceinline__ size_t chk_place(size_t i, size_t n, int* err) {
+    if (i >= n) {
+        atomicOr(err, 4);
+        return 0;
+    }
+    return i;
+}
 #else
 __device__ __forceinline__ int chk(int i, int, int, int*) { return i; }
+__device__ __forceinline__ size_t chk_place(size_t i, size_t, int*) { return i; }
 #endif
 
 // one stage of a DUGKS step (fvDVM::evolution) on stream s; `launches` (may be

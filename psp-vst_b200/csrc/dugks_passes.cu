@@ -78,8 +78,8 @@ __device__ __forceinline__ Seg seg_at(const DevMesh& m, int s) {
         q.d0 = row * m.n1d + q.ix0;   // as seg_dv
         q.len = min(kSeg, m.n1d - q.ix0);
         const int2 t = __ldg(m.row_yz + row);
-        q.iy = t.x;
-        q.iz = t.y;
+        q.iy = chk(t.x, 0, m.n1d, m.err);
+        q.iz = chk(t.y, 0, m.n1d, m.err);
     }
     return q;
 }
@@ -758,7 +758,7 @@ template <bool GEN>
 __global__ void k_list_tangential(const DevMesh m, int2* list, unsigned long long* cursor, uint2* at, unsigned* seg) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     const size_t nF = static_cast<size_t>(m.nF);
-    const bool between = f < m.nIF && !in_tile_face(m, f, __ldg(m.fown + f));
+    const bool between = f < m.nIF && !in_tile_face(m, f, chk(__ldg(m.fown + f), 0, m.nC, m.err));
     const unsigned tiles = __ballot_sync(0xffffffffu, between);
     for (int s = blockIdx.y; s < m.n_seg; s += gridDim.y) {
         const Seg q = seg_at<GEN>(m, s);
@@ -801,9 +801,10 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
     for (long long i = blockIdx.x * static_cast<long long>(kStream) + threadIdx.x; i < m.n_tang;
          i += static_cast<long long>(gridDim.x) * kStream) {
         const int2 t = __ldg(m.tang + i);
-        const int f = chk(t.x, 0, m.nIF, a.ds.err), s = chk(t.y / kSeg, 0, m.n_seg, a.ds.err), j = t.y % kSeg;
+        const int f = chk(t.x, 0, m.nIF, a.ds.err), s = chk(t.y / kSeg, 0, m.n_seg, a.ds.err);
         if (s < a.seg0 || s >= a.seg1) continue;
         const Seg q = seg_at<GEN>(m, s);
+        const int j = chk(t.y % kSeg, 0, q.len, a.ds.err);
         const int o = chk(__ldg(m.fown + f), 0, m.nC, a.ds.err), n = chk(__ldg(m.fnei + f), 0, m.nC, a.ds.err);
         bool in_tile = false;
         if constexpr (sizeof(Real) == 4 && !GEN)
@@ -1039,7 +1040,7 @@ __device__ __noinline__ void finish_face(const StepArgs& a, const Consts& kc, in
         macros_from_moments(s, kc, rho, U, T, q, tau);
         const double fac = 2.0 * tau / (2.0 * tau + 0.5 * dt * kc.Pr);  // fvDVM.C:1300
         for (int i = 0; i < 3; ++i) q[i] *= fac;
-        const int fo = __ldg(m.forig + f);
+        const int fo = chk(__ldg(m.forig + f), 0, m.nF, a.ds.err);
         double* fm = a.ds.fm + static_cast<size_t>(fo) * 9;
         fm[0] = rho;
         fm[4] = T;
@@ -1464,7 +1465,7 @@ __global__ void __launch_bounds__(kFaces, 5) k_face_moments(const __grid_constan
         const uint2 t = __ldg(m.tang_at + static_cast<size_t>(wf0 / kLanes) * m.nv_loc + d);
         const unsigned bit = 1u << (threadIdx.x % kLanes);
         if (!(t.x & bit)) return;
-        const size_t i = t.y + static_cast<unsigned>(__popc(t.x & (bit - 1)));
+        const size_t i = chk_place(t.y + static_cast<unsigned>(__popc(t.x & (bit - 1))), m.n_tang, a.ds.err);
         g += double(a.ds.tang_res[i]);
         if (!HZ) h += double(a.ds.tang_res[m.n_tang + i]);
     };
