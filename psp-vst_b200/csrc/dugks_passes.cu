@@ -1283,8 +1283,10 @@ __device__ __forceinline__ Incoming load_incoming(const StepArgs& a, int b, int 
     return t;
 }
 
-// boundary faces of one chunk: by patch type (fvDVM.C:866-1027)
-template <int D, typename Real, bool HZ, bool GEN>
+// boundary faces of one chunk: by patch type (fvDVM.C:866-1027).  CUT: gbar+
+// is held in parts, and k_zero_gradient has stored the zero-gradient faces (as
+// a test at run time it cost a 3,721-cell step 1.5 of 216 us)
+template <int D, typename Real, bool HZ, bool GEN, bool CUT>
 __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x1, const double* w1, int f, int s0,
                                               int s1, int w, Finish& sm) {
     const DevMesh& m = a.dm;
@@ -1329,16 +1331,14 @@ __device__ __noinline__ void boundary_moments(const StepArgs& a, const double* x
             const double gr = dv_ref<Real, GEN>(m.gref, d), hr = dv_ref<Real, GEN>(m.href, d);
             double g, h = 0.0;
             if (zero_grad) {
-                // every DV: the owner cell's gbar+ (fvDVM.C:887-891), which
-                // k_zero_gradient has stored already where it is held in parts
-                const bool there = m.nv_bar < m.nv_loc;
+                // every DV: the owner cell's gbar+ (fvDVM.C:887-891)
                 const size_t oc = slot(own, m.nv_loc) + o;
-                const Real gc = there ? gv : reinterpret_cast<const Real*>(a.ds.gbar)[oc];
-                fg[o] = gc;
+                const Real gc = CUT ? gv : reinterpret_cast<const Real*>(a.ds.gbar)[oc];
+                if (!CUT) fg[o] = gc;
                 g = double(gc) + gr;
                 if (!HZ) {
-                    const Real hc = there ? hv : reinterpret_cast<const Real*>(a.ds.hbar)[oc];
-                    fh[o] = hc;
+                    const Real hc = CUT ? hv : reinterpret_cast<const Real*>(a.ds.hbar)[oc];
+                    if (!CUT) fh[o] = hc;
                     h = double(hc) + hr;
                 }
             } else if (sym) {
@@ -1414,7 +1414,7 @@ constexpr size_t ring_moments() {
 // Internal faces: reads each face value once (8 B per face, DV and FP64
 // field) and adds seven FP64 operations.  Boundary faces: 32 per CTA, the
 // segments split over its warps, as incoming DFs cost an exponential each.
-template <int D, typename Real, bool HZ, bool GEN>
+template <int D, typename Real, bool HZ, bool GEN, bool CUT>
 __global__ void __launch_bounds__(kFaces, 5) k_face_moments(const __grid_constant__ StepArgs a,
                                                             const __grid_constant__ Consts kc) {
     static_assert(kFaces == kLanes * kParts, "one CTA size for internal and boundary blocks");
@@ -1433,7 +1433,7 @@ __global__ void __launch_bounds__(kFaces, 5) k_face_moments(const __grid_constan
         const int f0 = m.nIF + bx * kLanes, count = min(kLanes, m.nF - f0), lane = threadIdx.x % kLanes;
         const int w = warp_id();
         Finish& sm = *reinterpret_cast<Finish*>(ring_raw);
-        if (lane < count) boundary_moments<D, Real, HZ, GEN>(a, x1, w1, f0 + lane, s0, s1, w, sm);
+        if (lane < count) boundary_moments<D, Real, HZ, GEN, CUT>(a, x1, w1, f0 + lane, s0, s1, w, sm);
         if (reduce_chunk(sm, a.ds.partF, nF, f0, count, a.ds.done + bx, a.fused != 0)) {
             sum_chunks(sm, a.ds.partF, nF, f0, count, gridDim.y);
             if (w == 0) finish_face(a, kc, lane < count ? f0 + lane : -1, gridDim.y, &sm);
@@ -1906,8 +1906,10 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
             if (m.nBF > 0) k_zero_gradient<Real><<<blocks(m.nBF, kLanes), kStream, 0, s>>>(a);
             break;
         case KERNEL_FACE_MOMENTS:
-            k_face_moments<D, Real, HZ, GEN>
-                <<<dim3(nbF, a.chunks_f), kFaces, ring_moments<Real, HZ>(), s>>>(a, k);
+            if (m.nv_bar < m.nv_loc)
+                k_face_moments<D, Real, HZ, GEN, true><<<dim3(nbF, a.chunks_f), kFaces, ring_moments<Real, HZ>(), s>>>(a, k);
+            else
+                k_face_moments<D, Real, HZ, GEN, false><<<dim3(nbF, a.chunks_f), kFaces, ring_moments<Real, HZ>(), s>>>(a, k);
             break;
         case KERNEL_FACE_FLUX: {
             k_face_flux<D, Real, HZ, GEN>
@@ -1933,11 +1935,12 @@ cudaError_t launch_kernel(const StepArgs& a, int which, cudaStream_t s) {
 // dynamic shared memory of the rings (above the default limit)
 template <int D, typename Real, bool HZ, bool GEN>
 cudaError_t allow_rings() {
-    cudaError_t e = cudaFuncSetAttribute(k_face_moments<D, Real, HZ, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(ring_moments<Real, HZ>()));
-    return e != cudaSuccess ? e
-                            : cudaFuncSetAttribute(k_face_flux<D, Real, HZ, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   static_cast<int>(ring_flux<Real, HZ, GEN>()));
+    auto allow = [](auto* kernel, size_t bytes) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    };
+    cudaError_t e = allow(k_face_moments<D, Real, HZ, GEN, false>, ring_moments<Real, HZ>());
+    if (e == cudaSuccess) e = allow(k_face_moments<D, Real, HZ, GEN, true>, ring_moments<Real, HZ>());
+    return e != cudaSuccess ? e : allow(k_face_flux<D, Real, HZ, GEN>, ring_flux<Real, HZ, GEN>());
 }
 
 template <int D, typename Real>
