@@ -579,7 +579,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
         (st = upload(h, &d_invV, invV)) || (st = upload(h, &d_bpl, h->bface_patch_local)) ||
         (st = upload(h, &d_bpt, h->bface_ptype)) || (st = upload(h, &d_bown, bown)) || (st = upload(h, &d_dc, h->dc)) ||
         (st = upload(h, &d_bS, bS)) || (st = upload(h, &d_bmir, h->bface_mirror)) ||
-        (st = dev_alloc(h, &d_upw, 2 * static_cast<size_t>(n_seg) * nF)) || (st = dev_alloc(h, &d_count, 2))) {
+        (st = dev_alloc(h, &d_upw, 2 * static_cast<size_t>(n_seg) * nF)) || (st = dev_alloc(h, &d_count, 4))) {
         *out = h;
         return st;
     }
@@ -600,7 +600,7 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     dm.forig = d_for;
     dm.upw = d_upw;
     dm.tang = nullptr;
-    dm.n_tang = 0;
+    dm.n_tang = dm.n_rest = 0;
     dm.tang_at = nullptr;
     dm.tang_seg = nullptr;
     dm.bface_patch_local = d_bpl;
@@ -711,29 +711,31 @@ static int create_impl(const dugks_mesh* mesh, const dugks_dv_set* dv, const dug
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, cudaGetErrorString(ce));
     ce = dugks::configure_kernels(h->D, h->precision);
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, std::string("configure kernels: ") + cudaGetErrorString(ce));
-    unsigned long long n_tang = 0;
-    ce = cudaMemsetAsync(d_count, 0, 2 * sizeof(unsigned long long), h->stream);
+    // tangential pairs: all of them, and those whose rests the moments add
+    unsigned long long n_tang[2] = {0, 0};
+    ce = cudaMemsetAsync(d_count, 0, 4 * sizeof(unsigned long long), h->stream);
     if (ce == cudaSuccess) ce = dugks::launch_upwind_bits(dm, d_upw, d_count, h->stream);
     if (ce == cudaSuccess)
-        ce = cudaMemcpyAsync(&n_tang, d_count, sizeof n_tang, cudaMemcpyDeviceToHost, h->stream);
+        ce = cudaMemcpyAsync(n_tang, d_count, sizeof n_tang, cudaMemcpyDeviceToHost, h->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);
-    if (ce == cudaSuccess && n_tang > 0) {
+    if (ce == cudaSuccess && n_tang[0] > 0) {
         int2* d_tang = nullptr;
-        if ((st = dev_alloc(h, &d_tang, n_tang))) return *out = h, st;
+        if ((st = dev_alloc(h, &d_tang, n_tang[0]))) return *out = h, st;
         uint2* at = nullptr;
         unsigned* seg = nullptr;
-        if (h->precision == DUGKS_FP32C && !dvl && n_tang < (1ull << 32)) {
+        if (n_tang[1] > 0 && n_tang[1] < (1ull << 32)) {
             if ((st = dev_alloc(h, &at, static_cast<size_t>(dm.pF / 32) * dm.nv_loc)) ||
                 (st = dev_alloc(h, &seg, static_cast<size_t>(dm.pF / 32) * n_seg)) ||
-                (st = dev_alloc(h, &ds.tang_res, 2 * n_tang)))
+                (st = dev_alloc(h, &ds.tang_res, 2 * n_tang[1])))
                 return *out = h, st;
             dm.tang_at = at;
             dm.tang_seg = seg;
+            dm.n_rest = static_cast<long long>(n_tang[1]);
         }
-        ce = dugks::launch_list_tangential(dm, d_tang, d_count + 1, at, seg, h->stream);
+        ce = dugks::launch_list_tangential(dm, d_tang, d_count + 2, at, seg, h->stream);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);
         dm.tang = d_tang;
-        dm.n_tang = static_cast<long long>(n_tang);
+        dm.n_tang = static_cast<long long>(n_tang[0]);
     }
     if (ce != cudaSuccess) return fail(DUGKS_ERR_CUDA, std::string("upwind bits: ") + cudaGetErrorString(ce));
     if ((st = alloc_bars(h, true, !can_skip_h(h)))) return *out = h, st;

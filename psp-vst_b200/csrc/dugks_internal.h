@@ -103,10 +103,10 @@ struct DevMesh {
     const int32_t* forig;          // [nF] the caller's face
     const uint32_t* upw;           // [n_seg][nF][2] upwind bits of a segment's DVs: owner side, neighbour side
     const int2* tang;              // [n_tang] exactly tangential pairs: internal face, segment * kSeg + DV in it
-    long long n_tang;
-    // FP32 storage of a tensor DV set: where the pairs are in the list, by
-    // face block (null without pairs): the faces between tiles that have one at
-    // a DV (a bit each) and the first one's place; and the DVs of a segment with any
+    long long n_tang, n_rest;      // n_rest: FP32 storage of a tensor DV set, those of faces between tiles
+    // where the rests of those are, by face block (null without any): the faces
+    // that have one at a DV (a bit each) and the first one's place; and the DVs
+    // of a segment with any
     const uint2* tang_at;          // [pF/32][nv_loc]
     const unsigned* tang_seg;      // [pF/32][n_seg]
     int done_cells;                // first cell-block counter in DevState::done (face blocks before it)
@@ -143,7 +143,7 @@ struct DevState {
     // then, relaxed and multiplied by xi.S, the flux
     void* fvg;
     void* fvh;         // (null while h is identically zero)
-    float* tang_res;   // [2][n_tang] g and h: what rounding took from the listed pairs' means (FP32, as tang_at)
+    float* tang_res;   // [2][n_rest] g and h: what rounding took from those pairs' means
     double* partF;     // [chunks_f][kNM][nF]
     double* partC;     // [chunks][kNM][nC]
     double* partX;     // [chunks][kFX][nC] DV-list macroFlux: moments of the flux term (else null)

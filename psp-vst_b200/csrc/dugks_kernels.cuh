@@ -85,9 +85,10 @@ cudaError_t launch_pass(const StepArgs& a, int precision, int which, cudaStream_
 cudaError_t launch_finish(const StepArgs& a, bool faces, cudaStream_t s);
 // kernel attributes on the current device
 cudaError_t configure_kernels(int D, int precision);
-// DevMesh::upw from the geometry and the DV set, with the number of tangential
-// (internal face, DV) pairs, and their list DevMesh::tang (counters start at 0)
-cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, unsigned long long* n_tang, cudaStream_t s);
+// DevMesh::upw from the geometry and the DV set, with the numbers n_tang and
+// n_rest of tangential (internal face, DV) pairs in n[2], and their list
+// DevMesh::tang with the places of the rests (n and cursor[2] start at 0)
+cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, unsigned long long* n, cudaStream_t s);
 cudaError_t launch_list_tangential(const DevMesh& m, int2* list, unsigned long long* cursor, uint2* at, unsigned* seg,
                                    cudaStream_t s);
 // partial moments of all chunks summed into chunk 0 (n doubles per chunk)

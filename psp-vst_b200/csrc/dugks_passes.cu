@@ -705,15 +705,25 @@ __global__ void __launch_bounds__(kCells, 2) k_face_values(const __grid_constant
     }
 }
 
+// whether internal face f of owner o lies inside a tile (cell face code, bit 1)
+__device__ __forceinline__ bool in_tile_face(const DevMesh& m, int f, int o) {
+    for (int k = 0; k < m.nf_max; ++k) {
+        const int code = __ldg(m.cface + static_cast<size_t>(k) * m.nC + o);
+        if (code >= 0 && (code >> 2) == f) return code & 2;
+    }
+    return false;
+}
+
 // upwind bits of every face and segment (geometry and DV set only; once at
 // creation).  Bit j of word (s, f, side): DV j of segment s leaves through
 // face f from that side -- internal faces by the switch of fvDVM.C:829-863
 // (neither side on an exactly tangential face), boundary faces the outgoing
 // DVs (:916-923), symmetry faces the tangential ones too (:1013-1023);
 // zero-gradient faces take the cell's value for every DV instead.  Counts the
-// tangential (face, DV) pairs of internal faces into *n_tang.
+// tangential (face, DV) pairs of internal faces into count[0], with `tiles`
+// those of faces between tiles into count[1].
 template <int D, bool GEN>
-__global__ void k_upwind_bits(const DevMesh m, uint32_t* upw, unsigned long long* n_tang) {
+__global__ void k_upwind_bits(const DevMesh m, uint32_t* upw, bool tiles, unsigned long long* count) {
     __shared__ double x1[kMaxN1d], w1[kMaxN1d];
     load_nodes(m, x1, w1);
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -740,26 +750,21 @@ __global__ void k_upwind_bits(const DevMesh m, uint32_t* upw, unsigned long long
         w[1] = nei;
         if (pt == 0) tangential += q.len - __popc(own) - __popc(nei);
     }
-    if (tangential) atomicAdd(n_tang, static_cast<unsigned long long>(tangential));
-}
-
-// whether internal face f of owner o lies inside a tile (cell face code, bit 1)
-__device__ __forceinline__ bool in_tile_face(const DevMesh& m, int f, int o) {
-    for (int k = 0; k < m.nf_max; ++k) {
-        const int code = __ldg(m.cface + static_cast<size_t>(k) * m.nC + o);
-        if (code >= 0 && (code >> 2) == f) return code & 2;
-    }
-    return false;
+    if (!tangential) return;
+    atomicAdd(count, static_cast<unsigned long long>(tangential));
+    if (tiles && !in_tile_face(m, f, chk(__ldg(m.fown + f), 0, m.nC, m.err)))
+        atomicAdd(count + 1, static_cast<unsigned long long>(tangential));
 }
 
 // the list of those pairs (DevMesh::tang), pairs of one DV and consecutive
-// faces together
+// faces together, and the places of the rests of faces between tiles (cursor:
+// pairs listed, rests placed)
 template <bool GEN>
 __global__ void k_list_tangential(const DevMesh m, int2* list, unsigned long long* cursor, uint2* at, unsigned* seg) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     const size_t nF = static_cast<size_t>(m.nF);
-    const bool between = f < m.nIF && !in_tile_face(m, f, chk(__ldg(m.fown + f), 0, m.nC, m.err));
-    const unsigned tiles = __ballot_sync(0xffffffffu, between);
+    const bool between = at && f < m.nIF && !in_tile_face(m, f, chk(__ldg(m.fown + f), 0, m.nC, m.err));
+    const unsigned tiles = __ballot_sync(0xffffffffu, between), lt = (1u << (threadIdx.x % 32)) - 1u;
     for (int s = blockIdx.y; s < m.n_seg; s += gridDim.y) {
         const Seg q = seg_at<GEN>(m, s);
         unsigned t = 0;
@@ -777,12 +782,12 @@ __global__ void k_list_tangential(const DevMesh m, int2* list, unsigned long lon
             unsigned long long base = 0;
             if (threadIdx.x % 32 == 0) base = atomicAdd(cursor, static_cast<unsigned long long>(__popc(who)));
             base = __shfl_sync(0xffffffffu, base, 0);
-            // a warp's pairs between tiles first
-            const unsigned lt = (1u << (threadIdx.x % 32)) - 1u, inter = who & tiles;
-            if (at && first) at[(f / 32) * static_cast<size_t>(m.nv_loc) + q.d0 + j] = make_uint2(inter, static_cast<unsigned>(base));
-            if ((t >> j) & 1u)
-                list[base + (between ? __popc(inter & lt) : __popc(inter) + __popc(who & ~inter & lt))] =
-                    make_int2(f, s * kSeg + j);
+            if (at && first) {
+                const unsigned inter = who & tiles;
+                at[(f / 32) * static_cast<size_t>(m.nv_loc) + q.d0 + j] =
+                    make_uint2(inter, static_cast<unsigned>(atomicAdd(cursor + 1, static_cast<unsigned long long>(__popc(inter)))));
+            }
+            if ((t >> j) & 1u) list[base + __popc(who & lt)] = make_int2(f, s * kSeg + j);
         }
     }
 }
@@ -806,12 +811,21 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
         const Seg q = seg_at<GEN>(m, s);
         const int j = chk(t.y % kSeg, 0, q.len, a.ds.err);
         const int o = chk(__ldg(m.fown + f), 0, m.nC, a.ds.err), n = chk(__ldg(m.fnei + f), 0, m.nC, a.ds.err);
-        bool in_tile = false;
-        if constexpr (sizeof(Real) == 4 && !GEN)
-            in_tile = in_tile_face(m, f, o);
-        const bool rounded = kRoundsRows<D, Real, GEN> && in_tile && rounds_node(q.ix0 + j);
+        bool rounded = false;
+        if constexpr (kRoundsRows<D, Real, GEN>) rounded = rounds_node(q.ix0 + j) && in_tile_face(m, f, o);
         const Dv v = dv_at<D, GEN>(m, q, x1, j);
         const size_t rc = 32 * static_cast<size_t>(q.d0 + j), rf = slot(f, m.nv_loc) + rc;
+        // the place of its rest, if the face is between tiles
+        size_t place = 0;
+        bool between = false;
+        if constexpr (sizeof(Real) == 4 && !GEN) {
+            if (m.tang_at) {
+                const uint2 w = __ldg(m.tang_at + static_cast<size_t>(f / 32) * m.nv_loc + q.d0 + j);
+                const unsigned bit = 1u << (f % 32);
+                between = w.x & bit;
+                place = between ? chk_place(w.y + static_cast<unsigned>(__popc(w.x & (bit - 1))), m.n_rest, a.ds.err) : 0;
+            }
+        }
         auto average = [&](const void* bar, void* fv, float* res) {
             const Real* b = reinterpret_cast<const Real*>(bar) + (rc - 32 * static_cast<size_t>(a.d_bar));
             const Real vn = recon_mem<D, Real, GEN>(m, b, f, 1, n, hdt, v, rounded, a.ds.err);
@@ -820,10 +834,10 @@ __global__ void __launch_bounds__(kStream) k_tangential(const __grid_constant__ 
             reinterpret_cast<Real*>(fv)[rf] = mean;
             // what the moments of a face between tiles add: its two halves, not their rounded sum
             if constexpr (sizeof(Real) == 4)
-                if (res) res[i] = in_tile ? 0.f : float(0.5 * double(vo) + 0.5 * double(vn) - double(mean));
+                if (between) res[place] = float(0.5 * double(vo) + 0.5 * double(vn) - double(mean));
         };
         average(a.ds.gbar, a.ds.fvg, a.ds.tang_res);
-        if (!HZ) average(a.ds.hbar, a.ds.fvh, a.ds.tang_res ? a.ds.tang_res + m.n_tang : nullptr);
+        if (!HZ) average(a.ds.hbar, a.ds.fvh, a.ds.tang_res + m.n_rest);
     }
 }
 
@@ -1465,9 +1479,9 @@ __global__ void __launch_bounds__(kFaces, 5) k_face_moments(const __grid_constan
         const uint2 t = __ldg(m.tang_at + static_cast<size_t>(wf0 / kLanes) * m.nv_loc + d);
         const unsigned bit = 1u << (threadIdx.x % kLanes);
         if (!(t.x & bit)) return;
-        const size_t i = chk_place(t.y + static_cast<unsigned>(__popc(t.x & (bit - 1))), m.n_tang, a.ds.err);
+        const size_t i = chk_place(t.y + static_cast<unsigned>(__popc(t.x & (bit - 1))), m.n_rest, a.ds.err);
         g += double(a.ds.tang_res[i]);
-        if (!HZ) h += double(a.ds.tang_res[m.n_tang + i]);
+        if (!HZ) h += double(a.ds.tang_res[m.n_rest + i]);
     };
     const bool ok = ring_walk<GEN, kStagesM>(
         m, full + w * kStagesM, s0, wf0 < m.nIF ? s1 : s0, NH * kLanes * sizeof(Real),
@@ -1986,15 +2000,17 @@ cudaError_t launch_cell_records(const StepArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, unsigned long long* n_tang, cudaStream_t s) {
+cudaError_t launch_upwind_bits(const DevMesh& m, uint32_t* upw, unsigned long long* n, cudaStream_t s) {
+    // (FP32 storage of a tensor DV set: DevMesh::tang_at)
+    const bool tiles = m.prec == DUGKS_FP32C && !m.general_dv;
     const int nb = blocks(m.nF, 128);
     const dim3 grid(nb, std::min(m.n_seg, std::max(1, m.sms * 32 / std::max(nb, 1))));
     if (m.general_dv) {
-        if (m.D == 3) k_upwind_bits<3, true><<<grid, 128, 0, s>>>(m, upw, n_tang);
-        else k_upwind_bits<2, true><<<grid, 128, 0, s>>>(m, upw, n_tang);
+        if (m.D == 3) k_upwind_bits<3, true><<<grid, 128, 0, s>>>(m, upw, tiles, n);
+        else k_upwind_bits<2, true><<<grid, 128, 0, s>>>(m, upw, tiles, n);
     } else {
-        if (m.D == 3) k_upwind_bits<3, false><<<grid, 128, 0, s>>>(m, upw, n_tang);
-        else k_upwind_bits<2, false><<<grid, 128, 0, s>>>(m, upw, n_tang);
+        if (m.D == 3) k_upwind_bits<3, false><<<grid, 128, 0, s>>>(m, upw, tiles, n);
+        else k_upwind_bits<2, false><<<grid, 128, 0, s>>>(m, upw, tiles, n);
     }
     return cudaGetLastError();
 }
