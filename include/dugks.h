@@ -171,7 +171,8 @@ typedef struct dugks_options {
     int32_t precision;              /* dugks_precision */
     int32_t ls_weighting;           /* dugks_ls_weighting */
     int32_t device;                 /* CUDA device ordinal */
-    int32_t tile_cells;             /* cells per tile; 0 = automatic */
+    int32_t tile_cells;             /* cells per mesh tile; 0 = automatic.  FP32 storage rounds
+                                       by tiles (last bits); no launch depends on it */
     int32_t dv_chunks;              /* DV chunks of the cell sums, the face sums' by the same
                                        factor; 0 = automatic */
     int32_t macro_flux;             /* fvDVMparas macroFlux: 0 "no" (cell macros from the
@@ -338,7 +339,7 @@ int dugks_set_step_record(dugks_handle* h, const double* rec);
 /* Many independent cases stepped together (no counterpart in the
  * reference, which runs one case per dugksFoam process).  One CUDA graph
  * holds two steps of every handle, each handle a parallel branch on its own
- * stream, so that the tiles of small cases share the GPU; dugks_batch_step
+ * stream, so that small cases share the GPU; dugks_batch_step
  * replays it (an odd step count ends with one ordinary step per handle).
  * The handles must be initialised (dugks_set_macros), on one device and
  * unsharded; dt[i] is handle i's fixed time step.  Every handle's result is
@@ -427,9 +428,10 @@ int64_t dugks_checkpoint_forward_steps(int32_t n_steps, int32_t n_snapshots);
  * maxwellWall and farField patches (the dugks_adjoint_run restrictions). */
 int dugks_boundary_fluxes(dugks_handle* h, double dt, double* flux);
 
-/* The launch layout dugks_create chose: cells per tile (after shrinking
- * to fit), number of tiles and DV chunks per tile.  An autotuner reads it
- * to scale dugks_options.tile_cells / dv_chunks from the automatic choice. */
+/* What dugks_create chose: cells per mesh tile (after shrinking to fit),
+ * number of tiles and DV chunks of the cell sums (the face sums have a count
+ * of their own).  An autotuner reads it to scale dugks_options.dv_chunks from
+ * the automatic choice; that count as an option gives the same launches. */
 int dugks_layout(const dugks_handle* h, int32_t* tile_cells, int32_t* n_tiles, int32_t* dv_chunks);
 
 /* Number of discrete velocities (nDV^D). */

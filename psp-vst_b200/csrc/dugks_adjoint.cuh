@@ -88,7 +88,7 @@ struct View {
     const double* ha;       // [nBF] objective: energy-flux weights
     const double* fw;       // [nBF][3] objective: momentum-flux weights
     // state of the step (input)
-    const double* g;        // [nv][nC]
+    const double* g;        // cells
     const double* h;
     const double* cm;       // [nC][9] rho U T q tau the step starts from
     // forward record of the step: the handle's face-value buffers, faces in

@@ -1,5 +1,5 @@
 // Internal declarations of the B200 DUGKS step library: device layout,
-// per-tile stencil tables and the handle.  Not part of the public ABI.
+// cell and face tables and the handle.  Not part of the public ABI.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -12,6 +12,8 @@
 
 namespace dugks {
 
+// tiles: what FP32 rounds by (Tiling) and dugks_layout reports; a mesh that does
+// not fit them is refused
 constexpr int kMaxTile = 128;      // cells per tile at most
 constexpr int kMaxLocal = 256;     // cells of a tile with its ring of neighbours at most
 constexpr int kMaxItems = 511;     // faces of a tile's cells at most
@@ -71,7 +73,7 @@ struct DevMesh {
     int sms;               // multiprocessors of the device
     int* err;              // DevState::err, for the bounds-checked build
     // DVs this device holds: global DVs dv_base .. dv_base + nv_loc - 1, the
-    // DV rows row_base ..; the state and face-value arrays are [nv_loc][..]
+    // DV rows row_base ..
     int nv_loc, dv_base, row_base;
     int prec;              // dugks_precision of the state and tables
     // DV set

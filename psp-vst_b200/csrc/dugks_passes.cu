@@ -30,7 +30,7 @@
 // 16 warps per SM, two or three CTA barriers per 8 to 16 DVs) issued on 30 % of
 // the cycles and recomputed gbar+ of each tile's ring.  24,576 cells and 16^3
 // DVs in FP64 (100 M updates): 9.4 ms tiled, 3.7 ms now: half step 0.29, face
-// values 1.16, tangential pairs 0.12, moments 0.44, flux 0.88, update 0.84.
+// values 1.16, tangential pairs 0.12, moments 0.41, flux 0.90, update 0.84.
 #include <algorithm>
 #include <type_traits>
 
@@ -403,7 +403,7 @@ __device__ __forceinline__ double cell_r(const StepArgs& a, int c) {
 // k_half_step
 // ---------------------------------------------------------------------
 // Reads g~ and writes gbar+: 16 B per (cell, DV) and FP64 field, bound by HBM
-// (100 M updates in 0.29 ms: 5.5 TB/s).
+// (100 M updates in 0.295 ms: 5.4 TB/s).
 template <int D, typename Real, bool HZ, bool GEN>
 __global__ void __launch_bounds__(kStream) k_half_step(const __grid_constant__ StepArgs a) {
     const DevMesh& m = a.dm;
@@ -469,9 +469,10 @@ __device__ __forceinline__ Real recon(Real gb, const Real* G, const Real* v) {
     return r;
 }
 
-// One component of v = Cf - C - xi dt/2 in the storage type.  FP32 results
-// are held to the last bit, and this decides them: along a row the x product
-// is fused and the y and z products are rounded first; a DV list rounds all.
+// One component of v = Cf - C - xi dt/2 in the storage type.  Along a row the x
+// product is fused and the y and z products are rounded first; a DV list rounds
+// all.  Nothing in the method asks for this: it is how the compiler contracted the
+// former kernels' loops, kept so that FP32 runs give what they gave.
 template <typename Real>
 __device__ __forceinline__ Real fused_dist(Real d, Real hdt, double x) {
     return fma(-hdt, Real(x), d);
@@ -481,8 +482,8 @@ __device__ __forceinline__ Real rounded_dist(Real d, Real hdt, double x) {
     if constexpr (sizeof(Real) == 4) return __fsub_rn(d, __fmul_rn(hdt, Real(x)));
     else return fma(-hdt, x, d);
 }
-// (2-D rows round the x product too at the first and last of every eight
-// nodes, on faces inside a tile)
+// (likewise, 2-D rows round the x product too at the first and last of every
+// eight nodes, on faces inside a tile: the former kernel's batches and tiles)
 template <int D, typename Real, bool GEN>
 constexpr bool kRoundsRows = D == 2 && sizeof(Real) == 4 && !GEN;
 __device__ __forceinline__ bool rounds_node(int ix) { return ((ix + 1) & 6) == 0; }

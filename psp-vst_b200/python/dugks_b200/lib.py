@@ -346,7 +346,7 @@ class Solver:
         return out
 
     def layout(self) -> dict:
-        """dugks_layout: cells per tile, tiles and DV chunks the handle uses."""
+        """dugks_layout: cells per mesh tile, tiles and DV chunks of the cell sums."""
         t, n, c = C.c_int32(), C.c_int32(), C.c_int32()
         self._check(self.lib.dugks_layout(self.h, C.byref(t), C.byref(n), C.byref(c)))
         return {"tile_cells": t.value, "n_tiles": n.value, "dv_chunks": c.value}
@@ -516,8 +516,9 @@ class Batch:
 def tune_batch(cases, dt, precision: int = FP32C, tiles=(0, 96, 64), chunk_scales=(0.25, 0.5, 1.0, 2.0),
                steps: int = 4, warmup: int = 2, device: int = 0):
     """Autotuner of the batched launch.  Every candidate is a cell count per
-    tile (0: the automatic 128, shrunk to fit) and a factor on each case's
-    automatic DV-chunk count; it is measured as what it will run as -- the
+    tile (0: the automatic 128, shrunk to fit; tiles no longer decide a launch,
+    so candidates that differ in them alone time the same) and a factor on each
+    case's automatic DV-chunk count; it is measured as what it will run as -- the
     whole batch of cases in one graph, CUDA-event time of `steps` steps after
     `warmup` -- and the fastest wins.  Returns (best, table): best holds the
     tile and scale and the per-case Solver keyword arguments, table every
