@@ -1622,6 +1622,10 @@ void* take_kept(int device, size_t bytes) {
 }
 
 void keep(int device, void* p, size_t bytes) {
+    if (bytes > kKeep) {
+        cudaFree(p);
+        return;
+    }
     std::lock_guard<std::mutex> g(kept_lock);
     kept.push_back({p, bytes, device});
     size_t total = 0;

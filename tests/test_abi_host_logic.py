@@ -111,6 +111,9 @@ def test_memory_kept_between_runs_is_bounded_and_given_back(memory):
     # 2 GiB a device at most, over all handles
     for m in (600, 700, 900, 3000):
         assert _run(memory, b, m) == 0 and kept() <= 2048
+    # a block over the bound takes no other's place
+    at = kept()
+    assert _run(memory, b, 3000) == 0 and kept() == at
     # no allocation of any handle fails while memory is kept
     assert _run(memory, a, 1000, 900) == 0
     memory.fake_capacity(0, memory.fake_used(0))
